@@ -133,6 +133,26 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+  """The native host side (csrc/host.cpp): the modules' calls without the Python and ctypes steps.
+  Its functions return NotImplemented for arguments that only the Python forms handle."""
+  global _host
+  if _host is None:
+    load()
+    from recurrentgemma_b200 import modules
+    try:
+      from recurrentgemma_b200 import _host as ext
+    except ImportError as e:
+      raise RuntimeError("recurrentgemma_b200/_host.so cannot be loaded: build it with "
+                         f"`python -m recurrentgemma_b200.build` ({e})") from e
+    ext.init(LIB_PATH, _workspaces, workspace, check, modules.RecurrentBlockCache)
+    _host = ext
+  return _host
+
+
 def check(rc: int) -> None:
   if rc != 0:
     raise RgkError(rc, load().rgk_last_error().decode(errors="replace"))

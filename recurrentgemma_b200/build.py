@@ -1,4 +1,5 @@
-"""Builds recurrentgemma_b200/librgk.so from csrc/*.cu with nvcc for sm_100a (in-tree).
+"""Builds recurrentgemma_b200/librgk.so from csrc/*.cu with nvcc for sm_100a, and _host.so (the
+native host side of the modules' calls) from csrc/host.cpp, both in-tree.
 
     python -m recurrentgemma_b200.build [--force] [--verbose] [--checks]
 
@@ -14,11 +15,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "librgk.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -65,11 +68,12 @@ def _compile_one(nvcc: str, src: str, obj: str, verbose: bool, checks: bool = Fa
 
 
 def build_library(force: bool = False, verbose: bool = False, checks: bool = False) -> str:
-  """Compiles every .cu under csrc/ and links librgk.so; returns its path.  checks=True builds
+  """Compiles every .cu under csrc/ and links librgk.so (and builds _host.so); returns librgk's path.  checks=True builds
   librgk_checks.so instead: the same library with -DRGK_CHECKS, in which computed indices of the
   look-back records, states and outputs are range-checked (a bad one raises the status word to -8
   and the access is skipped; nothing traps)."""
   nvcc = _nvcc()
+  build_host(force and not checks)
   os.makedirs(OBJ_DIR, exist_ok=True)
   deps = _deps()
   jobs = []
@@ -90,6 +94,28 @@ def build_library(force: bool = False, verbose: bool = False, checks: bool = Fal
     if r.returncode != 0:
       raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
   return lib_path
+
+
+def build_host(force: bool = False) -> str:
+  """Compiles csrc/host.cpp against torch's headers into the extension module _host.so."""
+  src = os.path.join(CSRC, "host.cpp")
+  if not force and not _stale(HOST_PATH, [src, *_deps()]):
+    return HOST_PATH
+  import torch
+  root = os.path.join(os.path.dirname(torch.__file__))
+  inc = os.path.join(root, "include")
+  cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+  cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+         "-I", sysconfig.get_paths()["include"], "-I", inc,
+         "-I", os.path.join(inc, "torch", "csrc", "api", "include"),
+         "-I", os.path.join(cuda, "include"), src, "-o", HOST_PATH,
+         "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+         "-lc10", "-lc10_cuda"]
+  r = subprocess.run(cmd, capture_output=True, text=True)
+  if r.returncode != 0:
+    raise RuntimeError(f"g++ failed for {src}:\n{r.stdout}\n{r.stderr}")
+  return HOST_PATH
 
 
 def main():

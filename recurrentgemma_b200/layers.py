@@ -285,6 +285,9 @@ class RGLRU(nn.Module):
       return_cache: bool = True,
   ) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """Returns (y [B,T,E] in x.dtype, last hidden state [B,E] float32 or None)."""
+    done = _lib.host().rglru(self, x, segment_pos, cache, return_cache)
+    if done is not NotImplemented:
+      return done
     bs, l, e = x.shape
     assert e == self.width
     dev = _lib.require_cuda(x, segment_pos, cache, self.a_param)

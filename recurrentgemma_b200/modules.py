@@ -48,6 +48,10 @@ def recurrent_path(
   input projections and `linear_out` (recurrentgemma/torch/modules.py:631-646).  With `inplace`
   a decode step overwrites the tensors of `cache` and returns that cache (an extension for
   decode loops that run as a CUDA graph; the reference always returns new tensors)."""
+  done = _lib.host().recurrent_path(xb, yb, segment_pos, conv_1d, rg_lru, cache, return_cache, out,
+                                    inplace)
+  if done is not NotImplemented:
+    return done
   bs, l, e = xb.shape
   dev = _lib.require_cuda(xb, yb, segment_pos, conv_1d.w, rg_lru.a_param)
   layers._same_dtype(xb, conv_1d.w, conv_1d.b, rg_lru.a_param, rg_lru.input_gate.w,
