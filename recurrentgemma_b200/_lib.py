@@ -39,6 +39,17 @@ class RgkBlockParams(ctypes.Structure):
       "linear_y_w", "linear_y_b", "linear_x_w", "linear_x_b", "linear_out_w", "linear_out_b")]
 
 
+class RgkChannelParams(ctypes.Structure):
+  """struct rgk_channel_params of include/rgk.h."""
+  _fields_ = [(n, _vp) for n in ("norm_scale", "packed_up", "down_w", "down_b")] + [
+      ("eps", ctypes.c_float)]
+
+
+class RgkAttentionParams(ctypes.Structure):
+  """struct rgk_attention_params of include/rgk.h."""
+  _fields_ = [(n, _vp) for n in ("q_w", "k_w", "v_w", "final_w", "final_b")]
+
+
 # name -> (restype, argtypes); mirrors include/rgk.h declaration by declaration.
 SIGNATURES = {
     "rgk_abi_version": (_int, []),
@@ -90,6 +101,16 @@ SIGNATURES = {
     "rgk_dense_linear_small": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _int, _vp, _vp, _vp]),
     "rgk_dense_linear_small_pair": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _int, _vp,
                                            _vp, _vp, _vp]),
+    "rgk_residual_decode_rows": (_int, []),
+    "rgk_residual_decode_workspace_bytes": (_sz, [_i64, _i64, _i64, _i64, _int, _int]),
+    "rgk_recurrent_residual_decode": (_int, [
+        _vp, _vp, _int, ctypes.POINTER(RgkBlockParams), _vp, ctypes.c_float,
+        ctypes.POINTER(RgkChannelParams), _vp, _vp, _i64, _i64, _i64, _i64, _int, _int, _int, _int,
+        _vp, _vp, _vp, _int, _vp, _sz, _vp]),
+    "rgk_attention_residual_decode": (_int, [
+        _vp, _vp, _int, ctypes.POINTER(RgkAttentionParams), _vp, ctypes.c_float,
+        ctypes.POINTER(RgkChannelParams), _vp, _vp, _vp, _i64, _i64, _i64, _int, _int, _int, _int,
+        _int, _vp, _int, _vp, _sz, _vp]),
     "rgk_embed": (_int, [_vp, _int, _vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp]),
     "rgk_logits": (_int, [_vp, _vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp, _vp]),
     "rgk_argmax": (_int, [_vp, _i64, _i64, _int, _vp, _vp]),
@@ -148,7 +169,12 @@ def host():
     except ImportError as e:
       raise RuntimeError("recurrentgemma_b200/_host.so cannot be loaded: build it with "
                          f"`python -m recurrentgemma_b200.build` ({e})") from e
-    ext.init(LIB_PATH, _workspaces, workspace, check, modules.RecurrentBlockCache)
+    from torch.nn.modules import module as nn_module
+    ext.init(LIB_PATH, _workspaces, workspace, check,
+             (modules.RecurrentBlockCache, modules.AttentionBlockCache, modules.layers.RMSNorm,
+              modules.RecurrentBlock, modules.LocalAttentionBlock, modules.MLPBlock,
+              modules.ResidualBlock),
+             nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks)
     _host = ext
   return _host
 
@@ -200,8 +226,11 @@ def stream_ptr(dev: torch.device) -> int:
 
 
 # One growing scratch buffer per (device, stream): calls on one stream are ordered, so they can
-# share it; different streams get different buffers.
+# share it; different streams get different buffers.  A buffer that has become too small is retired,
+# not freed: a CUDA graph captured while it was current holds its address.  Buffers at least double,
+# so the retired ones of a stream together are no larger than its current one.
 _workspaces = {}
+_retired = {}
 
 
 def workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
@@ -209,13 +238,13 @@ def workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
          torch.cuda.current_stream(dev).cuda_stream)
   buf = _workspaces.get(key)
   if buf is None or buf.numel() < nbytes:
+    size = max(nbytes, 1 << 20) if buf is None else max(nbytes, 2 * buf.numel())
     with torch.cuda.device(dev):
-      new = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
+      new = torch.empty(size, dtype=torch.uint8, device=dev)
       # the status word (first int): kernels only ever raise it, nobody but its reader clears it
-      if buf is None:
-        new[:4].zero_()
-      else:
-        new[:4].copy_(buf[:4])
+      new[:4].zero_()
+    if buf is not None:
+      _retired.setdefault(key, []).append(buf)
     _workspaces[key] = buf = new
   return buf
 
@@ -249,4 +278,5 @@ def check_status(device: Optional[torch.device] = None) -> None:
   for (dev_index, stream), buf in list(_workspaces.items()):
     if index is None or dev_index == index:
       with torch.cuda.device(dev_index):
-        workspace_status(buf, stream)
+        for b in [buf, *_retired.get((dev_index, stream), [])]:
+          workspace_status(b, stream)

@@ -62,12 +62,16 @@ class GreedySampler:
                "next_token": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "positions": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "cache": _own(cache), "logits": None}
-      # one eager step creates every lazily made buffer of a decode step; capturing then records
-      # the launches without running them
-      self._step(state)
+      # one eager step on the capture stream creates every lazily made buffer of a decode step (the
+      # stream's workspace among them, which must not come from the graph's own memory pool: it
+      # outlives this graph); capturing then records the launches without running them
+      stream = _capture_stream(dev)
+      stream.wait_stream(torch.cuda.current_stream(dev))
+      with torch.cuda.stream(stream):
+        self._step(state)
       graph = torch.cuda.CUDAGraph()
       torch.cuda.synchronize(dev)
-      with torch.cuda.graph(graph):
+      with torch.cuda.graph(graph, stream=stream):
         self._step(state)
       self._state, self._graph, self._graph_key = state, graph, (b, dev)
     for name, c in cache.items():
@@ -146,6 +150,17 @@ class GreedySampler:
     if check_status:
       _lib.check_status(dev)
     return SamplerOutput(out_tokens, out_logits)
+
+
+_capture_streams = {}
+
+
+def _capture_stream(dev: torch.device) -> torch.cuda.Stream:
+  """The one stream per device that samplers capture their graphs on."""
+  index = dev.index if dev.index is not None else torch.cuda.current_device()
+  if index not in _capture_streams:
+    _capture_streams[index] = torch.cuda.Stream(index)
+  return _capture_streams[index]
 
 
 def _own(cache):
