@@ -387,6 +387,51 @@ RGK_API int rgk_local_attention_decode(const void* q, const void* k_new, const v
                                        void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * ResidualBlock.forward with a cache: one token per sequence through a whole residual block
+ * (recurrentgemma/torch/modules.py:897-911), either kind of temporal block, as one call:
+ *   r = temporal_block(rmsnorm(x)) + x;  out = mlp(rmsnorm(r)) + r        x, out [B,D] (B tokens)
+ * The norms, biases, activations and residual adds run inside the projection kernels, and the
+ * kernels follow one another as programmatic dependents: each fetches its weights while its
+ * predecessor finishes.  bfloat16, B <= rgk_residual_decode_rows(), head width / head dimension 256,
+ * W = 4; RGK_ESHAPE otherwise.  The caches may be updated in place (h_out = h_in, conv_out = conv_in;
+ * the attention ring always is, see rgk_local_attention_decode).
+ * chained != 0: the last work enqueued on the stream is another such call, so that no kernel that may
+ * still be running writes weights, and this call may fetch its first weights ahead of its turn.
+ * workspace: rgk_residual_decode_workspace_bytes(B, D, E, X, N, window) bytes, 256-byte aligned (for
+ * a recurrent block N = window = 0, for an attention block E = D); first word: status.
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct rgk_channel_params {
+  const void* norm_scale; /* channel_pre_norm.scale          [D] */
+  const void* packed_up;  /* output of rgk_pack_mlp_up           */
+  const void* down_w;     /* mlp_block.ffw_down.weight    [D, X] */
+  const void* down_b;     /* mlp_block.ffw_down.bias         [D] */
+  float eps;
+} rgk_channel_params;
+
+typedef struct rgk_attention_params {
+  const void* q_w;        /* proj_q.weight                [D, D] */
+  const void* k_w;        /* proj_k.weight              [256, D] */
+  const void* v_w;        /* proj_v.weight              [256, D] */
+  const void* final_w;    /* proj_final.weight            [D, D] */
+  const void* final_b;    /* proj_final.bias                 [D] */
+} rgk_attention_params;
+
+RGK_API int rgk_residual_decode_rows(void);
+RGK_API size_t rgk_residual_decode_workspace_bytes(int64_t B, int64_t D, int64_t E, int64_t X, int N,
+                                                   int window);
+RGK_API int rgk_recurrent_residual_decode(
+    const void* x, const void* segment_pos, int pos_dtype, const rgk_block_params* p,
+    const void* norm_scale, float eps, const rgk_channel_params* channel, const float* h_in,
+    const void* conv_cache_in, int64_t B, int64_t D, int64_t E, int64_t X, int H, int W, int dtype,
+    int gates_impl, void* out, float* h_out, void* conv_cache_out, int chained, void* workspace,
+    size_t workspace_bytes, void* stream);
+RGK_API int rgk_attention_residual_decode(
+    const void* x, const void* segment_pos, int pos_dtype, const rgk_attention_params* p,
+    const void* norm_scale, float eps, const rgk_channel_params* channel, void* keys, void* values,
+    int* num_tokens, int64_t B, int64_t D, int64_t X, int N, int head_dim, int window, int dtype,
+    int update, void* out, int chained, void* workspace, size_t workspace_bytes, void* stream);
+
+/* ------------------------------------------------------------------------------------------------
  * The two ends of Griffin.forward around the residual blocks, and greedy sampling.
  * rgk_embed: Embedder.encode (recurrentgemma/torch/modules.py:991-998): out [M,D] =
  *   table[tokens[m], :] * scale (scale = sqrt(D) rounded to bfloat16, or 1), tokens RGK_I32 or

@@ -490,6 +490,28 @@ int rgk_dense_linear(const void* x, const void* weight, const void* bias, int64_
   return RGK_OK;
 }
 
+// Projections of few rows on the kernel for their number: up to kRowsGemm rows the one that streams
+// weights into registers, above that the one with 128-feature tensor-core tiles.
+static constexpr int kRowsGemm = 8;
+static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats,
+                                   const void* residual, int64_t M, int K, int act, float cap, int* status,
+                                   bool early, bool wide, cudaStream_t s) {
+  if (M <= kRowsGemm)
+    return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
+  return rgk::launch_dense_small(x, mats, n_mats, residual, M, K, act, cap, status, early, wide, s);
+}
+
+// The same with RMSNorm of the rows in front: inside the kernel, or as one of its own into xn.
+static cudaError_t few_rows_norm_linear(const void* x, const void* scale, float eps, void* xn,
+                                        const rgk::RowsMatrix* mats, int n_mats, int64_t M, int K, int act,
+                                        int* status, bool early, cudaStream_t s) {
+  if (M <= kRowsGemm && rgk::rows_gemm_supported(RGK_BF16, M, K, 8, true))
+    return rgk::launch_rows_gemm(x, scale, eps, mats, n_mats, nullptr, M, K, act, 0.0f, early, s);
+  cudaError_t e = rgk::launch_rmsnorm_rows(x, scale, M, K, eps, early, xn, s);
+  if (e != cudaSuccess) return e;
+  return few_rows_linear(xn, mats, n_mats, nullptr, M, K, act, 0.0f, status, true, true, s);
+}
+
 int rgk_dense_linear_small(const void* x, const void* weight, const void* bias, const void* residual,
                            int64_t M, int64_t K, int64_t N, int dtype, int act, void* out,
                            int* status, void* stream) {
@@ -504,13 +526,14 @@ int rgk_dense_linear_small(const void* x, const void* weight, const void* bias, 
               "multiple of 64, N=%lld) and no residual", (long long)N);
   RGK_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(out) && aligned16(bias) &&
               aligned16(residual), RGK_EALIGN, "pointers must be 16-byte aligned");
-  RGK_REQUIRE(rgk::dense_small_supported(dtype, M > 0 ? M : 1, K, N), RGK_ESHAPE,
+  RGK_REQUIRE(M <= 256 && rgk::dense_small_supported(dtype, M > 0 ? M : 1, K, N), RGK_ESHAPE,
               "the few-row linear covers bfloat16 with M <= 256 and K and N multiples of 8 "
               "(dtype %d, M=%lld, K=%lld, N=%lld)", dtype, (long long)M, (long long)K, (long long)N);
   if (M == 0) return RGK_OK;
   RGK_CHECK_DEVICE();
-  RGK_CUDA(rgk::launch_dense_small(x, weight, bias, nullptr, nullptr, residual, M, (int)K, (int)N, 0,
-                                   act, out, nullptr, status, static_cast<cudaStream_t>(stream)),
+  const rgk::RowsMatrix mat = {weight, bias, out, (int)N};
+  RGK_CUDA(few_rows_linear(x, &mat, 1, residual, M, (int)K, act, 0.0f, status, false, true,
+                           static_cast<cudaStream_t>(stream)),
            "few-row dense linear launch");
   return RGK_OK;
 }
@@ -527,15 +550,16 @@ int rgk_dense_linear_small_pair(const void* x, const void* weight_a, const void*
   RGK_REQUIRE(aligned16(x) && aligned16(weight_a) && aligned16(weight_b) && aligned16(out_a) &&
               aligned16(out_b) && aligned16(bias_a) && aligned16(bias_b), RGK_EALIGN,
               "pointers must be 16-byte aligned");
-  RGK_REQUIRE(rgk::dense_small_supported(dtype, M > 0 ? M : 1, K, N_a + N_b) && N_a % 128 == 0 &&
+  RGK_REQUIRE(M <= 256 && rgk::dense_small_supported(dtype, M > 0 ? M : 1, K, N_a + N_b) && N_a % 128 == 0 &&
               N_b % 8 == 0, RGK_ESHAPE,
               "the paired few-row linear covers bfloat16 with M <= 256, K and N_b multiples of 8 and "
               "N_a a multiple of 128 (dtype %d, M=%lld, K=%lld, N_a=%lld, N_b=%lld)", dtype,
               (long long)M, (long long)K, (long long)N_a, (long long)N_b);
   if (M == 0) return RGK_OK;
   RGK_CHECK_DEVICE();
-  RGK_CUDA(rgk::launch_dense_small(x, weight_a, bias_a, weight_b, bias_b, nullptr, M, (int)K, (int)N_a,
-                                   (int)N_b, 0, out_a, out_b, status, static_cast<cudaStream_t>(stream)),
+  const rgk::RowsMatrix mats[2] = {{weight_a, bias_a, out_a, (int)N_a}, {weight_b, bias_b, out_b, (int)N_b}};
+  RGK_CUDA(few_rows_linear(x, mats, 2, nullptr, M, (int)K, 0, 0.0f, status, false, true,
+                           static_cast<cudaStream_t>(stream)),
            "paired few-row dense linear launch");
   return RGK_OK;
 }
@@ -573,6 +597,13 @@ int rgk_logits(const void* x, const void* table, int64_t M, int64_t D, int64_t V
               "(dtype %d, D=%lld, V=%lld)", dtype, (long long)D, (long long)V);
   if (M == 0) return RGK_OK;
   RGK_CHECK_DEVICE();
+  if (M <= 256) {
+    const rgk::RowsMatrix mat = {table, nullptr, out, (int)V};
+    RGK_CUDA(few_rows_linear(x, &mat, 1, nullptr, M, (int)D, 0, cap, status, false, true,
+                             static_cast<cudaStream_t>(stream)),
+             "logits launch");
+    return RGK_OK;
+  }
   RGK_CUDA(rgk::launch_dense_tc(x, table, nullptr, nullptr, M, (int)D, (int)V, 0, out, status,
                                 static_cast<cudaStream_t>(stream), cap),
            "logits launch");
@@ -952,6 +983,25 @@ int rgk_local_attention_decode(const void* q, const void* k_new, const void* v_n
   return RGK_OK;
 }
 
+// One decode step of the sub-path on the kernel for its batch: up to kDecodeRows rows the one whose
+// CTAs serve 16 rows, above that the one with 128-row tensor-core tiles.
+static constexpr int kDecodeRows = 96;
+static cudaError_t path_decode_bf16(const void* xb, const void* yb, const void* pos, int pos64,
+                                    const rgk_params* p, const void* packed, const float* h_in,
+                                    const void* conv_in, int64_t B, int H, int gates_impl, void* out,
+                                    float* h_out, void* conv_out, void* ws_header, cudaStream_t s,
+                                    bool early) {
+  const int math = gates_impl == RGK_GATES_FUSED_EXACT || gates_impl == RGK_GATES_TCGEN05
+                       ? rgk::kMathExact : rgk::kMathFast;
+  if (B <= kDecodeRows)
+    return rgk::launch_path_decode_rows(xb, yb, pos, pos64, p->conv_w, p->conv_b, p->a_param, p->gate_x_b,
+                                        p->gate_a_b, packed, h_in, conv_in, B, H, out, h_out, conv_out,
+                                        s, math, early);
+  return rgk::launch_path_decode_tc(xb, yb, pos, pos64, p->conv_w, p->conv_b, p->a_param, p->gate_x_b,
+                                    p->gate_a_b, packed, h_in, conv_in, B, H, out, h_out, conv_out,
+                                    ws_header, s, math);
+}
+
 int rgk_recurrent_path_decode(const void* xb, const void* yb, const void* segment_pos,
                               int pos_dtype, const rgk_params* p, const float* h_in,
                               const void* conv_cache_in, int64_t B, int64_t E, int H, int W,
@@ -990,12 +1040,8 @@ int rgk_recurrent_path_decode(const void* xb, const void* yb, const void* segmen
                "pack_gate_weights launch");
       packed = w.wpack;
     }
-    RGK_CUDA(rgk::launch_path_decode_tc(xb, yb, segment_pos, pos_dtype, p->conv_w, p->conv_b,
-                                        p->a_param, p->gate_x_b, p->gate_a_b, packed, h_in,
-                                        conv_cache_in, B, H, out, h_out, conv_cache_out, workspace,
-                                        s, (gates_impl == RGK_GATES_FUSED_EXACT ||
-                                            gates_impl == RGK_GATES_TCGEN05) ? rgk::kMathExact
-                                                                             : rgk::kMathFast),
+    RGK_CUDA(path_decode_bf16(xb, yb, segment_pos, pos_dtype, p, packed, h_in, conv_cache_in, B, H,
+                              gates_impl, out, h_out, conv_cache_out, workspace, s, false),
              "fused decode launch");
     return RGK_OK;
   }
@@ -1008,6 +1054,137 @@ int rgk_recurrent_path_decode(const void* xb, const void* yb, const void* segmen
   RGK_CUDA(rgk::launch_decode_update(w.a, w.xn, h_in, yb, B, E, dtype, out, h_out, s),
            "decode_update launch");
   return RGK_OK;
+}
+
+// ---- one token through a whole residual block ---------------------------------------------------------
+
+int rgk_residual_decode_rows(void) { return 256; }
+
+// [header | four tensors [B, E] | two [B, D] | the hidden activations [B, X] | ring attention]
+size_t rgk_residual_decode_workspace_bytes(int64_t B, int64_t D, int64_t E, int64_t X, int N, int window) {
+  if (B < 0 || D < 1 || E < 1 || X < 1 || N < 0 || window < 0) return 0;
+  if (B < 1) B = 1;
+  const size_t ring = N > 0 && window > 0 ? rgk::attention_decode_workspace_bytes(B, N, window) : 0;
+  return 256 + 4 * up256((size_t)B * E * 2) + 2 * up256((size_t)B * D * 2) + up256((size_t)B * X * 2) + ring;
+}
+
+static int check_residual_decode(const void* x, const void* segment_pos, int pos_dtype,
+                                 const void* norm_scale, const rgk_channel_params* c, int64_t B,
+                                 int64_t D, int64_t E, int64_t X, int N, int window, int dtype,
+                                 const void* out, void* workspace, size_t workspace_bytes) {
+  RGK_REQUIRE(dtype == RGK_BF16, RGK_ESHAPE, "the residual decode step is bfloat16 only (dtype %d)", dtype);
+  RGK_REQUIRE(pos_dtype == RGK_I32 || pos_dtype == RGK_I64, RGK_EINVAL, "unknown index dtype");
+  RGK_REQUIRE(B >= 0, RGK_EINVAL, "negative batch");
+  RGK_REQUIRE(B <= rgk_residual_decode_rows(), RGK_ESHAPE, "the residual decode step covers up to %d "
+              "sequences (B=%lld)", rgk_residual_decode_rows(), (long long)B);
+  RGK_REQUIRE(x && segment_pos && norm_scale && out && c && c->norm_scale && c->packed_up && c->down_w,
+              RGK_EINVAL, "NULL pointer argument");
+  RGK_REQUIRE(aligned16(x) && aligned16(norm_scale) && aligned16(out) && aligned16(c->norm_scale) &&
+                  aligned16(c->packed_up) && aligned16(c->down_w) && aligned16(c->down_b),
+              RGK_EALIGN, "pointers must be 16-byte aligned");
+  RGK_REQUIRE(D >= 8 && D % 8 == 0 && X >= 64 && X % 64 == 0 && D < (1 << 24) && X < (1 << 23) &&
+                  rgk::rmsnorm_supported(dtype, D),
+              RGK_ESHAPE, "widths the residual decode step does not cover (D=%lld, X=%lld)", (long long)D,
+              (long long)X);
+  const size_t need = rgk_residual_decode_workspace_bytes(B, D, E, X, N, window);
+  RGK_REQUIRE(workspace != nullptr && workspace_bytes >= need, RGK_EWORKSPACE,
+              "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+  RGK_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, RGK_EALIGN,
+              "workspace must be 256-byte aligned");
+  return RGK_OK;
+}
+
+// The channel half, r -> out, with `hidden` [B, X] as scratch; always behind kernels of this call.
+static int channel_decode(const void* r, const rgk_channel_params* c, int64_t B, int64_t D, int64_t X,
+                          void* xn, void* hidden, void* out, int* status, cudaStream_t s) {
+  const char* pw = static_cast<const char*>(c->packed_up);
+  const rgk::RowsMatrix up = {pw, pw + mlp_pack_w_bytes(D, X), hidden, (int)(2 * X)};
+  RGK_CUDA(few_rows_norm_linear(r, c->norm_scale, c->eps, xn, &up, 1, B, (int)D, 2, status, true, s),
+           "ffw_up launch");
+  const rgk::RowsMatrix down = {c->down_w, c->down_b, out, (int)D};
+  RGK_CUDA(few_rows_linear(hidden, &down, 1, r, B, (int)X, 0, 0.0f, status, true, false, s),
+           "ffw_down launch");
+  return RGK_OK;
+}
+
+int rgk_recurrent_residual_decode(const void* x, const void* segment_pos, int pos_dtype,
+                                  const rgk_block_params* p, const void* norm_scale, float eps,
+                                  const rgk_channel_params* channel, const float* h_in,
+                                  const void* conv_cache_in, int64_t B, int64_t D, int64_t E, int64_t X,
+                                  int H, int W, int dtype, int gates_impl, void* out, float* h_out,
+                                  void* conv_cache_out, int chained, void* workspace,
+                                  size_t workspace_bytes, void* stream) {
+  int rc = check_block_args(x, segment_pos, pos_dtype, p, B, 1, D, E, H, W, dtype, out, h_out,
+                            conv_cache_out);
+  if (rc) return rc;
+  if ((rc = check_residual_decode(x, segment_pos, pos_dtype, norm_scale, channel, B, D, E, X, 0, 0, dtype,
+                                  out, workspace, workspace_bytes)))
+    return rc;
+  RGK_REQUIRE(gates_impl >= RGK_GATES_AUTO && gates_impl <= RGK_GATES_FUSED_EXACT &&
+                  gates_impl != RGK_GATES_SIMT, RGK_EINVAL, "unknown gates_impl %d", gates_impl);
+  RGK_REQUIRE(h_in && conv_cache_in && h_out && conv_cache_out && p->path.gates_packed, RGK_EINVAL,
+              "NULL pointer argument");
+  RGK_REQUIRE(aligned16(h_in) && aligned16(conv_cache_in), RGK_EALIGN, "pointers must be 16-byte aligned");
+  if (B == 0) return RGK_OK;
+  RGK_CHECK_DEVICE();
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  char* yb = static_cast<char*>(workspace) + 256;
+  const size_t act = up256((size_t)B * E * 2), wide = up256((size_t)B * D * 2);
+  char *xb = yb + act, *z = xb + act, *r = z + 2 * act, *xn = r + wide, *hidden = xn + wide;
+  int* status = static_cast<int*>(workspace);
+  const rgk::RowsMatrix in[2] = {{p->linear_y_w, p->linear_y_b, yb, (int)E},
+                                 {p->linear_x_w, p->linear_x_b, xb, (int)E}};
+  RGK_CUDA(few_rows_norm_linear(x, norm_scale, eps, xn, in, 2, B, (int)D, 0, status, chained != 0, s),
+           "linear_y, linear_x launch");
+  RGK_CUDA(path_decode_bf16(xb, yb, segment_pos, pos_dtype, &p->path, p->path.gates_packed, h_in,
+                            conv_cache_in, B, H, gates_impl, z, h_out, conv_cache_out, workspace, s, true),
+           "fused decode launch");
+  const rgk::RowsMatrix last = {p->linear_out_w, p->linear_out_b, r, (int)D};
+  RGK_CUDA(few_rows_linear(z, &last, 1, x, B, (int)E, 0, 0.0f, status, true, false, s),
+           "linear_out launch");
+  return channel_decode(r, channel, B, D, X, xn, hidden, out, status, s);
+}
+
+int rgk_attention_residual_decode(const void* x, const void* segment_pos, int pos_dtype,
+                                  const rgk_attention_params* p, const void* norm_scale, float eps,
+                                  const rgk_channel_params* channel, void* keys, void* values,
+                                  int* num_tokens, int64_t B, int64_t D, int64_t X, int N, int head_dim,
+                                  int window, int dtype, int update, void* out, int chained,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+  RGK_REQUIRE(N >= 1 && window >= 1, RGK_EINVAL, "bad size (heads=%d window=%d)", N, window);
+  int rc = check_residual_decode(x, segment_pos, pos_dtype, norm_scale, channel, B, D, D, X, N, window,
+                                 dtype, out, workspace, workspace_bytes);
+  if (rc) return rc;
+  RGK_REQUIRE(p && p->q_w && p->k_w && p->v_w && p->final_w && keys && values && num_tokens, RGK_EINVAL,
+              "NULL pointer argument");
+  RGK_REQUIRE(aligned16(p->q_w) && aligned16(p->k_w) && aligned16(p->v_w) && aligned16(p->final_w) &&
+                  aligned16(p->final_b) && aligned16(keys) && aligned16(values),
+              RGK_EALIGN, "pointers must be 16-byte aligned");
+  RGK_REQUIRE(rgk::attention_decode_supported(head_dim, N, window) && D == (int64_t)N * head_dim, RGK_ESHAPE,
+              "the decode attention kernel covers head dimension 256 and 1/2/4/8/10 query heads "
+              "(head_dim %d, heads %d, window %d)", head_dim, N, window);
+  if (B == 0) return RGK_OK;
+  RGK_CHECK_DEVICE();
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  char* q = static_cast<char*>(workspace) + 256;
+  const size_t wide = up256((size_t)B * D * 2);
+  char *k = q + wide, *v = k + up256((size_t)B * head_dim * 2), *enc = q + 3 * wide, *r = enc + wide;
+  char *xn = r + wide, *hidden = xn + wide;
+  int* status = static_cast<int*>(workspace);
+  char* ring = hidden + up256((size_t)B * X * 2);
+  const rgk::RowsMatrix in[3] = {{p->q_w, nullptr, q, (int)D}, {p->k_w, nullptr, k, head_dim},
+                                 {p->v_w, nullptr, v, head_dim}};
+  RGK_CUDA(few_rows_norm_linear(x, norm_scale, eps, xn, in, 3, B, (int)D, 0, status, chained != 0, s),
+           "proj_q, proj_k, proj_v launch");
+  RGK_CUDA(rgk::launch_rope(q, segment_pos, pos_dtype == RGK_I64, B, N, head_dim, dtype, s), "rope launch");
+  RGK_CUDA(rgk::launch_rope(k, segment_pos, pos_dtype == RGK_I64, B, 1, head_dim, dtype, s), "rope launch");
+  RGK_CUDA(rgk::launch_attention_decode(q, k, v, keys, values, num_tokens, B, N, window, dtype, update,
+                                        enc, ring, s),
+           "decode attention launch");
+  const rgk::RowsMatrix last = {p->final_w, p->final_b, r, (int)D};
+  RGK_CUDA(few_rows_linear(enc, &last, 1, x, B, (int)D, 0, 0.0f, status, true, false, s),
+           "proj_final launch");
+  return channel_decode(r, channel, B, D, X, xn, hidden, out, status, s);
 }
 
 }  // extern "C"

@@ -36,8 +36,9 @@ static_assert(kSmemG <= 232448, "exceeds the 227 KiB of shared memory a CTA may 
 constexpr uint32_t kIdescG = tc_idesc_bf16(BM, BN);
 
 // kMode 0: bias only; 1: gelu_tanh of the rounded result; 2: + residual (rounded again);
-// 3: GeGLU - W holds, per group of 128 rows, 64 gate rows then the 64 value rows of the same
-//    features (see pack_mlp_up_kernel); out [M, N/2] = gelu_tanh(gate) * value, where gate and
+// 3: GeGLU - W holds, per group of 8 rows, 4 gate rows then the 4 value rows of the same features
+//    (see pack_mlp_up_kernel: groups this small leave every kernel free to cut tiles at multiples of
+//    8 rows); out [M, N/2] = gelu_tanh(gate) * value, where gate and
 //    value are round(round(acc) + bias): the contraction and the bias add are two tensor operations
 //    in the reference (torch/layers.py:700-703, torch/modules.py:749-751);
 // 4: logits soft cap - round(tanh(round(round(acc) / cap)) * cap), the three tensor operations of
@@ -102,28 +103,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     }
   } else if (warp == kEpi + 1) {
     // ------------------------------ MMA issue -----------------------------------------------------
-    if (lane == 0) {
-      unsigned it = 0;
-      bool ok = true;
-      for (int t = 0; t < n_my && ok; ++t) {
-        const int as = t & 1;
-        ok = mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort);
-        if (!ok) break;
-        tc_fence_after();
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          ok = mbar_wait(bar_full(s), (it / kStages) & 1, s_abort);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a0 = s_base + kOffRing + s * kStageBytes, b0 = a0 + kABytes;
-#pragma unroll
-          for (int ks = 0; ks < BK / 16; ++ks)
-            tc_mma_bf16(tmem_base + as * BN, smem_desc_sw128(a0 + ks * 32),
-                        smem_desc_sw128(b0 + ks * 32), kIdescG, (kb | ks) != 0 ? 1u : 0u);
-          tc_commit(bar_empty(s));
-        }
-        if (ok) tc_commit(bar_acc_full(as));
-      }
+    RingPos at;
+    bool ok = true;
+    for (int t = 0; t < n_my; ++t) {
+      const int as = t & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+      if (!ok) break;
+      tc_fence_after();
+      ok = mma_ring<BK / 16>(tmem_base + as * BN, smem_desc_sw128(s_base + kOffRing),
+                             smem_desc_sw128(s_base + kOffRing + kABytes), kStageBytes >> 4, kIdescG, k_blocks,
+                             kStages, bar_full(0), bar_empty(0), at, s_abort);
+      if (!ok) break;
+      if (elect_one()) tc_commit(bar_acc_full(as));
+      __syncwarp();
     }
   } else {
     // ------------------------------ epilogue ------------------------------------------------------
@@ -142,40 +134,37 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + as * BN +
                              col_half * 128;
       if constexpr (kMode == 3) {
-        // this warp's 128 accumulator columns are one group: gate columns 0-63, value columns 64-127
         const int n_out = N / 2;
-        const int oc0 = n0 / 2;                // first output feature of the group
+        const int oc0 = n0 / 2;                // first output feature of this warp's 128 columns
 #pragma unroll 1
         for (int cc = 0; cc < 2; ++cc) {       // 32 features at a time
           uint4 ov[4];
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {     // 16 features: bounded register use
-            uint32_t ag[16], av[16];
-            tc_ld_32x16(t_row + cc * 32 + hf * 16, ag);
-            tc_ld_32x16(t_row + 64 + cc * 32 + hf * 16, av);
-            const int nb = n0 + cc * 32 + hf * 16;
-            uint4 bg[2], bvv[2];
+          for (int hf = 0; hf < 2; ++hf) {     // 32 columns = 16 features: bounded register use
+            uint32_t acc[32];
+            tc_ld_32x32(t_row + cc * 64 + hf * 32, acc);
+            const int nb = n0 + cc * 64 + hf * 32;
+            uint4 bv[4];                       // 4 gate biases, then 4 value biases
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              bg[j] = *reinterpret_cast<const uint4*>(bias + nb + 8 * j);
-              bvv[j] = *reinterpret_cast<const uint4*>(bias + nb + 64 + 8 * j);
-            }
+            for (int j = 0; j < 4; ++j) bv[j] = nb + 8 * j < N ? *reinterpret_cast<const uint4*>(bias + nb + 8 * j)
+                                                               : make_uint4(0u, 0u, 0u, 0u);
             tc_wait_ld();
+            uint32_t o[8];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const uint32_t bgp[4] = {bg[j].x, bg[j].y, bg[j].z, bg[j].w};
-              const uint32_t bvp[4] = {bvv[j].x, bvv[j].y, bvv[j].z, bvv[j].w};
-              uint32_t o[4];
+            for (int j = 0; j < 4; ++j) {
 #pragma unroll
-              for (int p = 0; p < 4; ++p) {
+              for (int p = 0; p < 2; ++p) {
                 const int n = j * 8 + p * 2;
-                const uint32_t g2 = badd2(pack_bf16x2(__uint_as_float(ag[n]), __uint_as_float(ag[n + 1])), bgp[p]);
-                const uint32_t v2 = badd2(pack_bf16x2(__uint_as_float(av[n]), __uint_as_float(av[n + 1])), bvp[p]);
+                const uint32_t g2 = badd2(pack_bf16x2(__uint_as_float(acc[n]), __uint_as_float(acc[n + 1])),
+                                          p == 0 ? bv[j].x : bv[j].y);
+                const uint32_t v2 = badd2(pack_bf16x2(__uint_as_float(acc[n + 4]), __uint_as_float(acc[n + 5])),
+                                          p == 0 ? bv[j].z : bv[j].w);
                 const uint32_t a2 = pack_bf16x2(gelu_tanh_<true>(bf16_lo(g2)), gelu_tanh_<true>(bf16_hi(g2)));
-                o[p] = bmul2(a2, v2);
+                o[j * 2 + p] = bmul2(a2, v2);
               }
-              ov[hf * 2 + j] = make_uint4(o[0], o[1], o[2], o[3]);
             }
+            ov[hf * 2] = make_uint4(o[0], o[1], o[2], o[3]);
+            ov[hf * 2 + 1] = make_uint4(o[4], o[5], o[6], o[7]);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
@@ -278,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 }
 
 // ffw_up of the MLP block: w [2, D, X] (in, out) and b [2, X] into the K-major, gate/value
-// interleaved layout of mode 3: packed row g*128 + c*64 + i = column (feature) g*64 + i of w[c].
+// interleaved layout of mode 3: packed row g*8 + c*4 + i = column (feature) g*4 + i of w[c].
 __global__ void pack_mlp_up_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                                    int D, int X, __nv_bfloat16* __restrict__ packed_w,
                                    __nv_bfloat16* __restrict__ packed_b) {
@@ -294,7 +283,7 @@ __global__ void pack_mlp_up_kernel(const __nv_bfloat16* __restrict__ w, const __
   for (int r = threadIdx.y; r < 32; r += 8) {                      // r walks features, x walks k
     const int f = f0 + r, k = k0 + threadIdx.x;
     if (f < X && k < D) {
-      const int64_t row = (int64_t)(f / 64) * 128 + c * 64 + (f % 64);
+      const int64_t row = (int64_t)(f / 4) * 8 + c * 4 + (f % 4);
       packed_w[row * D + k] = tile[threadIdx.x][r];
       if (k == 0) packed_b[row] = b[(int64_t)c * X + f];
     }

@@ -27,8 +27,10 @@ struct Lib {
   decltype(&rgk_recurrent_path_prefill) path_prefill;
   decltype(&rgk_recurrent_path_decode) path_decode;
   decltype(&rgk_rglru_forward) rglru_forward;
-  decltype(&rgk_conv1d_prefill) conv1d_prefill;
-  decltype(&rgk_conv1d_decode) conv1d_decode;
+  decltype(&rgk_residual_decode_rows) residual_decode_rows;
+  decltype(&rgk_residual_decode_workspace_bytes) residual_decode_workspace_bytes;
+  decltype(&rgk_recurrent_residual_decode) recurrent_residual_decode;
+  decltype(&rgk_attention_residual_decode) attention_residual_decode;
 } g_lib;
 bool g_ready = false;
 
@@ -37,10 +39,17 @@ PyObject* g_workspaces = nullptr;        // _lib._workspaces: (device, stream) -
 PyObject* g_make_workspace = nullptr;    // _lib.workspace(device, nbytes): grows it
 PyObject* g_raise = nullptr;             // _lib.check(rc): raises RgkError with the library's text
 PyObject* g_cache_cls = nullptr;         // modules.RecurrentBlockCache
+PyObject* g_ring_cls = nullptr;          // modules.AttentionBlockCache
+PyObject *g_norm_cls, *g_recurrent_cls, *g_attention_cls, *g_mlp_cls, *g_residual_cls;   // module classes
+PyObject *g_hooks, *g_pre_hooks;         // torch's hooks for every module
 
 // interned attribute names
 #define NAMES(X) X(_parameters) X(_modules) X(w) X(b) X(a_param) X(input_gate) X(a_gate) X(num_heads) \
-  X(gates_impl) X(temporal_width) X(width) X(_pack_key) X(_pack_buf) X(_packed_gates)
+  X(gates_impl) X(temporal_width) X(width) X(_pack_key) X(_pack_buf) X(_packed_gates) \
+  X(_packed_up) X(_forward_hooks) X(_forward_pre_hooks) X(weight) X(bias) X(scale) X(eps) X(conv_1d) \
+  X(rg_lru) X(linear_x) X(linear_y) X(linear_out) X(ffw_up) X(ffw_down) X(proj_q) X(proj_k) X(proj_v) \
+  X(proj_final) X(window_size) X(expanded_width) X(lru_width) X(recurrent_block) \
+  X(attention_block) X(temporal_pre_norm) X(channel_pre_norm) X(mlp_block)
 #define DECL(n) PyObject* s_##n = nullptr;
 NAMES(DECL)
 #undef DECL
@@ -163,21 +172,25 @@ bool succeeded(int rc) {
   return false;
 }
 
-// RGLRU._packed_gates: the packed copy if its key still describes the weights, else whatever the
-// module's own method makes of it.  False: a Python error is set.
-bool packed_gates(PyObject* lru, const at::Tensor& wx, const at::Tensor& wa, int dt, const void** out) {
-  Ref key(PyObject_GetAttr(lru, s__pack_key));
+// The packed copy a module keeps of two of its parameters (RGLRU._packed_gates, MLPBlock._packed_up),
+// if its key still describes them, else whatever the module's own method makes of it.  The key is
+// (address, version) of both and, for the gates, the dtype.  *made: a packing kernel was enqueued.  False: a Python error is set.
+bool packed(PyObject* module, const at::Tensor& p0, const at::Tensor& p1, int dt, PyObject* method,
+            const void** out, bool* made = nullptr) {
+  Ref key(PyObject_GetAttr(module, s__pack_key));
   if (key.p == nullptr) PyErr_Clear();
-  if (key.p != nullptr && PyTuple_Check(key.p) && PyTuple_GET_SIZE(key.p) == 5) {
-    const unsigned long long want[5] = {(unsigned long long)(uintptr_t)wx.const_data_ptr(), (unsigned long long)wx._version(),
-                                        (unsigned long long)(uintptr_t)wa.const_data_ptr(), (unsigned long long)wa._version(),
-                                        (unsigned long long)dt};
+  const Py_ssize_t n = dt >= 0 ? 5 : 4;
+  if (key.p != nullptr && PyTuple_Check(key.p) && PyTuple_GET_SIZE(key.p) == n) {
+    const unsigned long long want[5] = {(unsigned long long)(uintptr_t)p0.const_data_ptr(),
+                                        (unsigned long long)p0._version(),
+                                        (unsigned long long)(uintptr_t)p1.const_data_ptr(),
+                                        (unsigned long long)p1._version(), (unsigned long long)dt};
     bool same = true;
-    for (int i = 0; i < 5 && same; ++i)
+    for (Py_ssize_t i = 0; i < n && same; ++i)
       same = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(key.p, i)) == want[i];
     if (PyErr_Occurred()) PyErr_Clear();
     if (same) {
-      Ref buf(PyObject_GetAttr(lru, s__pack_buf));
+      Ref buf(PyObject_GetAttr(module, s__pack_buf));
       if (buf.p != nullptr && THPVariable_Check(buf.p)) {
         *out = THPVariable_Unpack(buf.p).const_data_ptr();
         return true;
@@ -185,7 +198,8 @@ bool packed_gates(PyObject* lru, const at::Tensor& wx, const at::Tensor& wa, int
       PyErr_Clear();
     }
   }
-  Ref r(PyObject_CallMethodNoArgs(lru, s__packed_gates));
+  if (made != nullptr) *made = true;
+  Ref r(PyObject_CallMethodNoArgs(module, method));
   if (r.p == nullptr) return false;
   *out = r.p == Py_None ? nullptr : PyLong_AsVoidPtr(r.p);
   return !(PyErr_Occurred());
@@ -194,7 +208,7 @@ bool packed_gates(PyObject* lru, const at::Tensor& wx, const at::Tensor& wa, int
 // The parameters of Conv1D (may be absent) + RGLRU.
 enum class Found { yes, no, error };
 Found path_params(PyObject* conv, PyObject* lru, Params& pr, int dt, long width, rgk_params* p,
-                  long* heads, long* impl) {
+                  long* heads, long* impl, bool* made = nullptr) {
   PyObject* gx = submodule(lru, s_input_gate);
   PyObject* ga = submodule(lru, s_a_gate);
   const at::Tensor* wx = pr.get(gx, s_w);
@@ -215,7 +229,7 @@ Found path_params(PyObject* conv, PyObject* lru, Params& pr, int dt, long width,
   p->gate_x_w = wx->const_data_ptr();
   p->gate_a_w = wa->const_data_ptr();
   p->gates_packed = nullptr;
-  if (!packed_gates(lru, *wx, *wa, dt, &p->gates_packed)) return Found::error;
+  if (!packed(lru, *wx, *wa, dt, s__packed_gates, &p->gates_packed, made)) return Found::error;
   return Found::yes;
 }
 
@@ -348,12 +362,177 @@ PyObject* rglru(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return PyTuple_Pack(2, ry.p, rh.p);
 }
 
+// ---- the decode step of a residual block ------------------------------------------------------------
+// The decode step of a few sequences through a whole residual block, one library call.
+
+bool no_hooks(PyObject* module) {
+  for (PyObject* name : {s__forward_hooks, s__forward_pre_hooks}) {
+    Ref d(PyObject_GetAttr(module, name));
+    if (d.p == nullptr || !PyDict_Check(d.p) || PyDict_Size(d.p) != 0) return false;
+  }
+  return true;
+}
+bool exactly(PyObject* module, PyObject* cls) { return (PyObject*)Py_TYPE(module) == cls; }
+bool float_attr(PyObject* o, PyObject* name, float* v) {
+  Ref a(PyObject_GetAttr(o, name));
+  if (a.p == nullptr) return false;
+  *v = (float)PyFloat_AsDouble(a.p);
+  return !PyErr_Occurred();
+}
+// An activation-sized tensor of one token per sequence: [B, 1, width] or the ring's tensors.
+bool shaped(const at::Tensor* t, at::ScalarType dtype, c10::Device dev, at::IntArrayRef sizes) {
+  return t != nullptr && t->scalar_type() == dtype && t->device() == dev && t->sizes() == sizes;
+}
+
+PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* block, PyObject* norm2,
+               PyObject* mlp, PyObject* cache, bool want, bool inplace, bool chained) {
+  const at::Tensor *x = dense(x_arg), *pos = dense(pos_arg);
+  const bool recurrent = exactly(block, g_recurrent_cls);
+  if (x == nullptr || pos == nullptr || !PyTuple_Check(cache) || x->scalar_type() != at::kBFloat16 ||
+      x->dim() != 3 || x->size(1) != 1 || pos->dim() != 2 || pos_code(*pos) < 0 ||
+      pos->device() != x->device() || pos->size(0) != x->size(0) || pos->size(1) != 1)
+    return not_here();
+  const int64_t B = x->size(0), D = x->size(2);
+  const c10::Device dev = x->device();
+  if (B == 0 || B > g_lib.residual_decode_rows() || D == 0) return not_here();
+  if (!(recurrent || exactly(block, g_attention_cls)) || !exactly(norm1, g_norm_cls) ||
+      !exactly(norm2, g_norm_cls) || !exactly(mlp, g_mlp_cls) || PyDict_Size(g_hooks) != 0 ||
+      PyDict_Size(g_pre_hooks) != 0 || !no_hooks(norm1) || !no_hooks(block) || !no_hooks(mlp))
+    return not_here();
+  Guard guard(dev.index());
+  Params pr{at::kBFloat16, dev};
+  // the channel half
+  long X = 0, w1 = 0, w2 = 0, w3 = 0;
+  float eps1 = 0.0f;
+  rgk_channel_params c = {};
+  PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
+  const at::Tensor *up_w = pr.get(up, s_w), *up_b = pr.get(up, s_b);
+  c.norm_scale = pr.ptr(norm2, s_scale);
+  c.down_w = pr.ptr(down, s_weight);
+  c.down_b = pr.ptr(down, s_bias);
+  const void* scale1 = pr.ptr(norm1, s_scale);
+  if (!pr.ok || down == nullptr || !no_hooks(down) || !int_attr(mlp, s_expanded_width, &X) ||
+      !int_attr(mlp, s_width, &w1) || !int_attr(norm1, s_width, &w2) || !int_attr(norm2, s_width, &w3) ||
+      w1 != D || w2 != D || w3 != D || X % 64 != 0 || D % 8 != 0 || !float_attr(norm1, s_eps, &eps1) ||
+      !float_attr(norm2, s_eps, &c.eps))
+    return not_here();
+  const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int pc = pos_code(*pos);
+  Workspace ws;
+  bool made = false;                               // a packing kernel was enqueued by this call
+  if (recurrent) {
+    if (PyTuple_GET_SIZE(cache) != 2) return not_here();
+    const at::Tensor *h_in = dense(PyTuple_GET_ITEM(cache, 0)), *c_in = dense(PyTuple_GET_ITEM(cache, 1));
+    long E = 0, heads = 0, impl = 0, width = 0;
+    if (!int_attr(block, s_lru_width, &E) || !int_attr(block, s_width, &width) || width != D ||
+        !shaped(h_in, at::kFloat, dev, {B, E}) || !shaped(c_in, at::kBFloat16, dev, {B, 3, E}))
+      return not_here();
+    PyObject *ly = submodule(block, s_linear_y), *lx = submodule(block, s_linear_x),
+             *lo = submodule(block, s_linear_out);
+    rgk_block_params p = {};
+    p.linear_y_w = pr.ptr(ly, s_weight); p.linear_y_b = pr.ptr(ly, s_bias);
+    p.linear_x_w = pr.ptr(lx, s_weight); p.linear_x_b = pr.ptr(lx, s_bias);
+    p.linear_out_w = pr.ptr(lo, s_weight); p.linear_out_b = pr.ptr(lo, s_bias);
+    PyObject *conv = submodule(block, s_conv_1d), *lru = submodule(block, s_rg_lru);
+    if (!pr.ok || conv == nullptr || lru == nullptr) return not_here();
+    switch (path_params(conv, lru, pr, RGK_BF16, E, &p.path, &heads, &impl, &made)) {
+      case Found::no: return not_here();
+      case Found::error: return nullptr;
+      case Found::yes: break;
+    }
+    if (E != heads * 256 || impl == RGK_GATES_SIMT || p.path.gates_packed == nullptr) return not_here();
+    if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
+    if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, E, X, 0, 0), &ws)) return nullptr;
+    at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
+    at::Tensor h = inplace ? *h_in : empty({B, E}, at::kFloat, dev);
+    at::Tensor cc = inplace ? *c_in : empty({B, 3, E}, at::kBFloat16, dev);
+    if (!succeeded(g_lib.recurrent_residual_decode(
+            x->const_data_ptr(), pos->const_data_ptr(), pc, &p, scale1, eps1, &c,
+            static_cast<const float*>(h_in->const_data_ptr()), c_in->const_data_ptr(), B, D, E, X,
+            (int)heads, 4, RGK_BF16, (int)impl, out.mutable_data_ptr(),
+            static_cast<float*>(h.mutable_data_ptr()), cc.mutable_data_ptr(), chained && !made ? 1 : 0,
+            ws.ptr, ws.bytes, s)))
+      return nullptr;
+    Ref o(wrap(std::move(out)));
+    if (!want) return PyTuple_Pack(2, o.p, Py_None);
+    Ref state(inplace ? make_cache(Py_NewRef(PyTuple_GET_ITEM(cache, 0)), Py_NewRef(PyTuple_GET_ITEM(cache, 1)))
+                      : make_cache(wrap(std::move(h)), wrap(std::move(cc))));
+    if (o.p == nullptr || state.p == nullptr) return nullptr;
+    return PyTuple_Pack(2, o.p, state.p);
+  }
+  if (PyTuple_GET_SIZE(cache) != 3) return not_here();
+  const at::Tensor *keys = dense(PyTuple_GET_ITEM(cache, 0)), *values = dense(PyTuple_GET_ITEM(cache, 1)),
+                   *seen = dense(PyTuple_GET_ITEM(cache, 2));
+  long heads = 0, window = 0, width = 0;
+  if (!int_attr(block, s_num_heads, &heads) || !int_attr(block, s_window_size, &window) ||
+      !int_attr(block, s_width, &width) || width != D || heads * 256 != D ||
+      !(heads == 1 || heads == 2 || heads == 4 || heads == 8 || heads == 10) ||
+      !shaped(keys, at::kBFloat16, dev, {B, window, 1, 256}) ||
+      !shaped(values, at::kBFloat16, dev, {B, window, 1, 256}) || !shaped(seen, at::kInt, dev, {B}))
+    return not_here();
+  rgk_attention_params p = {};
+  p.q_w = pr.ptr(submodule(block, s_proj_q), s_weight);
+  p.k_w = pr.ptr(submodule(block, s_proj_k), s_weight);
+  p.v_w = pr.ptr(submodule(block, s_proj_v), s_weight);
+  p.final_w = pr.ptr(submodule(block, s_proj_final), s_weight);
+  p.final_b = pr.ptr(submodule(block, s_proj_final), s_bias);
+  if (!pr.ok) return not_here();
+  if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
+  if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, D, X, (int)heads, (int)window), &ws))
+    return nullptr;
+  at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
+  // the kernels work on the ring in place; the functional form is the same step on a copy
+  const bool copy = want && !inplace;
+  at::Tensor k = copy ? keys->clone() : *keys, v = copy ? values->clone() : *values,
+             seen_out = copy ? seen->clone() : *seen;
+  if (!succeeded(g_lib.attention_residual_decode(
+          x->const_data_ptr(), pos->const_data_ptr(), pc, &p, scale1, eps1, &c, k.mutable_data_ptr(),
+          v.mutable_data_ptr(), static_cast<int*>(seen_out.mutable_data_ptr()), B, D, X, (int)heads, 256,
+          (int)window, RGK_BF16, want ? 1 : 0, out.mutable_data_ptr(), chained && !made ? 1 : 0, ws.ptr,
+          ws.bytes, s)))
+    return nullptr;
+  Ref o(wrap(std::move(out)));
+  if (o.p == nullptr) return nullptr;
+  if (!want) return PyTuple_Pack(2, o.p, Py_None);
+  if (!copy) return PyTuple_Pack(2, o.p, cache);
+  Ref rk(wrap(std::move(k))), rv(wrap(std::move(v))), rs(wrap(std::move(seen_out)));
+  if (rk.p == nullptr || rv.p == nullptr || rs.p == nullptr) return nullptr;
+  Ref ring(PyObject_CallFunctionObjArgs(g_ring_cls, rk.p, rv.p, rs.p, nullptr));
+  if (ring.p == nullptr) return nullptr;
+  return PyTuple_Pack(2, o.p, ring.p);
+}
+
+// residual_step(x, segment_pos, norm, temporal block, norm, mlp, cache, return_cache, inplace)
+PyObject* residual_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (!g_ready || n != 9) return not_here();
+  return step(args[0], args[1], args[2], args[3], args[4], args[5], args[6], PyObject_IsTrue(args[7]) == 1,
+              PyObject_IsTrue(args[8]) == 1, false);
+}
+
+// block_step(ResidualBlock, x, segment_pos, cache, return_cache, inplace, chained): the same for a
+// module; chained: the last work on the stream is another block's step (see rgk.h).
+PyObject* block_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (!g_ready || n != 7) return not_here();
+  PyObject* m = args[0];
+  if (!exactly(m, g_residual_cls) || !no_hooks(m)) return not_here();
+  PyObject* temporal = submodule(m, s_recurrent_block);
+  if (temporal == nullptr) temporal = submodule(m, s_attention_block);
+  PyObject *norm1 = submodule(m, s_temporal_pre_norm), *norm2 = submodule(m, s_channel_pre_norm),
+           *mlp = submodule(m, s_mlp_block);
+  if (temporal == nullptr || norm1 == nullptr || norm2 == nullptr || mlp == nullptr) return not_here();
+  return step(args[1], args[2], norm1, temporal, norm2, mlp, args[3], PyObject_IsTrue(args[4]) == 1,
+              PyObject_IsTrue(args[5]) == 1, PyObject_IsTrue(args[6]) == 1);
+}
+
 // ---- set-up --------------------------------------------------------------------------------------
-// init(librgk path, _workspaces, workspace, check, RecurrentBlockCache)
+// init(librgk path, _workspaces, workspace, check, (RecurrentBlockCache, AttentionBlockCache, RMSNorm,
+// RecurrentBlock, LocalAttentionBlock, MLPBlock, ResidualBlock), torch's global forward hooks and pre-hooks)
 PyObject* init(PyObject*, PyObject* args) {
   const char* path = nullptr;
-  PyObject *spaces, *make, *raise, *cache_cls;
-  if (!PyArg_ParseTuple(args, "sO!OOO", &path, &PyDict_Type, &spaces, &make, &raise, &cache_cls))
+  PyObject *spaces, *make, *raise, *cls[7], *hooks, *pre_hooks;
+  if (!PyArg_ParseTuple(args, "sO!OO(OOOOOOO)O!O!", &path, &PyDict_Type, &spaces, &make, &raise, &cls[0],
+                        &cls[1], &cls[2], &cls[3], &cls[4], &cls[5], &cls[6], &PyDict_Type, &hooks, &PyDict_Type,
+                        &pre_hooks))
     return nullptr;
   void* so = dlopen(path, RTLD_NOW | RTLD_LOCAL);        // already loaded by ctypes: the same handle
   if (so == nullptr) {
@@ -369,8 +548,10 @@ PyObject* init(PyObject*, PyObject* args) {
   find(&g_lib.path_prefill, "rgk_recurrent_path_prefill");
   find(&g_lib.path_decode, "rgk_recurrent_path_decode");
   find(&g_lib.rglru_forward, "rgk_rglru_forward");
-  find(&g_lib.conv1d_prefill, "rgk_conv1d_prefill");
-  find(&g_lib.conv1d_decode, "rgk_conv1d_decode");
+  find(&g_lib.residual_decode_rows, "rgk_residual_decode_rows");
+  find(&g_lib.residual_decode_workspace_bytes, "rgk_residual_decode_workspace_bytes");
+  find(&g_lib.recurrent_residual_decode, "rgk_recurrent_residual_decode");
+  find(&g_lib.attention_residual_decode, "rgk_attention_residual_decode");
   if (PyErr_Occurred()) return nullptr;
 #define INTERN(n) if (s_##n == nullptr) s_##n = PyUnicode_InternFromString(#n);
   NAMES(INTERN)
@@ -378,7 +559,11 @@ PyObject* init(PyObject*, PyObject* args) {
   g_workspaces = Py_NewRef(spaces);
   g_make_workspace = Py_NewRef(make);
   g_raise = Py_NewRef(raise);
-  g_cache_cls = Py_NewRef(cache_cls);
+  PyObject** to[7] = {&g_cache_cls, &g_ring_cls, &g_norm_cls, &g_recurrent_cls, &g_attention_cls, &g_mlp_cls,
+                      &g_residual_cls};
+  for (int i = 0; i < 7; ++i) *to[i] = Py_NewRef(cls[i]);
+  g_hooks = Py_NewRef(hooks);
+  g_pre_hooks = Py_NewRef(pre_hooks);
   g_ready = true;
   Py_RETURN_NONE;
 }
@@ -388,6 +573,8 @@ PyMethodDef methods[] = {
     {"init", init, METH_VARARGS, nullptr},
     FAST(recurrent_path),
     FAST(rglru),
+    FAST(residual_step),
+    FAST(block_step),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr,
                           nullptr};

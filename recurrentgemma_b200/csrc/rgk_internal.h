@@ -127,16 +127,39 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
 // [M,N] tensor to the rounded result and rounds again (not together with gelu).  cap != 0 (no bias,
 // gelu or residual) is the logits soft cap: tanh(acc / cap) * cap with every rounding of the
 // reference.  status: optional device int raised on a bounded-wait timeout.
-// gemm_small_tc.cu: the same projection for M <= 256 rows, weights split over all SMs (the K
-// slices of a feature tile are a thread-block cluster and add up in distributed shared memory).
-// act 0: bias; 1: gelu_tanh of the rounded result; 2: GeGLU over the packed up-projection of the
-// MLP (w as pack_mlp_up_kernel writes it, N = 2 X rows, out [M, X]).  w2 != nullptr: a second
-// projection of the same x (N2 features, own bias and output) in the same launch; N a multiple of
-// 128 then.
+// gemm_rows.cu: up to three projections (matrices) of the same M <= 16 rows in one launch, with
+// RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as above behind; one
+// residual for a single matrix.  early: no kernel in front of this one on the stream that could still be
+// running writes weights (it is one of the library's own, launched by the same call), so they may
+// be fetched before it ends.
+struct RowsMatrix {
+  const void* w;
+  const void* bias;
+  void* out;
+  int n;
+};
+bool rows_gemm_supported(int dtype, int64_t M, int64_t K, int64_t N, bool norm);
+cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, const RowsMatrix* mats,
+                             int n_mats, const void* residual, int64_t M, int K, int act, float cap,
+                             bool early, cudaStream_t s);
+// gemm_small_tc.cu: the same projections (no norm) for up to some hundreds of rows, weights split over
+// all SMs (the K slices of a feature tile are a thread-block cluster and add up in distributed
+// shared memory).  act 0: bias; 1: gelu_tanh of the rounded result; 2: GeGLU over the packed
+// up-projection of the MLP (w as pack_mlp_up_kernel writes it, n = 2 X rows, out [M, X]).  status:
+// optional device int raised on a bounded-wait timeout.  early as for launch_rows_gemm; wide: CTAs
+// that never share an SM with another of the same launch (kernels in a chain alternate).
 bool dense_small_supported(int dtype, int64_t M, int64_t K, int64_t N);
-cudaError_t launch_dense_small(const void* x, const void* w, const void* bias, const void* w2,
-                               const void* bias2, const void* residual, int64_t M, int K, int N,
-                               int N2, int act, void* out, void* out2, int* status, cudaStream_t s);
+cudaError_t launch_dense_small(const void* x, const RowsMatrix* mats, int n_mats, const void* residual,
+                               int64_t M, int K, int act, float cap, int* status, bool early, bool wide,
+                               cudaStream_t s);
+// decode_rows.cu: launch_path_decode_tc for small batches; early as for launch_rows_gemm.
+cudaError_t launch_path_decode_rows(const void* xb, const void* yb, const void* pos, int pos64,
+                                    const void* conv_w, const void* conv_b, const void* a_param,
+                                    const void* bx, const void* ba, const void* packed_w,
+                                    const float* h_in, const void* cache_in, int64_t B, int H,
+                                    void* out, float* h_out, void* cache_out, cudaStream_t s,
+                                    int math, bool early);
+
 bool dense_tc_supported(int dtype, int64_t M, int64_t K, int64_t N);
 cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, const void* residual,
                             int64_t M, int K, int N, int gelu, void* out, int* status,
@@ -182,6 +205,10 @@ bool rmsnorm_supported(int dtype, int64_t D);
 cudaError_t launch_rmsnorm(const void* x, const void* scale, int64_t M, int64_t D, float eps,
                            int dtype, void* out, cudaStream_t s, const void* addend = nullptr,
                            void* sum_out = nullptr);
+// The same for few bfloat16 rows: a block per row, launched as a programmatic dependent; early as for
+// launch_rows_gemm.
+cudaError_t launch_rmsnorm_rows(const void* x, const void* scale, int64_t M, int64_t D, float eps, bool early,
+                                void* out, cudaStream_t s);
 
 // scan.cu
 size_t scan_workspace_bytes(int64_t B, int64_t T, int64_t E, int dtype);

@@ -109,6 +109,66 @@ rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ addend, const T* _
   }
 }
 
+// Few rows (a decode step): one block of four warps per row, because with a warp per row a handful of
+// SMs would each wait through ten dependent-latency rounds (7 us for 64 rows of 2560; 2.5 us this
+// way), and a programmatic dependent launch, so that the projection behind it can set up and fetch
+// weights meanwhile.  bfloat16, no addend.
+constexpr int kRowThreads = 128;
+
+template <int kPacks>
+__global__ void __launch_bounds__(kRowThreads)
+rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ scale, int D,
+                   float eps, int early, __nv_bfloat16* __restrict__ out) {
+  __shared__ float s_sum[kRowThreads / 32];
+  const int packs = D / 8, tid = threadIdx.x;
+  const int64_t row = blockIdx.x;
+  if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (the kernel behind may fetch weights as soon as it starts, see launch_rows_gemm)
+  if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  uint4 v[kPacks], sc[kPacks];
+#pragma unroll
+  for (int i = 0; i < kPacks; ++i) {
+    const int p = tid + i * kRowThreads;
+    v[i] = sc[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (p < packs) {
+      v[i] = *reinterpret_cast<const uint4*>(x + row * D + p * 8);
+      sc[i] = *reinterpret_cast<const uint4*>(scale + p * 8);
+    }
+  }
+  float sum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kPacks; ++i) {
+    const uint32_t w[4] = {bf2mul(v[i].x, v[i].x), bf2mul(v[i].y, v[i].y), bf2mul(v[i].z, v[i].z),
+                           bf2mul(v[i].w, v[i].w)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sum += bf16_lo(w[k]) + bf16_hi(w[k]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((tid & 31) == 0) s_sum[tid >> 5] = sum;
+  __syncthreads();
+  sum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kRowThreads / 32; ++i) sum += s_sum[i];
+  const float var = round_bf16(sum / (float)D);
+  const float r = round_bf16(1.0f / sqrtf(round_bf16(var + eps)));
+  const uint32_t r2 = pack_bf16x2(r, r);
+  constexpr uint32_t kOne = 0x3f803f80u;
+#pragma unroll
+  for (int i = 0; i < kPacks; ++i) {
+    const int p = tid + i * kRowThreads;
+    if (p < packs) {
+      uint4 o;
+      o.x = bf2mul(bf2mul(v[i].x, r2), bf2add(sc[i].x, kOne));
+      o.y = bf2mul(bf2mul(v[i].y, r2), bf2add(sc[i].y, kOne));
+      o.z = bf2mul(bf2mul(v[i].z, r2), bf2add(sc[i].z, kOne));
+      o.w = bf2mul(bf2mul(v[i].w, r2), bf2add(sc[i].w, kOne));
+      *reinterpret_cast<uint4*>(out + row * D + p * 8) = o;
+    }
+  }
+}
+
 template <typename T>
 cudaError_t launch_typed(const void* x, const void* addend, const void* scale, int64_t M, int64_t D,
                          float eps, void* sum_out, void* out, cudaStream_t s) {
@@ -138,6 +198,27 @@ cudaError_t launch_rmsnorm(const void* x, const void* scale, int64_t M, int64_t 
   if (M == 0) return cudaSuccess;
   return dtype ? launch_typed<__nv_bfloat16>(x, addend, scale, M, D, eps, sum_out, out, s)
                : launch_typed<float>(x, addend, scale, M, D, eps, sum_out, out, s);
+}
+
+cudaError_t launch_rmsnorm_rows(const void* x, const void* scale, int64_t M, int64_t D, float eps, bool early,
+                                void* out, cudaStream_t s) {
+  if (M == 0) return cudaSuccess;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)M);
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  using T_ = __nv_bfloat16;
+  const int packs = (int)((D / 8 + kRowThreads - 1) / kRowThreads);
+#define RGK_ROW(P) cudaLaunchKernelEx(&cfg, rmsnorm_row_kernel<P>, (const T_*)x, (const T_*)scale, (int)D, eps, \
+                                      early ? 1 : 0, (T_*)out)
+  cudaError_t e = packs <= 1 ? RGK_ROW(1) : packs <= 3 ? RGK_ROW(3) : packs <= 4 ? RGK_ROW(4) : RGK_ROW(8);
+#undef RGK_ROW
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace rgk

@@ -126,9 +126,53 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
   return d;
 }
 
+// The loop of the warp that issues the MMAs of one accumulator over a TMA ring: for each of n_kb
+// stages wait, issue kSteps instructions of K 16, release the stage.  The whole warp runs it and one
+// elected lane issues: with the loop under `if (lane == 0)` the compiler keeps descriptors and
+// addresses in per-thread registers and a stage of four instructions took 600 cycles whatever its
+// size, more than four instructions of N = 256 execute in.  The barrier of the next stage is asked about
+// before this stage's instructions are issued.  desc_a, desc_b: descriptors of stage 0; `step`:
+// descriptor distance of two stages (bytes / 16).  Returns false if a wait gave up.
+struct RingPos {
+  int stage = 0;
+  uint32_t phase = 0;
+  bool ready = false;                              // the stage was already full when last asked
+};
+template <int kSteps>
+__device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
+                                         uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
+                                         uint32_t bar_empty0, RingPos& at, volatile int* abort_flag);
+
 // Instruction descriptor of tcgen05.mma kind::f16: D float32, A and B bfloat16, both K-major.
 constexpr uint32_t tc_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+template <int kSteps>
+__device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
+                                         uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
+                                         uint32_t bar_empty0, RingPos& at, volatile int* abort_flag) {
+  for (int i = 0; i < n_kb; ++i) {
+    if (!at.ready) {
+      bool ok = mbar_wait(bar_full0 + 8u * at.stage, at.phase, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) return false;
+    }
+    tc_fence_after();
+    const int next = at.stage + 1 == n_stages ? 0 : at.stage + 1;
+    const uint32_t next_phase = next == 0 ? at.phase ^ 1 : at.phase;
+    at.ready = __all_sync(0xffffffffu, mbar_test(bar_full0 + 8u * next, next_phase));
+    const uint64_t da = desc_a + (uint64_t)(at.stage * step), db = desc_b + (uint64_t)(at.stage * step);
+    if (elect_one()) {
+#pragma unroll
+      for (int ks = 0; ks < kSteps; ++ks)
+        tc_mma_bf16(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
+      tc_commit(bar_empty0 + 8u * at.stage);
+    }
+    __syncwarp();
+    at.stage = next;
+    at.phase = next_phase;
+  }
+  return true;
 }
 
 // packed bfloat16x2 arithmetic, each lane rounded to nearest even (what torch does per element)

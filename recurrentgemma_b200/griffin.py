@@ -13,6 +13,7 @@ from typing import Dict, NamedTuple, Optional, Tuple
 import torch
 from torch import nn
 
+from recurrentgemma_b200 import _lib
 from recurrentgemma_b200 import layers
 from recurrentgemma_b200 import modules
 
@@ -102,9 +103,19 @@ class Griffin(nn.Module):
       return None, None
     x = self.embedder.encode(tokens)
     new_cache = {}
+    # decode steps of few sequences take the blocks as a chain of native calls: each may fetch its
+    # first weights while the block in front of it finishes
+    step = None if cache is None else _lib.host().block_step
+    chained = False
     for i, block in enumerate(self.blocks):
       name = f"blocks.{i}"
       block_cache = None if cache is None else cache[name]
+      if step is not None:
+        done = step(block, x, segment_pos, block_cache, return_cache, inplace_cache, chained)
+        chained = done is not NotImplemented
+        if chained:
+          x, new_cache[name] = done
+          continue
       x, new_cache[name] = block(x, segment_pos, block_cache, return_cache, inplace_cache)
     if not return_logits:
       return None, new_cache

@@ -480,6 +480,12 @@ def residual_block(
   r = temporal_block(temporal_pre_norm(x)) + x;  out = mlp_block(channel_pre_norm(r)) + r.
   Returns (out, updated cache of the temporal block or None).  `inplace`: a decode step overwrites
   the tensors of `cache` instead of returning new ones."""
+  if cache is not None:
+    # a decode step of a few sequences is one library call
+    done = _lib.host().residual_step(x, segment_pos, temporal_pre_norm, temporal_block,
+                                     channel_pre_norm, mlp_block, cache, return_cache, inplace)
+    if done is not NotImplemented:
+      return done
   if (isinstance(temporal_block, RecurrentBlock) and temporal_block._fusable(x, cache)
       and temporal_pre_norm.width == temporal_block.width):
     # bfloat16 prefill of the recurrent kind: each half is one library call
