@@ -63,30 +63,6 @@ constexpr int kWideS = 114 * 1024;
 static_assert(2 * (kWideS + 1024) > 233472, "two wide CTAs would fit an SM");
 static_assert(kWideS + kDataHalfS + kTailS + 2 * 1024 <= 233472, "wide and narrow do not fit an SM");
 
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-// Cluster barrier halves; every thread of every CTA of the cluster executes each of them, warps
-// converged.
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t peer_smem(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
 // Shared memory of this CTA -> shared memory of a peer; completion on the peer's mbarrier.
 __device__ __forceinline__ void bulk_to_peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
   asm volatile(

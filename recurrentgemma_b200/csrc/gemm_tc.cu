@@ -2,13 +2,18 @@
 // torch/modules.py:531-548, 627-631, 647) on the 5th-generation tensor cores, bfloat16 in and out,
 // float32 accumulation, optional gelu_tanh epilogue (the y branch, torch/modules.py:628).
 //
-// x [M, K] and W [N, K] are both K-contiguous, i.e. K-major operands as they are: TMA brings
-// 128 x 64 (x) and 256 x 64 (W) boxes with the 128-byte swizzle into a 4-stage ring, a single
-// thread issues tcgen05.mma.cta_group::1.kind::f16 (M 128, N 256, K 16) into one of two TMEM
-// accumulators, and 16 epilogue warps drain the other: tcgen05.ld, + bias in float32, one rounding
-// to bfloat16 (then gelu and a second rounding if asked, as torch does for a separate gelu op),
-// a 32 x 32 transposition through shared memory and 64-byte-contiguous stores.  Persistent CTAs
-// walk the output tiles n-fastest so that the CTAs running together share x rows and all of W in L2.
+// x [M, K] and W [N, K] are both K-contiguous, i.e. K-major operands as they are.  Two CTAs of a
+// cluster share one tile of 256 rows x BN columns (tcgen05.mma.cta_group::2, M 256): each brings its
+// 128 rows of x and its HALF of the tile's columns of W (128 x 64 and BN/2 x 64 boxes, 128-byte
+// swizzle) into a ring of its own and keeps the accumulator of its rows, so an SM reads 32 KB per K
+// block of a 256-wide tile where a CTA by itself reads 48 KB.  At 32768 rows both kinds of tile are
+// bound by what the SMs can fetch from L2 and by the power limit: 2560 x 2560 345 -> 284 us,
+// 7680 -> 2560 924 -> 813 us, 2560 -> 15360 2407 -> 1934 us; at 3002 rows 38.0 -> 30.1 us,
+// 95.7 -> 85.7 us, 228 -> 172 us.  One thread of the even CTA issues into one of two accumulators in
+// the TMEM of both, and 16 epilogue warps per CTA drain the other: tcgen05.ld, + bias in float32, one
+// rounding to bfloat16 (then gelu and a second rounding if asked, as torch does for a separate gelu
+// op), a 32 x 32 transposition through shared memory and 64-byte-contiguous stores.  Persistent pairs
+// walk the output tiles in groups of rows (kGroupRows); BN is chosen per call (tile_columns).
 //
 // Every mbarrier wait is bounded; on expiry WsHeader::status (if given) is raised and the CTA leaves.
 #include <cuda.h>
@@ -20,20 +25,20 @@
 namespace rgk {
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, kStages = 4;
+constexpr int BM = 128, BK = 64;                 // rows of a CTA (a pair: 256), K per stage
+constexpr int kBnMax = 256;                      // columns of a tile at most
 constexpr int kABytes = BM * BK * 2;             // 16 KiB
-constexpr int kBBytes = BN * BK * 2;             // 32 KiB
-constexpr int kStageBytes = kABytes + kBBytes;   // 48 KiB
+constexpr int kRingBytes = 192 * 1024;           // 6 stages of a 256-wide tile, 9 of a 64-wide one
+constexpr int kMaxStages = 9;
 constexpr int kEpi = 16;
 constexpr int kThreadsG = (kEpi + 2) * 32;
 constexpr int kOffRing = 0;
-constexpr int kOffStageOut = kStages * kStageBytes;              // 196608: per-warp 2 KiB staging
-constexpr int kOffBarG = kOffStageOut + kEpi * 2048;             // full[4] empty[4] acc_full[2] acc_empty[2]
-constexpr int kOffTmemG = kOffBarG + (2 * kStages + 4) * 8;
+constexpr int kOffStageOut = kRingBytes;                         // per-warp 2 KiB staging
+constexpr int kOffBarG = kOffStageOut + kEpi * 2048;             // full[] empty[] acc_full[2] acc_empty[2]
+constexpr int kOffTmemG = kOffBarG + (2 * kMaxStages + 4) * 8;
 constexpr int kOffAbortG = kOffTmemG + 4;
 constexpr int kSmemG = kOffAbortG + 4 + 1024;
 static_assert(kSmemG <= 232448, "exceeds the 227 KiB of shared memory a CTA may use");
-constexpr uint32_t kIdescG = tc_idesc_bf16(BM, BN);
 
 // kMode 0: bias only; 1: gelu_tanh of the rounded result; 2: + residual (rounded again);
 // 3: GeGLU - W holds, per group of 8 rows, 4 gate rows then the 4 value rows of the same features
@@ -43,12 +48,21 @@ constexpr uint32_t kIdescG = tc_idesc_bf16(BM, BN);
 //    in the reference (torch/layers.py:700-703, torch/modules.py:749-751);
 // 4: logits soft cap - round(tanh(round(round(acc) / cap)) * cap), the three tensor operations of
 //    torch/griffin.py:183-185 after the contraction of torch/modules.py:1003.
+// Where tile number `tile` lies: groups of `group` rows of tiles, m-fastest within a group and n-fastest
+// across it.
+__device__ __forceinline__ void tile_at(int tile, int m_tiles, int n_tiles, int group, int* m, int* n) {
+  const int g = tile / (group * n_tiles), in = tile - g * group * n_tiles;
+  const int rows = min(group, m_tiles - g * group);
+  *n = in / rows;
+  *m = g * group + in - *n * rows;
+}
+
 template <int kMode>
 __global__ void __launch_bounds__(kThreadsG, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual,
                int64_t M, int N, int K, int m_tiles,
-               int n_tiles, __nv_bfloat16* __restrict__ out, int* status, float cap) {
+               int n_tiles, int group, int bn, __nv_bfloat16* __restrict__ out, int* status, float cap) {
   extern __shared__ uint8_t smem_raw[];
   // aligned by an offset into the shared array, so that the address space stays known to the
   // compiler (shared-memory load/store instructions instead of generic ones)
@@ -56,88 +70,131 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const uint32_t s_base = smem_u32(smem);
   const uint32_t bar0 = s_base + kOffBarG;
   auto bar_full = [&](int s) { return bar0 + 8u * s; };
-  auto bar_empty = [&](int s) { return bar0 + 8u * (kStages + s); };
-  auto bar_acc_full = [&](int s) { return bar0 + 8u * (2 * kStages + s); };
-  auto bar_acc_empty = [&](int s) { return bar0 + 8u * (2 * kStages + 2 + s); };
+  auto bar_empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
+  auto bar_acc_full = [&](int s) { return bar0 + 8u * (2 * kMaxStages + s); };
+  auto bar_acc_empty = [&](int s) { return bar0 + 8u * (2 * kMaxStages + 2 + s); };
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmemG);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbortG);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();            // cluster = (2, 1, 1)
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int k_blocks = (K + BK - 1) / BK;
-  const int total_tiles = m_tiles * n_tiles;
-  const int n_my = (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int n_my = (m_tiles * n_tiles - pair + pairs - 1) / pairs;
+  const uint32_t stage_bytes = kABytes + (uint32_t)bn * (BK * 2 / 2);
+  const int n_stages = min(kMaxStages, kRingBytes / (int)stage_bytes);
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
-    for (int s = 0; s < kStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), kEpi / 2); }
+    for (int s = 0; s < n_stages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), 2 * kEpi); }
     mbar_fence_init();
   }
   if (warp == kEpi + 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                  :: "r"(s_base + kOffTmemG), "r"(512) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_arrive();
+  cluster_wait();                                  // the peer's barriers are set up, its TMEM is there
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  // everything up to here overlaps the kernel in front
+  grid_dependency_wait();
+  grid_launch_dependents();
 
   if (warp == kEpi) {
     // ------------------------------ TMA producer --------------------------------------------------
     if (lane == 0) {
-      unsigned it = 0;
+      const uint32_t full0 = peer_smem(bar_full(0), 0);  // the loads of both CTAs report to the even one
+      int s = 0;
+      uint32_t phase = 1;
       bool ok = true;
       for (int t = 0; t < n_my && ok; ++t) {
-        const int tile = blockIdx.x + t * gridDim.x;
-        const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          ok = mbar_wait(bar_empty(s), ((it / kStages) & 1) ^ 1, s_abort);
+        int m0, n0;
+        tile_at(pair + t * pairs, m_tiles, n_tiles, group, &m0, &n0);
+        m0 = m0 * (2 * BM) + rank * BM;
+        n0 = n0 * bn + rank * (bn / 2);
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          ok = mbar_wait(bar_empty(s), phase, s_abort);
           if (!ok) break;
-          mbar_expect_tx(bar_full(s), kStageBytes);
-          tma_load_2d(s_base + kOffRing + s * kStageBytes, &map_x, kb * BK, m0, bar_full(s));
-          tma_load_2d(s_base + kOffRing + s * kStageBytes + kABytes, &map_w, kb * BK, n0, bar_full(s));
+          if (rank == 0) mbar_expect_tx(bar_full(s), 2 * stage_bytes);
+          const uint32_t st = s_base + kOffRing + s * stage_bytes;
+          tma_load_2d_pair(st, &map_x, kb * BK, m0, full0 + 8u * s);
+          tma_load_2d_pair(st + kABytes, &map_w, kb * BK, n0, full0 + 8u * s);
+          if (++s == n_stages) { s = 0; phase ^= 1; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == kEpi + 1) {
-    // ------------------------------ MMA issue -----------------------------------------------------
-    RingPos at;
-    bool ok = true;
-    for (int t = 0; t < n_my; ++t) {
-      const int as = t & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
-      if (!ok) break;
-      tc_fence_after();
-      ok = mma_ring<BK / 16>(tmem_base + as * BN, smem_desc_sw128(s_base + kOffRing),
-                             smem_desc_sw128(s_base + kOffRing + kABytes), kStageBytes >> 4, kIdescG, k_blocks,
-                             kStages, bar_full(0), bar_empty(0), at, s_abort);
-      if (!ok) break;
-      if (elect_one()) tc_commit(bar_acc_full(as));
-      __syncwarp();
+    // ------------------------------ MMA issue: the even CTA for both -------------------------------
+    if (rank == 0) {
+      RingPos at;
+      bool ok = true;
+      for (int t = 0; t < n_my; ++t) {
+        const int as = t & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+        if (!ok) break;
+        tc_fence_after();
+        ok = mma_ring<BK / 16, 2>(tmem_base + as * kBnMax, smem_desc_sw128(s_base + kOffRing),
+                                  smem_desc_sw128(s_base + kOffRing + kABytes), stage_bytes >> 4,
+                                  tc_idesc_bf16(2 * BM, bn), k_blocks, n_stages, bar_full(0), bar_empty(0),
+                                  at, s_abort);
+        if (!ok) break;
+        if (elect_one()) tc_commit_pair(bar_acc_full(as));
+        __syncwarp();
+      }
     }
   } else {
     // ------------------------------ epilogue ------------------------------------------------------
-    const int as = warp >> 3;                // accumulator = tile parity
+    // all warps on every tile: what a pair does behind its last MMA is as short as it can be
     const int lane_base = (warp & 3) * 32;   // TMEM lanes this warp may read
-    const int col_half = (warp >> 2) & 1;    // which 128 of the tile's 256 columns
+    const int col_group = warp >> 2;         // takes every fourth group of columns
     uint8_t* stage = smem + kOffStageOut + warp * 2048;
     bool ok = true;
-    for (int t = as; t < n_my && ok; t += 2) {
-      const int tile = blockIdx.x + t * gridDim.x;
-      const int64_t m0 = (int64_t)(tile / n_tiles) * BM;
-      const int n0 = (tile % n_tiles) * BN + col_half * 128;
+    for (int t = 0; t < n_my && ok; ++t) {
+      const int as = t & 1;                  // accumulator
+      int mt, n0;
+      tile_at(pair + t * pairs, m_tiles, n_tiles, group, &mt, &n0);
+      const int64_t m0 = (int64_t)mt * (2 * BM) + rank * BM;
+      n0 *= bn;
+      // bias and residual of a chunk of 32 columns, the latter as the pieces this thread will add
+      // after the transposition; the first chunk's are loaded ahead of the wait for the accumulator
+      [[maybe_unused]] uint32_t bv[16];
+      [[maybe_unused]] uint4 rv[4];
+      auto load_chunk = [&](int cc) {
+        const int nc = n0 + cc * 32;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 b4 = make_uint4(0u, 0u, 0u, 0u);
+          if (bias != nullptr && nc + 8 * j < N) b4 = *reinterpret_cast<const uint4*>(bias + nc + 8 * j);
+          bv[4 * j] = b4.x; bv[4 * j + 1] = b4.y; bv[4 * j + 2] = b4.z; bv[4 * j + 3] = b4.w;
+        }
+        if constexpr (kMode == 2) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int64_t grow = m0 + lane_base + (lane >> 2) + 8 * k;
+            const int gcol = nc + (lane & 3) * 8;
+            rv[k] = (grow < M && gcol < N) ? ld_stream(residual + grow * N + gcol)
+                                           : make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+      };
+      if constexpr (kMode != 3) {
+        if (col_group < bn / 32) load_chunk(col_group);
+      }
       ok = mbar_wait(bar_acc_full(as), (t >> 1) & 1, s_abort);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + as * BN +
-                             col_half * 128;
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + as * kBnMax;
       if constexpr (kMode == 3) {
         const int n_out = N / 2;
-        const int oc0 = n0 / 2;                // first output feature of this warp's 128 columns
+        const int oc0 = n0 / 2;                // first output feature of the tile
 #pragma unroll 1
-        for (int cc = 0; cc < 2; ++cc) {       // 32 features at a time
+        for (int cc = col_group; cc < bn / 64; cc += 4) {   // 32 features at a time
           uint4 ov[4];
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {     // 32 columns = 16 features: bounded register use
@@ -182,29 +239,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         }
       } else {
 #pragma unroll 1
-      for (int cc = 0; cc < 4; ++cc) {
+      for (int cc = col_group; cc < bn / 32; cc += 4) {
         uint32_t acc[32];
         tc_ld_32x32(t_row + cc * 32, acc);
         const int nc = n0 + cc * 32;         // first output column of this chunk
-        // the residual pieces this thread will add after the transposition: in flight during the
-        // epilogue arithmetic
-        uint4 rv[4];
-        if constexpr (kMode == 2) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int64_t grow = m0 + lane_base + (lane >> 2) + 8 * k;
-            const int gcol = nc + (lane & 3) * 8;
-            rv[k] = (grow < M && gcol < N) ? ld_stream(residual + grow * N + gcol)
-                                           : make_uint4(0u, 0u, 0u, 0u);
-          }
-        }
-        float bv[32];
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          uint32_t b2 = 0u;
-          if (bias != nullptr && nc + j < N) b2 = *reinterpret_cast<const uint32_t*>(bias + nc + j);
-          bv[j] = bf16_lo(b2); bv[j + 1] = bf16_hi(b2);
-        }
         tc_wait_ld();
         uint4 ov[4];
 #pragma unroll
@@ -213,7 +251,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 #pragma unroll
           for (int p = 0; p < 4; ++p) {
             const int n = j * 8 + p * 2;
-            float v0 = __uint_as_float(acc[n]) + bv[n], v1 = __uint_as_float(acc[n + 1]) + bv[n + 1];
+            const uint32_t b2 = bv[j * 4 + p];
+            float v0 = __uint_as_float(acc[n]) + bf16_lo(b2), v1 = __uint_as_float(acc[n + 1]) + bf16_hi(b2);
             uint32_t pk = pack_bf16x2(v0, v1);
             if constexpr (kMode == 1) pk = pack_bf16x2(gelu_tanh_<true>(bf16_lo(pk)), gelu_tanh_<true>(bf16_hi(pk)));
             if constexpr (kMode == 4) {
@@ -247,21 +286,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             *reinterpret_cast<uint4*>(out + grow * N + gcol) = v;
           }
         }
+        if (cc + 4 < bn / 32) load_chunk(cc + 4);
         __syncwarp();
       }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_acc_empty(as));
+      if (lane == 0) mbar_arrive_cluster(peer_smem(bar_acc_empty(as), 0));
     }
   }
 
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *s_abort && status != nullptr) atomicExch(status, kStatusTimeout);
+  cluster_arrive();
+  cluster_wait();                                  // the peer signals this CTA no more
   if (warp == kEpi + 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
                  : "memory");
   }
 }
@@ -292,6 +334,28 @@ __global__ void pack_mlp_up_kernel(const __nv_bfloat16* __restrict__ w, const __
 
 
 
+// Columns of a tile: the width with the least expected time.  A wave (one tile per pair) takes, per 40
+// K blocks, 8.2, 8.6, 9.3 and 12.5 us at 64, 128, 192 and 256 columns - up to 192 the time to fetch
+// the operands from L2 (16 KB of x whatever the width), from there on the MMAs themselves.  So a tall
+// problem takes 256, and a short one the width that fills the last wave.  The GeGLU epilogue works on
+// 64 columns at a time, the others on 32.
+int tile_columns(int64_t m_tiles, int N, int pairs, int step) {
+  int best = kBnMax;
+  double least = 1e300;
+  for (int bn = kBnMax; bn >= 64; bn -= step) {
+    const int64_t tiles = m_tiles * ((N + bn - 1) / bn);
+    const double wave = bn <= 192 ? 7.7 + bn / 120.0 : 9.3 + (bn - 192) / 20.0;
+    const double t = (double)((tiles + pairs - 1) / pairs) * wave;
+    if (t < least) { least = t; best = bn; }
+  }
+  return best;
+}
+
+// Rows of tiles that a group takes: the pairs running together then read about as many rows of x as
+// of W, where the same number of tiles in one row would read all of W for each of them (2560 -> 15360
+// at 3002 rows 180 -> 162 us, at 8192 445 -> 405 us; 8 to 16 make no difference).
+constexpr int kGroupRows = 12;
+
 }  // namespace
 
 bool dense_tc_supported(int dtype, int64_t M, int64_t K, int64_t N) {
@@ -303,10 +367,6 @@ cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, cons
                             int64_t M, int K, int N, int gelu, void* out, int* status,
                             cudaStream_t s, float cap) {
   if (M == 0) return cudaSuccess;
-  CUtensorMap map_x, map_w;
-  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, BM, BK, true) ||
-      !tensor_map_2d(&map_w, w, (uint64_t)N, (uint64_t)K, BN, BK, true))
-    return cudaErrorInvalidValue;
   static PerDeviceOnce once;
   int num_sms = 0;
   cudaError_t e0 = once.run([] {
@@ -318,20 +378,39 @@ cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, cons
     return cudaFuncSetAttribute(gemm_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG);
   }, &num_sms);
   if (e0 != cudaSuccess) return e0;
-  const int m_tiles = (int)((M + BM - 1) / BM), n_tiles = (N + BN - 1) / BN;
-  const int total = m_tiles * n_tiles;
-  const int grid = total < num_sms ? total : num_sms;
+  const int64_t m_tiles = (M + 2 * BM - 1) / (2 * BM);
+  const int bn = tile_columns(m_tiles, N, num_sms / 2, gelu == 2 ? 64 : 32), n_tiles = (N + bn - 1) / bn;
+  CUtensorMap map_x, map_w;
+  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, BM, BK, true) ||
+      !tensor_map_2d(&map_w, w, (uint64_t)N, (uint64_t)K, (uint32_t)(bn / 2), BK, true))
+    return cudaErrorInvalidValue;
+  if (m_tiles * n_tiles > 0x7fffffff) return cudaErrorInvalidValue;
+  const int total = (int)(m_tiles * n_tiles);
+  const int64_t groups = (m_tiles + kGroupRows - 1) / kGroupRows;
+  const int group = (int)((m_tiles + groups - 1) / groups);
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2u * (unsigned)(total < num_sms / 2 ? total : num_sms / 2));
+  cfg.blockDim = dim3(kThreadsG);
+  cfg.dynamicSmemBytes = kSmemG;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   using T_ = __nv_bfloat16;
   if ((gelu != 0) + (residual != nullptr) > 1) return cudaErrorInvalidValue;
-#define RGK_GEMM(MODE)                                                                          \
-  gemm_tc_kernel<MODE><<<grid, kThreadsG, kSmemG, s>>>(map_x, map_w, (const T_*)bias,           \
-                                                       (const T_*)residual, M, N, K, m_tiles,   \
-                                                       n_tiles, (T_*)out, status, cap)
+#define RGK_GEMM(MODE)                                                                               \
+  e0 = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MODE>, map_x, map_w, (const T_*)bias, (const T_*)residual, \
+                          M, N, K, (int)m_tiles, n_tiles, group, bn, (T_*)out, status, cap)
   if (cap != 0.0f && (gelu != 0 || residual != nullptr || bias != nullptr)) return cudaErrorInvalidValue;
   if (cap != 0.0f) RGK_GEMM(4);
   else if (gelu == 2) RGK_GEMM(3); else if (gelu) RGK_GEMM(1); else if (residual) RGK_GEMM(2); else RGK_GEMM(0);
 #undef RGK_GEMM
-  return cudaGetLastError();
+  return e0 != cudaSuccess ? e0 : cudaGetLastError();
 }
 
 cudaError_t launch_pack_mlp_up(const void* w, const void* b, int D, int X, void* packed_w,

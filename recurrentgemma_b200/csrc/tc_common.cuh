@@ -55,6 +55,20 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, ui
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Pair forms (cta_group::2): the MMA of the two CTAs of a cluster, issued by the even one over the
+// operands at the same offsets of both; its commit arrives at this barrier of both.
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               :: "r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                 uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
 // The same with operand A read from tensor memory: row = lane, a 32-bit column holds two
 // consecutive K elements, so a K step of 16 bfloat16 is 8 columns.
 __device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
@@ -138,7 +152,7 @@ struct RingPos {
   uint32_t phase = 0;
   bool ready = false;                              // the stage was already full when last asked
 };
-template <int kSteps>
+template <int kSteps, int kCtas = 1>
 __device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
                                          uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
                                          uint32_t bar_empty0, RingPos& at, volatile int* abort_flag);
@@ -148,7 +162,7 @@ constexpr uint32_t tc_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-template <int kSteps>
+template <int kSteps, int kCtas>
 __device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
                                          uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
                                          uint32_t bar_empty0, RingPos& at, volatile int* abort_flag) {
@@ -164,15 +178,63 @@ __device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint6
     const uint64_t da = desc_a + (uint64_t)(at.stage * step), db = desc_b + (uint64_t)(at.stage * step);
     if (elect_one()) {
 #pragma unroll
-      for (int ks = 0; ks < kSteps; ++ks)
-        tc_mma_bf16(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
-      tc_commit(bar_empty0 + 8u * at.stage);
+      for (int ks = 0; ks < kSteps; ++ks) {
+        if constexpr (kCtas == 2) tc_mma_bf16_pair(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
+        else tc_mma_bf16(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
+      }
+      if constexpr (kCtas == 2) tc_commit_pair(bar_empty0 + 8u * at.stage);
+      else tc_commit(bar_empty0 + 8u * at.stage);
     }
     __syncwarp();
     at.stage = next;
     at.phase = next_phase;
   }
   return true;
+}
+
+// Programmatic dependent launch: wait until every kernel in front has completed and its writes are
+// visible; let the kernel behind be placed (it does the same wait before it touches memory).
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Cluster barrier halves; every thread of every CTA of the cluster executes each of them, warps
+// converged.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t peer_smem(uint32_t local_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
+  return r;
+}
+// An arrival at a barrier of any CTA of the cluster, and the wait that takes such arrivals.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (unsigned i = 0; i < kWaitLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitHintNs) : "memory");
+    if (ok) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
 }
 
 // packed bfloat16x2 arithmetic, each lane rounded to nearest even (what torch does per element)
