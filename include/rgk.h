@@ -354,7 +354,7 @@ RGK_API int rgk_residual_channel(const void* residual_in, const void* norm_scale
  * rgk_local_attention_prefill: the attention proper without a cache - logits of rotated queries
  *   q [B,T,N,head_dim] and keys k [B,T,head_dim] (one key/value head), the causal / window / same
  *   document mask of torch/modules.py:89-140, float32 softmax of the bfloat16-rounded logits,
- *   probabilities rounded to bfloat16, product with v [B,T,head_dim] -> out [B,T,N*head_dim].
+ *   weights rounded to bfloat16 (before the division by their sum), product with v [B,T,head_dim] -> out [B,T,N*head_dim].
  *   bfloat16 with head_dim 256; RGK_ESHAPE otherwise.
  * workspace: rgk_attention_workspace_bytes(B, T) bytes, 256-byte aligned (first word: status).
  * ---------------------------------------------------------------------------------------------- */
@@ -419,6 +419,18 @@ typedef struct rgk_attention_params {
 RGK_API int rgk_residual_decode_rows(void);
 RGK_API size_t rgk_residual_decode_workspace_bytes(int64_t B, int64_t D, int64_t E, int64_t X, int N,
                                                    int window);
+/* LocalAttentionBlock.forward without a cache (recurrentgemma/torch/modules.py:399-493), for bfloat16
+ * with head_dim 256 and D = N * head_dim: projections, rotary embedding, attention, output projection;
+ * with norm_scale the temporal half of a residual block, x + block(RMSNorm(x)) (torch/modules.py:
+ * 897-902).  keys, values [B,window,head_dim], num_tokens [B] int32: the ring cache of the prompt
+ * (torch/modules.py:238-258), or all NULL.  Workspace as elsewhere, 256-byte aligned. */
+RGK_API size_t rgk_attention_block_workspace_bytes(int64_t B, int64_t T, int64_t D);
+RGK_API int rgk_attention_block_prefill(
+    const void* x, const void* segment_pos, int pos_dtype, const rgk_attention_params* p,
+    const void* norm_scale, float eps, int64_t B, int64_t T, int64_t D, int N, int head_dim, int window,
+    int dtype, void* out, void* keys, void* values, int* num_tokens, void* workspace,
+    size_t workspace_bytes, void* stream);
+
 RGK_API int rgk_recurrent_residual_decode(
     const void* x, const void* segment_pos, int pos_dtype, const rgk_block_params* p,
     const void* norm_scale, float eps, const rgk_channel_params* channel, const float* h_in,

@@ -95,6 +95,10 @@ SIGNATURES = {
     "rgk_attention_workspace_bytes": (_sz, [_i64, _i64]),
     "rgk_local_attention_prefill": (_int, [_vp, _vp, _vp, _vp, _int, _i64, _i64, _int, _int, _int,
                                            _int, _vp, _vp, _sz, _vp]),
+    "rgk_attention_block_workspace_bytes": (_sz, [_i64, _i64, _i64]),
+    "rgk_attention_block_prefill": (_int, [
+        _vp, _vp, _int, ctypes.POINTER(RgkAttentionParams), _vp, ctypes.c_float, _i64, _i64, _i64, _int,
+        _int, _int, _int, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "rgk_attention_decode_workspace_bytes": (_sz, [_i64, _int, _int]),
     "rgk_local_attention_decode": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _int, _int, _int, _int,
                                           _int, _vp, _vp, _sz, _vp]),

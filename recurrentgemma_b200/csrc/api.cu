@@ -484,8 +484,9 @@ int rgk_dense_linear(const void* x, const void* weight, const void* bias, int64_
               "(dtype %d, K=%lld, N=%lld)", dtype, (long long)K, (long long)N);
   if (M == 0) return RGK_OK;
   RGK_CHECK_DEVICE();
-  RGK_CUDA(rgk::launch_dense_tc(x, weight, bias, nullptr, M, (int)K, (int)N, act == RGK_ACT_GELU_TANH, out,
-                                status, static_cast<cudaStream_t>(stream)),
+  const rgk::RowsMatrix mat = {weight, bias, out, (int)N};
+  RGK_CUDA(rgk::launch_dense_tc(x, &mat, 1, nullptr, M, (int)K, act == RGK_ACT_GELU_TANH, status,
+                                static_cast<cudaStream_t>(stream)),
            "dense linear launch");
   return RGK_OK;
 }
@@ -510,6 +511,27 @@ static cudaError_t few_rows_norm_linear(const void* x, const void* scale, float 
   cudaError_t e = rgk::launch_rmsnorm_rows(x, scale, M, K, eps, early, xn, s);
   if (e != cudaSuccess) return e;
   return few_rows_linear(xn, mats, n_mats, nullptr, M, K, act, 0.0f, status, true, true, s);
+}
+
+// Projections of a prompt's rows.  Up to 256 rows the few-row kernels: every SM has weights to stream
+// there, where a pair of CTAs walks all of K for its tile (128 rows: 2560 x 2560 9.3 against 13.1 us,
+// 7680 -> 2560 14.8 against 29.8); longer inner dimensions keep them ahead longer (400 rows: 29.5
+// against 31.3), wide outputs less long (2560 -> 15360 at 199 rows: 21.1 against 20.8).  act 1 needs
+// more rows than that and applies to the first matrix.
+static bool few_rows(int64_t M, int64_t K, int64_t N) {
+  return M <= (N >= 4 * K ? 192 : (K >= 2 * N ? 384 : 256));
+}
+static cudaError_t prompt_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats, const void* residual,
+                                 int64_t M, int K, int act, int* status, cudaStream_t s) {
+  if (few_rows(M, K, mats[0].n) && (act != 1 || n_mats == 1))
+    return few_rows_linear(x, mats, n_mats, residual, M, K, act, 0.0f, status, false, true, s);
+  return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s);
+}
+// RMSNorm of a prompt's rows: a block per row while the warps of the other kernel would not fill the chip.
+static cudaError_t prompt_norm(const void* x, const void* scale, int64_t M, int64_t D, float eps, void* out,
+                               cudaStream_t s) {
+  return M <= 512 ? rgk::launch_rmsnorm_rows(x, scale, M, D, eps, false, out, s)
+                  : rgk::launch_rmsnorm(x, scale, M, D, eps, RGK_BF16, out, s);
 }
 
 int rgk_dense_linear_small(const void* x, const void* weight, const void* bias, const void* residual,
@@ -604,8 +626,9 @@ int rgk_logits(const void* x, const void* table, int64_t M, int64_t D, int64_t V
              "logits launch");
     return RGK_OK;
   }
-  RGK_CUDA(rgk::launch_dense_tc(x, table, nullptr, nullptr, M, (int)D, (int)V, 0, out, status,
-                                static_cast<cudaStream_t>(stream), cap),
+  const rgk::RowsMatrix mat = {table, nullptr, out, (int)V};
+  RGK_CUDA(rgk::launch_dense_tc(x, &mat, 1, nullptr, M, (int)D, 0, status, static_cast<cudaStream_t>(stream),
+                                cap),
            "logits launch");
   return RGK_OK;
 }
@@ -660,25 +683,25 @@ static int block_prefill_impl(const void* x_in, const void* residual, const void
   int* status = static_cast<int*>(workspace);
   const int64_t M = B * T;
   int rc;
-  // y branch with its gelu in the GEMM epilogue, x branch plain
-  RGK_CUDA(rgk::launch_dense_tc(x_in, p->linear_y_w, p->linear_y_b, nullptr, M, (int)D, (int)E, 1, yb,
-                                status, s),
-           "linear_y launch");
-  RGK_CUDA(rgk::launch_dense_tc(x_in, p->linear_x_w, p->linear_x_b, nullptr, M, (int)D, (int)E, 0, xb,
-                                status, s),
-           "linear_x launch");
+  // both input projections in one launch; the y branch's gelu in the GEMM's epilogue, or (few rows) in
+  // the join of the RG-LRU kernel
+  const bool few = few_rows(M, D, E);
+  const rgk::RowsMatrix in[2] = {{p->linear_y_w, p->linear_y_b, yb, (int)E},
+                                 {p->linear_x_w, p->linear_x_b, xb, (int)E}};
+  RGK_CUDA(prompt_linear(x_in, in, 2, nullptr, M, (int)D, few ? 0 : 1, status, s),
+           "linear_y, linear_x launch");
   // Conv1D inside the RG-LRU kernel where that kernel applies (the joined output y * gelu(yb) then
   // goes to the conv-output buffer, which the fused form does not use), else as its own kernel
   // (a warp reads its tile of yb before it writes the same tile of the output); with a separate
   // conv kernel xb has been consumed by then and receives the output
   const bool fused = rgk::rglru_chan_supported(dtype, (int)(E / H), B, T) && conv_fusion_enabled();
   char* joined = fused ? yb : xb;
-  if ((rc = run_rglru(w.c, segment_pos, pos_dtype, &p->path, nullptr, yb, 1, B, T, E, H, dtype,
-                      RGK_GATES_AUTO, w.wpack, w.a, w.xn, w.scan, joined, h_last, s, xb,
+  if ((rc = run_rglru(w.c, segment_pos, pos_dtype, &p->path, nullptr, yb, few ? 0 : 1, B, T, E, H,
+                      dtype, RGK_GATES_AUTO, w.wpack, w.a, w.xn, w.scan, joined, h_last, s, xb,
                       conv_cache_out)))
     return rc;
-  RGK_CUDA(rgk::launch_dense_tc(joined, p->linear_out_w, p->linear_out_b, residual, M, (int)E, (int)D,
-                                0, out, status, s),
+  const rgk::RowsMatrix last = {p->linear_out_w, p->linear_out_b, out, (int)D};
+  RGK_CUDA(prompt_linear(joined, &last, 1, residual, M, (int)E, 0, status, s),
            "linear_out launch");
   return RGK_OK;
 }
@@ -795,7 +818,7 @@ int rgk_residual_block_prefill(const void* x, const void* segment_pos, int pos_d
   RGK_CHECK_DEVICE();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   void* xn = static_cast<char*>(workspace) + block;      // temporal_pre_norm(x)
-  RGK_CUDA(rgk::launch_rmsnorm(x, norm_scale, B * T, D, eps, dtype, xn, s), "rmsnorm launch");
+  RGK_CUDA(prompt_norm(x, norm_scale, B * T, D, eps, xn, s), "rmsnorm launch");
   return block_prefill_impl(xn, x, segment_pos, pos_dtype, p, B, T, D, E, H, dtype, out, h_last,
                             conv_cache_out, workspace, s);
 }
@@ -840,11 +863,10 @@ static int mlp_impl(const void* x_in, const void* packed_up, const void* down_w,
   int* status = static_cast<int*>(workspace);
   char* act = static_cast<char*>(workspace) + 256;
   const char* pw = static_cast<const char*>(packed_up);
-  RGK_CUDA(rgk::launch_dense_tc(x_in, pw, pw + mlp_pack_w_bytes(D, X), nullptr, M, (int)D,
-                                (int)(2 * X), 2, act, status, s),
-           "ffw_up launch");
-  RGK_CUDA(rgk::launch_dense_tc(act, down_w, down_b, residual, M, (int)X, (int)D, 0, out, status, s),
-           "ffw_down launch");
+  const rgk::RowsMatrix up = {pw, pw + mlp_pack_w_bytes(D, X), act, (int)(2 * X)};
+  RGK_CUDA(prompt_linear(x_in, &up, 1, nullptr, M, (int)D, 2, status, s), "ffw_up launch");
+  const rgk::RowsMatrix down = {down_w, down_b, out, (int)D};
+  RGK_CUDA(prompt_linear(act, &down, 1, residual, M, (int)X, 0, status, s), "ffw_down launch");
   return RGK_OK;
 }
 
@@ -897,7 +919,7 @@ int rgk_residual_channel(const void* residual_in, const void* norm_scale, float 
   RGK_CHECK_DEVICE();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   void* xn = static_cast<char*>(workspace) + 256 + up256(static_cast<size_t>(M) * X * 2);
-  RGK_CUDA(rgk::launch_rmsnorm(residual_in, norm_scale, M, D, eps, dtype, xn, s), "rmsnorm launch");
+  RGK_CUDA(prompt_norm(residual_in, norm_scale, M, D, eps, xn, s), "rmsnorm launch");
   return mlp_impl(xn, packed_up, down_w, down_b, residual_in, M, D, X, out, workspace, s);
 }
 
@@ -943,9 +965,69 @@ int rgk_local_attention_prefill(const void* q, const void* k, const void* v, con
               "workspace must be 256-byte aligned");
   RGK_CHECK_DEVICE();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RGK_CUDA(rgk::launch_attention_prefill(q, k, v, segment_pos, pos_dtype == RGK_I64, B, T, N, window,
-                                         out, workspace, s),
+  RGK_CUDA(rgk::launch_attention_prefill(const_cast<void*>(q), const_cast<void*>(k), v, segment_pos,
+                                         pos_dtype == RGK_I64, B, T, N, window, false, nullptr, nullptr,
+                                         nullptr, out, workspace, s),
            "attention launch");
+  return RGK_OK;
+}
+
+// [attention workspace | q, later the encoded heads | k | v | the normalised input]
+size_t rgk_attention_block_workspace_bytes(int64_t B, int64_t T, int64_t D) {
+  if (B < 0 || T < 0 || D < 256) return 0;
+  const size_t m = static_cast<size_t>(B < 1 ? 1 : B) * (T < 1 ? 1 : T);
+  return up256(rgk_attention_workspace_bytes(B, T)) + 2 * up256(m * D * 2) + 2 * up256(m * 512);
+}
+
+int rgk_attention_block_prefill(const void* x, const void* segment_pos, int pos_dtype,
+                                const rgk_attention_params* p, const void* norm_scale, float eps, int64_t B,
+                                int64_t T, int64_t D, int N, int head_dim, int window, int dtype, void* out,
+                                void* keys, void* values, int* num_tokens, void* workspace,
+                                size_t workspace_bytes, void* stream) {
+  RGK_REQUIRE(pos_dtype == RGK_I32 || pos_dtype == RGK_I64, RGK_EINVAL, "unknown index dtype");
+  RGK_REQUIRE(B >= 0 && T >= 0 && N >= 1 && window >= 1, RGK_EINVAL, "bad size");
+  RGK_REQUIRE(x && segment_pos && out && p && p->q_w && p->k_w && p->v_w && p->final_w, RGK_EINVAL,
+              "NULL pointer argument");
+  RGK_REQUIRE((keys == nullptr) == (values == nullptr) && (keys == nullptr) == (num_tokens == nullptr),
+              RGK_EINVAL, "the cache tensors go together");
+  RGK_REQUIRE(aligned16(x) && aligned16(out) && aligned16(norm_scale) && aligned16(keys) && aligned16(values) &&
+                  aligned16(p->q_w) && aligned16(p->k_w) && aligned16(p->v_w) && aligned16(p->final_w) &&
+                  aligned16(p->final_b),
+              RGK_EALIGN, "pointers must be 16-byte aligned");
+  RGK_REQUIRE(rgk::attention_supported(dtype, head_dim, B > 0 ? B : 1, T > 0 ? T : 1, N) &&
+                  D == (int64_t)N * head_dim && window < (1 << 24),
+              RGK_ESHAPE, "the attention block covers bfloat16 with head dimension 256 and as many heads as "
+              "the width holds (dtype %d, head_dim %d, width %lld)", dtype, head_dim, (long long)D);
+  RGK_REQUIRE(norm_scale == nullptr || rgk::rmsnorm_supported(dtype, D), RGK_ESHAPE,
+              "block width %lld is not covered by the RMSNorm kernel", (long long)D);
+  if (B * T == 0) return RGK_OK;
+  const size_t need = rgk_attention_block_workspace_bytes(B, T, D);
+  RGK_REQUIRE(workspace != nullptr && workspace_bytes >= need, RGK_EWORKSPACE,
+              "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+  RGK_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, RGK_EALIGN,
+              "workspace must be 256-byte aligned");
+  RGK_CHECK_DEVICE();
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t M = B * T;
+  int* status = static_cast<int*>(workspace);
+  char* q = static_cast<char*>(workspace) + up256(rgk_attention_workspace_bytes(B, T));
+  char* k = q + up256((size_t)M * D * 2);
+  char* v = k + up256((size_t)M * 512);
+  char* xn = v + up256((size_t)M * 512);
+  const void* in = x;
+  if (norm_scale != nullptr) {
+    RGK_CUDA(prompt_norm(x, norm_scale, M, D, eps, xn, s), "rmsnorm launch");
+    in = xn;
+  }
+  const rgk::RowsMatrix qkv[3] = {{p->q_w, nullptr, q, (int)D}, {p->k_w, nullptr, k, head_dim},
+                                  {p->v_w, nullptr, v, head_dim}};
+  RGK_CUDA(prompt_linear(in, qkv, 3, nullptr, M, (int)D, 0, status, s), "proj_q, proj_k, proj_v launch");
+  RGK_CUDA(rgk::launch_attention_prefill(q, k, v, segment_pos, pos_dtype == RGK_I64, B, T, N, window, true,
+                                         keys, values, num_tokens, q, workspace, s),
+           "attention launch");
+  const rgk::RowsMatrix last = {p->final_w, p->final_b, out, (int)D};
+  RGK_CUDA(prompt_linear(q, &last, 1, norm_scale != nullptr ? x : nullptr, M, (int)D, 0, status, s),
+           "proj_final launch");
   return RGK_OK;
 }
 

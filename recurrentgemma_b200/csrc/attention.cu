@@ -1,30 +1,35 @@
 // Local (sliding-window) multi-query attention of the attention residual blocks, prefill form
 // (recurrentgemma torch/modules.py:399-493 with the helpers at 58-140), bfloat16, head dimension
 // 256, one key/value head:
-//   rope_kernel         rotary embedding of queries and keys (torch/modules.py:58-86);
-//   attn_bounds_kernel  per token the first visible key: max(start of its document, t - window)
-//                       (the mask of torch/modules.py:89-140 is "lo(t) <= s <= t": documents are
-//                       contiguous, so "same segment" is "not before the start of mine");
-//   transpose_v_kernel  values [B,T,256] -> [B,256,Tp], key index contiguous, zero padded: the
-//                       second contraction then has a K-major B operand like the first;
+//   attn_prepare_kernel everything between the projections and the attention in one launch: rotary
+//                       embedding of queries and keys in place (torch/modules.py:58-86), the ring
+//                       cache a prompt leaves behind (torch/modules.py:238-258), per token the first
+//                       visible key max(start of its document, t - window) (the mask of
+//                       torch/modules.py:89-140 is "lo(t) <= s <= t": documents are contiguous, so
+//                       "same segment" is "not before the start of mine"), and the values as
+//                       [B,256,Tp], key index contiguous, zero padded: the second contraction then
+//                       has a K-major B operand like the first;
 //   attn_prefill_kernel the attention itself on tcgen05.
 //
-// The reference rounds the logits to bfloat16, takes the softmax of the masked logits in float32
-// over the WHOLE row and casts the normalised probabilities to bfloat16 before the second
-// contraction.  To round what the reference rounds, the kernel makes two passes over the key tiles
-// of a query tile: pass 1 computes every row's maximum and sum (online), pass 2 recomputes the
-// logits, forms the normalised probabilities, rounds them, and accumulates P V on the tensor cores.
+// The logits are rounded to bfloat16 as the reference rounds them; the softmax runs in float32 in one
+// pass over the key tiles with a running reference m per row: P = 2^(s - m) rounded to bfloat16, O and
+// the row sum l in float32, O / l at the end.  m follows the row's maximum only when a tile exceeds it
+// by more than 2^8 (p and the sums stay far inside their ranges, and relative roundings do not depend
+// on the reference), so that O is hardly ever rescaled.  An earlier version computed Q K^T twice to
+// round the normalised probabilities: half again as many tensor instructions and twice the softmax
+// work, 451 us for 4 x 4096 tokens, 10 heads, window 2048.
 //
 // A unit of work is (sequence, query head, 128 queries); units are dealt out round-robin to
-// persistent CTAs.  Roles in a CTA (18 warps):
+// persistent CTAs, longest first.  Roles in a CTA (20 warps):
 //   warps 0-15 softmax: group g = (warp / 4) % 2 takes the key tiles of parity g (its own S
 //              accumulator); a thread owns a query row (TMEM lane quarter warp % 4) and the 64 keys
-//              of column half warp / 8 of every tile of its group.  In pass 2 it writes the rounded
-//              probabilities back into tensor memory over the logits it has just read (two
-//              bfloat16 per 32-bit column, the layout of an operand A held in tensor memory);
-//   warp 16    TMA producer: the query tile once per unit (four slices of 64 of the head dimension,
-//              resident for both passes) and the key tiles as slices of 64 into a 5-slot ring;
-//   warp 19    TMA producer of the transposed values (two 64-key slices per key tile of pass 2);
+//              of column half warp / 8 of every tile of its group.  The reference of a row passes
+//              from tile to tile through shared memory (bar_m), early in each tile's turn.  The
+//              rounded probabilities go back into tensor memory over the logits (two bfloat16 per
+//              32-bit column, the layout of an operand A held in tensor memory);
+//   warp 16    TMA producer: the query tile once per unit (four slices of 64 of the head dimension)
+//              and the key tiles as slices of 64 into a 5-slot ring;
+//   warp 19    TMA producer of the transposed values (two 64-key slices per key tile);
 //   warp 17    TMEM allocation and issue of S = Q K^T (M 128, N 128, 16 K-steps) into S[parity];
 //   warp 18    issue of O += P V (M 128, N 256, 8 K-steps, A = P from tensor memory) once the
 //              group has written P.  Two issuing warps, so that a P V never queues behind the
@@ -71,37 +76,170 @@ __global__ void rope_kernel(T* __restrict__ x, const void* __restrict__ pos, int
   h[i + quarter] = (T)o1;
 }
 
-// lo[b, t] = max(start of the document of token t, t - window); one warp per sequence.
-__global__ void attn_bounds_kernel(const void* __restrict__ pos, int pos64, int B, int T_, int window,
-                                   int* __restrict__ lo) {
-  const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (b >= B) return;
-  int start = 0;                                // tokens before the first document start: segment 0
-  for (int t0 = 0; t0 < T_; t0 += 32) {
-    const int t = t0 + lane;
-    const bool z = t < T_ && pos_is_zero(pos, pos64, (int64_t)b * T_ + t);
-    const unsigned m = __ballot_sync(0xffffffffu, z);
-    const unsigned upto = m & (lane == 31 ? 0xffffffffu : ((2u << lane) - 1u));
-    const int mine = upto ? t0 + 31 - __clz(upto) : start;
-    if (t < T_) lo[(int64_t)b * T_ + t] = max(mine, t - window);
-    if (m) start = t0 + 31 - __clz(m);
-  }
+// Blocks by role: [0, B) the visible ranges (and token counts) of one sequence each; then blocks of 32
+// tokens: rotary embedding, cache rows, transposed values.  A thread of the latter owns 8 of the 64
+// rotated pairs of a row and walks the heads, so that sine and cosine are computed once per row and
+// position and not once per head (a kernel with a thread per pair and head took 95 us for 16384 rows
+// of 10 heads; the memory it touches, 20).
+constexpr int kPrepRows = 32;
+struct PrepArgs {
+  __nv_bfloat16 *q, *k;
+  const __nv_bfloat16* v;
+  const void* pos;
+  int pos64, B, T, Tp, N, window;
+  int rotate;                            // 0: q and k are rotated already
+  int* lo;
+  __nv_bfloat16* vt;
+  __nv_bfloat16 *cache_k, *cache_v;      // [B, window, 256], or NULL
+  int* num_tokens;
+};
+
+__device__ __forceinline__ int pos_at(const PrepArgs& a, int64_t i) {
+  return a.pos64 ? (int)reinterpret_cast<const long long*>(a.pos)[i] : reinterpret_cast<const int*>(a.pos)[i];
 }
 
-// v [B, T, 256] -> vt [B, 256, Tp]; columns T .. Tp-1 are zero.
-__global__ void transpose_v_kernel(const __nv_bfloat16* __restrict__ v, int T_, int Tp,
-                                   __nv_bfloat16* __restrict__ vt) {
-  __shared__ __nv_bfloat16 tile[32][33];
-  const int b = blockIdx.z, t0 = blockIdx.x * 32, d0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const int t = t0 + r;
-    tile[r][threadIdx.x] = t < T_ ? v[((int64_t)b * T_ + t) * 256 + d0 + threadIdx.x] : __float2bfloat16(0.0f);
+// bfloat16 pairs (a, b) of one register each, rotated with the reference's roundings
+__device__ __forceinline__ void rotate2(uint32_t& a2, uint32_t& b2, uint32_t cs2, uint32_t sn2) {
+  const uint32_t a = a2, b = b2;
+  a2 = bsub2(bmul2(a, cs2), bmul2(b, sn2));
+  b2 = badd2(bmul2(b, cs2), bmul2(a, sn2));
+}
+
+__global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepArgs a) {
+  __shared__ __align__(16) uint4 s_tile[kPrepRows * 33];      // a value row per 33 packs; also the scan's scratch
+  const int tid = threadIdx.x;
+  const int T_ = a.T;
+  if ((int)blockIdx.x < a.B) {
+    // ---- visible ranges: a thread scans a chunk for document starts, then a maximum over the chunks
+    // in front (the first token starts a document whatever its position)
+    int* s_last = reinterpret_cast<int*>(s_tile);
+    const int b = blockIdx.x;
+    const int64_t base = (int64_t)b * T_;
+    const int chunk = (T_ + 255) / 256, t0 = tid * chunk, t1 = min(t0 + chunk, T_);
+    int last = 0;
+    for (int t = t0; t < t1; ++t)
+      if (pos_is_zero(a.pos, a.pos64, base + t)) last = t;
+    int incl = last;
+    const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl = max(incl, o);
+    }
+    if (lane == 31) s_last[warp] = incl;
+    __syncthreads();
+    int start = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) start = 0;
+    for (int w = 0; w < warp; ++w) start = max(start, s_last[w]);
+    for (int t = t0; t < t1; ++t) {
+      if (pos_is_zero(a.pos, a.pos64, base + t)) start = t;
+      a.lo[base + t] = max(start, t - a.window);
+    }
+    if (tid == 0 && a.num_tokens != nullptr) a.num_tokens[b] = pos_at(a, base + T_ - 1) + 1;
+    return;
   }
+  // a sequence's rows, and behind them the ring slots a short prompt leaves empty
+  const int slots = min(a.window, T_);
+  const int rows = a.cache_k != nullptr ? T_ + (a.window - slots) : T_;
+  const int per_seq = (max(rows, a.Tp) + kPrepRows - 1) / kPrepRows;
+  const int blk = (int)blockIdx.x - a.B;
+  const int b = blk / per_seq, t_base = (blk - b * per_seq) * kPrepRows;
+  const int r = tid >> 3, part = tid & 7;
+  const int t = t_base + r;
+  const int64_t row = (int64_t)b * T_ + t;
+  uint4 vv[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) vv[j] = make_uint4(0u, 0u, 0u, 0u);
+  if (t < T_) {
+    uint4* kr = reinterpret_cast<uint4*>(a.k + row * 256);
+    uint4 k0 = kr[part], k1 = kr[part + 8];
+    const uint4* vr = reinterpret_cast<const uint4*>(a.v + row * 256);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) vv[j] = vr[part + 8 * j];
+    if (a.rotate) {
+      const float p = a.pos64 ? (float)reinterpret_cast<const long long*>(a.pos)[row]
+                              : (float)reinterpret_cast<const int*>(a.pos)[row];
+      uint32_t cs[4], sn[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float c[2], s[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float exponent = 2.0f * (float)(part * 8 + j * 2 + e) / 128.0f;
+          const float ang = p * (1.0f / powf(10000.0f, exponent));
+          s[e] = sinf(ang);
+          c[e] = cosf(ang);
+        }
+        cs[j] = pack_bf16x2(c[0], c[1]);
+        sn[j] = pack_bf16x2(s[0], s[1]);
+      }
+      auto rotate = [&](uint4& x, uint4& y) {
+        rotate2(x.x, y.x, cs[0], sn[0]);
+        rotate2(x.y, y.y, cs[1], sn[1]);
+        rotate2(x.z, y.z, cs[2], sn[2]);
+        rotate2(x.w, y.w, cs[3], sn[3]);
+      };
+      uint4* qr = reinterpret_cast<uint4*>(a.q + row * a.N * 256);
+      int h = 0;
+      for (; h + 2 <= a.N; h += 2) {
+        uint4 x0 = qr[h * 32 + part], y0 = qr[h * 32 + 8 + part];
+        uint4 x1 = qr[h * 32 + 32 + part], y1 = qr[h * 32 + 40 + part];
+        rotate(x0, y0);
+        rotate(x1, y1);
+        qr[h * 32 + part] = x0;
+        qr[h * 32 + 8 + part] = y0;
+        qr[h * 32 + 32 + part] = x1;
+        qr[h * 32 + 40 + part] = y1;
+      }
+      if (h < a.N) {
+        uint4 x0 = qr[h * 32 + part], y0 = qr[h * 32 + 8 + part];
+        rotate(x0, y0);
+        qr[h * 32 + part] = x0;
+        qr[h * 32 + 8 + part] = y0;
+      }
+      rotate(k0, k1);
+      kr[part] = k0;
+      kr[part + 8] = k1;
+    }
+    const int u = t - (T_ - slots);              // place among the tokens the ring keeps
+    if (a.cache_k != nullptr && u >= 0) {
+      // the ring's slot: position modulo the window (rolled by the number of tokens)
+      const int seen = pos_at(a, (int64_t)b * T_ + T_ - 1) + 1;
+      int shift = seen % a.window;
+      if (shift < 0) shift += a.window;
+      const int slot = (int)(((int64_t)u + shift) % slots);
+      uint4* ck = reinterpret_cast<uint4*>(a.cache_k + ((int64_t)b * a.window + slot) * 256);
+      uint4* cv = reinterpret_cast<uint4*>(a.cache_v + ((int64_t)b * a.window + slot) * 256);
+      ck[part] = k0;
+      ck[part + 8] = k1;
+      ck[part + 16] = kr[part + 16];
+      ck[part + 24] = kr[part + 24];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cv[part + 8 * j] = vv[j];
+    }
+  } else if (t < rows) {
+    const int64_t at = ((int64_t)b * a.window + slots + (t - T_)) * 256;
+    uint4 *ck = reinterpret_cast<uint4*>(a.cache_k + at), *cv = reinterpret_cast<uint4*>(a.cache_v + at);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      ck[part + 8 * j] = make_uint4(0u, 0u, 0u, 0u);
+      cv[part + 8 * j] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  if (t_base >= a.Tp) return;
+  // transposed values: a thread gathers one of the 256 dimensions over the block's 32 tokens
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s_tile[r * 33 + part + 8 * j] = vv[j];
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const int t = t0 + threadIdx.x;
-    if (t < Tp) vt[((int64_t)b * 256 + d0 + r) * Tp + t] = tile[threadIdx.x][r];
+  const uint16_t* col = reinterpret_cast<const uint16_t*>(s_tile) + tid;
+  __nv_bfloat16* dst = a.vt + ((int64_t)b * 256 + tid) * a.Tp + t_base;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      w[e] = col[(j * 8 + 2 * e) * 264] | ((uint32_t)col[(j * 8 + 2 * e + 1) * 264] << 16);
+    if (t_base + j * 8 < a.Tp) *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -117,11 +255,13 @@ constexpr int kVStage = kHd * kSl * 2;               // a 64-key slice of V^T: 3
 constexpr int kOffQ = 0;                             // the query tile, four slices
 constexpr int kOffK = (kHd / kSl) * kSlice;          //  65536
 constexpr int kOffV = kOffK + kRingK * kSlice;       // 147456
-// The partial (max, sum) of a row, float2 [2 groups x 2 column halves][128 rows], exchanged between
-// the passes.
-constexpr int kOffMl = kOffV + 2 * kVStage;          // 212992
-constexpr int kOffBarA = kOffMl + 4 * kTq * 8;       // 217088
-constexpr int kNumBarA = 2 + 2 * kRingK + 4 + 8 + 2; // q, key ring, v, s_full/s_empty/p_full/pv_done [2], o
+// A row's maximum over the 64 keys of each thread [group][half][row]; its reference after the last tile
+// of each parity [group][row]; its partial sums [unit parity][group, half][row].
+constexpr int kOffMx = kOffV + 2 * kVStage;          // 212992
+constexpr int kOffRef = kOffMx + 4 * kTq * 4;
+constexpr int kOffSum = kOffRef + 2 * kTq * 4;
+constexpr int kOffBarA = kOffSum + 8 * kTq * 4;
+constexpr int kNumBarA = 2 + 2 * kRingK + 4 + 10 + 2; // q, key ring, v, s_full/s_empty/p_full/pv_done/m [2], o
 constexpr int kOffTmemA = kOffBarA + kNumBarA * 8;
 constexpr int kOffAbortA = kOffTmemA + 4;
 constexpr int kSmemA = kOffAbortA + 4 + 1024;
@@ -131,14 +271,8 @@ constexpr int kThreadsA = (kSoftWarps + 4) * 32;
 constexpr uint32_t kIdescS = tc_idesc_bf16(kTq, kTk);
 constexpr uint32_t kIdescO = tc_idesc_bf16(kTq, kHd);
 constexpr float kNegBig = -3.0e38f;
-
-// Two floats rounded to bfloat16 and widened again, through the packed conversion (the scalar one
-// occupies the special-function pipe that the exponentials need).
-__device__ __forceinline__ void round2_bf16(float a, float b, float& ra, float& rb) {
-  const uint32_t pk = pack_bf16x2(a, b);
-  ra = __uint_as_float(pk << 16);
-  rb = __uint_as_float(pk & 0xffff0000u);
-}
+constexpr float kLogitScale = 0.0625f * 1.4426950408889634f;  // hd^-1/2 log2(e): exponent per logit unit
+constexpr float kSlack = 8.0f / kLogitScale;         // logits a row may exceed its reference by: p <= 2^8
 
 __global__ void __launch_bounds__(kThreadsA, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -158,11 +292,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   auto bar_s_empty = [&](int g) { return bar0 + 8u * (2 + 2 * kRingK + 6 + g); };
   auto bar_p_full = [&](int g) { return bar0 + 8u * (2 + 2 * kRingK + 8 + g); };
   auto bar_pv_done = [&](int g) { return bar0 + 8u * (2 + 2 * kRingK + 10 + g); };
-  const uint32_t bar_o_full = bar0 + 8u * (2 + 2 * kRingK + 12);
-  const uint32_t bar_o_empty = bar0 + 8u * (2 + 2 * kRingK + 13);
+  auto bar_m = [&](int g) { return bar0 + 8u * (2 + 2 * kRingK + 12 + g); };
+  const uint32_t bar_o_full = bar0 + 8u * (2 + 2 * kRingK + 14);
+  const uint32_t bar_o_empty = bar0 + 8u * (2 + 2 * kRingK + 15);
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmemA);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbortA);
-  float2* s_ml = reinterpret_cast<float2*>(smem + kOffMl);
+  float* s_mx = reinterpret_cast<float*>(smem + kOffMx);
+  float* s_ref = reinterpret_cast<float*>(smem + kOffRef);
+  float* s_sum = reinterpret_cast<float*>(smem + kOffSum);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q_tiles = (T_ + kTq - 1) / kTq;
@@ -178,9 +315,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_init(bar_s_full(s), 1); mbar_init(bar_s_empty(s), 8);
       mbar_init(bar_p_full(s), 8);
       mbar_init(bar_pv_done(s), 1);
+      mbar_init(bar_m(s), 8);
     }
     mbar_init(bar_o_full, 1);
-    mbar_init(bar_o_empty, 8);
+    mbar_init(bar_o_empty, kSoftWarps);
     mbar_fence_init();
   }
   if (warp == kSoftWarps + 1) {
@@ -196,7 +334,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // unit -> (sequence, head, query tile); the key tiles it needs
   auto unit_of = [&](int i, int& b, int& n, int& t0, int& j_lo, int& j_hi) {
     const int u = blockIdx.x + i * gridDim.x;
-    const int qt = u % q_tiles, bn = u / q_tiles;
+    const int qt = q_tiles - 1 - u / (B * N), bn = u % (B * N);   // longest first
     n = bn % N;
     b = bn / N;
     t0 = qt * kTq;
@@ -224,20 +362,18 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tma_load_3d(s_base + kOffQ + ks * kSlice, &map_q, n * kHd + ks * kSl, t0, b, bar_q_full);
         }
         __syncwarp();
-        for (int pass = 0; pass < 2 && ok; ++pass) {
-          for (int j = j_lo; j <= j_hi && ok; ++j) {
+        for (int j = j_lo; j <= j_hi && ok; ++j) {
 #pragma unroll
-            for (int ks = 0; ks < kHd / kSl; ++ks) {
-              if (ok) ok = mbar_wait(bar_empty(slot), slot_phase, s_abort);
-              if (!ok) break;
-              if (elect_one()) {
-                mbar_expect_tx(bar_full(slot), kSlice);
-                tma_load_3d(s_base + kOffK + slot * kSlice, &map_k, ks * kSl, j * kTk, b,
-                            bar_full(slot));
-              }
-              __syncwarp();
-              if (++slot == kRingK) { slot = 0; slot_phase ^= 1; }
+          for (int ks = 0; ks < kHd / kSl; ++ks) {
+            if (ok) ok = mbar_wait(bar_empty(slot), slot_phase, s_abort);
+            if (!ok) break;
+            if (elect_one()) {
+              mbar_expect_tx(bar_full(slot), kSlice);
+              tma_load_3d(s_base + kOffK + slot * kSlice, &map_k, ks * kSl, j * kTk, b,
+                          bar_full(slot));
             }
+            __syncwarp();
+            if (++slot == kRingK) { slot = 0; slot_phase ^= 1; }
           }
         }
       }
@@ -318,9 +454,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         unit_of(i, b, n, t0, j_lo, j_hi);
         const int nt = j_hi - j_lo + 1;
         ok = mbar_wait(bar_q_full, i & 1, s_abort);
-        // pass 1: logits only
-        for (int j = 0; j < nt && ok; ++j) issue_qk(j & 1);
-        // pass 2: the logits again; the other warp issues P V for tile j once its P is written
+        // the other warp issues P V for tile j once its P is written
         for (int j = 0; j < nt && ok; ++j) {
           issue_qk(j & 1);
           ++pv_issued[j & 1];
@@ -380,9 +514,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int g = (warp >> 2) & 1, quarter = warp & 3, chalf = warp >> 3;
     const int row = quarter * 32 + lane;                     // query row inside the tile = TMEM lane
     const uint32_t t_s = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + g * kTk + chalf * 64;
-    const uint32_t t_o = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 2 * kTk + chalf * 128;
-    constexpr float kScale = 0.0625f * 1.4426950408889634f;  // hd^-1/2 log2(e): exponent per logit unit
-    unsigned cs = 0;
+    const uint32_t t_orow = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 2 * kTk;
+    unsigned mine = 0, theirs = 0;             // tiles of this and of the other group in earlier units
     bool ok = true;
     for (int i = 0; i < n_my; ++i) {
       int b, n, t0, j_lo, j_hi;
@@ -393,88 +526,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       // visible keys of this row: lo .. t (a row past the end sees key 0 only; it is never stored)
       const int lo = row_ok ? lo_all[(int64_t)b * T_ + t] : 0;
       const int hi = row_ok ? t : 0;
-
-      // ---- pass 1: row maximum and sum over this thread's keys ------------------------------------
-      float m = kNegBig, l = 0.0f;
+      float m = kNegBig, l = 0.0f;             // the reference l is relative to, this thread's part of l
       for (int j = g; j < nt; j += 2) {
-        if (ok) ok = mbar_wait(bar_s_full(g), cs & 1, s_abort);
-        ++cs;
-        tc_fence_after();
-        const int s0 = (j_lo + j) * kTk + chalf * 64;
-#pragma unroll 1
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t acc[32];
-          if (ok) {
-            tc_ld_32x32(t_s + cc * 32, acc);
-            tc_wait_ld();
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) acc[c] = 0u;
-          }
-          const int sc = s0 + cc * 32;
-          float v[32];
-          float cm = kNegBig;
-          if (sc > hi || sc + 31 < lo) {                    // nothing visible in these 32 keys
-#pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = kNegBig;
-          } else if (sc >= lo && sc + 31 <= hi) {           // all visible: the common case
-#pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-              round2_bf16(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]), v[c], v[c + 1]);
-              cm = fmaxf(cm, fmaxf(v[c], v[c + 1]));
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-              round2_bf16(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]), v[c], v[c + 1]);
-              if (!(sc + c >= lo && sc + c <= hi)) v[c] = kNegBig;
-              if (!(sc + c + 1 >= lo && sc + c + 1 <= hi)) v[c + 1] = kNegBig;
-              cm = fmaxf(cm, fmaxf(v[c], v[c + 1]));
-            }
-          }
-          if (cm > kNegBig) {
-            const float m_new = fmaxf(m, cm);
-            const float off = -m_new * kScale;
-            float add = 0.0f;
-            // a masked key contributes 2^(-huge) = 0
-#pragma unroll
-            for (int c = 0; c < 32; ++c) add += ex2f(fmaf(v[c], kScale, off));
-            l = l * ex2f(fmaxf((m - m_new) * kScale, -200.0f)) + add;
-            m = m_new;
-          }
-          __syncwarp();
-        }
-        tc_fence_before();
+        const unsigned k = mine + (j >> 1);    // which of this group's tiles
+        if (ok) ok = mbar_wait(bar_s_full(g), k & 1, s_abort);
         __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(bar_s_empty(g));
-      }
-      // the four partial (m, l) of a row -> its final ones
-      s_ml[(g * 2 + chalf) * kTq + row] = make_float2(m, l);
-      named_bar_sync(1, kSoftWarps * 32);
-      {
-        float m_all = kNegBig;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) m_all = fmaxf(m_all, s_ml[k * kTq + row].x);
-        float l_all = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 o = s_ml[k * kTq + row];
-          if (o.x > kNegBig) l_all += o.y * ex2f((o.x - m_all) * kScale);
-        }
-        m = m_all;
-        l = l_all;
-      }
-      named_bar_sync(1, kSoftWarps * 32);      // the exchange area may be rewritten from here on
-      // p = 2^(s k - (m k + log2 l)): the normalisation rides in the exponent
-      const float off2 = -(m * kScale + log2f(fmaxf(l, 1e-30f)));
-
-      // ---- pass 2: normalised probabilities, rounded, into P[g] -----------------------------------
-      for (int j = g; j < nt; j += 2) {
-        if (ok) ok = mbar_wait(bar_s_full(g), cs & 1, s_abort);
-        ++cs;
         tc_fence_after();
         const int s0 = (j_lo + j) * kTk + chalf * 64;
-#pragma unroll 1
+        uint32_t v[32];                        // the 64 logits, rounded, in pairs
+        uint32_t mx2 = 0xff80ff80u;
+#pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           uint32_t acc[32];
           if (ok) {
@@ -485,32 +546,77 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int c = 0; c < 32; ++c) acc[c] = 0u;
           }
           const int sc = s0 + cc * 32;
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            v[cc * 16 + c] = pack_bf16x2(__uint_as_float(acc[2 * c]), __uint_as_float(acc[2 * c + 1]));
+          if (!(sc >= lo && sc + 31 <= hi)) {  // some key is not visible: its logit is -inf
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              const int key = sc + 2 * c;
+              uint32_t& x = v[cc * 16 + c];
+              if (!(key >= lo && key <= hi)) x = (x & 0xffff0000u) | 0xff80u;
+              if (!(key + 1 >= lo && key + 1 <= hi)) x = (x & 0xffffu) | 0xff800000u;
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 16; ++c) mx2 = bmax2(mx2, v[cc * 16 + c]);
+        }
+        // the row's maximum over the tile, and its reference after the tile in front
+        float tmax = fmaxf(bf16_lo(mx2), bf16_hi(mx2));
+        s_mx[(g * 2 + chalf) * kTq + row] = tmax;
+        named_bar_sync(2 + g, 256);
+        tmax = fmaxf(tmax, s_mx[(g * 2 + (chalf ^ 1)) * kTq + row]);
+        float before = kNegBig;
+        if (j > 0) {
+          if (ok) ok = mbar_wait(bar_m(g ^ 1), (theirs + ((j - 1) >> 1)) & 1, s_abort);
+          __syncwarp();
+          before = s_ref[(g ^ 1) * kTq + row];
+        }
+        // (a row without a visible key so far has no reference: -inf is below kNegBig)
+        const float ref = tmax > before + (before > kNegBig ? kSlack : 0.0f) ? tmax : before;
+        if (chalf == 0) s_ref[g * kTq + row] = ref;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_m(g));
+        if (__any_sync(0xffffffffu, ref > before && before > kNegBig)) {
+          // rare: O follows, once the tile in front has been added
+          if (ok) ok = mbar_wait(bar_pv_done(g ^ 1), (theirs + ((j - 1) >> 1)) & 1, s_abort);
+          __syncwarp();
+          tc_fence_after();
+          const float f = before > kNegBig ? ex2f(fmaxf((before - ref) * kLogitScale, -200.0f)) : 1.0f;
+          if (ok) {
+#pragma unroll 1
+            for (int cc = 0; cc < 8; ++cc) {
+              uint32_t acc[16];
+              tc_ld_32x16(t_orow + chalf * 128 + cc * 16, acc);
+              tc_wait_ld();
+#pragma unroll
+              for (int c = 0; c < 16; ++c) acc[c] = __float_as_uint(__uint_as_float(acc[c]) * f);
+              tc_st_32x16(t_orow + chalf * 128 + cc * 16, acc);
+            }
+            tc_wait_st();
+          }
+        }
+        if (ref != m) {
+          l *= ex2f(fmaxf((m - ref) * kLogitScale, -200.0f));
+          m = ref;
+        }
+        const float off = -ref * kLogitScale;
+        float add[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
           uint32_t pk[16];
-          if (sc >= lo && sc + 31 <= hi) {                  // all visible
 #pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-              float s0v, s1v;
-              round2_bf16(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]), s0v, s1v);
-              pk[c >> 1] = pack_bf16x2(ex2f(fmaf(s0v, kScale, off2)), ex2f(fmaf(s1v, kScale, off2)));
-            }
-          } else if (sc > hi || sc + 31 < lo) {             // none visible
-#pragma unroll
-            for (int c = 0; c < 16; ++c) pk[c] = 0u;
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-              float s0v, s1v;
-              round2_bf16(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]), s0v, s1v);
-              const float p0 = (sc + c >= lo && sc + c <= hi) ? ex2f(fmaf(s0v, kScale, off2)) : 0.0f;
-              const float p1 =
-                  (sc + c + 1 >= lo && sc + c + 1 <= hi) ? ex2f(fmaf(s1v, kScale, off2)) : 0.0f;
-              pk[c >> 1] = pack_bf16x2(p0, p1);
-            }
+          for (int c = 0; c < 16; ++c) {
+            const uint32_t x = v[cc * 16 + c];
+            const float p0 = ex2f(fmaf(bf16_lo(x), kLogitScale, off)), p1 = ex2f(fmaf(bf16_hi(x), kLogitScale, off));
+            add[(2 * c) & 3] += p0;
+            add[(2 * c + 1) & 3] += p1;
+            pk[c] = pack_bf16x2(p0, p1);
           }
           // 32 keys = 16 columns, over logits this thread has already read
-          __syncwarp();
           if (ok) tc_st_32x16(t_s + cc * 16, pk);
         }
+        l += (add[0] + add[1]) + (add[2] + add[3]);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -519,38 +625,54 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           mbar_arrive(bar_p_full(g));
         }
       }
+      mine += (unsigned)((nt + 1 - g) >> 1);
+      theirs += (unsigned)((nt + g) >> 1);
 
-      // ---- epilogue (group 0): O -> bfloat16 -> encoded [B, T, N * 256] ---------------------------
-      if (g == 0) {
-        if (ok) ok = mbar_wait(bar_o_full, i & 1, s_abort);
-        tc_fence_after();
-        __nv_bfloat16* orow = out + ((int64_t)b * T_ + t) * ((int64_t)N * kHd) + (int64_t)n * kHd +
-                              chalf * 128;
-#pragma unroll 1
-        for (int cc = 0; cc < 4; ++cc) {
-          uint32_t acc[32];
-          if (ok) {
-            tc_ld_32x32(t_o + cc * 32, acc);
-            tc_wait_ld();
-          } else {
+      // ---- the four partial sums of a row, and O / l -> bfloat16 -> encoded [B, T, N * 256]: a thread
+      // takes 64 columns.  The sums alternate between two places, so one barrier a unit is enough.
+      float* sums = s_sum + (i & 1) * 4 * kTq;
+      float last = m;
+      if (g != ((nt - 1) & 1)) {
+        // the other group took the last tile: its reference is the final one
+        if (ok) ok = mbar_wait(bar_m(g ^ 1), (theirs - 1) & 1, s_abort);
+        __syncwarp();
+        last = s_ref[(g ^ 1) * kTq + row];
+      }
+      sums[(g * 2 + chalf) * kTq + row] = l * ex2f(fmaxf((m - last) * kLogitScale, -200.0f));
+      named_bar_sync(1, kSoftWarps * 32);
+      const float sum = (sums[row] + sums[kTq + row]) + (sums[2 * kTq + row] + sums[3 * kTq + row]);
+      const float inv = 1.0f / sum;
+      if (ok) ok = mbar_wait(bar_o_full, i & 1, s_abort);
+      __syncwarp();
+      tc_fence_after();
+      const int c0 = (g * 2 + chalf) * 64;
+      __nv_bfloat16* orow = out + ((int64_t)b * T_ + t) * ((int64_t)N * kHd) + (int64_t)n * kHd + c0;
 #pragma unroll
-            for (int c = 0; c < 32; ++c) acc[c] = 0u;
-          }
-          if (row_ok) {
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t acc[32];
+        if (ok) {
+          tc_ld_32x32(t_orow + c0 + cc * 32, acc);
+          tc_wait_ld();
+        } else {
 #pragma unroll
-            for (int u4 = 0; u4 < 4; ++u4) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(acc[8 * u4]), __uint_as_float(acc[8 * u4 + 1]));
-              o.y = pack_bf16x2(__uint_as_float(acc[8 * u4 + 2]), __uint_as_float(acc[8 * u4 + 3]));
-              o.z = pack_bf16x2(__uint_as_float(acc[8 * u4 + 4]), __uint_as_float(acc[8 * u4 + 5]));
-              o.w = pack_bf16x2(__uint_as_float(acc[8 * u4 + 6]), __uint_as_float(acc[8 * u4 + 7]));
-              *reinterpret_cast<uint4*>(orow + cc * 32 + u4 * 8) = o;
-            }
+          for (int c = 0; c < 32; ++c) acc[c] = 0u;
+        }
+        if (cc == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0 && ok) mbar_arrive(bar_o_empty);
+        }
+        if (row_ok) {
+#pragma unroll
+          for (int u4 = 0; u4 < 4; ++u4) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              o[e] = pack_bf16x2(__uint_as_float(acc[8 * u4 + 2 * e]) * inv,
+                                 __uint_as_float(acc[8 * u4 + 2 * e + 1]) * inv);
+            *reinterpret_cast<uint4*>(orow + cc * 32 + u4 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(bar_o_empty);
       }
     }
   }
@@ -590,10 +712,12 @@ bool attention_supported(int dtype, int hd, int64_t B, int64_t T, int N) {
          B * N * ((T + kTq - 1) / kTq) < ((int64_t)1 << 31);
 }
 
-// q [B,T,N,256] and k [B,T,256] already rotated, v [B,T,256]; out [B,T,N*256].
-cudaError_t launch_attention_prefill(const void* q, const void* k, const void* v, const void* pos,
-                                     int pos64, int64_t B, int64_t T, int N, int window, void* out,
-                                     void* ws, cudaStream_t s) {
+// q [B,T,N,256] and k [B,T,256], rotated in place first if `rotate`, v [B,T,256]; out [B,T,N*256] may be q (a unit reads
+// the queries it will overwrite before it writes).  cache_k, cache_v, num_tokens: the ring cache of
+// the prompt, or NULL.
+cudaError_t launch_attention_prefill(void* q, void* k, const void* v, const void* pos, int pos64, int64_t B,
+                                     int64_t T, int N, int window, bool rotate, void* cache_k,
+                                     void* cache_v, int* num_tokens, void* out, void* ws, cudaStream_t s) {
   using T_ = __nv_bfloat16;
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const int64_t Tp = (T + 7) / 8 * 8;
@@ -601,12 +725,30 @@ cudaError_t launch_attention_prefill(const void* q, const void* k, const void* v
   int* status = reinterpret_cast<int*>(base);
   int* lo = reinterpret_cast<int*>(base + 256);
   T_* vt = reinterpret_cast<T_*>(base + 256 + up((size_t)B * T * sizeof(int)));
-  attn_bounds_kernel<<<(unsigned)((B + 3) / 4), 128, 0, s>>>(pos, pos64, (int)B, (int)T, window, lo);
+  PrepArgs a = {};
+  a.q = static_cast<T_*>(q);
+  a.k = static_cast<T_*>(k);
+  a.v = static_cast<const T_*>(v);
+  a.pos = pos;
+  a.pos64 = pos64;
+  a.B = (int)B;
+  a.T = (int)T;
+  a.Tp = (int)Tp;
+  a.N = N;
+  a.window = window;
+  a.rotate = rotate ? 1 : 0;
+  a.lo = lo;
+  a.vt = vt;
+  a.cache_k = static_cast<T_*>(cache_k);
+  a.cache_v = static_cast<T_*>(cache_v);
+  a.num_tokens = num_tokens;
+  int64_t rows = Tp;
+  if (cache_k != nullptr && T < window) rows = rows > window ? rows : window;
+  const int64_t blocks = B + B * ((rows + kPrepRows - 1) / kPrepRows);
+  if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+  attn_prepare_kernel<<<(unsigned)blocks, 256, 0, s>>>(a);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  transpose_v_kernel<<<dim3((unsigned)((Tp + 31) / 32), kHd / 32, (unsigned)B), dim3(32, 8), 0, s>>>(
-      (const T_*)v, (int)T, (int)Tp, vt);
-  if ((err = cudaGetLastError()) != cudaSuccess) return err;
   CUtensorMap map_q, map_k, map_vt;
   if (!tensor_map_bte(&map_q, q, (uint64_t)B, (uint64_t)T, (uint64_t)N * kHd, kTq, kSl, true) ||
       !tensor_map_bte(&map_k, k, (uint64_t)B, (uint64_t)T, kHd, kTk, kSl, true) ||

@@ -40,7 +40,7 @@ constexpr int kOffAbortG = kOffTmemG + 4;
 constexpr int kSmemG = kOffAbortG + 4 + 1024;
 static_assert(kSmemG <= 232448, "exceeds the 227 KiB of shared memory a CTA may use");
 
-// kMode 0: bias only; 1: gelu_tanh of the rounded result; 2: + residual (rounded again);
+// kMode 0: bias only; 1: gelu_tanh of the rounded result of the first matrix; 2: + residual (rounded again);
 // 3: GeGLU - W holds, per group of 8 rows, 4 gate rows then the 4 value rows of the same features
 //    (see pack_mlp_up_kernel: groups this small leave every kernel free to cut tiles at multiples of
 //    8 rows); out [M, N/2] = gelu_tanh(gate) * value, where gate and
@@ -57,12 +57,24 @@ __device__ __forceinline__ void tile_at(int tile, int m_tiles, int n_tiles, int 
   *m = g * group + in - *n * rows;
 }
 
+struct DenseMat {
+  const __nv_bfloat16* bias;
+  __nv_bfloat16* out;
+  int n, tile0;                        // columns, number of the first tile
+};
+struct DenseArgs {
+  DenseMat mat[3];                     // absent ones start behind the last tile
+  const __nv_bfloat16* residual;
+  int64_t M;
+  int k_blocks, m_tiles, n_tiles, group, bn;
+  float cap;
+};
+
 template <int kMode>
 __global__ void __launch_bounds__(kThreadsG, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-               const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual,
-               int64_t M, int N, int K, int m_tiles,
-               int n_tiles, int group, int bn, __nv_bfloat16* __restrict__ out, int* status, float cap) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
+               const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2,
+               const __grid_constant__ DenseArgs a, int* status) {
   extern __shared__ uint8_t smem_raw[];
   // aligned by an offset into the shared array, so that the address space stays known to the
   // compiler (shared-memory load/store instructions instead of generic ones)
@@ -79,7 +91,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();            // cluster = (2, 1, 1)
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int k_blocks = (K + BK - 1) / BK;
+  const int k_blocks = a.k_blocks, m_tiles = a.m_tiles, n_tiles = a.n_tiles, group = a.group, bn = a.bn;
+  const int64_t M = a.M;
   const int n_my = (m_tiles * n_tiles - pair + pairs - 1) / pairs;
   const uint32_t stage_bytes = kABytes + (uint32_t)bn * (BK * 2 / 2);
   const int n_stages = min(kMaxStages, kRingBytes / (int)stage_bytes);
@@ -115,15 +128,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       for (int t = 0; t < n_my && ok; ++t) {
         int m0, n0;
         tile_at(pair + t * pairs, m_tiles, n_tiles, group, &m0, &n0);
+        const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
+        const CUtensorMap* map_w = mi == 0 ? &map_w0 : (mi == 1 ? &map_w1 : &map_w2);
         m0 = m0 * (2 * BM) + rank * BM;
-        n0 = n0 * bn + rank * (bn / 2);
+        n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn + rank * (bn / 2);
         for (int kb = 0; kb < k_blocks; ++kb) {
           ok = mbar_wait(bar_empty(s), phase, s_abort);
           if (!ok) break;
           if (rank == 0) mbar_expect_tx(bar_full(s), 2 * stage_bytes);
           const uint32_t st = s_base + kOffRing + s * stage_bytes;
           tma_load_2d_pair(st, &map_x, kb * BK, m0, full0 + 8u * s);
-          tma_load_2d_pair(st + kABytes, &map_w, kb * BK, n0, full0 + 8u * s);
+          tma_load_2d_pair(st + kABytes, map_w, kb * BK, n0, full0 + 8u * s);
           if (++s == n_stages) { s = 0; phase ^= 1; }
         }
       }
@@ -160,7 +175,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       int mt, n0;
       tile_at(pair + t * pairs, m_tiles, n_tiles, group, &mt, &n0);
       const int64_t m0 = (int64_t)mt * (2 * BM) + rank * BM;
-      n0 *= bn;
+      // (copies, so that nothing indexes the parameters dynamically)
+      const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
+      const __nv_bfloat16* bias = mi == 0 ? a.mat[0].bias : (mi == 1 ? a.mat[1].bias : a.mat[2].bias);
+      __nv_bfloat16* out = mi == 0 ? a.mat[0].out : (mi == 1 ? a.mat[1].out : a.mat[2].out);
+      const int N = mi == 0 ? a.mat[0].n : (mi == 1 ? a.mat[1].n : a.mat[2].n);
+      n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn;
       // bias and residual of a chunk of 32 columns, the latter as the pieces this thread will add
       // after the transposition; the first chunk's are loaded ahead of the wait for the accumulator
       [[maybe_unused]] uint32_t bv[16];
@@ -178,7 +198,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           for (int k = 0; k < 4; ++k) {
             const int64_t grow = m0 + lane_base + (lane >> 2) + 8 * k;
             const int gcol = nc + (lane & 3) * 8;
-            rv[k] = (grow < M && gcol < N) ? ld_stream(residual + grow * N + gcol)
+            rv[k] = (grow < M && gcol < N) ? ld_stream(a.residual + grow * N + gcol)
                                            : make_uint4(0u, 0u, 0u, 0u);
           }
         }
@@ -254,8 +274,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             const uint32_t b2 = bv[j * 4 + p];
             float v0 = __uint_as_float(acc[n]) + bf16_lo(b2), v1 = __uint_as_float(acc[n + 1]) + bf16_hi(b2);
             uint32_t pk = pack_bf16x2(v0, v1);
-            if constexpr (kMode == 1) pk = pack_bf16x2(gelu_tanh_<true>(bf16_lo(pk)), gelu_tanh_<true>(bf16_hi(pk)));
+            if (kMode == 1 && mi == 0) pk = pack_bf16x2(gelu_tanh_<true>(bf16_lo(pk)), gelu_tanh_<true>(bf16_hi(pk)));
             if constexpr (kMode == 4) {
+              const float cap = a.cap;
               uint32_t t = pack_bf16x2(__fdiv_rn(bf16_lo(pk), cap), __fdiv_rn(bf16_hi(pk), cap));
               t = pack_bf16x2(tanhf(bf16_lo(t)), tanhf(bf16_hi(t)));
               pk = pack_bf16x2(bf16_lo(t) * cap, bf16_hi(t) * cap);
@@ -339,11 +360,13 @@ __global__ void pack_mlp_up_kernel(const __nv_bfloat16* __restrict__ w, const __
 // the operands from L2 (16 KB of x whatever the width), from there on the MMAs themselves.  So a tall
 // problem takes 256, and a short one the width that fills the last wave.  The GeGLU epilogue works on
 // 64 columns at a time, the others on 32.
-int tile_columns(int64_t m_tiles, int N, int pairs, int step) {
+int tile_columns(int64_t m_tiles, const RowsMatrix* mats, int n_mats, int pairs, int step) {
   int best = kBnMax;
   double least = 1e300;
   for (int bn = kBnMax; bn >= 64; bn -= step) {
-    const int64_t tiles = m_tiles * ((N + bn - 1) / bn);
+    int64_t tiles = 0;
+    for (int i = 0; i < n_mats; ++i) tiles += (mats[i].n + bn - 1) / bn;
+    tiles *= m_tiles;
     const double wave = bn <= 192 ? 7.7 + bn / 120.0 : 9.3 + (bn - 192) / 20.0;
     const double t = (double)((tiles + pairs - 1) / pairs) * wave;
     if (t < least) { least = t; best = bn; }
@@ -363,37 +386,61 @@ bool dense_tc_supported(int dtype, int64_t M, int64_t K, int64_t N) {
          N % 8 == 0 && K < (1 << 24) && N < (1 << 24);
 }
 
-cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, const void* residual,
-                            int64_t M, int K, int N, int gelu, void* out, int* status,
-                            cudaStream_t s, float cap) {
+cudaError_t launch_dense_tc(const void* x, const RowsMatrix* mats, int n_mats, const void* residual, int64_t M,
+                            int K, int act, int* status, cudaStream_t s, float cap) {
   if (M == 0) return cudaSuccess;
+  if (n_mats < 1 || n_mats > 3 || (n_mats > 1 && (act == 2 || residual != nullptr || cap != 0.0f)))
+    return cudaErrorInvalidValue;
+  if ((act != 0) + (residual != nullptr) > 1) return cudaErrorInvalidValue;
+  if (cap != 0.0f && (act != 0 || residual != nullptr || mats[0].bias != nullptr)) return cudaErrorInvalidValue;
   static PerDeviceOnce once;
   int num_sms = 0;
-  cudaError_t e0 = once.run([] {
-    cudaError_t e;
-    if ((e = cudaFuncSetAttribute(gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(gemm_tc_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(gemm_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG);
+  cudaError_t e = once.run([] {
+    cudaError_t r = cudaSuccess;
+    auto set = [&](auto* kernel) {
+      if (r == cudaSuccess)
+        r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG);
+    };
+    set(gemm_tc_kernel<0>);
+    set(gemm_tc_kernel<1>);
+    set(gemm_tc_kernel<2>);
+    set(gemm_tc_kernel<3>);
+    set(gemm_tc_kernel<4>);
+    return r;
   }, &num_sms);
-  if (e0 != cudaSuccess) return e0;
+  if (e != cudaSuccess) return e;
   const int64_t m_tiles = (M + 2 * BM - 1) / (2 * BM);
-  const int bn = tile_columns(m_tiles, N, num_sms / 2, gelu == 2 ? 64 : 32), n_tiles = (N + bn - 1) / bn;
-  CUtensorMap map_x, map_w;
-  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, BM, BK, true) ||
-      !tensor_map_2d(&map_w, w, (uint64_t)N, (uint64_t)K, (uint32_t)(bn / 2), BK, true))
-    return cudaErrorInvalidValue;
+  DenseArgs a = {};
+  a.bn = tile_columns(m_tiles, mats, n_mats, num_sms / 2, act == 2 ? 64 : 32);
+  int64_t n_tiles = 0;
+  CUtensorMap map_x, map_w[3];
+  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, BM, BK, true)) return cudaErrorInvalidValue;
+  for (int i = 0; i < n_mats; ++i) {
+    a.mat[i] = {static_cast<const __nv_bfloat16*>(mats[i].bias), static_cast<__nv_bfloat16*>(mats[i].out),
+                mats[i].n, (int)n_tiles};
+    n_tiles += (mats[i].n + a.bn - 1) / a.bn;
+    if (!tensor_map_2d(&map_w[i], mats[i].w, (uint64_t)mats[i].n, (uint64_t)K, (uint32_t)(a.bn / 2), BK, true))
+      return cudaErrorInvalidValue;
+  }
+  for (int i = n_mats; i < 3; ++i) {
+    a.mat[i].tile0 = 0x7fffffff;
+    map_w[i] = map_w[0];
+  }
   if (m_tiles * n_tiles > 0x7fffffff) return cudaErrorInvalidValue;
-  const int total = (int)(m_tiles * n_tiles);
-  const int64_t groups = (m_tiles + kGroupRows - 1) / kGroupRows;
-  const int group = (int)((m_tiles + groups - 1) / groups);
+  const int64_t total = m_tiles * n_tiles, groups = (m_tiles + kGroupRows - 1) / kGroupRows;
+  a.residual = static_cast<const __nv_bfloat16*>(residual);
+  a.M = M;
+  a.k_blocks = (K + BK - 1) / BK;
+  a.m_tiles = (int)m_tiles;
+  a.n_tiles = (int)n_tiles;
+  a.group = (int)((m_tiles + groups - 1) / groups);
+  a.cap = cap;
   cudaLaunchAttribute attr[2];
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2u * (unsigned)(total < num_sms / 2 ? total : num_sms / 2));
   cfg.blockDim = dim3(kThreadsG);
@@ -401,16 +448,12 @@ cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, cons
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  using T_ = __nv_bfloat16;
-  if ((gelu != 0) + (residual != nullptr) > 1) return cudaErrorInvalidValue;
-#define RGK_GEMM(MODE)                                                                               \
-  e0 = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MODE>, map_x, map_w, (const T_*)bias, (const T_*)residual, \
-                          M, N, K, (int)m_tiles, n_tiles, group, bn, (T_*)out, status, cap)
-  if (cap != 0.0f && (gelu != 0 || residual != nullptr || bias != nullptr)) return cudaErrorInvalidValue;
-  if (cap != 0.0f) RGK_GEMM(4);
-  else if (gelu == 2) RGK_GEMM(3); else if (gelu) RGK_GEMM(1); else if (residual) RGK_GEMM(2); else RGK_GEMM(0);
+#define RGK_GEMM(MODE) \
+  cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MODE>, map_x, map_w[0], map_w[1], map_w[2], a, status)
+  e = cap != 0.0f ? RGK_GEMM(4) : act == 2 ? RGK_GEMM(3) : act == 1 ? RGK_GEMM(1)
+                  : residual != nullptr ? RGK_GEMM(2) : RGK_GEMM(0);
 #undef RGK_GEMM
-  return e0 != cudaSuccess ? e0 : cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_pack_mlp_up(const void* w, const void* b, int D, int X, void* packed_w,

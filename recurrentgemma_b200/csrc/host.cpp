@@ -31,6 +31,14 @@ struct Lib {
   decltype(&rgk_residual_decode_workspace_bytes) residual_decode_workspace_bytes;
   decltype(&rgk_recurrent_residual_decode) recurrent_residual_decode;
   decltype(&rgk_attention_residual_decode) attention_residual_decode;
+  decltype(&rgk_block_workspace_bytes) block_workspace_bytes;
+  decltype(&rgk_residual_workspace_bytes) residual_workspace_bytes;
+  decltype(&rgk_recurrent_block_prefill) recurrent_block_prefill;
+  decltype(&rgk_residual_block_prefill) residual_block_prefill;
+  decltype(&rgk_attention_block_workspace_bytes) attention_block_workspace_bytes;
+  decltype(&rgk_attention_block_prefill) attention_block_prefill;
+  decltype(&rgk_mlp_workspace_bytes) mlp_workspace_bytes;
+  decltype(&rgk_residual_channel) residual_channel;
 } g_lib;
 bool g_ready = false;
 
@@ -49,7 +57,7 @@ PyObject *g_hooks, *g_pre_hooks;         // torch's hooks for every module
   X(_packed_up) X(_forward_hooks) X(_forward_pre_hooks) X(weight) X(bias) X(scale) X(eps) X(conv_1d) \
   X(rg_lru) X(linear_x) X(linear_y) X(linear_out) X(ffw_up) X(ffw_down) X(proj_q) X(proj_k) X(proj_v) \
   X(proj_final) X(window_size) X(expanded_width) X(lru_width) X(recurrent_block) \
-  X(attention_block) X(temporal_pre_norm) X(channel_pre_norm) X(mlp_block)
+  X(attention_block) X(conv1d_temporal_width) X(temporal_pre_norm) X(channel_pre_norm) X(mlp_block)
 #define DECL(n) PyObject* s_##n = nullptr;
 NAMES(DECL)
 #undef DECL
@@ -384,6 +392,29 @@ bool shaped(const at::Tensor* t, at::ScalarType dtype, c10::Device dev, at::IntA
   return t != nullptr && t->scalar_type() == dtype && t->device() == dev && t->sizes() == sizes;
 }
 
+// The parameters of a RecurrentBlock of RG-LRU width E.
+Found recurrent_params(PyObject* block, Params& pr, long E, rgk_block_params* p, long* heads, long* impl,
+                       bool* made) {
+  PyObject *ly = submodule(block, s_linear_y), *lx = submodule(block, s_linear_x),
+           *lo = submodule(block, s_linear_out);
+  p->linear_y_w = pr.ptr(ly, s_weight); p->linear_y_b = pr.ptr(ly, s_bias);
+  p->linear_x_w = pr.ptr(lx, s_weight); p->linear_x_b = pr.ptr(lx, s_bias);
+  p->linear_out_w = pr.ptr(lo, s_weight); p->linear_out_b = pr.ptr(lo, s_bias);
+  PyObject *conv = submodule(block, s_conv_1d), *lru = submodule(block, s_rg_lru);
+  if (!pr.ok || conv == nullptr || lru == nullptr) return Found::no;
+  return path_params(conv, lru, pr, RGK_BF16, E, &p->path, heads, impl, made);
+}
+// The parameters of a LocalAttentionBlock; pr.ok says whether they are all there.
+rgk_attention_params attention_params(PyObject* block, Params& pr) {
+  rgk_attention_params p = {};
+  p.q_w = pr.ptr(submodule(block, s_proj_q), s_weight);
+  p.k_w = pr.ptr(submodule(block, s_proj_k), s_weight);
+  p.v_w = pr.ptr(submodule(block, s_proj_v), s_weight);
+  p.final_w = pr.ptr(submodule(block, s_proj_final), s_weight);
+  p.final_b = pr.ptr(submodule(block, s_proj_final), s_bias);
+  return p;
+}
+
 PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* block, PyObject* norm2,
                PyObject* mlp, PyObject* cache, bool want, bool inplace, bool chained) {
   const at::Tensor *x = dense(x_arg), *pos = dense(pos_arg);
@@ -427,15 +458,8 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
     if (!int_attr(block, s_lru_width, &E) || !int_attr(block, s_width, &width) || width != D ||
         !shaped(h_in, at::kFloat, dev, {B, E}) || !shaped(c_in, at::kBFloat16, dev, {B, 3, E}))
       return not_here();
-    PyObject *ly = submodule(block, s_linear_y), *lx = submodule(block, s_linear_x),
-             *lo = submodule(block, s_linear_out);
     rgk_block_params p = {};
-    p.linear_y_w = pr.ptr(ly, s_weight); p.linear_y_b = pr.ptr(ly, s_bias);
-    p.linear_x_w = pr.ptr(lx, s_weight); p.linear_x_b = pr.ptr(lx, s_bias);
-    p.linear_out_w = pr.ptr(lo, s_weight); p.linear_out_b = pr.ptr(lo, s_bias);
-    PyObject *conv = submodule(block, s_conv_1d), *lru = submodule(block, s_rg_lru);
-    if (!pr.ok || conv == nullptr || lru == nullptr) return not_here();
-    switch (path_params(conv, lru, pr, RGK_BF16, E, &p.path, &heads, &impl, &made)) {
+    switch (recurrent_params(block, pr, E, &p, &heads, &impl, &made)) {
       case Found::no: return not_here();
       case Found::error: return nullptr;
       case Found::yes: break;
@@ -470,12 +494,7 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
       !shaped(keys, at::kBFloat16, dev, {B, window, 1, 256}) ||
       !shaped(values, at::kBFloat16, dev, {B, window, 1, 256}) || !shaped(seen, at::kInt, dev, {B}))
     return not_here();
-  rgk_attention_params p = {};
-  p.q_w = pr.ptr(submodule(block, s_proj_q), s_weight);
-  p.k_w = pr.ptr(submodule(block, s_proj_k), s_weight);
-  p.v_w = pr.ptr(submodule(block, s_proj_v), s_weight);
-  p.final_w = pr.ptr(submodule(block, s_proj_final), s_weight);
-  p.final_b = pr.ptr(submodule(block, s_proj_final), s_bias);
+  const rgk_attention_params p = attention_params(block, pr);
   if (!pr.ok) return not_here();
   if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
   if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, D, X, (int)heads, (int)window), &ws))
@@ -500,6 +519,164 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
   Ref ring(PyObject_CallFunctionObjArgs(g_ring_cls, rk.p, rv.p, rs.p, nullptr));
   if (ring.p == nullptr) return nullptr;
   return PyTuple_Pack(2, o.p, ring.p);
+}
+
+// ---- prefill of a temporal block, alone or inside its residual block -------------------------------
+
+// The linear maps of a block that a caller may have replaced or hooked.
+bool plain_children(PyObject* block) {
+  Ref d(PyObject_GetAttr(block, s__modules));
+  if (d.p == nullptr || !PyDict_Check(d.p)) return false;
+  PyObject *key, *child;
+  Py_ssize_t at = 0;
+  while (PyDict_Next(d.p, &at, &key, &child))
+    if (child == Py_None || !no_hooks(child)) return false;
+  return true;
+}
+
+// x, segment_pos -> [norm ->] temporal block [-> + x], with the cache of the prompt.  Yes: *out and, if
+// wanted, *cache are set.
+Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* norm, PyObject* block, bool want,
+                       at::Tensor* out, PyObject** cache) {
+  const bool recurrent = exactly(block, g_recurrent_cls);
+  if (!(recurrent || exactly(block, g_attention_cls)) || PyDict_Size(g_hooks) != 0 ||
+      PyDict_Size(g_pre_hooks) != 0 || !plain_children(block))
+    return Found::no;
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
+  const c10::Device dev = x.device();
+  Params pr{at::kBFloat16, dev};
+  const void* scale = nullptr;
+  float eps = 0.0f;
+  long w1 = 0, width = 0;
+  if (norm != nullptr) {
+    if (!exactly(norm, g_norm_cls) || !no_hooks(norm) || !no_hooks(block)) return Found::no;
+    scale = pr.ptr(norm, s_scale);
+    if (!pr.ok || !int_attr(norm, s_width, &w1) || w1 != D || !float_attr(norm, s_eps, &eps)) return Found::no;
+  }
+  if (!int_attr(block, s_width, &width) || width != D || D % 8 != 0) return Found::no;
+  const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int pc = pos_code(pos);
+  Workspace ws;
+  if (recurrent) {
+    long E = 0, heads = 0, impl = 0, tw = 0;
+    rgk_block_params p = {};
+    if (!int_attr(block, s_lru_width, &E) || !int_attr(block, s_conv1d_temporal_width, &tw) || tw != 4)
+      return Found::no;
+    const Found f = recurrent_params(block, pr, E, &p, &heads, &impl, nullptr);
+    if (f != Found::yes) return f;
+    if (E != heads * 256 || impl == RGK_GATES_SIMT) return Found::no;
+    if (!workspace(x, s, norm != nullptr ? g_lib.residual_workspace_bytes(B, T, D, E, RGK_BF16)
+                                         : g_lib.block_workspace_bytes(B, T, D, E, RGK_BF16), &ws))
+      return Found::error;
+    *out = empty(x.sizes(), at::kBFloat16, dev);
+    at::Tensor h, c;
+    if (want) {
+      h = empty({B, E}, at::kFloat, dev);
+      c = empty({B, 3, E}, at::kBFloat16, dev);
+    }
+    float* hp = want ? static_cast<float*>(h.mutable_data_ptr()) : nullptr;
+    void* cp = want ? c.mutable_data_ptr() : nullptr;
+    const int rc = norm != nullptr
+        ? g_lib.residual_block_prefill(x.const_data_ptr(), pos.const_data_ptr(), pc, &p, scale, eps, B, T, D, E,
+                                       (int)heads, 4, RGK_BF16, out->mutable_data_ptr(), hp, cp, ws.ptr,
+                                       ws.bytes, s)
+        : g_lib.recurrent_block_prefill(x.const_data_ptr(), pos.const_data_ptr(), pc, &p, B, T, D, E,
+                                        (int)heads, 4, RGK_BF16, out->mutable_data_ptr(), hp, cp, ws.ptr,
+                                        ws.bytes, s);
+    if (!succeeded(rc)) return Found::error;
+    if (want) *cache = make_cache(wrap(std::move(h)), wrap(std::move(c)));
+  } else {
+    long heads = 0, window = 0;
+    const rgk_attention_params p = attention_params(block, pr);
+    if (!pr.ok || !int_attr(block, s_num_heads, &heads) || !int_attr(block, s_window_size, &window) ||
+        heads * 256 != D || window < 1)
+      return Found::no;
+    if (!workspace(x, s, g_lib.attention_block_workspace_bytes(B, T, D), &ws)) return Found::error;
+    *out = empty(x.sizes(), at::kBFloat16, dev);
+    at::Tensor k, v, seen;
+    if (want) {
+      k = empty({B, window, 1, 256}, at::kBFloat16, dev);
+      v = empty({B, window, 1, 256}, at::kBFloat16, dev);
+      seen = empty({B}, at::kInt, dev);
+    }
+    if (!succeeded(g_lib.attention_block_prefill(
+            x.const_data_ptr(), pos.const_data_ptr(), pc, &p, scale, eps, B, T, D, (int)heads, 256, (int)window,
+            RGK_BF16, out->mutable_data_ptr(), want ? k.mutable_data_ptr() : nullptr,
+            want ? v.mutable_data_ptr() : nullptr,
+            want ? static_cast<int*>(seen.mutable_data_ptr()) : nullptr, ws.ptr, ws.bytes, s)))
+      return Found::error;
+    if (want) {
+      Ref rk(wrap(std::move(k))), rv(wrap(std::move(v))), rs(wrap(std::move(seen)));
+      if (rk.p == nullptr || rv.p == nullptr || rs.p == nullptr) return Found::error;
+      *cache = PyObject_CallFunctionObjArgs(g_ring_cls, rk.p, rv.p, rs.p, nullptr);
+    }
+  }
+  return want && *cache == nullptr ? Found::error : Found::yes;
+}
+
+// The arguments of a prefill call: dense bfloat16 [B, T, D] and positions [B, T] on the same device.
+bool prompt_args(const at::Tensor* x, const at::Tensor* pos) {
+  return x != nullptr && pos != nullptr && x->scalar_type() == at::kBFloat16 && x->dim() == 3 &&
+         pos->dim() == 2 && pos_code(*pos) >= 0 && pos->device() == x->device() &&
+         pos->size(0) == x->size(0) && pos->size(1) == x->size(1) && x->numel() > 0;
+}
+
+// prefill(temporal block, x, segment_pos, return_cache): its forward without a cache
+PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (!g_ready || n != 4) return not_here();
+  const at::Tensor *x = dense(args[1]), *pos = dense(args[2]);
+  if (!prompt_args(x, pos)) return not_here();
+  Guard guard(x->device().index());
+  at::Tensor out;
+  PyObject* cache = nullptr;
+  switch (temporal_prefill(*x, *pos, nullptr, args[0], PyObject_IsTrue(args[3]) == 1, &out, &cache)) {
+    case Found::no: return not_here();
+    case Found::error: return nullptr;
+    case Found::yes: break;
+  }
+  Ref o(wrap(std::move(out))), c(cache != nullptr ? cache : Py_NewRef(Py_None));
+  return o.p == nullptr ? nullptr : PyTuple_Pack(2, o.p, c.p);
+}
+
+// residual_prefill(x, segment_pos, norm, temporal block, norm, mlp, return_cache)
+PyObject* residual_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (!g_ready || n != 7) return not_here();
+  const at::Tensor *x = dense(args[0]), *pos = dense(args[1]);
+  PyObject *norm2 = args[4], *mlp = args[5];
+  if (!prompt_args(x, pos) || !exactly(norm2, g_norm_cls) || !exactly(mlp, g_mlp_cls) || !no_hooks(norm2) ||
+      !no_hooks(mlp) || !plain_children(mlp))
+    return not_here();
+  const int64_t M = x->size(0) * x->size(1), D = x->size(2);
+  const c10::Device dev = x->device();
+  Guard guard(dev.index());
+  Params pr{at::kBFloat16, dev};
+  long X = 0, w1 = 0, w2 = 0;
+  float eps = 0.0f;
+  PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
+  const at::Tensor *up_w = pr.get(up, s_w), *up_b = pr.get(up, s_b);
+  const void *scale = pr.ptr(norm2, s_scale), *down_w = pr.ptr(down, s_weight), *down_b = pr.ptr(down, s_bias);
+  if (!pr.ok || !int_attr(mlp, s_expanded_width, &X) || !int_attr(mlp, s_width, &w1) ||
+      !int_attr(norm2, s_width, &w2) || w1 != D || w2 != D || X % 64 != 0 || !float_attr(norm2, s_eps, &eps))
+    return not_here();
+  const void* packed_up = nullptr;
+  if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &packed_up)) return nullptr;
+  at::Tensor r;
+  PyObject* cache = nullptr;
+  switch (temporal_prefill(*x, *pos, args[2], args[3], PyObject_IsTrue(args[6]) == 1, &r, &cache)) {
+    case Found::no: return not_here();
+    case Found::error: return nullptr;
+    case Found::yes: break;
+  }
+  Ref c(cache != nullptr ? cache : Py_NewRef(Py_None));
+  const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  Workspace ws;
+  if (!workspace(*x, s, g_lib.mlp_workspace_bytes(M, D, X, RGK_BF16), &ws)) return nullptr;
+  at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
+  if (!succeeded(g_lib.residual_channel(r.const_data_ptr(), scale, eps, packed_up, down_w, down_b, M, D, X,
+                                        RGK_BF16, out.mutable_data_ptr(), ws.ptr, ws.bytes, s)))
+    return nullptr;
+  Ref o(wrap(std::move(out)));
+  return o.p == nullptr ? nullptr : PyTuple_Pack(2, o.p, c.p);
 }
 
 // residual_step(x, segment_pos, norm, temporal block, norm, mlp, cache, return_cache, inplace)
@@ -552,6 +729,14 @@ PyObject* init(PyObject*, PyObject* args) {
   find(&g_lib.residual_decode_workspace_bytes, "rgk_residual_decode_workspace_bytes");
   find(&g_lib.recurrent_residual_decode, "rgk_recurrent_residual_decode");
   find(&g_lib.attention_residual_decode, "rgk_attention_residual_decode");
+  find(&g_lib.block_workspace_bytes, "rgk_block_workspace_bytes");
+  find(&g_lib.residual_workspace_bytes, "rgk_residual_workspace_bytes");
+  find(&g_lib.recurrent_block_prefill, "rgk_recurrent_block_prefill");
+  find(&g_lib.residual_block_prefill, "rgk_residual_block_prefill");
+  find(&g_lib.attention_block_workspace_bytes, "rgk_attention_block_workspace_bytes");
+  find(&g_lib.attention_block_prefill, "rgk_attention_block_prefill");
+  find(&g_lib.mlp_workspace_bytes, "rgk_mlp_workspace_bytes");
+  find(&g_lib.residual_channel, "rgk_residual_channel");
   if (PyErr_Occurred()) return nullptr;
 #define INTERN(n) if (s_##n == nullptr) s_##n = PyUnicode_InternFromString(#n);
   NAMES(INTERN)
@@ -575,6 +760,8 @@ PyMethodDef methods[] = {
     FAST(rglru),
     FAST(residual_step),
     FAST(block_step),
+    FAST(prefill),
+    FAST(residual_prefill),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr,
                           nullptr};

@@ -121,12 +121,6 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
                               void* out, float* h_last, void* ws, int math, cudaStream_t s,
                               const void* conv_w = nullptr, const void* conv_b = nullptr);
 
-// gemm_tc.cu: out [M,N] = x [M,K] W[N,K]^T + bias (bfloat16, float32 accumulation) on tcgen05;
-// gelu == 1 applies gelu_tanh to the rounded result; gelu == 2 is the GeGLU epilogue of the MLP
-// block (W and bias packed by launch_pack_mlp_up, N = 2 X, out [M, X]); residual != null adds a
-// [M,N] tensor to the rounded result and rounds again (not together with gelu).  cap != 0 (no bias,
-// gelu or residual) is the logits soft cap: tanh(acc / cap) * cap with every rounding of the
-// reference.  status: optional device int raised on a bounded-wait timeout.
 // gemm_rows.cu: up to three projections (matrices) of the same M <= 16 rows in one launch, with
 // RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as above behind; one
 // residual for a single matrix.  early: no kernel in front of this one on the stream that could still be
@@ -160,10 +154,17 @@ cudaError_t launch_path_decode_rows(const void* xb, const void* yb, const void* 
                                     void* out, float* h_out, void* cache_out, cudaStream_t s,
                                     int math, bool early);
 
+// gemm_tc.cu: out [M,N] = x [M,K] W[N,K]^T + bias (bfloat16, float32 accumulation) on tcgen05;
+// act == 1 applies gelu_tanh to the rounded result; act == 2 is the GeGLU epilogue of the MLP
+// block (W and bias packed by launch_pack_mlp_up, N = 2 X, out [M, X]); residual != null adds a
+// [M,N] tensor to the rounded result and rounds again (not together with gelu).  cap != 0 (no bias,
+// gelu or residual) is the logits soft cap: tanh(acc / cap) * cap with every rounding of the
+// reference.  status: optional device int raised on a bounded-wait timeout.
+// Any number of rows, up to three matrices of the same K in one launch; act 1 applies to the first
+// matrix, act 2, cap and a residual take a single one.
 bool dense_tc_supported(int dtype, int64_t M, int64_t K, int64_t N);
-cudaError_t launch_dense_tc(const void* x, const void* w, const void* bias, const void* residual,
-                            int64_t M, int K, int N, int gelu, void* out, int* status,
-                            cudaStream_t s, float cap = 0.0f);
+cudaError_t launch_dense_tc(const void* x, const RowsMatrix* mats, int n_mats, const void* residual, int64_t M,
+                            int K, int act, int* status, cudaStream_t s, float cap = 0.0f);
 
 // attention_decode.cu: one new token per sequence against the ring cache keys / values [B,W,256]
 // (num_tokens [B] int32 tokens seen so far): q [B,N,256] and k_new [B,256] rotated, v_new [B,256]
@@ -190,14 +191,16 @@ cudaError_t launch_pack_mlp_up(const void* w, const void* b, int D, int X, void*
 
 // attention.cu: rotary embedding in place (x [rows, heads, hd], the first half of each head), and
 // the local multi-query attention of the attention blocks in prefill form: q [B,T,N,256] and
-// k [B,T,256] rotated, v [B,T,256], bfloat16 -> out [B,T,N*256].  ws: attention_workspace_bytes.
+// k [B,T,256] (rotated in place first if `rotate`), v [B,T,256], bfloat16 -> out [B,T,N*256], which may
+// be q.  cache_k, cache_v [B,window,256] and num_tokens [B]: the ring cache a prompt leaves behind, or
+// NULL.  ws: attention_workspace_bytes.
 cudaError_t launch_rope(void* x, const void* pos, int pos64, int64_t rows, int heads, int hd,
                         int dtype, cudaStream_t s);
 bool attention_supported(int dtype, int hd, int64_t B, int64_t T, int N);
 size_t attention_workspace_bytes(int64_t B, int64_t T);
-cudaError_t launch_attention_prefill(const void* q, const void* k, const void* v, const void* pos,
-                                     int pos64, int64_t B, int64_t T, int N, int window, void* out,
-                                     void* ws, cudaStream_t s);
+cudaError_t launch_attention_prefill(void* q, void* k, const void* v, const void* pos, int pos64, int64_t B,
+                                     int64_t T, int N, int window, bool rotate, void* cache_k,
+                                     void* cache_v, int* num_tokens, void* out, void* ws, cudaStream_t s);
 
 // rmsnorm.cu: out [M,D] = x * rsqrt(mean(x^2) + eps) * (scale + 1) with the reference's roundings
 // (torch/layers.py:65-73); one warp per row held in registers.

@@ -102,6 +102,7 @@ class Griffin(nn.Module):
     if not return_logits and not return_cache:
       return None, None
     x = self.embedder.encode(tokens)
+    segment_pos = segment_pos.contiguous()       # once for all blocks
     new_cache = {}
     # decode steps of few sequences take the blocks as a chain of native calls: each may fetch its
     # first weights while the block in front of it finishes

@@ -252,6 +252,10 @@ class RecurrentBlock(nn.Module):
     """Returns (block output [B,T,width], updated cache or None).  `inplace`: see
     `recurrent_path`."""
     dev = _lib.require_cuda(x, segment_pos, self.linear_x.weight)
+    if cache is None:
+      done = _lib.host().prefill(self, x, segment_pos, return_cache)
+      if done is not NotImplemented:
+        return done
     if self._fusable(x, cache):
       return self._forward_fused(x, segment_pos, return_cache, dev)
     yb, xb = linear_pair(x, self.linear_y, self.linear_x)
@@ -484,8 +488,12 @@ def residual_block(
     # a decode step of a few sequences is one library call
     done = _lib.host().residual_step(x, segment_pos, temporal_pre_norm, temporal_block,
                                      channel_pre_norm, mlp_block, cache, return_cache, inplace)
-    if done is not NotImplemented:
-      return done
+  else:
+    # bfloat16 prefill: two library calls
+    done = _lib.host().residual_prefill(x, segment_pos, temporal_pre_norm, temporal_block,
+                                        channel_pre_norm, mlp_block, return_cache)
+  if done is not NotImplemented:
+    return done
   if (isinstance(temporal_block, RecurrentBlock) and temporal_block._fusable(x, cache)
       and temporal_pre_norm.width == temporal_block.width):
     # bfloat16 prefill of the recurrent kind: each half is one library call
@@ -588,6 +596,10 @@ class LocalAttentionBlock(nn.Module):
     writes the new key and value into their ring slot of `cache` and bumps its `num_tokens`
     (an extension for decode loops that run as a CUDA graph) instead of cloning the ring."""
     dev = _lib.require_cuda(x, segment_pos, self.proj_q.weight)
+    if cache is None:
+      done = _lib.host().prefill(self, x, segment_pos, return_cache)   # bfloat16, head dimension 256
+      if done is not NotImplemented:
+        return done
     layers._same_dtype(x, self.proj_q.weight, self.proj_k.weight, self.proj_v.weight,
                        self.proj_final.weight, self.proj_final.bias)
     b, t, _ = x.shape
