@@ -439,8 +439,8 @@ RGK_API int rgk_recurrent_residual_decode(
     size_t workspace_bytes, void* stream);
 RGK_API int rgk_attention_residual_decode(
     const void* x, const void* segment_pos, int pos_dtype, const rgk_attention_params* p,
-    const void* norm_scale, float eps, const rgk_channel_params* channel, void* keys, void* values,
-    int* num_tokens, int64_t B, int64_t D, int64_t X, int N, int head_dim, int window, int dtype,
+    const void* norm_scale, float eps, const rgk_channel_params* channel, const void* keys_in,
+    const void* values_in, const int* num_tokens_in, void* keys, void* values, int* num_tokens, int64_t B, int64_t D, int64_t X, int N, int head_dim, int window, int dtype,
     int update, void* out, int chained, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------

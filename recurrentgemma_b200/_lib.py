@@ -113,8 +113,8 @@ SIGNATURES = {
         _vp, _vp, _vp, _int, _vp, _sz, _vp]),
     "rgk_attention_residual_decode": (_int, [
         _vp, _vp, _int, ctypes.POINTER(RgkAttentionParams), _vp, ctypes.c_float,
-        ctypes.POINTER(RgkChannelParams), _vp, _vp, _vp, _i64, _i64, _i64, _int, _int, _int, _int,
-        _int, _vp, _int, _vp, _sz, _vp]),
+        ctypes.POINTER(RgkChannelParams), _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _int,
+        _int, _int, _int, _vp, _int, _vp, _sz, _vp]),
     "rgk_embed": (_int, [_vp, _int, _vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp]),
     "rgk_logits": (_int, [_vp, _vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp, _vp]),
     "rgk_argmax": (_int, [_vp, _i64, _i64, _int, _vp, _vp]),

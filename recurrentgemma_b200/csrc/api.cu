@@ -1058,9 +1058,13 @@ int rgk_local_attention_decode(const void* q, const void* k_new, const void* v_n
   RGK_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, RGK_EALIGN,
               "workspace must be 256-byte aligned");
   RGK_CHECK_DEVICE();
-  RGK_CUDA(rgk::launch_attention_decode(q, k_new, v_new, keys, values, num_tokens, B, N, window,
-                                        dtype, update, out, workspace,
-                                        static_cast<cudaStream_t>(stream)),
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  RGK_CUDA(dtype == RGK_BF16
+               ? rgk::launch_attention_decode_ring(q, k_new, v_new, nullptr, 0, keys, values, num_tokens, keys,
+                                                   values, num_tokens, B, N, window, update, out,
+                                                   static_cast<int*>(workspace), s)
+               : rgk::launch_attention_decode(q, k_new, v_new, keys, values, num_tokens, B, N, window, update,
+                                              out, workspace, s),
            "decode attention launch");
   return RGK_OK;
 }
@@ -1142,12 +1146,11 @@ int rgk_recurrent_path_decode(const void* xb, const void* yb, const void* segmen
 
 int rgk_residual_decode_rows(void) { return 256; }
 
-// [header | four tensors [B, E] | two [B, D] | the hidden activations [B, X] | ring attention]
+// [header | four tensors [B, E] | two [B, D] | the hidden activations [B, X]]
 size_t rgk_residual_decode_workspace_bytes(int64_t B, int64_t D, int64_t E, int64_t X, int N, int window) {
   if (B < 0 || D < 1 || E < 1 || X < 1 || N < 0 || window < 0) return 0;
   if (B < 1) B = 1;
-  const size_t ring = N > 0 && window > 0 ? rgk::attention_decode_workspace_bytes(B, N, window) : 0;
-  return 256 + 4 * up256((size_t)B * E * 2) + 2 * up256((size_t)B * D * 2) + up256((size_t)B * X * 2) + ring;
+  return 256 + 4 * up256((size_t)B * E * 2) + 2 * up256((size_t)B * D * 2) + up256((size_t)B * X * 2);
 }
 
 static int check_residual_decode(const void* x, const void* segment_pos, int pos_dtype,
@@ -1229,7 +1232,8 @@ int rgk_recurrent_residual_decode(const void* x, const void* segment_pos, int po
 
 int rgk_attention_residual_decode(const void* x, const void* segment_pos, int pos_dtype,
                                   const rgk_attention_params* p, const void* norm_scale, float eps,
-                                  const rgk_channel_params* channel, void* keys, void* values,
+                                  const rgk_channel_params* channel, const void* keys_in,
+                                  const void* values_in, const int* num_tokens_in, void* keys, void* values,
                                   int* num_tokens, int64_t B, int64_t D, int64_t X, int N, int head_dim,
                                   int window, int dtype, int update, void* out, int chained,
                                   void* workspace, size_t workspace_bytes, void* stream) {
@@ -1237,8 +1241,11 @@ int rgk_attention_residual_decode(const void* x, const void* segment_pos, int po
   int rc = check_residual_decode(x, segment_pos, pos_dtype, norm_scale, channel, B, D, D, X, N, window,
                                  dtype, out, workspace, workspace_bytes);
   if (rc) return rc;
-  RGK_REQUIRE(p && p->q_w && p->k_w && p->v_w && p->final_w && keys && values && num_tokens, RGK_EINVAL,
-              "NULL pointer argument");
+  RGK_REQUIRE(p && p->q_w && p->k_w && p->v_w && p->final_w && keys_in && values_in && num_tokens_in &&
+                  keys && values && num_tokens, RGK_EINVAL, "NULL pointer argument");
+  RGK_REQUIRE(aligned16(keys_in) && aligned16(values_in), RGK_EALIGN, "pointers must be 16-byte aligned");
+  RGK_REQUIRE((keys_in == keys) == (values_in == values) && (keys_in == keys) == (num_tokens_in == num_tokens),
+              RGK_EINVAL, "the cache tensors are updated in place together or not at all");
   RGK_REQUIRE(aligned16(p->q_w) && aligned16(p->k_w) && aligned16(p->v_w) && aligned16(p->final_w) &&
                   aligned16(p->final_b) && aligned16(keys) && aligned16(values),
               RGK_EALIGN, "pointers must be 16-byte aligned");
@@ -1253,15 +1260,13 @@ int rgk_attention_residual_decode(const void* x, const void* segment_pos, int po
   char *k = q + wide, *v = k + up256((size_t)B * head_dim * 2), *enc = q + 3 * wide, *r = enc + wide;
   char *xn = r + wide, *hidden = xn + wide;
   int* status = static_cast<int*>(workspace);
-  char* ring = hidden + up256((size_t)B * X * 2);
   const rgk::RowsMatrix in[3] = {{p->q_w, nullptr, q, (int)D}, {p->k_w, nullptr, k, head_dim},
                                  {p->v_w, nullptr, v, head_dim}};
   RGK_CUDA(few_rows_norm_linear(x, norm_scale, eps, xn, in, 3, B, (int)D, 0, status, chained != 0, s),
            "proj_q, proj_k, proj_v launch");
-  RGK_CUDA(rgk::launch_rope(q, segment_pos, pos_dtype == RGK_I64, B, N, head_dim, dtype, s), "rope launch");
-  RGK_CUDA(rgk::launch_rope(k, segment_pos, pos_dtype == RGK_I64, B, 1, head_dim, dtype, s), "rope launch");
-  RGK_CUDA(rgk::launch_attention_decode(q, k, v, keys, values, num_tokens, B, N, window, dtype, update,
-                                        enc, ring, s),
+  RGK_CUDA(rgk::launch_attention_decode_ring(q, k, v, segment_pos, pos_dtype == RGK_I64, keys_in, values_in,
+                                             num_tokens_in, keys, values, num_tokens, B, N, window, update,
+                                             enc, status, s),
            "decode attention launch");
   const rgk::RowsMatrix last = {p->final_w, p->final_b, r, (int)D};
   RGK_CUDA(few_rows_linear(enc, &last, 1, x, B, (int)D, 0, 0.0f, status, true, false, s),

@@ -253,20 +253,21 @@ cudaError_t launch_path_decode_rows(const void* xb, const void* yb, const void* 
   // 32 channels per CTA while all CTAs then run at once (two per SM, in clusters of eight), 64 from
   // there on: half the conv work in all, and twice the rest per CTA
   const int cg = B <= 48 ? 1 : 2, ctas = kHeadR / (32 * cg);
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;      // the channel groups of a head
   attr[1].val.clusterDim.x = (unsigned)ctas;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
+  attr[2] = smem_carveout(2 * 30 * 1024);                // two CTAs
   cudaLaunchConfig_t cfg = {};
   const unsigned row_tiles = (unsigned)((B + kRowsR - 1) / kRowsR);
   cfg.gridDim = dim3((unsigned)(H * ctas), row_tiles);
   cfg.blockDim = dim3(kThreadsR);
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = 3;
   cudaError_t e;
 #define RGK_DEC(MUL, MATH)                                                        \
   (cg == 1 ? cudaLaunchKernelEx(&cfg, decode_rows_kernel<MUL, MATH, 1>, a)        \

@@ -347,17 +347,19 @@ cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, c
   const bool staged = (int64_t)M * a.pitch <= (norm_scale != nullptr ? kXBudget : 48 * 1024);
   if (norm_scale != nullptr && !staged) return cudaErrorInvalidValue;
 
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  const int slots = num_sms * (staged && (int64_t)M * a.pitch > kXThree ? 2 : kCtasPerSm);
+  const int per_sm = staged && (int64_t)M * a.pitch > kXThree ? 2 : kCtasPerSm;
+  const int slots = num_sms * per_sm;
+  attr[1] = smem_carveout(per_sm * ((staged ? (size_t)M * a.pitch : 0) + 6 * 1024));
   cfg.gridDim = dim3((unsigned)(a.units < slots ? a.units : slots));
   cfg.blockDim = dim3(kRowsThreads);
   cfg.dynamicSmemBytes = staged ? (size_t)M * a.pitch : 0;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const bool two = M > 8;
 #define RGK_ROWS(MODE) (two ? launch_rows_t<MODE, true>(cfg, staged, a) : launch_rows_t<MODE, false>(cfg, staged, a))
   cudaError_t e;

@@ -500,12 +500,13 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
   if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, D, X, (int)heads, (int)window), &ws))
     return nullptr;
   at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
-  // the kernels work on the ring in place; the functional form is the same step on a copy
-  const bool copy = want && !inplace;
-  at::Tensor k = copy ? keys->clone() : *keys, v = copy ? values->clone() : *values,
-             seen_out = copy ? seen->clone() : *seen;
+  const bool fresh = want && !inplace;             // a new ring, written as the old one is read
+  at::Tensor k = fresh ? empty(keys->sizes(), at::kBFloat16, dev) : *keys,
+             v = fresh ? empty(values->sizes(), at::kBFloat16, dev) : *values,
+             seen_out = fresh ? empty(seen->sizes(), at::kInt, dev) : *seen;
   if (!succeeded(g_lib.attention_residual_decode(
-          x->const_data_ptr(), pos->const_data_ptr(), pc, &p, scale1, eps1, &c, k.mutable_data_ptr(),
+          x->const_data_ptr(), pos->const_data_ptr(), pc, &p, scale1, eps1, &c, keys->const_data_ptr(),
+          values->const_data_ptr(), static_cast<const int*>(seen->const_data_ptr()), k.mutable_data_ptr(),
           v.mutable_data_ptr(), static_cast<int*>(seen_out.mutable_data_ptr()), B, D, X, (int)heads, 256,
           (int)window, RGK_BF16, want ? 1 : 0, out.mutable_data_ptr(), chained && !made ? 1 : 0, ws.ptr,
           ws.bytes, s)))
@@ -513,7 +514,7 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
   Ref o(wrap(std::move(out)));
   if (o.p == nullptr) return nullptr;
   if (!want) return PyTuple_Pack(2, o.p, Py_None);
-  if (!copy) return PyTuple_Pack(2, o.p, cache);
+  if (!fresh) return PyTuple_Pack(2, o.p, cache);
   Ref rk(wrap(std::move(k))), rv(wrap(std::move(v))), rs(wrap(std::move(seen_out)));
   if (rk.p == nullptr || rv.p == nullptr || rs.p == nullptr) return nullptr;
   Ref ring(PyObject_CallFunctionObjArgs(g_ring_cls, rk.p, rv.p, rs.p, nullptr));

@@ -39,6 +39,19 @@ class PerDeviceOnce {
   int sms_[kMaxDevices] = {};
 };
 
+// The share of an SM's 228 KB that a launch asks to be shared memory rather than L1, for kernels that
+// stream through L1: without it they inherit whatever the kernel in front left, and behind one that used
+// all of it the projections of one row took 26 us instead of 11.5 (28 KB of L1 for 120 KB of loads in
+// flight).  `bytes`: shared memory of the CTAs of an SM; 64 KB at least, so that the kernels of a decode
+// step of a few sequences agree and the SMs are not reconfigured between them.
+inline cudaLaunchAttribute smem_carveout(size_t bytes) {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  const size_t kb = bytes > 64 * 1024 ? (bytes + 1023) / 1024 : 64;
+  a.val.sharedMemCarveout = kb >= 228 ? 100 : (unsigned)((kb * 100 + 227) / 228);
+  return a;
+}
+
 // How the fused RG-LRU kernel evaluates the two sigmoids of the gates and the gelu of the join.
 //   kMathExact  sigmoids as 1 / (1 + 2^(-z log2 e)) in float32 with one reciprocal for the four
 //               denominators of a token pair (both gates), gelu as z / (1 + 2^w) with one reciprocal
@@ -167,14 +180,21 @@ cudaError_t launch_dense_tc(const void* x, const RowsMatrix* mats, int n_mats, c
                             int K, int act, int* status, cudaStream_t s, float cap = 0.0f);
 
 // attention_decode.cu: one new token per sequence against the ring cache keys / values [B,W,256]
-// (num_tokens [B] int32 tokens seen so far): q [B,N,256] and k_new [B,256] rotated, v_new [B,256]
+// (num_tokens [B] int32 tokens seen so far): q [B,N,256], k_new [B,256], v_new [B,256]
 // -> out [B,N*256]; update != 0 then stores k_new / v_new in ring slot num_tokens % W and adds one
-// to num_tokens.  ws: attention_decode_workspace_bytes.
+// to num_tokens.
+// float32, q and k_new rotated: the ring is updated in place.  ws: attention_decode_workspace_bytes.
 bool attention_decode_supported(int hd, int N, int W);
 size_t attention_decode_workspace_bytes(int64_t B, int N, int W);
 cudaError_t launch_attention_decode(const void* q, const void* k_new, const void* v_new, void* keys,
                                     void* values, int* num_tokens, int64_t B, int N, int W,
-                                    int dtype, int update, void* out, void* ws, cudaStream_t s);
+                                    int update, void* out, void* ws, cudaStream_t s);
+// bfloat16; q and k_new are rotated by the positions pos [B], unless it is NULL.  The updated ring goes to
+// keys, values, seen, which may be the tensors it is read from; status: raised if a bounded wait gives up.
+cudaError_t launch_attention_decode_ring(const void* q, const void* k_new, const void* v_new, const void* pos,
+                                         int pos64, const void* keys_in, const void* values_in,
+                                         const int* seen_in, void* keys, void* values, int* seen, int64_t B,
+                                         int N, int W, int update, void* out, int* status, cudaStream_t s);
 
 // embed.cu: rows of the embedding table scaled by a constant (Embedder.encode), and the index of
 // the first maximum of every row of a [M, V] matrix (greedy sampling).
