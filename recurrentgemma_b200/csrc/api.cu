@@ -152,7 +152,9 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
     cudaError_t e = fuse_conv
         ? rgk::launch_conv1d_cache(xb, pos, pos64, B, T, E, dtype, conv_cache_out, s)
         : rgk::launch_conv1d_prefill(xb, pos, pos64, p->conv_w, p->conv_b, B, T, E, dtype,
-                                     const_cast<void*>(c), conv_cache_out, s);
+                                     const_cast<void*>(c), conv_cache_out, s,
+                                    chan_route ? rgk::rglru_chan_prep(scan_ws, p->a_param, B, T, H)
+                                               : rgk::ChanPrep());
     if (e != cudaSuccess) return cuda_fail(e, "conv1d launch");
   }
   const bool fused_ok = rgk::rglru_chan_supported(dtype, bw, B, T);
@@ -171,7 +173,7 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
     cudaError_t e = rgk::launch_rglru_chan(fuse_conv ? xb : c, pos, pos64, p->a_param, p->gate_x_b,
                                            p->gate_a_b, packed, h0, yb, y_activated, B, T, H, out,
                                            h_last, scan_ws, math, s, fuse_conv ? p->conv_w : nullptr,
-                                           fuse_conv ? p->conv_b : nullptr);
+                                           fuse_conv ? p->conv_b : nullptr, xb != nullptr && !fuse_conv);
     if (e != cudaSuccess) return cuda_fail(e, "fused RG-LRU launch");
     return RGK_OK;
   }

@@ -109,6 +109,8 @@ __global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepArgs a) {
   __shared__ __align__(16) uint4 s_tile[kPrepRows * 33];      // a value row per 33 packs; also the scan's scratch
   const int tid = threadIdx.x;
   const int T_ = a.T;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if ((int)blockIdx.x < a.B) {
     // ---- visible ranges: a thread scans a chunk for document starts, then a maximum over the chunks
     // in front (the first token starts a document whatever its position)
@@ -330,6 +332,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  grid_dependency_wait();
+  grid_launch_dependents();
 
   // unit -> (sequence, head, query tile); the key tiles it needs
   auto unit_of = [&](int i, int& b, int& n, int& t0, int& j_lo, int& j_hi) {
@@ -746,8 +750,7 @@ cudaError_t launch_attention_prefill(void* q, void* k, const void* v, const void
   if (cache_k != nullptr && T < window) rows = rows > window ? rows : window;
   const int64_t blocks = B + B * ((rows + kPrepRows - 1) / kPrepRows);
   if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
-  attn_prepare_kernel<<<(unsigned)blocks, 256, 0, s>>>(a);
-  cudaError_t err = cudaGetLastError();
+  cudaError_t err = launch_dependent(attn_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, s, a);
   if (err != cudaSuccess) return err;
   CUtensorMap map_q, map_k, map_vt;
   if (!tensor_map_bte(&map_q, q, (uint64_t)B, (uint64_t)T, (uint64_t)N * kHd, kTq, kSl, true) ||
@@ -763,9 +766,8 @@ cudaError_t launch_attention_prefill(void* q, void* k, const void* v, const void
   const int q_tiles = (int)((T + kTq - 1) / kTq);
   const int n_units = (int)(B * N * q_tiles);
   const int grid = n_units < num_sms ? n_units : num_sms;
-  attn_prefill_kernel<<<grid, kThreadsA, kSmemA, s>>>(map_q, map_k, map_vt, lo, (int)B, (int)T, N,
-                                                      window, n_units, (T_*)out, status);
-  return cudaGetLastError();
+  return launch_dependent(attn_prefill_kernel, dim3(grid), dim3(kThreadsA), kSmemA, s, map_q, map_k, map_vt, lo,
+                          (int)B, (int)T, N, window, n_units, (T_*)out, status);
 }
 
 }  // namespace rgk

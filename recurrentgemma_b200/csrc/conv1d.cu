@@ -69,9 +69,16 @@ template <typename T>
 __global__ void __launch_bounds__(kConvThreads)
 conv1d_prefill_kernel(const T* __restrict__ x, const void* __restrict__ pos, int pos64,
                       const T* __restrict__ w, const T* __restrict__ bias, int T_, int E,
-                      T* __restrict__ out, T* __restrict__ cache_out) {
+                      T* __restrict__ out, T* __restrict__ cache_out, const ChanPrep prep) {
   constexpr int kPack = Traits<T>::kPack;
   using Ops = PackOps<T>;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  if (prep.E > 0) {                              // for the RG-LRU kernel behind
+    const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    chan_prepare(prep, block * kConvThreads + threadIdx.x,
+                 (int64_t)gridDim.x * gridDim.y * gridDim.z * kConvThreads);
+  }
   const int pack_idx = blockIdx.x * kConvThreads + threadIdx.x;
   const int e0 = pack_idx * kPack;
   if (e0 >= E) return;
@@ -221,22 +228,19 @@ conv1d_decode_kernel(const T* x, const T* cache_in, const T* __restrict__ w,
 
 cudaError_t launch_conv1d_prefill(const void* x, const void* pos, int pos64, const void* w,
                                   const void* b, int64_t B, int64_t T, int64_t E, int dtype,
-                                  void* out, void* cache_out, cudaStream_t s) {
+                                  void* out, void* cache_out, cudaStream_t s, const ChanPrep& prep) {
   if (B == 0 || T == 0 || E == 0) return cudaSuccess;
   const int pack = dtype ? 8 : 4;
   dim3 grid((unsigned)((E / pack + kConvThreads - 1) / kConvThreads),
             (unsigned)((T + kConvRows - 1) / kConvRows), (unsigned)B);
   if (dtype) {
     using T_ = __nv_bfloat16;
-    conv1d_prefill_kernel<T_><<<grid, kConvThreads, 0, s>>>(
-        (const T_*)x, pos, pos64, (const T_*)w, (const T_*)b, (int)T, (int)E, (T_*)out,
-        (T_*)cache_out);
-  } else {
-    conv1d_prefill_kernel<float><<<grid, kConvThreads, 0, s>>>(
-        (const float*)x, pos, pos64, (const float*)w, (const float*)b, (int)T, (int)E, (float*)out,
-        (float*)cache_out);
+    return launch_dependent(conv1d_prefill_kernel<T_>, grid, dim3(kConvThreads), 0, s, (const T_*)x, pos, pos64,
+                            (const T_*)w, (const T_*)b, (int)T, (int)E, (T_*)out, (T_*)cache_out, prep);
   }
-  return cudaGetLastError();
+  return launch_dependent(conv1d_prefill_kernel<float>, grid, dim3(kConvThreads), 0, s, (const float*)x, pos,
+                          pos64, (const float*)w, (const float*)b, (int)T, (int)E, (float*)out,
+                          (float*)cache_out, prep);
 }
 
 cudaError_t launch_conv1d_cache(const void* x, const void* pos, int pos64, int64_t B, int64_t T,

@@ -137,6 +137,28 @@ template <bool kFast> __device__ __forceinline__ float sqrt_(float v) {
 // torch softplus defaults: beta 1, threshold 20.
 __device__ __forceinline__ float softplus_(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
 
+// Programmatic dependent launch: wait until every kernel in front has completed and its writes are
+// visible; let the kernel behind be placed (it does the same wait before it touches memory).
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// thread `at` of `of` doing its share of a ChanPrep (rgk_internal.h)
+template <typename Prep>
+__device__ __forceinline__ void chan_prepare(const Prep& p, int64_t at, int64_t of) {
+  for (int64_t i = at; i < p.n_zero; i += of) p.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int64_t e = at; e < p.E; e += of) {
+    // rounded as the reference rounds its factors; clamped to the range of the kernel's table of
+    // exp(log_a): beyond it a = exp(log_a) is 0 in float32 either way (the gate would have to be below
+    // 0.7 at softplus(a_param) above 16)
+    const float s = round_bf16(softplus_(__bfloat162float(p.a_param[e])));
+    p.m8sp[e] = __float2bfloat16_rn(fmaxf(-8.0f * s, -127.5f));
+  }
+}
+
 // gelu(approximate="tanh") written through the logistic function:
 // 0.5 (1 + tanh(u)) = sigmoid(2u), u = sqrt(2/pi) (z + 0.044715 z^3).
 template <bool kFast> __device__ __forceinline__ float gelu_tanh_(float z) {

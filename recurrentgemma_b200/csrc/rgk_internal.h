@@ -2,6 +2,7 @@
 // arguments first.  Each returns the cudaError_t of its last launch.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -39,6 +40,36 @@ class PerDeviceOnce {
   int sms_[kMaxDevices] = {};
 };
 
+// A launch that may be placed while the kernel in front still runs (programmatic dependent launch): every
+// CTA of `kernel` executes griddepcontrol.wait before it touches memory that a kernel may have written
+// or still reads.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// What rglru_chan_kernel finds prepared: the words that states (and maps) arrive in without their tokens,
+// and -8 softplus(a_param).  The kernel in front does it on the side (launch_conv1d_prefill), or a small
+// one of its own.
+struct ChanPrep {
+  uint4* zero = nullptr;
+  int64_t n_zero = 0;                    // in packs of 16 bytes
+  const __nv_bfloat16* a_param = nullptr;
+  __nv_bfloat16* m8sp = nullptr;
+  int E = 0;
+};
+
 // The share of an SM's 228 KB that a launch asks to be shared memory rather than L1, for kernels that
 // stream through L1: without it they inherit whatever the kernel in front left, and behind one that used
 // all of it the projections of one row took 26 us instead of 11.5 (28 KB of L1 for 120 KB of loads in
@@ -68,7 +99,8 @@ enum { kMathExact = 0, kMathFast = 1 };
 // conv1d.cu
 cudaError_t launch_conv1d_prefill(const void* x, const void* pos, int pos64, const void* w,
                                   const void* b, int64_t B, int64_t T, int64_t E, int dtype,
-                                  void* out, void* cache_out, cudaStream_t s);
+                                  void* out, void* cache_out, cudaStream_t s,
+                                  const ChanPrep& prep = ChanPrep());
 // the cache a prefill returns, alone (the fused RG-LRU kernel computes the convolution itself)
 cudaError_t launch_conv1d_cache(const void* x, const void* pos, int pos64, int64_t B, int64_t T,
                                 int64_t E, int dtype, void* cache_out, cudaStream_t s);
@@ -128,11 +160,14 @@ cudaError_t launch_path_decode_tc(const void* xb, const void* yb, const void* po
 // ws: rglru_chan_workspace_bytes(B, T, E) bytes whose first word is the caller's status word.
 bool rglru_chan_supported(int dtype, int bw, int64_t B, int64_t T);
 size_t rglru_chan_workspace_bytes(int64_t B, int64_t T, int64_t E);
+// what the launch below does first unless `prepared`
+ChanPrep rglru_chan_prep(void* ws, const void* a_param, int64_t B, int64_t T, int H);
 cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const void* a_param,
                               const void* bx, const void* ba, const void* packed_w, const float* h0,
                               const void* yb, int y_activated, int64_t B, int64_t T, int H,
                               void* out, float* h_last, void* ws, int math, cudaStream_t s,
-                              const void* conv_w = nullptr, const void* conv_b = nullptr);
+                              const void* conv_w = nullptr, const void* conv_b = nullptr,
+                              bool prepared = false);
 
 // gemm_rows.cu: up to three projections (matrices) of the same M <= 16 rows in one launch, with
 // RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as above behind; one

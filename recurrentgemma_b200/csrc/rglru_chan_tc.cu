@@ -273,7 +273,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
                   const __grid_constant__ CUtensorMap map_ct, const __grid_constant__ CUtensorMap map_yt,
                   const __grid_constant__ CUtensorMap map_ot, const void* __restrict__ pos, int pos64,
                   const __nv_bfloat16* __restrict__ bias_x, const __nv_bfloat16* __restrict__ bias_a,
-                  const __nv_bfloat16* __restrict__ m8sp, const float* __restrict__ h0, int B, int T_,
+                  const __nv_bfloat16* m8sp, const float* __restrict__ h0, int B, int T_,
                   int E, int groups, int n_units, float* __restrict__ h_last, WsHeader* hdr,
                   unsigned long long* agg, unsigned long long* incl, int use_agg,
                   const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ conv_b) {
@@ -326,6 +326,9 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  // everything up to here, the table above all, overlaps the kernel in front; the one behind is not let
+  // in before this one ends (its waiting warps cost this kernel, which is bound by issue, 6%)
+  grid_dependency_wait();
 
   if (warp == kEpi) {
     // ------------------------------ TMA producer of the MMA operands ------------------------------
@@ -544,7 +547,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
       const int e = chan0(u) + lane;
       bxv = __ldg(reinterpret_cast<const uint16_t*>(bias_x) + e);
       bav = __ldg(reinterpret_cast<const uint16_t*>(bias_a) + e);
-      spv = __ldg(reinterpret_cast<const uint16_t*>(m8sp) + e);
+      spv = reinterpret_cast<const uint16_t*>(m8sp)[e];
     };
     if (n_my > 0) load_consts(cur);
 
@@ -763,24 +766,13 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   }
 }
 
-// -8 softplus(a_param), rounded as the reference rounds its factors, one value per channel.
-__global__ void m8sp_chan_kernel(const __nv_bfloat16* __restrict__ a_param, int E,
-                                 __nv_bfloat16* __restrict__ m8sp) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < E) {
-    const float s = round_bf16(softplus_(__bfloat162float(a_param[e])));
-    // clamped to the range of the kernel's table of exp(log_a): beyond it a = exp(log_a) is 0 in
-    // float32 either way (the gate would have to be below 0.7 at softplus(a_param) above 16)
-    m8sp[e] = __float2bfloat16_rn(fmaxf(-8.0f * s, kLogAFloor));
-  }
+// The preparation where no kernel in front does it on the side.
+__global__ void chan_prepare_kernel(const ChanPrep p) {
+  static_assert(kLogAFloor == -127.5f, "the clamp of chan_prepare");
+  grid_dependency_wait();
+  grid_launch_dependents();
+  chan_prepare(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
-
-// Tensor map of a row-major bfloat16 matrix [rows, cols] with boxes of box_rows x box_cols.
-
-
-// Tensor map of bfloat16 activations [B, T, E] with boxes of box_rows tokens x box_cols channels of
-// one sequence: rows past the end of a sequence read as zero and are dropped from stores.
-
 
 struct ChanLayout {
   int64_t n_units, n_rec;
@@ -821,6 +813,11 @@ cudaError_t chan_device_setup(int* num_sms) {
   }, num_sms);
 }
 
+// With fewer units per time tile than CTAs, consecutive tiles of a chain are in flight at once
+// and carries are resolved from published maps; otherwise a tile's predecessor was dealt out a
+// round earlier and only its state is ever waited for.
+bool chan_uses_maps(int64_t B, int groups, int grid) { return B * groups < grid; }
+
 }  // namespace
 
 bool rglru_chan_supported(int dtype, int bw, int64_t B, int64_t T) {
@@ -832,11 +829,29 @@ size_t rglru_chan_workspace_bytes(int64_t B, int64_t T, int64_t E) {
   return chan_layout(B, T, E).total;
 }
 
+// State words (and map words, where used) start without their token; the status word in front of them
+// belongs to the caller.
+ChanPrep rglru_chan_prep(void* ws, const void* a_param, int64_t B, int64_t T, int H) {
+  ChanPrep p;
+  int num_sms = 0;
+  if (chan_device_setup(&num_sms) != cudaSuccess) return p;
+  const int E = H * kHW;
+  const ChanLayout L = chan_layout(B, T, E);
+  char* base = static_cast<char*>(ws);
+  const int grid = (int)(L.n_units < num_sms ? L.n_units : num_sms);
+  p.zero = reinterpret_cast<uint4*>(base + L.incl_off);
+  p.n_zero = (int64_t)(((chan_uses_maps(B, 2 * H, grid) ? L.m8sp_off : L.agg_off) - L.incl_off) / 16);
+  p.a_param = static_cast<const __nv_bfloat16*>(a_param);
+  p.m8sp = reinterpret_cast<__nv_bfloat16*>(base + L.m8sp_off);
+  p.E = E;
+  return p;
+}
+
 cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const void* a_param,
                               const void* bx, const void* ba, const void* packed_w, const float* h0,
                               const void* yb, int y_activated, int64_t B, int64_t T, int H,
                               void* out, float* h_last, void* ws, int math, cudaStream_t s,
-                              const void* conv_w, const void* conv_b) {
+                              const void* conv_w, const void* conv_b, bool prepared) {
   using T_ = __nv_bfloat16;
   const bool conv = conv_w != nullptr;       // `c` is then the block input, the kernel convolves it
   const int E = H * kHW;
@@ -848,17 +863,15 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
   const int groups = 2 * H;
   const int n_units = (int)L.n_units;
   const int grid = n_units < num_sms ? n_units : num_sms;   // all CTAs resident: look-back may spin
-  // With fewer units per time tile than CTAs, consecutive tiles of a chain are in flight at once
-  // and carries are resolved from published maps; otherwise a tile's predecessor was dealt out a
-  // round earlier and only its state is ever waited for.
-  const int use_agg = (int64_t)B * groups < grid ? 1 : 0;
-  // state words (and map words, where used) start without their token; the status word before
-  // them belongs to the caller
-  err = cudaMemsetAsync(base + sizeof(int), 0, (use_agg ? L.m8sp_off : L.agg_off) - sizeof(int), s);
-  if (err != cudaSuccess) return err;
-  T_* m8sp = reinterpret_cast<T_*>(base + L.m8sp_off);
-  m8sp_chan_kernel<<<(E + 255) / 256, 256, 0, s>>>((const T_*)a_param, E, m8sp);
-  if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  const int use_agg = chan_uses_maps(B, groups, grid) ? 1 : 0;
+  const ChanPrep prep = rglru_chan_prep(ws, a_param, B, T, H);
+  if (!prepared) {
+    const int64_t n = prep.n_zero > prep.E ? prep.n_zero : prep.E, blocks = (n + 1023) / 1024;
+    err = launch_dependent(chan_prepare_kernel, dim3((unsigned)(blocks < 8 * num_sms ? blocks : 8 * num_sms)),
+                           dim3(256), 0, s, prep);
+    if (err != cudaSuccess) return err;
+  }
+  const T_* m8sp = prep.m8sp;
 
   CUtensorMap map_c, map_w, map_ct, map_yt, map_ot;
   const uint64_t Bu = (uint64_t)B, Tu = (uint64_t)T, Eu = (uint64_t)E;
@@ -870,12 +883,13 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
       !tensor_map_bte_sw64(&map_yt, yb != nullptr ? yb : out, Bu, Tu, Eu, kSub, kSub))
     return cudaErrorInvalidValue;
 #define RGK_CHAN_C(J, M, C, THREADS)                                                             \
-  rglru_chan_kernel<J, M, C><<<grid, THREADS, kSmem, s>>>(                                       \
-      map_c, map_w, map_ct, map_yt, map_ot, pos, pos64, (const T_*)bx, (const T_*)ba, m8sp, h0,  \
-      (int)B, (int)T, E, groups, n_units, h_last, reinterpret_cast<WsHeader*>(base),             \
-      reinterpret_cast<unsigned long long*>(base + L.agg_off),                                   \
-      reinterpret_cast<unsigned long long*>(base + L.incl_off), use_agg, (const T_*)conv_w,      \
-      (const T_*)conv_b)
+  err = launch_dependent(rglru_chan_kernel<J, M, C>, dim3(grid), dim3(THREADS), kSmem, s,        \
+                         map_c, map_w, map_ct, map_yt, map_ot, pos, pos64, (const T_*)bx,        \
+                         (const T_*)ba, m8sp, h0, (int)B, (int)T, E, groups, n_units, h_last,    \
+                         reinterpret_cast<WsHeader*>(base),                                      \
+                         reinterpret_cast<unsigned long long*>(base + L.agg_off),                \
+                         reinterpret_cast<unsigned long long*>(base + L.incl_off), use_agg,      \
+                         (const T_*)conv_w, (const T_*)conv_b)
 #define RGK_CHAN(J, M)                                                                           \
   do { if (conv) RGK_CHAN_C(J, M, true, kThreadsConv); else RGK_CHAN_C(J, M, false, kThreads); } while (0)
 #define RGK_CHAN_J(M)                                                                            \
@@ -889,7 +903,7 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
 #undef RGK_CHAN_J
 #undef RGK_CHAN
 #undef RGK_CHAN_C
-  return cudaGetLastError();
+  return err;
 }
 
 }  // namespace rgk

@@ -35,6 +35,8 @@ rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ addend, const T* _
   constexpr bool kBf16 = Traits<T>::kBf16;
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kNormWarps + (threadIdx.x >> 5);
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (row >= M) return;
   const int packs = D / kPack;                 // packs in a row
   const T* xr = x + row * D;
@@ -175,15 +177,14 @@ cudaError_t launch_typed(const void* x, const void* addend, const void* scale, i
   const int packs_per_lane = (int)((D / Traits<T>::kPack + 31) / 32);
   const unsigned grid = (unsigned)((M + kNormWarps - 1) / kNormWarps);
   const dim3 block(kNormWarps * 32);
-#define RGK_NORM(P)                                                                           \
-  rmsnorm_kernel<T, P><<<grid, block, 0, s>>>((const T*)x, (const T*)addend, (const T*)scale, M, (int)D, \
-                                              eps, (T*)sum_out, (T*)out)
-  if (packs_per_lane <= 4) RGK_NORM(4);
-  else if (packs_per_lane <= 10) RGK_NORM(10);
-  else if (packs_per_lane <= 16) RGK_NORM(16);
-  else RGK_NORM(kMaxPacks);
+#define RGK_NORM(P)                                                                                     \
+  launch_dependent(rmsnorm_kernel<T, P>, dim3(grid), block, 0, s, (const T*)x, (const T*)addend,        \
+                   (const T*)scale, M, (int)D, eps, (T*)sum_out, (T*)out)
+  if (packs_per_lane <= 4) return RGK_NORM(4);
+  if (packs_per_lane <= 10) return RGK_NORM(10);
+  if (packs_per_lane <= 16) return RGK_NORM(16);
+  return RGK_NORM(kMaxPacks);
 #undef RGK_NORM
-  return cudaGetLastError();
 }
 
 }  // namespace

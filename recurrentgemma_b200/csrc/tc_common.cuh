@@ -192,14 +192,6 @@ __device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint6
   return true;
 }
 
-// Programmatic dependent launch: wait until every kernel in front has completed and its writes are
-// visible; let the kernel behind be placed (it does the same wait before it touches memory).
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 // Cluster barrier halves; every thread of every CTA of the cluster executes each of them, warps
 // converged.
 __device__ __forceinline__ void cluster_arrive() {
@@ -217,6 +209,9 @@ __device__ __forceinline__ uint32_t peer_smem(uint32_t local_addr, uint32_t rank
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
+}
+__device__ __forceinline__ void st_peer_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(addr), "r"(v) : "memory");
 }
 // An arrival at a barrier of any CTA of the cluster, and the wait that takes such arrivals.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {

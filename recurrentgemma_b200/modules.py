@@ -839,13 +839,15 @@ class Embedder(nn.Module):
 
 
 @torch.no_grad()
-def argmax(logits: torch.Tensor) -> torch.Tensor:
+def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
   """torch.argmax(logits, dim=-1) as int32 (greedy sampling,
-  recurrentgemma/torch/sampler.py:131-132): the first maximum of every row."""
+  recurrentgemma/torch/sampler.py:131-132): the first maximum of every row, into `out` if given."""
   dev = _lib.require_cuda(logits)
   v = logits.shape[-1]
   xc = logits.contiguous()
-  out = torch.empty(logits.shape[:-1], dtype=torch.int32, device=dev)
+  if out is None:
+    out = torch.empty(logits.shape[:-1], dtype=torch.int32, device=dev)
+  assert out.shape == logits.shape[:-1] and out.dtype == torch.int32 and out.is_contiguous()
   with torch.cuda.device(dev):
     _lib.check(_lib.load().rgk_argmax(xc.data_ptr(), xc.numel() // v, v,
                                       _lib.dtype_code(logits.dtype), out.data_ptr(),

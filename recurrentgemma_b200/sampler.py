@@ -60,7 +60,6 @@ class GreedySampler:
     dev = self.device
     if self._graph_key != (b, dev):
       state = {"last_token": torch.zeros((b, 1), dtype=torch.int32, device=dev),
-               "next_token": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "positions": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "cache": _own(cache), "logits": None}
       # one eager step on the capture stream creates every lazily made buffer of a decode step (the
@@ -94,12 +93,12 @@ class GreedySampler:
 
   def _step(self, state) -> None:
     """One sampling step (recurrentgemma/torch/sampler.py:137-187) on static buffers: reads
-    `last_token` and `positions`, updates the cache in place, writes `next_token`, `logits`."""
+    `last_token` and `positions`, updates the cache in place, writes `last_token` (the next token is
+    the last one from here on) and `logits`."""
     logits, _ = self.model(state["last_token"], state["positions"], state["cache"],
                            return_logits=True, return_cache=True, inplace_cache=True)
     state["logits"] = logits
-    state["next_token"].copy_(modules.argmax(logits[:, 0])[:, None])
-    state["last_token"].copy_(state["next_token"])
+    modules.argmax(logits[:, 0], out=state["last_token"][:, 0])
     state["positions"].add_(1)
 
   @torch.no_grad()
@@ -146,14 +145,13 @@ class GreedySampler:
       state["positions"].copy_(pos[:, -1:] + 1)
     else:
       state = {"last_token": first[:, None].clone(),
-               "next_token": torch.empty((b, 1), dtype=torch.int32, device=dev),
                "positions": (pos[:, -1:] + 1).contiguous(), "cache": _own(cache), "logits": None}
     for step in range(1, total_generation_steps):
       if graph is None:
         self._step(state)
       else:
         graph.replay()
-      out_tokens[:, step] = state["next_token"][:, 0]
+      out_tokens[:, step] = state["last_token"][:, 0]
       if return_logits:
         out_logits[:, step] = state["logits"][:, 0]
     if self.eos_id is not None:
