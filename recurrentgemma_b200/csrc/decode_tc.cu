@@ -6,13 +6,18 @@
 // head (64 channels); the four CTAs of a head form a cluster.  The A operand - the conv output of
 // the 128 rows for all 256 channels of the head, computed from the new token and the three cached
 // rows with the reference's bfloat16 roundings, in the 128-byte-swizzled K-major layout tcgen05
-// reads - is built once per cluster: each CTA computes the slice of its own 64 channels and stores it
-// into the shared memory of all four (distributed shared memory), while TMA brings the CTA's 64
-// x-gate and 64 a-gate weight rows (64 KiB, pre-packed K-major).  Sixteen tcgen05.mma (M 128, N 128, K 16) leave both gates of every channel in TMEM;
-// the epilogue does the gate arithmetic, the state update h = a h + x in float32 (stored
-// unrounded), the join with gelu(y branch), and writes out / state / shifted conv cache.
+// reads - is built once per cluster: each CTA computes the slice of its own 64 channels in its shared
+// memory and sends it to the other three with one bulk copy each (stores of every thread into the
+// peers' memory, as an earlier version had them, moved 64 KiB per CTA at 25 GB/s), while TMA brings
+// the CTA's 64 x-gate and 64 a-gate weight rows (64 KiB, pre-packed K-major).  Sixteen tcgen05.mma
+// (M 128, N 128, K 16) leave both gates of every channel in TMEM, a lane a row; the epilogue does the
+// gate arithmetic, the state update h = a h + x in float32 (stored unrounded) and the join with
+// gelu(y branch).  State and y branch come through shared memory, rows in whole 256- and 128-byte
+// pieces, loaded before the conv is computed and written back over themselves: a thread reading its
+// row's 16 channels from global memory touches 32 rows per instruction, which took 4.6 us.
+// Per layer of 2560 channels at 256 rows: 11.2 -> 9.7 us in a chain of 26.
 //
-// Both mbarrier waits are bounded; on expiry WsHeader::status is raised and the CTA leaves.
+// Every mbarrier wait is bounded; on expiry WsHeader::status is raised and the CTA leaves.
 #include <cuda.h>
 
 #include "rgk_common.cuh"
@@ -31,9 +36,11 @@ constexpr int kASlice = kRowsM * 128;            // 16 KiB
 constexpr int kBSlice = kN * 128;                // 16 KiB
 constexpr int kOffB = 0;
 constexpr int kOffA = kSlices * kBSlice;                       // 65536
-constexpr int kOffConst = kOffA + kSlices * kASlice;           // 131072
-constexpr int kOffBar = kOffConst + 3 * (kChanCta / 2) * 4;    // two mbarriers
-constexpr int kOffTmem = kOffBar + 16;
+constexpr int kOffH = kOffA + kSlices * kASlice;               // 131072: state, 128 rows of 256 bytes
+constexpr int kOffY = kOffH + kRowsM * kChanCta * 4;           // the other branch, 128 rows of 128 bytes
+constexpr int kOffConst = kOffY + kRowsM * kChanCta * 2;
+constexpr int kOffBar = kOffConst + 3 * (kChanCta / 2) * 4;    // weights, MMAs, the peers' slices
+constexpr int kOffTmem = kOffBar + 24;
 constexpr int kOffAbort = kOffTmem + 4;
 constexpr int kOffLutDec = (kOffAbort + 4 + 15) & ~15;        // {a, multiplier} by log_a (tc_common.cuh)
 constexpr int kSmem = kOffLutDec + kLutEntries * 4 + 1024;
@@ -66,7 +73,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t s_base = smem_u32(smem);
   uint32_t* s_const = reinterpret_cast<uint32_t*>(smem + kOffConst);
-  const uint32_t bar_b = s_base + kOffBar, bar_mma = s_base + kOffBar + 8;
+  const uint32_t bar_b = s_base + kOffBar, bar_mma = bar_b + 8, bar_a = bar_b + 16;
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
@@ -82,7 +89,9 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     *s_abort = 0;
     mbar_init(bar_b, 1);
     mbar_init(bar_mma, 1);
+    mbar_init(bar_a, 1);
     mbar_fence_init();
+    mbar_expect_tx(bar_a, 3 * kASlice);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -129,13 +138,14 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   }
   tc_fence_before();
   __syncthreads();
+  cluster_arrive();                                // this CTA's barriers are set up
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
 
   // ---- weights: 64 x-gate rows and 64 a-gate rows of this quarter, per K slice -------------------
   // (After the dependency wait: the packed copy may have been written by the kernel just before.)
   if (tid == 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_dependency_wait();
     mbar_expect_tx(bar_b, kSlices * kBSlice);
     const int group_row = (head * 2 + (quarter >> 1)) * 256 + (quarter & 1) * kChanCta;
     for (int k = 0; k < kSlices; ++k) {
@@ -145,10 +155,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     }
   }
 
-  // ---- A operand: conv output of 128 rows x the head's 256 channels ------------------------------
-  // The four CTAs of a head (a cluster) need the same A tile.  Each computes the K slice of its own
-  // 64 channels and stores it into the shared memory of all four: a quarter of the loads and of the
-  // arithmetic per CTA.
+  // ---- this CTA's slice of the A operand: conv output of 128 rows x 64 channels -------------------
+  const int64_t row0 = (int64_t)tile * kRowsM;
   {
     const int pk = tid & 7;                       // 16-byte pack inside this CTA's slice of channels
     const int e = chan0 + pk * 8;
@@ -156,70 +164,88 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
 #pragma unroll
     for (int k = 0; k < 4; ++k) wv[k] = *reinterpret_cast<const uint4*>(conv_w + (int64_t)k * E + e);
     const uint4 bv = *reinterpret_cast<const uint4*>(conv_b + e);
-    uint32_t a_remote[4];                         // this slice inside each CTA of the cluster
-#pragma unroll
-    for (int d = 0; d < 4; ++d)
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                   : "=r"(a_remote[d]) : "r"(s_base + kOffA + quarter * kASlice), "r"(d));
     // Everything above (barriers, TMEM, the per-channel constants) is independent of the kernel
     // before this one on the stream, which in a decode loop is the previous layer: with
     // programmatic dependent launch it overlaps that kernel's tail.  The activations below are its
     // output, so wait for it here, then let the next layer's prologue start in turn.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // two rows per thread, their 8 loads all issued before the first use
+    grid_dependency_wait();
+    grid_launch_dependents();
+    // all loads before the first use: the windows of two rows per thread, then state and other branch
     constexpr int kPer = kRowsM * 8 / kThreadsDec;     // rows per thread: 2
     constexpr int kRowStep = kThreadsDec / 8;
     uint4 xv[kPer][4];
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int r = (tid >> 3) + kRowStep * i;
-      const int64_t m = min((int64_t)tile * kRowsM + r, (int64_t)M - 1);   // clamped: never out of range
+      const int64_t m = min(row0 + (tid >> 3) + kRowStep * i, (int64_t)M - 1);   // clamped: never out of range
       const __nv_bfloat16* cr = cache_in + m * 3 * E + e;
       xv[i][0] = *reinterpret_cast<const uint4*>(cr);
       xv[i][1] = *reinterpret_cast<const uint4*>(cr + E);
       xv[i][2] = *reinterpret_cast<const uint4*>(cr + 2 * (int64_t)E);
       xv[i][3] = *reinterpret_cast<const uint4*>(xb + m * E + e);
     }
-    // every CTA of the cluster is running before its shared memory is written from outside
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    constexpr int kHPer = kRowsM * 16 / kThreadsDec, kYPer = kRowsM * 8 / kThreadsDec;   // packs per thread
+    uint4 hp[kHPer], yp[kYPer];
+#pragma unroll
+    for (int i = 0; i < kHPer; ++i) {
+      const int64_t m = min(row0 + (tid >> 4) + (kThreadsDec / 16) * i, (int64_t)M - 1);
+      hp[i] = *reinterpret_cast<const uint4*>(h_in + m * E + chan0 + (tid & 15) * 4);
+    }
+    if constexpr (kMul) {
+#pragma unroll
+      for (int i = 0; i < kYPer; ++i) {
+        const int64_t m = min(row0 + (tid >> 3) + kRowStep * i, (int64_t)M - 1);
+        yp[i] = *reinterpret_cast<const uint4*>(yb + m * E + e);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       const int r = (tid >> 3) + kRowStep * i;
-      const int64_t m = (int64_t)tile * kRowsM + r;
+      const int64_t m = row0 + r;
       // newest tap first (torch/layers.py:491-517 with prompt_len = 3), then the bias
       uint4 acc = mul4(xv[i][3], wv[3]);
       acc = add4(acc, mul4(xv[i][2], wv[2]));
       acc = add4(acc, mul4(xv[i][1], wv[1]));
       acc = add4(acc, mul4(xv[i][0], wv[0]));
       acc = add4(acc, bv);
-      if (m < M) {
-        if (cache_out != nullptr) {               // these are this CTA's own channels: shift the cache
-          __nv_bfloat16* co = cache_out + m * 3 * E + e;
-          *reinterpret_cast<uint4*>(co) = xv[i][1];
-          *reinterpret_cast<uint4*>(co + E) = xv[i][2];
-          *reinterpret_cast<uint4*>(co + 2 * (int64_t)E) = xv[i][3];
-        }
-      } else {
-        acc = make_uint4(0u, 0u, 0u, 0u);
-      }
-      const uint32_t off = r * 128 + ((pk ^ (r & 7)) << 4);
+      if (m >= M) acc = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(smem + kOffA + quarter * kASlice + r * 128 + ((pk ^ (r & 7)) << 4)) = acc;
+    }
+    fence_proxy_async();                           // towards the copy engine and the tensor core
+    __syncthreads();
+    cluster_wait();                                // the peers' barriers are set up
+    if (tid < 3) {
+      const int d = (quarter + 1 + tid) & 3;       // each starts with another peer
+      const uint32_t slice = s_base + kOffA + quarter * kASlice;
+      bulk_to_peer(peer_smem(slice, d), slice, kASlice, peer_smem(bar_a, d));
+    }
+    // while the slices travel: the shifted window of this CTA's own channels, state and other branch
 #pragma unroll
-      for (int d = 0; d < 4; ++d)
-        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-                     :: "r"(a_remote[d] + off), "r"(acc.x), "r"(acc.y), "r"(acc.z), "r"(acc.w) : "memory");
+    for (int i = 0; i < kPer; ++i) {
+      const int64_t m = row0 + (tid >> 3) + kRowStep * i;
+      if (m < M && cache_out != nullptr) {
+        __nv_bfloat16* co = cache_out + m * 3 * E + e;
+        *reinterpret_cast<uint4*>(co) = xv[i][1];
+        *reinterpret_cast<uint4*>(co + E) = xv[i][2];
+        *reinterpret_cast<uint4*>(co + 2 * (int64_t)E) = xv[i][3];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kHPer; ++i) {
+      const int r = (tid >> 4) + (kThreadsDec / 16) * i;
+      *reinterpret_cast<uint4*>(smem + kOffH + r * 256 + (((tid & 15) ^ (r & 7)) << 4)) = hp[i];
+    }
+    if constexpr (kMul) {
+#pragma unroll
+      for (int i = 0; i < kYPer; ++i) {
+        const int r = (tid >> 3) + kRowStep * i;
+        *reinterpret_cast<uint4*>(smem + kOffY + r * 128 + ((pk ^ (r & 7)) << 4)) = yp[i];
+      }
     }
   }
-  // The tile is complete when all four CTAs have stored their slices: the generic-proxy writes are
-  // fenced towards the tensor core's (async) proxy, then released and acquired across the cluster.
-  asm volatile("fence.proxy.async;" ::: "memory");
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   // ---- MMA ------------------------------------------------------------------------------------------
   if (tid == 0) {
-    if (mbar_wait(bar_b, 0, s_abort)) {
+    if (mbar_wait(bar_b, 0, s_abort) && mbar_wait(bar_a, 0, s_abort)) {
       tc_fence_after();
 #pragma unroll
       for (int k = 0; k < kSlices; ++k) {
@@ -240,20 +266,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     const int r = lane_base + lane;
     const int64_t m = (int64_t)tile * kRowsM + r;
     const bool row_ok = m < M;
-    const int64_t m_ld = row_ok ? m : 0;
     const bool is_reset = row_ok && pos_is_zero(pos, pos64, m);
-    const int e = chan0 + col_grp * kEpiCols;
-    // inputs of the state update and of the join, in flight while the MMA runs
-    float4 hv[kEpiCols / 4];
-    uint4 yv[kEpiCols / 8];
-#pragma unroll
-    for (int j = 0; j < kEpiCols / 4; ++j)
-      hv[j] = *reinterpret_cast<const float4*>(h_in + m_ld * E + e + 4 * j);
-    if constexpr (kMul) {
-#pragma unroll
-      for (int j = 0; j < kEpiCols / 8; ++j)
-        yv[j] = *reinterpret_cast<const uint4*>(yb + m_ld * E + e + 8 * j);
-    }
+    __syncthreads();                               // state and other branch are in place
     if (mbar_wait(bar_mma, 0, s_abort)) {
       tc_fence_after();
       uint32_t zx[kEpiCols], za[kEpiCols];
@@ -266,6 +280,20 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
 #pragma unroll
       for (int j = 0; j < kEpiCols / 8; ++j)
         cv[j] = *reinterpret_cast<const uint4*>(a_row + (((col_grp * (kEpiCols / 8) + j) ^ (r & 7)) << 4));
+      float4* hs[kEpiCols / 4];                    // this row's state, and its other branch, in shared memory
+      uint4* ys[kEpiCols / 8];
+      float4 hv[kEpiCols / 4];
+      uint4 yv[kEpiCols / 8];
+#pragma unroll
+      for (int j = 0; j < kEpiCols / 4; ++j) {
+        hs[j] = reinterpret_cast<float4*>(smem + kOffH + r * 256 + (((col_grp * (kEpiCols / 4) + j) ^ (r & 7)) << 4));
+        hv[j] = *hs[j];
+      }
+#pragma unroll
+      for (int j = 0; j < kEpiCols / 8; ++j) {
+        ys[j] = reinterpret_cast<uint4*>(smem + kOffY + r * 128 + (((col_grp * (kEpiCols / 8) + j) ^ (r & 7)) << 4));
+        yv[j] = kMul ? *ys[j] : make_uint4(0u, 0u, 0u, 0u);
+      }
       tc_wait_ld();
 #pragma unroll
       for (int j = 0; j < kEpiCols / 8; ++j) {
@@ -310,17 +338,35 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
             }
           }
         }
-        if (row_ok) {
-          *reinterpret_cast<float4*>(h_out + m * E + e + 8 * j) = make_float4(hn[0], hn[1], hn[2], hn[3]);
-          *reinterpret_cast<float4*>(h_out + m * E + e + 8 * j + 4) = make_float4(hn[4], hn[5], hn[6], hn[7]);
-          *reinterpret_cast<uint4*>(out + m * E + e + 8 * j) = make_uint4(op[0], op[1], op[2], op[3]);
-        }
+        *hs[2 * j] = make_float4(hn[0], hn[1], hn[2], hn[3]);
+        *hs[2 * j + 1] = make_float4(hn[4], hn[5], hn[6], hn[7]);
+        *ys[j] = make_uint4(op[0], op[1], op[2], op[3]);
       }
     }
   }
-
   tc_fence_before();
   __syncthreads();
+  cluster_arrive();                                // every slice sent to this CTA has arrived
+
+  // ---- out and the new state, in whole rows ---------------------------------------------------------
+#pragma unroll
+  for (int i = 0; i < kRowsM * 16 / kThreadsDec; ++i) {
+    const int r = (tid >> 4) + (kThreadsDec / 16) * i;
+    const int64_t m = row0 + r;
+    if (m < M)
+      *reinterpret_cast<uint4*>(h_out + m * E + chan0 + (tid & 15) * 4) =
+          *reinterpret_cast<const uint4*>(smem + kOffH + r * 256 + (((tid & 15) ^ (r & 7)) << 4));
+  }
+#pragma unroll
+  for (int i = 0; i < kRowsM * 8 / kThreadsDec; ++i) {
+    const int r = (tid >> 3) + (kThreadsDec / 8) * i;
+    const int64_t m = row0 + r;
+    if (m < M)
+      *reinterpret_cast<uint4*>(out + m * E + chan0 + (tid & 7) * 8) =
+          *reinterpret_cast<const uint4*>(smem + kOffY + r * 128 + (((tid & 7) ^ (r & 7)) << 4));
+  }
+  cluster_wait();                                  // and so has every slice it sent
+
   if (tid == 0 && *s_abort) atomicExch(&hdr->status, kStatusTimeout);
   if (warp == 0) {
     tc_fence_after();

@@ -63,12 +63,6 @@ constexpr int kWideS = 114 * 1024;
 static_assert(2 * (kWideS + 1024) > 233472, "two wide CTAs would fit an SM");
 static_assert(kWideS + kDataHalfS + kTailS + 2 * 1024 <= 233472, "wide and narrow do not fit an SM");
 
-// Shared memory of this CTA -> shared memory of a peer; completion on the peer's mbarrier.
-__device__ __forceinline__ void bulk_to_peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      :: "r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
 __device__ __forceinline__ void tensor_prefetch_l2(const CUtensorMap* map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
                :: "l"(map), "r"(x), "r"(y) : "memory");
