@@ -161,6 +161,20 @@ __global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepArgs a) {
     if (a.rotate) {
       const float p = a.pos64 ? (float)reinterpret_cast<const long long*>(a.pos)[row]
                               : (float)reinterpret_cast<const int*>(a.pos)[row];
+      // five heads of the row at a time, the first ones on their way while sine and cosine are computed
+      constexpr int kHeads = 5;
+      uint4* qr = reinterpret_cast<uint4*>(a.q + row * a.N * 256);
+      uint4 qa[kHeads], qb[kHeads];
+      auto load_heads = [&](int h0) {
+#pragma unroll
+        for (int h = 0; h < kHeads; ++h) {
+          if (h0 + h < a.N) {
+            qa[h] = qr[(h0 + h) * 32 + part];
+            qb[h] = qr[(h0 + h) * 32 + 8 + part];
+          }
+        }
+      };
+      load_heads(0);
       uint32_t cs[4], sn[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -181,23 +195,16 @@ __global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepArgs a) {
         rotate2(x.z, y.z, cs[2], sn[2]);
         rotate2(x.w, y.w, cs[3], sn[3]);
       };
-      uint4* qr = reinterpret_cast<uint4*>(a.q + row * a.N * 256);
-      int h = 0;
-      for (; h + 2 <= a.N; h += 2) {
-        uint4 x0 = qr[h * 32 + part], y0 = qr[h * 32 + 8 + part];
-        uint4 x1 = qr[h * 32 + 32 + part], y1 = qr[h * 32 + 40 + part];
-        rotate(x0, y0);
-        rotate(x1, y1);
-        qr[h * 32 + part] = x0;
-        qr[h * 32 + 8 + part] = y0;
-        qr[h * 32 + 32 + part] = x1;
-        qr[h * 32 + 40 + part] = y1;
-      }
-      if (h < a.N) {
-        uint4 x0 = qr[h * 32 + part], y0 = qr[h * 32 + 8 + part];
-        rotate(x0, y0);
-        qr[h * 32 + part] = x0;
-        qr[h * 32 + 8 + part] = y0;
+      for (int h0 = 0; h0 < a.N; h0 += kHeads) {
+        if (h0 > 0) load_heads(h0);
+#pragma unroll
+        for (int h = 0; h < kHeads; ++h) {
+          if (h0 + h < a.N) {
+            rotate(qa[h], qb[h]);
+            qr[(h0 + h) * 32 + part] = qa[h];
+            qr[(h0 + h) * 32 + 8 + part] = qb[h];
+          }
+        }
       }
       rotate(k0, k1);
       kr[part] = k0;
@@ -305,7 +312,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q_tiles = (T_ + kTq - 1) / kTq;
-  const int n_my = (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  // whole rounds, and whether this CTA has a unit in the last one
+  const int rounds = n_units / (int)gridDim.x, rest = n_units - rounds * (int)gridDim.x;
+  const int last = (rounds & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+  const int n_my = rounds + (last < rest ? 1 : 0);
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
@@ -337,7 +347,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   // unit -> (sequence, head, query tile); the key tiles it needs
   auto unit_of = [&](int i, int& b, int& n, int& t0, int& j_lo, int& j_hi) {
-    const int u = blockIdx.x + i * gridDim.x;
+    // (back and forth over the CTAs, so that whoever took the longest of a round takes the shortest of
+    // the next)
+    const int u = i * gridDim.x + ((i & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     const int qt = q_tiles - 1 - u / (B * N), bn = u % (B * N);   // longest first
     n = bn % N;
     b = bn / N;
