@@ -11,15 +11,19 @@
 // K-slice, by the warps that later run the epilogue (hi written back over the slice the copy engine
 // delivered, lo beside it); the weights are split by a packing kernel into two K-major arrays.
 //
-// One CTA per (128-token tile, head, channel half): N = 256 accumulator columns = the 128 x-gate and
-// the 128 a-gate outputs of the half's channels, so that an epilogue thread finds both gates of a
-// channel in its own TMEM lane.  K = 256 arrives in sixteen slices of 16 (64-byte rows, 64-byte
-// swizzle) through a four-stage ring: activations 8 KiB, their low part 8 KiB (written by the
-// helper warps), weights hi and lo 16 KiB each - the per-slice hand-offs (copy engine -> split ->
-// tensor core -> release) of a CTA are serial, so more and smaller stages in flight hide them.  A single thread issues three
-// tcgen05.mma.cta_group::1.kind::tf32 (M 128, N 256, K 8) per K step.  The epilogue (16 warps: TMEM
-// lane quarter x 32-channel chunk) reads the accumulators, applies the float32-accurate gate
-// arithmetic and writes a and the normalised input for the scan kernel.
+// A CTA takes 128 tokens x kTN accumulator columns: the x-gate and the a-gate outputs of kTN / 2
+// channels, so that an epilogue thread finds both gates of a channel in its own TMEM lane.  K = 256
+// arrives in sixteen slices of 16 (64-byte rows, 64-byte swizzle) through a ring: activations 8 KiB, their
+// low part 8 KiB (written by the helper warps), weights hi and lo 16 KiB each (kTN = 256) - the
+// per-slice hand-offs (copy engine -> split -> tensor core -> release) of a CTA are serial, so more and
+// smaller stages in flight hide them.  A single thread issues three tcgen05.mma.cta_group::1.kind::tf32
+// (M 128, N kTN, K 8) per K step.  The epilogue (TMEM lane quarter x 32-channel chunks per warp) reads the
+// accumulators, applies the float32-accurate gate arithmetic and writes a and the normalised input for
+// the scan kernel.
+//
+// A tile costs some 640 KB of fetches, 6 us of contraction and 8 us of arithmetic (a hundred instructions
+// an element); with several tiles per SM two CTAs share it and overlap them (launch_gates_tf32).  (A
+// persistent form on pairs of CTAs, with warps of its own for the split, was slower: 1 us per slice.)
 //
 // Every mbarrier wait is bounded; on expiry WsHeader::status is raised and the CTA leaves.
 #include <cuda.h>
@@ -33,33 +37,31 @@ namespace {
 
 constexpr int kHW = 256;                 // head width = K
 constexpr int kTM = 128;                 // tokens per tile (MMA M)
-constexpr int kTN = 256;                 // accumulator columns: 128 x-gate + 128 a-gate
-constexpr int kHalf = 128;               // channels per CTA
-constexpr int kKS = 16;                  // K per slice: 16 float32 = 64 bytes (64-byte swizzle); 32 also works
+constexpr int kHalf = 128;               // channels of a group of packed weights (256 rows: both gates)
+constexpr int kKS = 16;                  // K per slice: 16 float32 = 64 bytes (64-byte swizzle)
 constexpr int kSlices = kHW / kKS;
-constexpr int kStages = 64 / kKS;        // 4 stages of 48 KiB, or 2 of 96 KiB
 constexpr int kABytes = kTM * kKS * 4;
-constexpr int kBBytes = kTN * kKS * 4;
-constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;     // A, A_lo, B_hi, B_lo
-constexpr bool kSw128 = kKS == 32;
-__device__ __forceinline__ uint64_t tf32_desc(uint32_t addr) {
-  return kSw128 ? smem_desc_sw128(addr) : smem_desc_sw64(addr);
-}
-constexpr int kEpi = 16;
-constexpr int kThreadsF = (kEpi + 2) * 32;
-constexpr int kOffSp = kStages * kStageBytes;               // float [3][128]: softplus(a_param), gate biases
-constexpr int kOffBarF = kOffSp + 3 * kHalf * 4;                // full[2] lo_full[2] empty[2] acc_full
-constexpr int kNumBarF = 3 * kStages + 1;
-constexpr int kOffTmemF = kOffBarF + kNumBarF * 8;
-constexpr int kOffAbortF = kOffTmemF + 4;
-constexpr int kSmemF = kOffAbortF + 4 + 1024;
-static_assert(kSmemF <= 232448, "exceeds the 227 KiB of shared memory a CTA may use");
+// kTN = 256 or 128 accumulator columns: both gates of kTN / 2 channels; kPerSm CTAs share an SM
+template <int kTN, int kPerSm>
+struct Cfg {
+  static constexpr int kEpi = kPerSm == 1 ? 16 : 8;
+  static constexpr int kThreads = (kEpi + 2) * 32;
+  static constexpr int kStages = kPerSm == 1 ? 4 : (kTN == 256 ? 2 : 3);
+  static constexpr int kBBytes = kTN * kKS * 4;
+  static constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;     // A, A_lo, B_hi, B_lo
+  static constexpr int kOffSp = kStages * kStageBytes;              // float [3][kTN / 2]: softplus(a_param), gate biases
+  static constexpr int kOffBar = kOffSp + 3 * (kTN / 2) * 4;        // full, lo_full, empty [stage], acc_full
+  static constexpr int kOffTmem = kOffBar + (3 * kStages + 1) * 8;
+  static constexpr int kOffAbort = kOffTmem + 4;
+  static constexpr int kSmem = kOffAbort + 4 + 1024;
+  static_assert(kPerSm * (kSmem + 1024) <= 233472, "too much shared memory");
+  static_assert(kEpi * 8192 <= kStages * kStageBytes, "the epilogue's blocks lie over the ring");
+};
 
 // Instruction descriptor of tcgen05.mma kind::tf32: D float32, A and B TF32, both K-major.
 constexpr uint32_t tc_idesc_tf32(int m, int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-constexpr uint32_t kIdescF = tc_idesc_tf32(kTM, kTN);
 
 __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate) {
@@ -76,28 +78,34 @@ __device__ __forceinline__ float tf32_high_part(float v) {
 }
 __device__ __forceinline__ float tf32_low_part(float v) { return v - tf32_high_part(v); }
 
-__global__ void __launch_bounds__(kThreadsF, 1)
+template <int kTN, int kPerSm>
+__global__ void __launch_bounds__((Cfg<kTN, kPerSm>::kThreads), kPerSm)
 gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wh,
                   const __grid_constant__ CUtensorMap map_wl, const float* __restrict__ x,
                   const void* __restrict__ pos, int pos64, const float* __restrict__ a_param,
                   const float* __restrict__ bias_x, const float* __restrict__ bias_a, int64_t M,
                   int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr) {
+  using C = Cfg<kTN, kPerSm>;
+  constexpr int kEpi = C::kEpi;
+  constexpr int kStages = C::kStages, kBBytes = C::kBBytes, kStageBytes = C::kStageBytes;
+  constexpr int kChans = kTN / 2;
+  constexpr uint32_t kIdescF = tc_idesc_tf32(kTM, kTN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t s_base = smem_u32(smem);
-  const uint32_t bar0 = s_base + kOffBarF;
+  const uint32_t bar0 = s_base + C::kOffBar;
   auto bar_full = [&](int s) { return bar0 + 8u * s; };
   auto bar_lo = [&](int s) { return bar0 + 8u * (kStages + s); };
   auto bar_empty = [&](int s) { return bar0 + 8u * (2 * kStages + s); };
   const uint32_t bar_acc = bar0 + 8u * (3 * kStages);
-  float* s_sp = reinterpret_cast<float*>(smem + kOffSp);
-  volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmemF);
-  volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbortF);
+  float* s_sp = reinterpret_cast<float*>(smem + C::kOffSp);
+  volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + C::kOffTmem);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(smem + C::kOffAbort);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, group = blockIdx.y;          // (head, half)
-  const int head = group >> 1, half = group & 1;
-  const int chan0 = head * kHW + half * kHalf;
+  const int n_tiles = E / kChans, tile = blockIdx.x / n_tiles, chan0 = (blockIdx.x - tile * n_tiles) * kChans;
+  const int head = chan0 / kHW;
+  const int wrow = chan0 / kHalf * (2 * kHalf) + chan0 % kHalf;      // packed rows: x-gate, kHalf behind a-gate
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
@@ -111,13 +119,14 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
   if (warp == kEpi + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 :: "r"(s_base + kOffTmemF), "r"(256) : "memory");
+                 :: "r"(s_base + C::kOffTmem), "r"(kTN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (threadIdx.x < kHalf) {
+  grid_dependency_wait();
+  if (threadIdx.x < kChans) {
     s_sp[threadIdx.x] = softplus_(a_param[chan0 + threadIdx.x]);
-    s_sp[kHalf + threadIdx.x] = bias_x[chan0 + threadIdx.x];
-    s_sp[2 * kHalf + threadIdx.x] = bias_a[chan0 + threadIdx.x];
+    s_sp[kChans + threadIdx.x] = bias_x[chan0 + threadIdx.x];
+    s_sp[2 * kChans + threadIdx.x] = bias_a[chan0 + threadIdx.x];
   }
   tc_fence_before();
   __syncthreads();
@@ -135,8 +144,12 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const uint32_t st = s_base + s * kStageBytes;
         mbar_expect_tx(bar_full(s), kABytes + 2 * kBBytes);
         tma_load_2d(st, &map_x, head * kHW + kb * kKS, tile * kTM, bar_full(s));
-        tma_load_2d(st + 2 * kABytes, &map_wh, kb * kKS, group * kTN, bar_full(s));
-        tma_load_2d(st + 2 * kABytes + kBBytes, &map_wl, kb * kKS, group * kTN, bar_full(s));
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {                      // x-gate rows, a-gate rows
+          const uint32_t w = st + 2 * kABytes + g * (kBBytes / 2);
+          tma_load_2d(w, &map_wh, kb * kKS, wrow + g * kHalf, bar_full(s));
+          tma_load_2d(w + kBBytes, &map_wl, kb * kKS, wrow + g * kHalf, bar_full(s));
+        }
       }
     }
   } else if (warp == kEpi + 1) {
@@ -153,8 +166,8 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const uint32_t b_hi = a_hi + 2 * kABytes, b_lo = b_hi + kBBytes;
 #pragma unroll
         for (int ks = 0; ks < kKS / 8; ++ks) {
-          const uint64_t dah = tf32_desc(a_hi + ks * 32), dal = tf32_desc(a_lo + ks * 32);
-          const uint64_t dbh = tf32_desc(b_hi + ks * 32), dbl = tf32_desc(b_lo + ks * 32);
+          const uint64_t dah = smem_desc_sw64(a_hi + ks * 32), dal = smem_desc_sw64(a_lo + ks * 32);
+          const uint64_t dbh = smem_desc_sw64(b_hi + ks * 32), dbl = smem_desc_sw64(b_lo + ks * 32);
           tc_mma_tf32(tmem_base, dah, dbh, kIdescF, (kb | ks) != 0 ? 1u : 0u);
           tc_mma_tf32(tmem_base, dal, dbh, kIdescF, 1u);
           tc_mma_tf32(tmem_base, dah, dbl, kIdescF, 1u);
@@ -195,67 +208,72 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // bytes: 16-byte piece j of row r sits at piece j ^ (r & 7), conflict-free both for the row
     // owner (lane = row) and for the copy pattern (8 lanes per row).
     const int lane_base = (warp & 3) * 32;
-    const int cq = warp >> 2;                                // 32-channel chunk of the half
     const int64_t row0 = (int64_t)tile * kTM + lane_base;
     const int64_t row = row0 + lane;
     const bool is_reset = row < M && pos_is_zero(pos, pos64, row);
-    const int e0 = chan0 + cq * 32;
     uint8_t* blk_a = smem + warp * 8192;                     // conv values in, a out
     uint8_t* blk_x = blk_a + 4096;                           // normalised input out
     const int cr = lane >> 3, cp = lane & 7;                 // copy pattern: row cr + 4 k, piece cp
-    // the conv values of the warp's block are asked for while the last MMAs run
-    float4 cin[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int r = cr + 4 * k;
-      cin[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row0 + r < M) cin[k] = __ldg(reinterpret_cast<const float4*>(x + (row0 + r) * E + e0 + cp * 4));
-    }
-    if (ok) ok = mbar_wait(bar_acc, 0, s_abort);             // every MMA has read the ring by now
-    tc_fence_after();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int r = cr + 4 * k;
-      *reinterpret_cast<float4*>(blk_a + r * 128 + ((cp ^ (r & 7)) << 4)) = cin[k];
-    }
-    __syncwarp();
-    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + cq * 32;
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      uint32_t zx[16], za[16];
-      tc_ld_32x16(t_row + cc * 16, zx);
-      tc_ld_32x16(t_row + kHalf + cc * 16, za);
-      tc_wait_ld();
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int piece = (cc * 4 + q) ^ (lane & 7);
-        const float4 cv = *reinterpret_cast<const float4*>(blk_a + lane * 128 + (piece << 4));
-        const float cvv[4] = {cv.x, cv.y, cv.z, cv.w};
-        float av[4], xv[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = q * 4 + j;
-          const int ch = cq * 32 + cc * 16 + n;            // channel within the half
-          gate_math<false, true>(cvv[j], __uint_as_float(zx[n]), __uint_as_float(za[n]), s_sp[kHalf + ch],
-                           s_sp[2 * kHalf + ch], s_sp[ch], is_reset, av[j], xv[j]);
-        }
-        *reinterpret_cast<float4*>(blk_a + lane * 128 + (piece << 4)) = make_float4(av[0], av[1], av[2], av[3]);
-        *reinterpret_cast<float4*>(blk_x + lane * 128 + (piece << 4)) = make_float4(xv[0], xv[1], xv[2], xv[3]);
-      }
-    }
-    __syncwarp();
-    if (ok) {
+    // (a warp takes the 32-channel chunks warp / 4 and, with eight warps, every second behind it)
+#pragma unroll 1
+    for (int cq = warp >> 2; cq < kChans / 32; cq += kEpi / 4) {
+      const int e0 = chan0 + cq * 32;
+      // the conv values of the warp's block are asked for while the last MMAs run
+      float4 cin[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int r = cr + 4 * k;
-        if (row0 + r < M) {
-          const int off = r * 128 + ((cp ^ (r & 7)) << 4);
-          *reinterpret_cast<float4*>(a_out + (row0 + r) * E + e0 + cp * 4) =
-              *reinterpret_cast<const float4*>(blk_a + off);
-          *reinterpret_cast<float4*>(xn_out + (row0 + r) * E + e0 + cp * 4) =
-              *reinterpret_cast<const float4*>(blk_x + off);
+        cin[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + r < M) cin[k] = __ldg(reinterpret_cast<const float4*>(x + (row0 + r) * E + e0 + cp * 4));
+      }
+      if (ok) ok = mbar_wait(bar_acc, 0, s_abort);             // every MMA has read the ring by now
+      __syncwarp();
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = cr + 4 * k;
+        *reinterpret_cast<float4*>(blk_a + r * 128 + ((cp ^ (r & 7)) << 4)) = cin[k];
+      }
+      __syncwarp();
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + cq * 32;
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t zx[16], za[16];
+        tc_ld_32x16(t_row + cc * 16, zx);
+        tc_ld_32x16(t_row + kChans + cc * 16, za);
+        tc_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int piece = (cc * 4 + q) ^ (lane & 7);
+          const float4 cv = *reinterpret_cast<const float4*>(blk_a + lane * 128 + (piece << 4));
+          const float cvv[4] = {cv.x, cv.y, cv.z, cv.w};
+          float av[4], xv[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int n = q * 4 + j;
+            const int ch = cq * 32 + cc * 16 + n;            // channel within the tile
+            gate_math<false, true>(cvv[j], __uint_as_float(zx[n]), __uint_as_float(za[n]), s_sp[kChans + ch],
+                             s_sp[2 * kChans + ch], s_sp[ch], is_reset, av[j], xv[j]);
+          }
+          *reinterpret_cast<float4*>(blk_a + lane * 128 + (piece << 4)) = make_float4(av[0], av[1], av[2], av[3]);
+          *reinterpret_cast<float4*>(blk_x + lane * 128 + (piece << 4)) = make_float4(xv[0], xv[1], xv[2], xv[3]);
         }
       }
+      __syncwarp();
+      if (ok) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = cr + 4 * k;
+          if (row0 + r < M) {
+            const int off = r * 128 + ((cp ^ (r & 7)) << 4);
+            *reinterpret_cast<float4*>(a_out + (row0 + r) * E + e0 + cp * 4) =
+                *reinterpret_cast<const float4*>(blk_a + off);
+            *reinterpret_cast<float4*>(xn_out + (row0 + r) * E + e0 + cp * 4) =
+                *reinterpret_cast<const float4*>(blk_x + off);
+          }
+        }
+      }
+      __syncwarp();
     }
   }
 
@@ -265,9 +283,31 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   if (threadIdx.x == 0 && *s_abort) atomicExch(&hdr->status, kStatusTimeout);
   if (warp == kEpi + 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(256)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(kTN)
                  : "memory");
   }
+}
+
+template <int kTN, int kPerSm>
+cudaError_t set_smem() {
+  return cudaFuncSetAttribute(gates_tf32_kernel<kTN, kPerSm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              Cfg<kTN, kPerSm>::kSmem);
+}
+
+template <int kTN, int kPerSm>
+cudaError_t launch_gates_t(const float* c, const void* pos, int pos64, const float* a_param, const float* bx,
+                           const float* ba, int64_t M, int E, const float* hi, const float* lo, float* a_out,
+                           float* xn_out, WsHeader* hdr, cudaStream_t s) {
+  const uint64_t w_rows = (uint64_t)E / kHalf * (2 * kHalf);
+  CUtensorMap map_x, map_wh, map_wl;
+  if (!tensor_map_2d(&map_x, c, (uint64_t)M, (uint64_t)E, kTM, kKS, false, 4, true) ||
+      !tensor_map_2d(&map_wh, hi, w_rows, kHW, kTN / 2, kKS, false, 4, true) ||
+      !tensor_map_2d(&map_wl, lo, w_rows, kHW, kTN / 2, kKS, false, 4, true))
+    return cudaErrorInvalidValue;
+  const int64_t tiles = (M + kTM - 1) / kTM * (E / (kTN / 2));
+  return launch_dependent(gates_tf32_kernel<kTN, kPerSm>, dim3((unsigned)tiles), dim3(Cfg<kTN, kPerSm>::kThreads),
+                          (size_t)Cfg<kTN, kPerSm>::kSmem, s, map_x, map_wh, map_wl, c, pos, pos64, a_param, bx, ba,
+                          M, E, a_out, xn_out, hdr);
 }
 
 // Splits the two gate weights [H, 256 (k), 256 (n)] float32 into K-major groups
@@ -283,7 +323,7 @@ __global__ void pack_gate_weights_tf32_kernel(const float* __restrict__ wx, cons
   for (int r = threadIdx.y; r < 32; r += 8)                        // r walks k, x walks n
     tile[r][threadIdx.x] = src[(int64_t)(k0 + r) * kHW + chan + threadIdx.x];
   __syncthreads();
-  const int64_t base = (int64_t)group * kTN * kHW;
+  const int64_t base = (int64_t)group * 2 * kHalf * kHW;
   for (int r = threadIdx.y; r < 32; r += 8) {                      // r walks n', x walks k
     const float v = tile[threadIdx.x][r];
     const float h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
@@ -294,7 +334,7 @@ __global__ void pack_gate_weights_tf32_kernel(const float* __restrict__ wx, cons
 
 }  // namespace
 
-size_t gates_tf32_packed_bytes(int H) { return (size_t)H * 2 * kTN * kHW * 4 * 2; }
+size_t gates_tf32_packed_bytes(int H) { return (size_t)H * 2 * 2 * kHalf * kHW * 4 * 2; }
 
 bool gates_tf32_supported(int dtype, int bw, int64_t M) {
   return dtype == 0 && bw == kHW && M >= 1 && M < ((int64_t)1 << 31);
@@ -303,8 +343,8 @@ bool gates_tf32_supported(int dtype, int bw, int64_t M) {
 cudaError_t launch_pack_gate_weights_tf32(const void* wx, const void* wa, int H, void* packed_w,
                                           cudaStream_t s) {
   float* hi = static_cast<float*>(packed_w);
-  float* lo = hi + (size_t)H * 2 * kTN * kHW;
-  pack_gate_weights_tf32_kernel<<<dim3(kHW / 32, kTN / 32, 2 * H), dim3(32, 8), 0, s>>>(
+  float* lo = hi + (size_t)H * 2 * 2 * kHalf * kHW;
+  pack_gate_weights_tf32_kernel<<<dim3(kHW / 32, 2 * kHalf / 32, 2 * H), dim3(32, 8), 0, s>>>(
       (const float*)wx, (const float*)wa, H, hi, lo);
   return cudaGetLastError();
 }
@@ -316,27 +356,29 @@ cudaError_t launch_gates_tf32(const void* c, const void* pos, int pos64, const v
   if (M == 0) return cudaSuccess;
   const int E = H * kHW;
   float* hi = static_cast<float*>(packed_w);
-  float* lo = hi + (size_t)H * 2 * kTN * kHW;
+  float* lo = hi + (size_t)H * 2 * 2 * kHalf * kHW;
   if (!packed_valid) {
     cudaError_t err = launch_pack_gate_weights_tf32(wx, wa, H, packed_w, s);
     if (err != cudaSuccess) return err;
   }
 
-  CUtensorMap map_x, map_wh, map_wl;
-  if (!tensor_map_2d(&map_x, c, (uint64_t)M, (uint64_t)E, kTM, kKS, kSw128, 4, !kSw128) ||
-      !tensor_map_2d(&map_wh, hi, (uint64_t)H * 2 * kTN, kHW, kTN, kKS, kSw128, 4, !kSw128) ||
-      !tensor_map_2d(&map_wl, lo, (uint64_t)H * 2 * kTN, kHW, kTN, kKS, kSw128, 4, !kSw128))
-    return cudaErrorInvalidValue;
   static PerDeviceOnce once;
+  int num_sms = 0;
   cudaError_t e0 = once.run([] {
-    return cudaFuncSetAttribute(gates_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF);
-  });
+    cudaError_t e = set_smem<256, 1>();
+    if (e == cudaSuccess) e = set_smem<256, 2>();
+    if (e == cudaSuccess) e = set_smem<128, 2>();
+    return e;
+  }, &num_sms);
   if (e0 != cudaSuccess) return e0;
-  const dim3 grid((unsigned)((M + kTM - 1) / kTM), (unsigned)(2 * H));
-  gates_tf32_kernel<<<grid, kThreadsF, kSmemF, s>>>(
-      map_x, map_wh, map_wl, (const float*)c, pos, pos64, (const float*)a_param, (const float*)bx,
-      (const float*)ba, M, E, (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header));
-  return cudaGetLastError();
+  // One tile an SM as long as there are no more: 700 tokens of 2560 channels 34 us, as two CTAs an SM 39.
+  // From there on two an SM, so that one's arithmetic runs under the other's contraction: 32768 tokens
+  // 829 -> 737 us with the scan behind.  Few tiles are cut in half: 200 tokens 29 -> 25 us.
+  const int64_t m_tiles = (M + kTM - 1) / kTM, tiles = m_tiles * (E / kHalf);
+  if (2 * tiles > 0x7fffffff) return cudaErrorInvalidValue;
+  auto launch = tiles > num_sms ? launch_gates_t<256, 2> : (2 * tiles > num_sms ? launch_gates_t<256, 1> : launch_gates_t<128, 2>);
+  return launch((const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba, M, E, hi, lo,
+                (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header), s);
 }
 
 }  // namespace rgk
