@@ -102,7 +102,7 @@ int check_params(const rgk_params* p, bool need_conv) {
 // Gate projections + gate arithmetic with the kernel `gates_impl` selects.
 int run_gates(const void* c, const void* pos, int pos64, const rgk_params* p, int64_t M, int H,
               int bw, int dtype, int gates_impl, void* wpack, void* a, void* xn, void* ws_header,
-              cudaStream_t s) {
+              cudaStream_t s, const rgk::ScanPrep& prep = rgk::ScanPrep()) {
   const bool tc_ok = rgk::gates_tc_supported(dtype, bw, M);
   const bool tf32_ok = rgk::gates_tf32_supported(dtype, bw, M);
   if (gates_impl == RGK_GATES_TCGEN05 && !tc_ok && !tf32_ok)
@@ -112,7 +112,7 @@ int run_gates(const void* c, const void* pos, int pos64, const rgk_params* p, in
     cudaError_t e = rgk::launch_gates_tf32(c, pos, pos64, p->a_param, p->gate_x_w, p->gate_x_b,
                                            p->gate_a_w, p->gate_a_b, M, H,
                                            p->gates_packed ? const_cast<void*>(p->gates_packed) : wpack,
-                                           p->gates_packed != nullptr, a, xn, ws_header, s);
+                                           p->gates_packed != nullptr, a, xn, ws_header, s, prep);
     if (e != cudaSuccess) return cuda_fail(e, "tcgen05 TF32 gates launch");
     return RGK_OK;
   }
@@ -177,12 +177,14 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
     if (e != cudaSuccess) return cuda_fail(e, "fused RG-LRU launch");
     return RGK_OK;
   }
-  int rc = run_gates(c, pos, pos64, p, B * T, H, bw, dtype,
-                     want_fused ? RGK_GATES_AUTO : gates_impl, wpack, a_buf,
-                     xn_buf, scan_ws, s);
+  // the float32 gate kernel clears what the scan wants cleared
+  const int impl = want_fused ? RGK_GATES_AUTO : gates_impl;
+  const bool prepared = rgk::gates_tf32_supported(dtype, bw, B * T) && impl != RGK_GATES_SIMT;
+  int rc = run_gates(c, pos, pos64, p, B * T, H, bw, dtype, impl, wpack, a_buf, xn_buf, scan_ws, s,
+                     prepared ? rgk::scan_prep(scan_ws, B, T, E, dtype) : rgk::ScanPrep());
   if (rc) return rc;
   cudaError_t e = rgk::launch_scan(xn_buf, a_buf, nullptr, nullptr, 0, h0, yb, y_activated, B, T, E,
-                                   dtype, out, h_last, scan_ws, s);
+                                   dtype, out, h_last, scan_ws, s, 0, 0, prepared);
   if (e != cudaSuccess) return cuda_fail(e, "scan launch");
   return RGK_OK;
 }

@@ -84,7 +84,7 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                   const __grid_constant__ CUtensorMap map_wl, const float* __restrict__ x,
                   const void* __restrict__ pos, int pos64, const float* __restrict__ a_param,
                   const float* __restrict__ bias_x, const float* __restrict__ bias_a, int64_t M,
-                  int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr) {
+                  int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr, const ScanPrep prep) {
   using C = Cfg<kTN, kPerSm>;
   constexpr int kEpi = C::kEpi;
   constexpr int kStages = C::kStages, kBBytes = C::kBBytes, kStageBytes = C::kStageBytes;
@@ -123,6 +123,12 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   grid_dependency_wait();
+  if (prep.ticket != nullptr) {                              // for the scan kernel behind
+    if (blockIdx.x == 0 && threadIdx.x == 0) *prep.ticket = 0u;
+    for (int64_t i = (int64_t)blockIdx.x * C::kThreads + threadIdx.x; i < prep.n_zero;
+         i += (int64_t)gridDim.x * C::kThreads)
+      prep.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
   if (threadIdx.x < kChans) {
     s_sp[threadIdx.x] = softplus_(a_param[chan0 + threadIdx.x]);
     s_sp[kChans + threadIdx.x] = bias_x[chan0 + threadIdx.x];
@@ -297,7 +303,7 @@ cudaError_t set_smem() {
 template <int kTN, int kPerSm>
 cudaError_t launch_gates_t(const float* c, const void* pos, int pos64, const float* a_param, const float* bx,
                            const float* ba, int64_t M, int E, const float* hi, const float* lo, float* a_out,
-                           float* xn_out, WsHeader* hdr, cudaStream_t s) {
+                           float* xn_out, WsHeader* hdr, cudaStream_t s, const ScanPrep& prep) {
   const uint64_t w_rows = (uint64_t)E / kHalf * (2 * kHalf);
   CUtensorMap map_x, map_wh, map_wl;
   if (!tensor_map_2d(&map_x, c, (uint64_t)M, (uint64_t)E, kTM, kKS, false, 4, true) ||
@@ -307,7 +313,7 @@ cudaError_t launch_gates_t(const float* c, const void* pos, int pos64, const flo
   const int64_t tiles = (M + kTM - 1) / kTM * (E / (kTN / 2));
   return launch_dependent(gates_tf32_kernel<kTN, kPerSm>, dim3((unsigned)tiles), dim3(Cfg<kTN, kPerSm>::kThreads),
                           (size_t)Cfg<kTN, kPerSm>::kSmem, s, map_x, map_wh, map_wl, c, pos, pos64, a_param, bx, ba,
-                          M, E, a_out, xn_out, hdr);
+                          M, E, a_out, xn_out, hdr, prep);
 }
 
 // Splits the two gate weights [H, 256 (k), 256 (n)] float32 into K-major groups
@@ -352,7 +358,7 @@ cudaError_t launch_pack_gate_weights_tf32(const void* wx, const void* wa, int H,
 cudaError_t launch_gates_tf32(const void* c, const void* pos, int pos64, const void* a_param,
                               const void* wx, const void* bx, const void* wa, const void* ba,
                               int64_t M, int H, void* packed_w, bool packed_valid, void* a_out,
-                              void* xn_out, void* ws_header, cudaStream_t s) {
+                              void* xn_out, void* ws_header, cudaStream_t s, const ScanPrep& prep) {
   if (M == 0) return cudaSuccess;
   const int E = H * kHW;
   float* hi = static_cast<float*>(packed_w);
@@ -378,7 +384,7 @@ cudaError_t launch_gates_tf32(const void* c, const void* pos, int pos64, const v
   if (2 * tiles > 0x7fffffff) return cudaErrorInvalidValue;
   auto launch = tiles > num_sms ? launch_gates_t<256, 2> : (2 * tiles > num_sms ? launch_gates_t<256, 1> : launch_gates_t<128, 2>);
   return launch((const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba, M, E, hi, lo,
-                (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header), s);
+                (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header), s, prep);
 }
 
 }  // namespace rgk

@@ -70,6 +70,14 @@ struct ChanPrep {
   int E = 0;
 };
 
+// What scan_kernel finds cleared: its ticket and its flags.  The gate kernel in front does it on the side
+// (launch_gates_tf32), or a memset.
+struct ScanPrep {
+  unsigned* ticket = nullptr;
+  uint4* zero = nullptr;
+  int64_t n_zero = 0;                    // in packs of 16 bytes
+};
+
 // The share of an SM's 228 KB that a launch asks to be shared memory rather than L1, for kernels that
 // stream through L1: without it they inherit whatever the kernel in front left, and behind one that used
 // all of it the projections of one row took 26 us instead of 11.5 (28 KB of L1 for 120 KB of loads in
@@ -136,7 +144,7 @@ cudaError_t launch_pack_gate_weights_tf32(const void* wx, const void* wa, int H,
 cudaError_t launch_gates_tf32(const void* c, const void* pos, int pos64, const void* a_param,
                               const void* wx, const void* bx, const void* wa, const void* ba,
                               int64_t M, int H, void* packed_w, bool packed_valid, void* a_out, void* xn_out,
-                              void* ws_header, cudaStream_t s);
+                              void* ws_header, cudaStream_t s, const ScanPrep& prep = ScanPrep());
 
 // Packs the gate weights only (the first step of launch_gates_tc), for callers that keep the
 // packed copy across calls; launch_gates_tc with packed_ready != 0 then skips its own packing.
@@ -273,10 +281,13 @@ size_t scan_workspace_bytes(int64_t B, int64_t T, int64_t E, int dtype);
 // y_mul (optional): the join y * gelu_tanh(y_mul), or y * y_mul when y_activated != 0 (the factor
 // was already passed through gelu by whoever produced it).  skip_time_tiles / spin_limit: only for
 // the wait-expiry self-test (rgk_selftest_wait_expiry); 0 = the whole problem, the default limit.
+// what the launch below clears first unless `prepared`
+ScanPrep scan_prep(void* ws, int64_t B, int64_t T, int64_t E, int dtype);
 cudaError_t launch_scan(const void* x, const void* a, const uint8_t* reset, const void* pos,
                         int pos64, const float* h0, const void* y_mul, int y_activated, int64_t B,
                         int64_t T, int64_t E, int dtype, void* y, float* h_last, void* ws,
-                        cudaStream_t s, int skip_time_tiles = 0, unsigned spin_limit = 0);
+                        cudaStream_t s, int skip_time_tiles = 0, unsigned spin_limit = 0,
+                        bool prepared = false);
 
 // The scan's built-in scratch (a __device__ array inside scan.cu): its size, and its address on the
 // current device (looked up with cudaGetSymbolAddress on first use per device).

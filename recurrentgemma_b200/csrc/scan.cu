@@ -123,6 +123,7 @@ scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
   const uint32_t bar = smem_u32(smem + Sm::kOffBar);
 
   const int tid = threadIdx.x;
+  grid_dependency_wait();
   if (tid == 0) {
     s_misc[0] = atomicAdd(&hdr->ticket, 1u) + ticket_base;
     mbar_init(bar, 1);
@@ -404,10 +405,9 @@ cudaError_t launch_scan_typed(const void* x, const void* a, const uint8_t* reset
                                 ScanSmem<T>::kBytes);
   });
   if (e != cudaSuccess) return e;
-  scan_kernel<T, kJoin><<<grid, kThreads, ScanSmem<T>::kBytes, s>>>(
-      map_x, map_a, reset, pos, pos64, h0, (const T*)y_mul, (int)B, (int)T_, (int)E, tiles_t, groups,
-      (T*)y, h_last, hdr, flags, agg, incl, ticket_base, spin_limit);
-  return cudaGetLastError();
+  return launch_dependent(scan_kernel<T, kJoin>, dim3(grid), dim3(kThreads), (size_t)ScanSmem<T>::kBytes, s, map_x,
+                          map_a, reset, pos, pos64, h0, (const T*)y_mul, (int)B, (int)T_, (int)E, tiles_t, groups,
+                          (T*)y, h_last, hdr, flags, agg, incl, ticket_base, spin_limit);
 }
 
 struct ScanLayout {
@@ -436,17 +436,29 @@ size_t scan_workspace_bytes(int64_t B, int64_t T, int64_t E, int dtype) {
   return scan_layout(B, T, E, dtype).total;
 }
 
+ScanPrep scan_prep(void* ws, int64_t B, int64_t T, int64_t E, int dtype) {
+  const ScanLayout L = scan_layout(B, T, E, dtype);
+  char* base = static_cast<char*>(ws);
+  ScanPrep p;
+  p.ticket = &reinterpret_cast<WsHeader*>(base)->ticket;
+  p.zero = reinterpret_cast<uint4*>(base + L.flags_off);
+  p.n_zero = (int64_t)((L.agg_off - L.flags_off) / 16);
+  return p;
+}
+
 cudaError_t launch_scan(const void* x, const void* a, const uint8_t* reset, const void* pos,
                         int pos64, const float* h0, const void* y_mul, int y_activated, int64_t B,
                         int64_t T, int64_t E, int dtype, void* y, float* h_last, void* ws,
-                        cudaStream_t s, int skip_time_tiles, unsigned spin_limit) {
+                        cudaStream_t s, int skip_time_tiles, unsigned spin_limit, bool prepared) {
   if (B == 0 || T == 0 || E == 0) return cudaSuccess;
   const ScanLayout L = scan_layout(B, T, E, dtype);
   char* base = static_cast<char*>(ws);
   // Ticket and flags start every launch at zero (the status word before them belongs to the
   // caller).
-  cudaError_t err = cudaMemsetAsync(base + sizeof(int), 0, L.agg_off - sizeof(int), s);
-  if (err != cudaSuccess) return err;
+  if (!prepared) {
+    const cudaError_t err = cudaMemsetAsync(base + sizeof(int), 0, L.agg_off - sizeof(int), s);
+    if (err != cudaSuccess) return err;
+  }
   WsHeader* hdr = reinterpret_cast<WsHeader*>(base);
   unsigned* flags = reinterpret_cast<unsigned*>(base + L.flags_off);
   float2* agg = reinterpret_cast<float2*>(base + L.agg_off);
