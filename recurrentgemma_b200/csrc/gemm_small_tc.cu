@@ -194,18 +194,23 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         tma_load_2d(s_base + i * stage_bytes + w_bytes, &map_x, (kb0 + i) * SK, row0, bar_full(i));
       }
-      bool ok = true;
-      int s = 0;
-      uint32_t phase = 0;                          // of the stage's previous contents
-      for (int i = pre; i < n_kb && ok; ++i) {
-        ok = mbar_wait(bar_empty(s), phase, s_abort);
-        if (!ok) break;
+    }
+    __syncwarp();
+    // the whole warp runs the loop and one elected lane issues (see mma_ring)
+    bool ok = true;
+    int s = 0;
+    uint32_t phase = 0;                            // of the stage's previous contents
+    for (int i = pre; i < n_kb; ++i) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_empty(s), phase, s_abort));
+      if (!ok) break;
+      if (elect_one()) {
         const uint32_t st = s_base + s * stage_bytes;
         mbar_expect_tx(bar_full(s), stage_bytes);
         tma_load_2d(st, map_w, (kb0 + i) * SK, f0, bar_full(s));
         tma_load_2d(st + w_bytes, &map_x, (kb0 + i) * SK, row0, bar_full(s));
-        if (++s == n_stages) { s = 0; phase ^= 1; }
       }
+      __syncwarp();
+      if (++s == n_stages) { s = 0; phase ^= 1; }
     }
     __syncwarp();
   } else if (warp == kEpiS + 1) {

@@ -31,7 +31,7 @@ constexpr int kABytes = BM * BK * 2;             // 16 KiB
 constexpr int kRingBytes = 192 * 1024;           // 6 stages of a 256-wide tile, 9 of a 64-wide one
 constexpr int kMaxStages = 9;
 constexpr int kEpi = 16;
-constexpr int kThreadsG = (kEpi + 2) * 32;
+constexpr int kThreadsG = (kEpi + 3) * 32;     // epilogue, two TMA producers around the MMA warp
 constexpr int kOffRing = 0;
 constexpr int kOffStageOut = kRingBytes;                         // per-warp 2 KiB staging
 constexpr int kOffBarG = kOffStageOut + kEpi * 2048;             // full[] empty[] acc_full[2] acc_empty[2]
@@ -118,32 +118,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   grid_dependency_wait();
   grid_launch_dependents();
 
-  if (warp == kEpi) {
-    // ------------------------------ TMA producer --------------------------------------------------
-    if (lane == 0) {
-      const uint32_t full0 = peer_smem(bar_full(0), 0);  // the loads of both CTAs report to the even one
-      int s = 0;
-      uint32_t phase = 1;
-      bool ok = true;
-      for (int t = 0; t < n_my && ok; ++t) {
-        int m0, n0;
-        tile_at(pair + t * pairs, m_tiles, n_tiles, group, &m0, &n0);
-        const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
-        const CUtensorMap* map_w = mi == 0 ? &map_w0 : (mi == 1 ? &map_w1 : &map_w2);
-        m0 = m0 * (2 * BM) + rank * BM;
-        n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn + rank * (bn / 2);
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          ok = mbar_wait(bar_empty(s), phase, s_abort);
+  if (warp == kEpi || warp == kEpi + 2) {
+    // ------------------------------ TMA producers -------------------------------------------------
+    // Two, for even and odd K blocks: a turn of this loop takes one 340 cycles, as long as the MMAs of a
+    // narrow tile's K blocks.  The whole warp runs it and one elected lane issues (see mma_ring).
+    const uint32_t full0 = peer_smem(bar_full(0), 0);  // the loads of both CTAs report to the even one
+    int kb = warp == kEpi ? 0 : 1, s = kb;
+    uint32_t phase = 1;
+    bool ok = true, ready = false;       // ready: the stage was already free when last asked
+    for (int t = 0; t < n_my && ok; ++t) {
+      int m0, n0;
+      tile_at(pair + t * pairs, m_tiles, n_tiles, group, &m0, &n0);
+      const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
+      const CUtensorMap* map_w = mi == 0 ? &map_w0 : (mi == 1 ? &map_w1 : &map_w2);
+      m0 = m0 * (2 * BM) + rank * BM;
+      n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn + rank * (bn / 2);
+      for (; kb < k_blocks; kb += 2) {
+        if (!ready) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_empty(s), phase, s_abort));
           if (!ok) break;
+        }
+        int next = s + 2;
+        uint32_t next_phase = phase;
+        if (next >= n_stages) { next -= n_stages; next_phase ^= 1; }
+        const bool free_next = mbar_test(bar_empty(next), next_phase);   // looked at behind the loads
+        if (elect_one()) {
           if (rank == 0) mbar_expect_tx(bar_full(s), 2 * stage_bytes);
           const uint32_t st = s_base + kOffRing + s * stage_bytes;
           tma_load_2d_pair(st, &map_x, kb * BK, m0, full0 + 8u * s);
           tma_load_2d_pair(st + kABytes, map_w, kb * BK, n0, full0 + 8u * s);
-          if (++s == n_stages) { s = 0; phase ^= 1; }
         }
+        __syncwarp();
+        ready = __all_sync(0xffffffffu, free_next);
+        s = next;
+        phase = next_phase;
       }
+      kb -= k_blocks;
     }
-    __syncwarp();
   } else if (warp == kEpi + 1) {
     // ------------------------------ MMA issue: the even CTA for both -------------------------------
     if (rank == 0) {

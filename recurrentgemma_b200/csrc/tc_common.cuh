@@ -140,54 +140,70 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
   return d;
 }
 
-// The loop of the warp that issues the MMAs of one accumulator over a TMA ring: for each of n_kb
-// stages wait, issue kSteps instructions of K 16, release the stage.  The whole warp runs it and one
-// elected lane issues: with the loop under `if (lane == 0)` the compiler keeps descriptors and
-// addresses in per-thread registers and a stage of four instructions took 600 cycles whatever its
-// size, more than four instructions of N = 256 execute in.  The barrier of the next stage is asked about
-// before this stage's instructions are issued.  desc_a, desc_b: descriptors of stage 0; `step`:
-// descriptor distance of two stages (bytes / 16).  Returns false if a wait gave up.
-struct RingPos {
-  int stage = 0;
-  uint32_t phase = 0;
-  bool ready = false;                              // the stage was already full when last asked
-};
-template <int kSteps, int kCtas = 1>
-__device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
-                                         uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
-                                         uint32_t bar_empty0, RingPos& at, volatile int* abort_flag);
-
 // Instruction descriptor of tcgen05.mma kind::f16: D float32, A and B bfloat16, both K-major.
 constexpr uint32_t tc_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-template <int kSteps, int kCtas>
+// The loop of the warp that issues the MMAs of one accumulator over a TMA ring: for each of n_kb
+// stages wait, issue kSteps instructions of K 16, release the stage.  The whole warp runs it and one
+// elected lane issues: with the loop under `if (lane == 0)` the compiler keeps descriptors and
+// addresses in per-thread registers and a stage of four instructions took 600 cycles whatever its
+// size, more than four instructions of N = 256 execute in.  What a stage takes is then this loop's own
+// latency wherever its instructions are narrow (waiting for nothing, 340 cycles for four instructions
+// that execute in 70 to 130), so two stages go together when both are there, and the barriers of the
+// two behind them are asked about in front of the instructions and looked at behind them.  desc_a,
+// desc_b: descriptors of stage 0; `step`: descriptor distance of two stages (bytes / 16).  Returns
+// false if a wait gave up.
+struct RingPos {
+  int stage = 0;
+  uint32_t phase = 0;
+  bool ready = false, ready2 = false;              // this stage, the one behind it: already full when last asked
+  __device__ __forceinline__ void advance(int n_stages) {
+    if (++stage == n_stages) { stage = 0; phase ^= 1; }
+  }
+};
+template <int kSteps, int kCtas = 1>
 __device__ __forceinline__ bool mma_ring(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t step,
                                          uint32_t idesc, int n_kb, int n_stages, uint32_t bar_full0,
                                          uint32_t bar_empty0, RingPos& at, volatile int* abort_flag) {
-  for (int i = 0; i < n_kb; ++i) {
+  // (a barrier may be asked about its next turn only when this turn's data have been used: with four
+  // stages or more that holds for the third ahead)
+  const bool may_pair = n_stages >= 4;
+  auto issue = [&](int stage, bool first) {
+    const uint64_t da = desc_a + (uint64_t)(stage * step), db = desc_b + (uint64_t)(stage * step);
+#pragma unroll
+    for (int ks = 0; ks < kSteps; ++ks) {
+      const uint32_t acc = (first && ks == 0) ? 0u : 1u;
+      if constexpr (kCtas == 2) tc_mma_bf16_pair(d_tmem, da + 2 * ks, db + 2 * ks, idesc, acc);
+      else tc_mma_bf16(d_tmem, da + 2 * ks, db + 2 * ks, idesc, acc);
+    }
+    if constexpr (kCtas == 2) tc_commit_pair(bar_empty0 + 8u * stage);
+    else tc_commit(bar_empty0 + 8u * stage);
+  };
+  for (int i = 0; i < n_kb;) {
     if (!at.ready) {
       bool ok = mbar_wait(bar_full0 + 8u * at.stage, at.phase, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) return false;
     }
     tc_fence_after();
-    const int next = at.stage + 1 == n_stages ? 0 : at.stage + 1;
-    const uint32_t next_phase = next == 0 ? at.phase ^ 1 : at.phase;
-    at.ready = __all_sync(0xffffffffu, mbar_test(bar_full0 + 8u * next, next_phase));
-    const uint64_t da = desc_a + (uint64_t)(at.stage * step), db = desc_b + (uint64_t)(at.stage * step);
+    const bool two = may_pair && at.ready2 && i + 2 <= n_kb;
+    const int s0 = at.stage;
+    at.advance(n_stages);
+    const int s1 = at.stage;
+    if (two) at.advance(n_stages);
+    RingPos behind = at;
+    behind.advance(n_stages);
+    const bool r = mbar_test(bar_full0 + 8u * at.stage, at.phase);
+    const bool r2 = may_pair && mbar_test(bar_full0 + 8u * behind.stage, behind.phase);
     if (elect_one()) {
-#pragma unroll
-      for (int ks = 0; ks < kSteps; ++ks) {
-        if constexpr (kCtas == 2) tc_mma_bf16_pair(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
-        else tc_mma_bf16(d_tmem, da + 2 * ks, db + 2 * ks, idesc, (i | ks) != 0 ? 1u : 0u);
-      }
-      if constexpr (kCtas == 2) tc_commit_pair(bar_empty0 + 8u * at.stage);
-      else tc_commit(bar_empty0 + 8u * at.stage);
+      issue(s0, i == 0);
+      if (two) issue(s1, false);
     }
     __syncwarp();
-    at.stage = next;
-    at.phase = next_phase;
+    at.ready = __all_sync(0xffffffffu, r);
+    at.ready2 = __all_sync(0xffffffffu, r2);
+    i += two ? 2 : 1;
   }
   return true;
 }
