@@ -495,6 +495,14 @@ int rgk_dense_linear(const void* x, const void* weight, const void* bias, int64_
   return RGK_OK;
 }
 
+// Up to how many rows the few-row kernels take a projection.  Every SM has weights to stream there, where
+// a pair of CTAs of the GEMM walks all of K for its tile: at 128 rows 9.2 us against 11.2 for 2560 x
+// 2560 and 14.9 against 24.1 for 7680 -> 2560, at 199 12.8 / 11.4 and 17.9 / 25.4, at 300 21.3 / 27.0 for
+// the latter; wide outputs fill the chip sooner (2560 -> 15360: 16.6 / 19.0 at 48 rows, 21.7 / 20.3 at 128).
+static bool few_rows(int64_t M, int64_t K, int64_t N) {
+  return M <= (N >= 4 * K ? 96 : (K >= 2 * N ? 352 : 160));
+}
+
 // Projections of few rows on the kernel for their number: up to kRowsGemm rows the one that streams
 // weights into registers, above that the one with 128-feature tensor-core tiles.
 static constexpr int kRowsGemm = 8;
@@ -503,6 +511,8 @@ static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, i
                                    bool early, bool wide, cudaStream_t s) {
   if (M <= kRowsGemm)
     return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
+  if (!few_rows(M, K, mats[0].n) && (act != 1 || n_mats == 1))
+    return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s, cap);
   return rgk::launch_dense_small(x, mats, n_mats, residual, M, K, act, cap, status, early, wide, s);
 }
 
@@ -517,14 +527,8 @@ static cudaError_t few_rows_norm_linear(const void* x, const void* scale, float 
   return few_rows_linear(xn, mats, n_mats, nullptr, M, K, act, 0.0f, status, true, true, s);
 }
 
-// Projections of a prompt's rows.  Up to 256 rows the few-row kernels: every SM has weights to stream
-// there, where a pair of CTAs walks all of K for its tile (128 rows: 2560 x 2560 9.3 against 13.1 us,
-// 7680 -> 2560 14.8 against 29.8); longer inner dimensions keep them ahead longer (400 rows: 29.5
-// against 31.3), wide outputs less long (2560 -> 15360 at 199 rows: 21.1 against 20.8).  act 1 needs
-// more rows than that and applies to the first matrix.
-static bool few_rows(int64_t M, int64_t K, int64_t N) {
-  return M <= (N >= 4 * K ? 192 : (K >= 2 * N ? 384 : 256));
-}
+// Projections of a prompt's rows.  act 1 on two matrices needs the GEMM of many rows and applies to the
+// first.
 static cudaError_t prompt_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats, const void* residual,
                                  int64_t M, int K, int act, int* status, cudaStream_t s) {
   if (few_rows(M, K, mats[0].n) && (act != 1 || n_mats == 1))
