@@ -501,8 +501,7 @@ def run_gpu(args, cfg):
     t_core = _time_loop(k_attn, ksteps, stream)
     t_full_att = _time_loop(lambda: rg.residual_block(x_in, pos, norm, att, norm, mlp), ksteps,
                             stream)
-    # 4 * head_dim flops per visible (query, key) pair; the kernel computes the logits twice
-    # (two-pass softmax), so its tensor work is 6 * head_dim per pair of every touched tile
+    # 4 * head_dim flops per visible (query, key) pair (the kernel works on whole tiles)
     pairs = b * heads * sum(min(i, window) + 1 for i in range(t))
     block_info["attention"] = {
         "what": "LocalAttentionBlock.forward prefill, 10 heads x 256, window 2048, same B and T",
@@ -566,8 +565,8 @@ def run_gpu(args, cfg):
                                                  "linear_scan_only", "parity")},
       "block_prefill": block_info,
       "clocks": clk,
-      # per pass: the conv kernel, the per-channel constant kernel and the fused RG-LRU kernel
-      "gpu_launches": 3 * passes * args.steps,
+      # per pass: the conv kernel and the fused RG-LRU kernel
+      "gpu_launches": 2 * passes * args.steps,
   }
   if long_scan is not None:
     line["long_scan"] = long_scan
@@ -906,7 +905,7 @@ def run_long_scan(args):
   if rank == 0:
     leg.update({"metric": "rglru_long_scan_tokens_per_s", "value": leg["tokens_per_s"],
                 "unit": "tokens/s", "higher_is_better": True, "dtype": "bf16", "data": "synthetic",
-                "gpu_launches": 3 * args.steps})
+                "gpu_launches": 2 * args.steps})     # what the RG-LRU kernel finds prepared, and the kernel
     print(json.dumps(leg), flush=True)
   if world > 1:
     dist.destroy_process_group()
@@ -1000,12 +999,12 @@ def run_griffin(args):
                 "d2h_bytes_per_step": b * gen_steps * 4,
                 "note": "the timed region is the public call on pinned host token ids, copies included"},
         "clocks": clk,
-        # this library's kernels per generation: a decode step launches 2 rmsnorm + geglu per block,
-        # the fused recurrent step per recurrent block, 2 rope + 3 ring kernels per attention
-        # block, the final rmsnorm, embed, logits and argmax; the prompt 8 per recurrent block
-        # (2 rmsnorm, conv, RG-LRU, 4 GEMMs... ) and 12 per attention block, twice (prompt, last token)
-        "gpu_launches": steps * (gen_steps * (3 * len(cfg.block_types) + n_rec + 5 * n_att + 4)
-                                 + 2 * (9 * n_rec + 12 * n_att + 3))}), flush=True)
+        # this library's kernels per generation: a block's decode step is 5 launches up to 8
+        # sequences (the norms ride in the projections) and 7 above, a step has the final norm,
+        # embed, logits and argmax on top; a block of the prompt is 8, and the last prompt token is
+        # a step of its own
+        "gpu_launches": steps * ((gen_steps + 1) * ((5 if b <= 8 else 7) * len(cfg.block_types) + 4)
+                                 + 8 * len(cfg.block_types) + 1)}), flush=True)
   if world > 1:
     dist.destroy_process_group()
 

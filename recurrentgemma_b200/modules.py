@@ -549,7 +549,7 @@ class LocalAttentionBlock(nn.Module):
   """Local multi-query attention (recurrentgemma/torch/modules.py:293-493): same constructor,
   parameter names (`proj_q/k/v.weight`, `proj_final.weight/.bias`), forward and cache.  bfloat16
   prefill with head dimension 256 runs on the library (projections on the tcgen05 GEMM, rotary
-  kernel, the two-pass tcgen05 attention kernel), and so does the decode step with head dimension
+  kernel, the tcgen05 attention kernel), and so does the decode step with head dimension
   256 (rotary kernel, the two ring kernels; projections of a handful of rows are library GEMMs);
   other shapes compose the rotary kernel with library contractions."""
 
