@@ -275,7 +275,7 @@ constexpr int kRows = 32;                          // ring slots of a stage
 constexpr int kSliceR = kRows * 128;               // 64 columns of them: 4 KiB
 constexpr int kStageR = 8 * kSliceR;               // four slices of keys, four of values
 constexpr int kStagesR = 3;
-constexpr int kMaxClusterR = 8;
+constexpr int kMaxClusterR = 16;                   // more than 8 has to be allowed per kernel
 constexpr int kQPitch = 528;                       // bytes of a query row, padded
 constexpr int kLogPitch = 17;                      // floats of a logits row
 constexpr int kPPitch = 80;                        // bytes of a head's 32 weights, padded
@@ -303,6 +303,52 @@ struct RingArgs {
   __nv_bfloat16* out;
   int* status;
 };
+
+// The last step of a CTA: its 256 / S columns of every head from the S CTAs' (maximum, sum, O), S up to kMax
+// (the loads of all are in flight together: with sixteen places for eight CTAs the step took 1 us longer).
+template <int kN, int kMax>
+__device__ __forceinline__ void combine_ctas(uint32_t s_base, float* s_w, int S, int split, int b,
+                                             __nv_bfloat16* __restrict__ out) {
+  const int tid = threadIdx.x;
+  if (tid < 16) {
+    float m = kMasked, sum = 0.0f;
+    float ms[kMax], ls[kMax];
+#pragma unroll
+    for (int c = 0; c < kMax; ++c) {
+      ms[c] = kMasked;
+      ls[c] = 0.0f;
+      if (c < S) {
+        const uint32_t peer = peer_smem(s_base + kOffStatR, c);
+        ms[c] = ld_peer_f32(peer + tid * 4);
+        ls[c] = ld_peer_f32(peer + 64 + tid * 4);
+      }
+      m = fmaxf(m, ms[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < kMax; ++c) {
+      ms[c] = __expf(ms[c] - m);
+      sum = fmaf(ls[c], ms[c], sum);
+    }
+#pragma unroll
+    for (int c = 0; c < kMax; ++c) s_w[c * 16 + tid] = ms[c] / sum;
+  }
+  __syncthreads();
+  const int cols = kHdD / S, pairs = cols / 2;
+  for (int i = tid; i < kN * pairs; i += 256) {
+    const int h = i / pairs, col = split * cols + (i - h * pairs) * 2;
+    float o0 = 0.0f, o1 = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kMax; ++c) {
+      if (c < S) {
+        const uint32_t src = peer_smem(s_base + (uint32_t)(h * kHdD + col) * 4, c);
+        const float w = s_w[c * 16 + h];
+        o0 = fmaf(ld_peer_f32(src), w, o0);
+        o1 = fmaf(ld_peer_f32(src + 4), w, o1);
+      }
+    }
+    *reinterpret_cast<uint32_t*>(out + ((int64_t)b * kN + h) * kHdD + col) = pack_bf16x2(o0, o1);
+  }
+}
 
 template <int kN>
 __global__ void __launch_bounds__(256, 2)
@@ -544,44 +590,8 @@ attn_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   __syncwarp();
   cluster_arrive();
   cluster_wait();
-  if (tid < 16) {
-    float m = kMasked, sum = 0.0f;
-    float ms[kMaxClusterR], ls[kMaxClusterR];
-#pragma unroll
-    for (int c = 0; c < kMaxClusterR; ++c) {
-      ms[c] = kMasked;
-      ls[c] = 0.0f;
-      if (c < S) {
-        const uint32_t peer = peer_smem(s_base + kOffStatR, c);
-        ms[c] = ld_peer_f32(peer + tid * 4);
-        ls[c] = ld_peer_f32(peer + 64 + tid * 4);
-      }
-      m = fmaxf(m, ms[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < kMaxClusterR; ++c) {
-      ms[c] = __expf(ms[c] - m);
-      sum = fmaf(ls[c], ms[c], sum);
-    }
-#pragma unroll
-    for (int c = 0; c < kMaxClusterR; ++c) s_w[c * 16 + tid] = ms[c] / sum;
-  }
-  __syncthreads();
-  const int cols = kHdD / S, pairs = cols / 2;
-  for (int i = tid; i < kN * pairs; i += 256) {
-    const int h = i / pairs, col = split * cols + (i - h * pairs) * 2;
-    float o0 = 0.0f, o1 = 0.0f;
-#pragma unroll
-    for (int c = 0; c < kMaxClusterR; ++c) {
-      if (c < S) {
-        const uint32_t src = peer_smem(s_base + (uint32_t)(h * kHdD + col) * 4, c);
-        const float w = s_w[c * 16 + h];
-        o0 = fmaf(ld_peer_f32(src), w, o0);
-        o1 = fmaf(ld_peer_f32(src + 4), w, o1);
-      }
-    }
-    *reinterpret_cast<uint32_t*>(a.out + ((int64_t)b * kN + h) * kHdD + col) = pack_bf16x2(o0, o1);
-  }
+  if (S <= 8) combine_ctas<kN, 8>(s_base, s_w, S, split, b, a.out);
+  else combine_ctas<kN, kMaxClusterR>(s_base, s_w, S, split, b, a.out);
   if (a.update && split == 0) {
     // every CTA of the sequence has read its slots (and written its copies)
     if (tid < 64) {
@@ -611,12 +621,17 @@ cudaError_t launch_ring(RingArgs a, const void* keys_in, const void* values_in, 
   static PerDeviceOnce once;
   int num_sms = 0;
   cudaError_t e = once.run([] {
-    return cudaFuncSetAttribute(attn_decode_ring_kernel<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemR);
+    const cudaError_t r =
+        cudaFuncSetAttribute(attn_decode_ring_kernel<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemR);
+    return r != cudaSuccess ? r : cudaFuncSetAttribute(attn_decode_ring_kernel<kN>,
+                                                       cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   }, &num_sms);
   if (e != cudaSuccess) return e;
-  // as many CTAs as run at once, two an SM
+  // as many CTAs as run at once, two an SM; sixteen only for a few sequences whose whole rings are gone
+  // through (one of 2048 slots 48.0 -> 43.5 us a block, but 65 -> 71 at 16 sequences: clusters that large
+  // do not all find a place at once; and a ring that is updated in place may hold a few slots only)
   int S = 1;
-  while (S < kMaxClusterR && 2 * S * B <= 2 * num_sms) S *= 2;
+  while (S < kMaxClusterR && 2 * S * B <= (S < 8 ? 2 : a.copy) * num_sms) S *= 2;
   if (S * B > 0x7fffffff) return cudaErrorInvalidValue;
   a.S = S;
   cudaLaunchAttribute attr[2];
