@@ -511,7 +511,7 @@ static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, i
                                    bool early, bool wide, cudaStream_t s) {
   if (M <= kRowsGemm)
     return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
-  if (!few_rows(M, K, mats[0].n) && (act != 1 || n_mats == 1))
+  if (!few_rows(M, K, mats[0].n))
     return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s, cap);
   return rgk::launch_dense_small(x, mats, n_mats, residual, M, K, act, cap, status, early, wide, s);
 }
@@ -527,11 +527,10 @@ static cudaError_t few_rows_norm_linear(const void* x, const void* scale, float 
   return few_rows_linear(xn, mats, n_mats, nullptr, M, K, act, 0.0f, status, true, true, s);
 }
 
-// Projections of a prompt's rows.  act 1 on two matrices needs the GEMM of many rows and applies to the
-// first.
+// Projections of a prompt's rows.
 static cudaError_t prompt_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats, const void* residual,
                                  int64_t M, int K, int act, int* status, cudaStream_t s) {
-  if (few_rows(M, K, mats[0].n) && (act != 1 || n_mats == 1))
+  if (few_rows(M, K, mats[0].n))
     return few_rows_linear(x, mats, n_mats, residual, M, K, act, 0.0f, status, false, true, s);
   return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s);
 }
@@ -691,12 +690,11 @@ static int block_prefill_impl(const void* x_in, const void* residual, const void
   int* status = static_cast<int*>(workspace);
   const int64_t M = B * T;
   int rc;
-  // both input projections in one launch; the y branch's gelu in the GEMM's epilogue, or (few rows) in
-  // the join of the RG-LRU kernel
-  const bool few = few_rows(M, D, E);
+  // both input projections in one launch; the y branch's gelu in its epilogue, in float32 (the join of the
+  // RG-LRU kernel would evaluate it with the packed bfloat16 tanh)
   const rgk::RowsMatrix in[2] = {{p->linear_y_w, p->linear_y_b, yb, (int)E},
                                  {p->linear_x_w, p->linear_x_b, xb, (int)E}};
-  RGK_CUDA(prompt_linear(x_in, in, 2, nullptr, M, (int)D, few ? 0 : 1, status, s),
+  RGK_CUDA(prompt_linear(x_in, in, 2, nullptr, M, (int)D, 1, status, s),
            "linear_y, linear_x launch");
   // Conv1D inside the RG-LRU kernel where that kernel applies (the joined output y * gelu(yb) then
   // goes to the conv-output buffer, which the fused form does not use), else as its own kernel
@@ -704,7 +702,7 @@ static int block_prefill_impl(const void* x_in, const void* residual, const void
   // conv kernel xb has been consumed by then and receives the output
   const bool fused = rgk::rglru_chan_supported(dtype, (int)(E / H), B, T) && conv_fusion_enabled();
   char* joined = fused ? yb : xb;
-  if ((rc = run_rglru(w.c, segment_pos, pos_dtype, &p->path, nullptr, yb, few ? 0 : 1, B, T, E, H,
+  if ((rc = run_rglru(w.c, segment_pos, pos_dtype, &p->path, nullptr, yb, 1, B, T, E, H,
                       dtype, RGK_GATES_AUTO, w.wpack, w.a, w.xn, w.scan, joined, h_last, s, xb,
                       conv_cache_out)))
     return rc;

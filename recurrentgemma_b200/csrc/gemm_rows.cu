@@ -57,7 +57,7 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1
 }
 __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// kMode: 0 bias, gelu if kGelu, residual if given; 2 GeGLU over the packed up-projection; 4 soft cap.
+// kMode: 0 bias, 1 gelu of the first matrix as well, residual if given; 2 GeGLU over the packed up-projection; 4 soft cap.
 // kTwo: rows 8-15 exist.  kStaged: x lies in shared memory (normalised if `scale` is given).
 // kFull: K is exactly 8 warps x chunks x kU blocks of 32 (2560, 7680), so no piece needs a test.
 enum { kPlain = 0, kGeluRows = 1, kGeglu = 2, kCap = 4 };
@@ -260,7 +260,7 @@ gemm_rows_kernel(const RowsArgs a) {
           out[(int64_t)em * a.mat[0].n + col] = __float2bfloat16_rn(round_bf16(tanhf(q)) * a.cap);
         } else {
           float y = round_bf16(sum + to_float(e_bias));
-          if constexpr (kMode == kGeluRows) y = round_bf16(gelu_tanh_<true>(y));
+          if (kMode == kGeluRows && mi == 0) y = round_bf16(gelu_tanh_<true>(y));
           if (a.residual != nullptr) y = y + to_float(e_other);
           out[(int64_t)em * a.mat[mi].n + col] = __float2bfloat16_rn(y);
         }

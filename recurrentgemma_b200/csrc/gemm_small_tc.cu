@@ -73,12 +73,12 @@ __device__ __forceinline__ float bf16_value(__nv_bfloat16 v) {
 
 enum { kActNone = 0, kActGelu = 1, kActGeglu = 2, kActCap = 3 };
 
-// One output value from its float32 sum: + bias, one rounding to bfloat16, then gelu or the soft cap
-// with their own roundings - the tensor operations of the reference, in its order.
+// One output value from its float32 sum: + bias, one rounding to bfloat16, then gelu (of the first matrix
+// only) or the soft cap with their own roundings - the tensor operations of the reference, in its order.
 template <int kAct>
-__device__ __forceinline__ float finish1(float sum, float bias, float cap) {
+__device__ __forceinline__ float finish1(float sum, float bias, float cap, bool first) {
   float y = round_bf16(sum + bias);
-  if constexpr (kAct == kActGelu) y = gelu_tanh_<true>(y);
+  if constexpr (kAct == kActGelu) y = first ? gelu_tanh_<true>(y) : y;
   if constexpr (kAct == kActCap) y = round_bf16(tanhf(round_bf16(__fdiv_rn(y, cap)))) * cap;
   return y;                                       // the caller's packing is the last rounding
 }
@@ -341,10 +341,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           } else {
             const float4 s0 = sum4(2 * p, lm), s1 = sum4(2 * p + 1, lm);
             const float b0 = s_bias[2 * p], b1 = s_bias[2 * p + 1];
-            v0[0] = finish1<kAct>(s0.x, b0, a.cap); v1[0] = finish1<kAct>(s1.x, b1, a.cap);
-            v0[1] = finish1<kAct>(s0.y, b0, a.cap); v1[1] = finish1<kAct>(s1.y, b1, a.cap);
-            v0[2] = finish1<kAct>(s0.z, b0, a.cap); v1[2] = finish1<kAct>(s1.z, b1, a.cap);
-            v0[3] = finish1<kAct>(s0.w, b0, a.cap); v1[3] = finish1<kAct>(s1.w, b1, a.cap);
+            v0[0] = finish1<kAct>(s0.x, b0, a.cap, mi == 0); v1[0] = finish1<kAct>(s1.x, b1, a.cap, mi == 0);
+            v0[1] = finish1<kAct>(s0.y, b0, a.cap, mi == 0); v1[1] = finish1<kAct>(s1.y, b1, a.cap, mi == 0);
+            v0[2] = finish1<kAct>(s0.z, b0, a.cap, mi == 0); v1[2] = finish1<kAct>(s1.z, b1, a.cap, mi == 0);
+            v0[3] = finish1<kAct>(s0.w, b0, a.cap, mi == 0); v1[3] = finish1<kAct>(s1.w, b1, a.cap, mi == 0);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -413,8 +413,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         tc_wait_ld();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float y0 = finish1<kAct>(__uint_as_float(acc[2 * j]), b, a.cap);
-          const float y1 = finish1<kAct>(__uint_as_float(acc[2 * j + 1]), b, a.cap);
+          const float y0 = finish1<kAct>(__uint_as_float(acc[2 * j]), b, a.cap, mi == 0);
+          const float y1 = finish1<kAct>(__uint_as_float(acc[2 * j + 1]), b, a.cap, mi == 0);
           const float got = __shfl_xor_sync(0xffffffffu, upper ? y0 : y1, 1);
           uint32_t y = upper ? pack_bf16x2(got, y1) : pack_bf16x2(y0, got);
           if (a.residual != nullptr) y = badd2(y, res[j]);

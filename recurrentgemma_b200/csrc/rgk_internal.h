@@ -178,7 +178,8 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
                               bool prepared = false);
 
 // gemm_rows.cu: up to three projections (matrices) of the same M <= 16 rows in one launch, with
-// RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as above behind; one
+// RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as below behind (act 1 on the
+// first matrix only); one
 // residual for a single matrix.  early: no kernel in front of this one on the stream that could still be
 // running writes weights (it is one of the library's own, launched by the same call), so they may
 // be fetched before it ends.
@@ -194,7 +195,7 @@ cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, c
                              bool early, cudaStream_t s);
 // gemm_small_tc.cu: the same projections (no norm) for up to some hundreds of rows, weights split over
 // all SMs (the K slices of a feature tile are a thread-block cluster and add up in distributed
-// shared memory).  act 0: bias; 1: gelu_tanh of the rounded result; 2: GeGLU over the packed
+// shared memory).  act 0: bias; 1: gelu_tanh of the first matrix's rounded result; 2: GeGLU over the packed
 // up-projection of the MLP (w as pack_mlp_up_kernel writes it, n = 2 X rows, out [M, X]).  status:
 // optional device int raised on a bounded-wait timeout.  early as for launch_rows_gemm; wide: CTAs
 // that never share an SM with another of the same launch (kernels in a chain alternate).
