@@ -504,14 +504,15 @@ static bool few_rows(int64_t M, int64_t K, int64_t N) {
 }
 
 // Projections of few rows on the kernel for their number: up to kRowsGemm rows the one that streams
-// weights into registers, above that the one with 128-feature tensor-core tiles.
+// weights into registers, above that the one with 128-feature tensor-core tiles, and the GEMM of many rows
+// where that is faster (its epilogues have gelu or a residual, not both).
 static constexpr int kRowsGemm = 8;
 static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats,
                                    const void* residual, int64_t M, int K, int act, float cap, int* status,
                                    bool early, bool wide, cudaStream_t s) {
   if (M <= kRowsGemm)
     return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
-  if (!few_rows(M, K, mats[0].n))
+  if (!few_rows(M, K, mats[0].n) && (act == 0 || residual == nullptr))
     return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s, cap);
   return rgk::launch_dense_small(x, mats, n_mats, residual, M, K, act, cap, status, early, wide, s);
 }

@@ -31,3 +31,25 @@ def test_gelu_of_the_y_branch_is_evaluated_in_float32(rows):
   want = (path.float() * gelu.float()).to(BF16)
   share = (got != want).float().mean().item()
   assert share <= 0.01, f"{share:.2%} of the outputs differ"
+
+
+# both sides of every change of kernel: 8 / 9 rows, 160 / 161 of a square shape, 96 / 97 of a wide one,
+# and the largest number of rows of each and of a narrow one
+@pytest.mark.parametrize("m,k,n", [(8, 512, 512), (9, 512, 512), (160, 512, 512), (161, 512, 512),
+                                   (256, 512, 512), (96, 256, 1024), (97, 256, 1024), (256, 1024, 256)])
+def test_gelu_and_residual_together(m, k, n):
+  """act(x W^T + b) + residual, which the few-row linear takes for every number of rows: float32 sum and
+  bias, one rounding, gelu and the sum with their own.  Another order of summation moves a value to its
+  neighbour (2^-8 of its size, 2^-7 of the next power of two) at each of the three roundings."""
+  from recurrentgemma_b200 import _lib, modules
+  torch.manual_seed(m + n)
+  x = torch.randn(m, k, device=DEV).to(BF16)
+  w = (torch.randn(n, k, device=DEV) / k ** 0.5).to(BF16)
+  b, res = (torch.randn(n, device=DEV) * 0.1).to(BF16), torch.randn(m, n, device=DEV).to(BF16)
+  got = modules.small_linear(x, w, b, act=_lib.ACT_GELU_TANH, residual=res)
+  y = (x.float() @ w.float().t() + b.float()).to(BF16)
+  y = torch.nn.functional.gelu(y.float(), approximate="tanh").to(BF16)
+  want = (y.float() + res.float()).to(BF16)
+  err = (got.float() - want.float()).abs().max() / want.float().abs().max()
+  assert err.item() <= 3 * 2.0 ** -8
+  assert (got != want).float().mean().item() <= 0.05
