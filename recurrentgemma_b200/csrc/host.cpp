@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/rgk.h"
@@ -75,10 +76,15 @@ PyObject* not_here() {
   Py_RETURN_NOTIMPLEMENTED;
 }
 
-// A dense CUDA tensor argument; null if it is anything else.
+// A dense CUDA tensor argument; null if it is anything else (a tensor that has its operations in Python or
+// no memory of its own - fake, batched, functional - among that).
 const at::Tensor* dense(PyObject* o) {
   if (o == nullptr || !THPVariable_Check(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
+  const c10::TensorImpl* impl = t.unsafeGetTensorImpl();
+  if (impl->is_python_dispatch() || !impl->has_storage() ||
+      impl->key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Functionalize, c10::DispatchKey::ZeroTensor})))
+    return nullptr;
   if (!t.is_cuda() || t.layout() != at::kStrided || !t.is_contiguous()) return nullptr;
   return &t;
 }
@@ -248,7 +254,7 @@ PyObject* make_cache(PyObject* h, PyObject* conv) {      // steals both
 }
 
 // ---- recurrent_path(xb, yb, segment_pos, conv_1d, rg_lru, cache, return_cache, out, inplace) -----
-PyObject* recurrent_path(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* recurrent_path(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 9) return not_here();
   const at::Tensor* x = dense(args[0]);
   const at::Tensor* y = args[1] == Py_None ? nullptr : dense(args[1]);
@@ -328,7 +334,7 @@ PyObject* recurrent_path(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---- RGLRU.forward: rglru(module, x, segment_pos, cache, return_cache) ---------------------------
-PyObject* rglru(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* rglru(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 5) return not_here();
   PyObject* lru = args[0];
   const at::Tensor *x = dense(args[1]), *pos = dense(args[2]);
@@ -623,7 +629,7 @@ bool prompt_args(const at::Tensor* x, const at::Tensor* pos) {
 }
 
 // prefill(temporal block, x, segment_pos, return_cache): its forward without a cache
-PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* prefill(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 4) return not_here();
   const at::Tensor *x = dense(args[1]), *pos = dense(args[2]);
   if (!prompt_args(x, pos)) return not_here();
@@ -640,7 +646,7 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // residual_prefill(x, segment_pos, norm, temporal block, norm, mlp, return_cache)
-PyObject* residual_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* residual_prefill(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 7) return not_here();
   const at::Tensor *x = dense(args[0]), *pos = dense(args[1]);
   PyObject *norm2 = args[4], *mlp = args[5];
@@ -681,7 +687,7 @@ PyObject* residual_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // residual_step(x, segment_pos, norm, temporal block, norm, mlp, cache, return_cache, inplace)
-PyObject* residual_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* residual_step(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 9) return not_here();
   return step(args[0], args[1], args[2], args[3], args[4], args[5], args[6], PyObject_IsTrue(args[7]) == 1,
               PyObject_IsTrue(args[8]) == 1, false);
@@ -689,7 +695,7 @@ PyObject* residual_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // block_step(ResidualBlock, x, segment_pos, cache, return_cache, inplace, chained): the same for a
 // module; chained: the last work on the stream is another block's step (see rgk.h).
-PyObject* block_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* block_step(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 7) return not_here();
   PyObject* m = args[0];
   if (!exactly(m, g_residual_cls) || !no_hooks(m)) return not_here();
@@ -754,7 +760,19 @@ PyObject* init(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
-#define FAST(fn) {#fn, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+// What CPython calls: torch's C++ exceptions (out of memory, no CUDA driver, the version of an inference
+// tensor) leave as the Python errors they are.
+template <PyObject* (*fn)(PyObject* const*, Py_ssize_t)>
+PyObject* entry_point(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  try {
+    return fn(args, n);
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
+}
+#define FAST(fn) \
+  {#fn, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(entry_point<fn>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"init", init, METH_VARARGS, nullptr},
     FAST(recurrent_path),
