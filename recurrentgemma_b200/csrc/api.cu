@@ -1002,7 +1002,7 @@ int rgk_attention_block_prefill(const void* x, const void* segment_pos, int pos_
                   aligned16(p->final_b),
               RGK_EALIGN, "pointers must be 16-byte aligned");
   RGK_REQUIRE(rgk::attention_supported(dtype, head_dim, B > 0 ? B : 1, T > 0 ? T : 1, N) &&
-                  D == (int64_t)N * head_dim && window < (1 << 24),
+                  D == (int64_t)N * head_dim,
               RGK_ESHAPE, "the attention block covers bfloat16 with head dimension 256 and as many heads as "
               "the width holds (dtype %d, head_dim %d, width %lld)", dtype, head_dim, (long long)D);
   RGK_REQUIRE(norm_scale == nullptr || rgk::rmsnorm_supported(dtype, D), RGK_ESHAPE,

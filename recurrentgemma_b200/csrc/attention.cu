@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepArgs a) {
   // a sequence's rows, and behind them the ring slots a short prompt leaves empty
   const int slots = min(a.window, T_);
   const int rows = a.cache_k != nullptr ? T_ + (a.window - slots) : T_;
-  const int per_seq = (max(rows, a.Tp) + kPrepRows - 1) / kPrepRows;
+  const int per_seq = (max(rows, a.Tp) - 1) / kPrepRows + 1;      // (a window of 2^31 - 1 does not overflow)
   const int blk = (int)blockIdx.x - a.B;
   const int b = blk / per_seq, t_base = (blk - b * per_seq) * kPrepRows;
   const int r = tid >> 3, part = tid & 7;

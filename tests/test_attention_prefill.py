@@ -62,3 +62,16 @@ def test_block(batch, seq, heads, window, doc, gain):
   # the same call again, without a cache: the same bits
   again, none = block(x, pos, return_cache=False)
   assert none is None and torch.equal(got, again)
+
+
+@pytest.mark.parametrize("window", [1 << 24, (1 << 31) - 1])
+def test_window_longer_than_any_prompt(window):
+  """Every window is taken where no cache is wanted: "no window at all" among them."""
+  import recurrentgemma_b200 as rg
+  block = rg.LocalAttentionBlock(512, 2, window, device=DEV, dtype=BF16)
+  x = torch.randn(2, 300, 512, device=DEV).to(BF16)
+  pos = torch.arange(300, device=DEV)[None].repeat(2, 1)
+  got, _ = block(x, pos, return_cache=False)
+  block.window_size = 300
+  want, _ = block(x, pos, return_cache=False)
+  assert torch.equal(got, want)
