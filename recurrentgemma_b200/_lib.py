@@ -177,7 +177,8 @@ def host():
     ext.init(LIB_PATH, _workspaces, workspace, check,
              (modules.RecurrentBlockCache, modules.AttentionBlockCache, modules.layers.RMSNorm,
               modules.RecurrentBlock, modules.LocalAttentionBlock, modules.MLPBlock,
-              modules.ResidualBlock),
+              modules.ResidualBlock, modules.layers.Conv1D, modules.layers.RGLRU,
+              modules.layers.Einsum, torch.nn.Linear),
              nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks)
     _host = ext
   return _host

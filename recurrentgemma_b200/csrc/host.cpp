@@ -7,7 +7,8 @@
 // device), so that every small call was bound by its host code.  Here they take a few microseconds.
 //
 // Every function returns NotImplemented for arguments it does not handle - a CPU tensor, a dtype
-// mismatch, a strided input, a subclass or a module with hooks where modules are fused - and the
+// mismatch, a strided input, and wherever a module's parameters stand for a
+// call of the module, one of another class, with hooks or with a forward of its own (`plain`) - and the
 // Python form of the same forward then runs, which also raises the errors.  Nothing is cached here:
 // parameters are looked up in the modules on every call.
 #include <ATen/ATen.h>
@@ -50,12 +51,13 @@ PyObject* g_raise = nullptr;             // _lib.check(rc): raises RgkError with
 PyObject* g_cache_cls = nullptr;         // modules.RecurrentBlockCache
 PyObject* g_ring_cls = nullptr;          // modules.AttentionBlockCache
 PyObject *g_norm_cls, *g_recurrent_cls, *g_attention_cls, *g_mlp_cls, *g_residual_cls;   // module classes
+PyObject *g_conv_cls, *g_lru_cls, *g_einsum_cls, *g_linear_cls;
 PyObject *g_hooks, *g_pre_hooks;         // torch's hooks for every module
 
 // interned attribute names
 #define NAMES(X) X(_parameters) X(_modules) X(w) X(b) X(a_param) X(input_gate) X(a_gate) X(num_heads) \
   X(gates_impl) X(temporal_width) X(width) X(_pack_key) X(_pack_buf) X(_packed_gates) \
-  X(_packed_up) X(_forward_hooks) X(_forward_pre_hooks) X(weight) X(bias) X(scale) X(eps) X(conv_1d) \
+  X(_packed_up) X(forward) X(_forward_hooks) X(_forward_pre_hooks) X(weight) X(bias) X(scale) X(eps) X(conv_1d) \
   X(rg_lru) X(linear_x) X(linear_y) X(linear_out) X(ffw_up) X(ffw_down) X(proj_q) X(proj_k) X(proj_v) \
   X(proj_final) X(window_size) X(expanded_width) X(lru_width) X(recurrent_block) \
   X(attention_block) X(conv1d_temporal_width) X(temporal_pre_norm) X(channel_pre_norm) X(mlp_block)
@@ -117,6 +119,19 @@ struct Params {
     return t == nullptr ? nullptr : t->const_data_ptr();
   }
 };
+
+// Whether calling `module` is running cls.forward on its parameters and nothing else.
+bool plain(PyObject* module, PyObject* cls) {
+  if (module == nullptr || (PyObject*)Py_TYPE(module) != cls) return false;
+  Ref d(PyObject_GenericGetDict(module, nullptr));
+  if (d.p == nullptr || !PyDict_Check(d.p) || PyDict_GetItemWithError(d.p, s_forward) != nullptr) return false;
+  for (PyObject* name : {s__forward_hooks, s__forward_pre_hooks}) {
+    PyObject* hooks = PyDict_GetItemWithError(d.p, name);
+    if (hooks == nullptr || !PyDict_Check(hooks) || PyDict_Size(hooks) != 0) return false;
+  }
+  return true;
+}
+bool no_global_hooks() { return PyDict_Size(g_hooks) == 0 && PyDict_Size(g_pre_hooks) == 0; }
 
 bool int_attr(PyObject* o, PyObject* name, long* v) {
   Ref a(PyObject_GetAttr(o, name));
@@ -223,6 +238,11 @@ bool packed(PyObject* module, const at::Tensor& p0, const at::Tensor& p1, int dt
 enum class Found { yes, no, error };
 Found path_params(PyObject* conv, PyObject* lru, Params& pr, int dt, long width, rgk_params* p,
                   long* heads, long* impl, bool* made = nullptr) {
+  long lru_width = 0;
+  if (!int_attr(lru, s_num_heads, heads) || !int_attr(lru, s_gates_impl, impl) ||
+      !int_attr(lru, s_width, &lru_width) || lru_width != width || *heads < 1 || width % *heads != 0)
+    return Found::no;
+  const long bw = width / *heads;
   PyObject* gx = submodule(lru, s_input_gate);
   PyObject* ga = submodule(lru, s_a_gate);
   const at::Tensor* wx = pr.get(gx, s_w);
@@ -236,10 +256,7 @@ Found path_params(PyObject* conv, PyObject* lru, Params& pr, int dt, long width,
     p->conv_b = pr.ptr(conv, s_b);
     if (!int_attr(conv, s_temporal_width, &tw) || tw != 4) return Found::no;
   }
-  long lru_width = 0;
-  if (!pr.ok || !int_attr(lru, s_num_heads, heads) || !int_attr(lru, s_gates_impl, impl) ||
-      !int_attr(lru, s_width, &lru_width) || lru_width != width || *heads < 1)
-    return Found::no;
+  if (!pr.ok) return Found::no;
   p->gate_x_w = wx->const_data_ptr();
   p->gate_a_w = wa->const_data_ptr();
   p->gates_packed = nullptr;
@@ -288,6 +305,7 @@ PyObject* recurrent_path(PyObject* const* args, Py_ssize_t n) {
         c_in->size(2) != E)
       return not_here();
   }
+  if (!plain(conv, g_conv_cls) || !plain(lru, g_lru_cls) || !no_global_hooks()) return not_here();
   Guard guard(x->device().index());
   Params pr{x->scalar_type(), x->device()};
   rgk_params p;
@@ -379,13 +397,6 @@ PyObject* rglru(PyObject* const* args, Py_ssize_t n) {
 // ---- the decode step of a residual block ------------------------------------------------------------
 // The decode step of a few sequences through a whole residual block, one library call.
 
-bool no_hooks(PyObject* module) {
-  for (PyObject* name : {s__forward_hooks, s__forward_pre_hooks}) {
-    Ref d(PyObject_GetAttr(module, name));
-    if (d.p == nullptr || !PyDict_Check(d.p) || PyDict_Size(d.p) != 0) return false;
-  }
-  return true;
-}
 bool exactly(PyObject* module, PyObject* cls) { return (PyObject*)Py_TYPE(module) == cls; }
 bool float_attr(PyObject* o, PyObject* name, float* v) {
   Ref a(PyObject_GetAttr(o, name));
@@ -398,27 +409,58 @@ bool shaped(const at::Tensor* t, at::ScalarType dtype, c10::Device dev, at::IntA
   return t != nullptr && t->scalar_type() == dtype && t->device() == dev && t->sizes() == sizes;
 }
 
-// The parameters of a RecurrentBlock of RG-LRU width E.
-Found recurrent_params(PyObject* block, Params& pr, long E, rgk_block_params* p, long* heads, long* impl,
+// The parameters of a RecurrentBlock of width D and RG-LRU width E.
+Found recurrent_params(PyObject* block, Params& pr, long D, long E, rgk_block_params* p, long* heads, long* impl,
                        bool* made) {
   PyObject *ly = submodule(block, s_linear_y), *lx = submodule(block, s_linear_x),
            *lo = submodule(block, s_linear_out);
+  PyObject *conv = submodule(block, s_conv_1d), *lru = submodule(block, s_rg_lru);
+  if (!plain(ly, g_linear_cls) || !plain(lx, g_linear_cls) || !plain(lo, g_linear_cls) ||
+      !plain(conv, g_conv_cls) || !plain(lru, g_lru_cls))
+    return Found::no;
   p->linear_y_w = pr.ptr(ly, s_weight); p->linear_y_b = pr.ptr(ly, s_bias);
   p->linear_x_w = pr.ptr(lx, s_weight); p->linear_x_b = pr.ptr(lx, s_bias);
   p->linear_out_w = pr.ptr(lo, s_weight); p->linear_out_b = pr.ptr(lo, s_bias);
-  PyObject *conv = submodule(block, s_conv_1d), *lru = submodule(block, s_rg_lru);
-  if (!pr.ok || conv == nullptr || lru == nullptr) return Found::no;
+  if (!pr.ok) return Found::no;
   return path_params(conv, lru, pr, RGK_BF16, E, &p->path, heads, impl, made);
 }
-// The parameters of a LocalAttentionBlock; pr.ok says whether they are all there.
-rgk_attention_params attention_params(PyObject* block, Params& pr) {
+// The parameters of a LocalAttentionBlock of width D and one key/value head of 256; pr.ok says whether they
+// are all there.
+rgk_attention_params attention_params(PyObject* block, Params& pr, long D) {
   rgk_attention_params p = {};
-  p.q_w = pr.ptr(submodule(block, s_proj_q), s_weight);
-  p.k_w = pr.ptr(submodule(block, s_proj_k), s_weight);
-  p.v_w = pr.ptr(submodule(block, s_proj_v), s_weight);
-  p.final_w = pr.ptr(submodule(block, s_proj_final), s_weight);
-  p.final_b = pr.ptr(submodule(block, s_proj_final), s_bias);
+  PyObject *q = submodule(block, s_proj_q), *k = submodule(block, s_proj_k), *v = submodule(block, s_proj_v),
+           *f = submodule(block, s_proj_final);
+  for (PyObject* m : {q, k, v, f}) pr.ok = pr.ok && plain(m, g_linear_cls);
+  if (!pr.ok) return p;
+  p.q_w = pr.ptr(q, s_weight);
+  p.k_w = pr.ptr(k, s_weight);
+  p.v_w = pr.ptr(v, s_weight);
+  p.final_w = pr.ptr(f, s_weight);
+  p.final_b = pr.ptr(f, s_bias);
   return p;
+}
+
+// The channel half of a residual block of width D: its norm and its MLP.
+struct Channel {
+  long X = 0;
+  float eps = 0.0f;
+  const void *scale = nullptr, *down_w = nullptr, *down_b = nullptr;
+  const at::Tensor *up_w = nullptr, *up_b = nullptr;       // ffw_up, which the kernels read packed
+};
+bool channel_params(PyObject* norm, PyObject* mlp, Params& pr, long D, Channel* c) {
+  long w = 0, wn = 0;
+  if (!plain(norm, g_norm_cls) || !plain(mlp, g_mlp_cls) || !int_attr(mlp, s_expanded_width, &c->X) ||
+      !int_attr(mlp, s_width, &w) || !int_attr(norm, s_width, &wn) || w != D || wn != D || c->X % 64 != 0 ||
+      D % 8 != 0 || !float_attr(norm, s_eps, &c->eps))
+    return false;
+  PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
+  if (!plain(up, g_einsum_cls) || !plain(down, g_linear_cls)) return false;
+  c->up_w = pr.get(up, s_w);
+  c->up_b = pr.get(up, s_b);
+  c->scale = pr.ptr(norm, s_scale);
+  c->down_w = pr.ptr(down, s_weight);
+  c->down_b = pr.ptr(down, s_bias);
+  return pr.ok;
 }
 
 PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* block, PyObject* norm2,
@@ -432,27 +474,25 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
   const int64_t B = x->size(0), D = x->size(2);
   const c10::Device dev = x->device();
   if (B == 0 || B > g_lib.residual_decode_rows() || D == 0) return not_here();
-  if (!(recurrent || exactly(block, g_attention_cls)) || !exactly(norm1, g_norm_cls) ||
-      !exactly(norm2, g_norm_cls) || !exactly(mlp, g_mlp_cls) || PyDict_Size(g_hooks) != 0 ||
-      PyDict_Size(g_pre_hooks) != 0 || !no_hooks(norm1) || !no_hooks(block) || !no_hooks(mlp))
+  if (!plain(block, recurrent ? g_recurrent_cls : g_attention_cls) || !plain(norm1, g_norm_cls) ||
+      !no_global_hooks())
     return not_here();
   Guard guard(dev.index());
   Params pr{at::kBFloat16, dev};
-  // the channel half
-  long X = 0, w1 = 0, w2 = 0, w3 = 0;
+  Channel ch;
+  long w1 = 0;
   float eps1 = 0.0f;
-  rgk_channel_params c = {};
-  PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
-  const at::Tensor *up_w = pr.get(up, s_w), *up_b = pr.get(up, s_b);
-  c.norm_scale = pr.ptr(norm2, s_scale);
-  c.down_w = pr.ptr(down, s_weight);
-  c.down_b = pr.ptr(down, s_bias);
-  const void* scale1 = pr.ptr(norm1, s_scale);
-  if (!pr.ok || down == nullptr || !no_hooks(down) || !int_attr(mlp, s_expanded_width, &X) ||
-      !int_attr(mlp, s_width, &w1) || !int_attr(norm1, s_width, &w2) || !int_attr(norm2, s_width, &w3) ||
-      w1 != D || w2 != D || w3 != D || X % 64 != 0 || D % 8 != 0 || !float_attr(norm1, s_eps, &eps1) ||
-      !float_attr(norm2, s_eps, &c.eps))
+  if (!channel_params(norm2, mlp, pr, D, &ch) || !int_attr(norm1, s_width, &w1) || w1 != D ||
+      !float_attr(norm1, s_eps, &eps1))
     return not_here();
+  const long X = ch.X;
+  rgk_channel_params c = {};
+  c.norm_scale = ch.scale;
+  c.down_w = ch.down_w;
+  c.down_b = ch.down_b;
+  c.eps = ch.eps;
+  const void* scale1 = pr.ptr(norm1, s_scale);
+  if (!pr.ok) return not_here();
   const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const int pc = pos_code(*pos);
   Workspace ws;
@@ -465,13 +505,13 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
         !shaped(h_in, at::kFloat, dev, {B, E}) || !shaped(c_in, at::kBFloat16, dev, {B, 3, E}))
       return not_here();
     rgk_block_params p = {};
-    switch (recurrent_params(block, pr, E, &p, &heads, &impl, &made)) {
+    switch (recurrent_params(block, pr, D, E, &p, &heads, &impl, &made)) {
       case Found::no: return not_here();
       case Found::error: return nullptr;
       case Found::yes: break;
     }
     if (E != heads * 256 || impl == RGK_GATES_SIMT || p.path.gates_packed == nullptr) return not_here();
-    if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
+    if (!packed(mlp, *ch.up_w, *ch.up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
     if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, E, X, 0, 0), &ws)) return nullptr;
     at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
     at::Tensor h = inplace ? *h_in : empty({B, E}, at::kFloat, dev);
@@ -500,9 +540,9 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
       !shaped(keys, at::kBFloat16, dev, {B, window, 1, 256}) ||
       !shaped(values, at::kBFloat16, dev, {B, window, 1, 256}) || !shaped(seen, at::kInt, dev, {B}))
     return not_here();
-  const rgk_attention_params p = attention_params(block, pr);
+  const rgk_attention_params p = attention_params(block, pr, D);
   if (!pr.ok) return not_here();
-  if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
+  if (!packed(mlp, *ch.up_w, *ch.up_b, -1, s__packed_up, &c.packed_up, &made)) return nullptr;
   if (!workspace(*x, s, g_lib.residual_decode_workspace_bytes(B, D, D, X, (int)heads, (int)window), &ws))
     return nullptr;
   at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
@@ -530,25 +570,12 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
 
 // ---- prefill of a temporal block, alone or inside its residual block -------------------------------
 
-// The linear maps of a block that a caller may have replaced or hooked.
-bool plain_children(PyObject* block) {
-  Ref d(PyObject_GetAttr(block, s__modules));
-  if (d.p == nullptr || !PyDict_Check(d.p)) return false;
-  PyObject *key, *child;
-  Py_ssize_t at = 0;
-  while (PyDict_Next(d.p, &at, &key, &child))
-    if (child == Py_None || !no_hooks(child)) return false;
-  return true;
-}
-
 // x, segment_pos -> [norm ->] temporal block [-> + x], with the cache of the prompt.  Yes: *out and, if
 // wanted, *cache are set.
 Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* norm, PyObject* block, bool want,
                        at::Tensor* out, PyObject** cache) {
   const bool recurrent = exactly(block, g_recurrent_cls);
-  if (!(recurrent || exactly(block, g_attention_cls)) || PyDict_Size(g_hooks) != 0 ||
-      PyDict_Size(g_pre_hooks) != 0 || !plain_children(block))
-    return Found::no;
+  if (!(recurrent || exactly(block, g_attention_cls)) || !no_global_hooks()) return Found::no;
   const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
   const c10::Device dev = x.device();
   Params pr{at::kBFloat16, dev};
@@ -556,7 +583,7 @@ Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* nor
   float eps = 0.0f;
   long w1 = 0, width = 0;
   if (norm != nullptr) {
-    if (!exactly(norm, g_norm_cls) || !no_hooks(norm) || !no_hooks(block)) return Found::no;
+    if (!plain(norm, g_norm_cls) || !plain(block, recurrent ? g_recurrent_cls : g_attention_cls)) return Found::no;
     scale = pr.ptr(norm, s_scale);
     if (!pr.ok || !int_attr(norm, s_width, &w1) || w1 != D || !float_attr(norm, s_eps, &eps)) return Found::no;
   }
@@ -569,7 +596,7 @@ Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* nor
     rgk_block_params p = {};
     if (!int_attr(block, s_lru_width, &E) || !int_attr(block, s_conv1d_temporal_width, &tw) || tw != 4)
       return Found::no;
-    const Found f = recurrent_params(block, pr, E, &p, &heads, &impl, nullptr);
+    const Found f = recurrent_params(block, pr, D, E, &p, &heads, &impl, nullptr);
     if (f != Found::yes) return f;
     if (E != heads * 256 || impl == RGK_GATES_SIMT) return Found::no;
     if (!workspace(x, s, norm != nullptr ? g_lib.residual_workspace_bytes(B, T, D, E, RGK_BF16)
@@ -594,7 +621,7 @@ Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* nor
     if (want) *cache = make_cache(wrap(std::move(h)), wrap(std::move(c)));
   } else {
     long heads = 0, window = 0;
-    const rgk_attention_params p = attention_params(block, pr);
+    const rgk_attention_params p = attention_params(block, pr, D);
     if (!pr.ok || !int_attr(block, s_num_heads, &heads) || !int_attr(block, s_window_size, &window) ||
         heads * 256 != D || window < 1)
       return Found::no;
@@ -650,23 +677,16 @@ PyObject* residual_prefill(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 7) return not_here();
   const at::Tensor *x = dense(args[0]), *pos = dense(args[1]);
   PyObject *norm2 = args[4], *mlp = args[5];
-  if (!prompt_args(x, pos) || !exactly(norm2, g_norm_cls) || !exactly(mlp, g_mlp_cls) || !no_hooks(norm2) ||
-      !no_hooks(mlp) || !plain_children(mlp))
-    return not_here();
+  if (!prompt_args(x, pos)) return not_here();
   const int64_t M = x->size(0) * x->size(1), D = x->size(2);
   const c10::Device dev = x->device();
   Guard guard(dev.index());
   Params pr{at::kBFloat16, dev};
-  long X = 0, w1 = 0, w2 = 0;
-  float eps = 0.0f;
-  PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
-  const at::Tensor *up_w = pr.get(up, s_w), *up_b = pr.get(up, s_b);
-  const void *scale = pr.ptr(norm2, s_scale), *down_w = pr.ptr(down, s_weight), *down_b = pr.ptr(down, s_bias);
-  if (!pr.ok || !int_attr(mlp, s_expanded_width, &X) || !int_attr(mlp, s_width, &w1) ||
-      !int_attr(norm2, s_width, &w2) || w1 != D || w2 != D || X % 64 != 0 || !float_attr(norm2, s_eps, &eps))
-    return not_here();
+  Channel ch;
+  if (!channel_params(norm2, mlp, pr, D, &ch)) return not_here();
+  const long X = ch.X;
   const void* packed_up = nullptr;
-  if (!packed(mlp, *up_w, *up_b, -1, s__packed_up, &packed_up)) return nullptr;
+  if (!packed(mlp, *ch.up_w, *ch.up_b, -1, s__packed_up, &packed_up)) return nullptr;
   at::Tensor r;
   PyObject* cache = nullptr;
   switch (temporal_prefill(*x, *pos, args[2], args[3], PyObject_IsTrue(args[6]) == 1, &r, &cache)) {
@@ -679,7 +699,7 @@ PyObject* residual_prefill(PyObject* const* args, Py_ssize_t n) {
   Workspace ws;
   if (!workspace(*x, s, g_lib.mlp_workspace_bytes(M, D, X, RGK_BF16), &ws)) return nullptr;
   at::Tensor out = empty(x->sizes(), at::kBFloat16, dev);
-  if (!succeeded(g_lib.residual_channel(r.const_data_ptr(), scale, eps, packed_up, down_w, down_b, M, D, X,
+  if (!succeeded(g_lib.residual_channel(r.const_data_ptr(), ch.scale, ch.eps, packed_up, ch.down_w, ch.down_b, M, D, X,
                                         RGK_BF16, out.mutable_data_ptr(), ws.ptr, ws.bytes, s)))
     return nullptr;
   Ref o(wrap(std::move(out)));
@@ -698,7 +718,7 @@ PyObject* residual_step(PyObject* const* args, Py_ssize_t n) {
 PyObject* block_step(PyObject* const* args, Py_ssize_t n) {
   if (!g_ready || n != 7) return not_here();
   PyObject* m = args[0];
-  if (!exactly(m, g_residual_cls) || !no_hooks(m)) return not_here();
+  if (!plain(m, g_residual_cls)) return not_here();
   PyObject* temporal = submodule(m, s_recurrent_block);
   if (temporal == nullptr) temporal = submodule(m, s_attention_block);
   PyObject *norm1 = submodule(m, s_temporal_pre_norm), *norm2 = submodule(m, s_channel_pre_norm),
@@ -710,13 +730,14 @@ PyObject* block_step(PyObject* const* args, Py_ssize_t n) {
 
 // ---- set-up --------------------------------------------------------------------------------------
 // init(librgk path, _workspaces, workspace, check, (RecurrentBlockCache, AttentionBlockCache, RMSNorm,
-// RecurrentBlock, LocalAttentionBlock, MLPBlock, ResidualBlock), torch's global forward hooks and pre-hooks)
+// RecurrentBlock, LocalAttentionBlock, MLPBlock, ResidualBlock, Conv1D, RGLRU, Einsum, nn.Linear), torch's
+// global forward hooks and pre-hooks)
 PyObject* init(PyObject*, PyObject* args) {
   const char* path = nullptr;
-  PyObject *spaces, *make, *raise, *cls[7], *hooks, *pre_hooks;
-  if (!PyArg_ParseTuple(args, "sO!OO(OOOOOOO)O!O!", &path, &PyDict_Type, &spaces, &make, &raise, &cls[0],
-                        &cls[1], &cls[2], &cls[3], &cls[4], &cls[5], &cls[6], &PyDict_Type, &hooks, &PyDict_Type,
-                        &pre_hooks))
+  PyObject *spaces, *make, *raise, *cls[11], *hooks, *pre_hooks;
+  if (!PyArg_ParseTuple(args, "sO!OO(OOOOOOOOOOO)O!O!", &path, &PyDict_Type, &spaces, &make, &raise, &cls[0],
+                        &cls[1], &cls[2], &cls[3], &cls[4], &cls[5], &cls[6], &cls[7], &cls[8], &cls[9], &cls[10],
+                        &PyDict_Type, &hooks, &PyDict_Type, &pre_hooks))
     return nullptr;
   void* so = dlopen(path, RTLD_NOW | RTLD_LOCAL);        // already loaded by ctypes: the same handle
   if (so == nullptr) {
@@ -751,9 +772,9 @@ PyObject* init(PyObject*, PyObject* args) {
   g_workspaces = Py_NewRef(spaces);
   g_make_workspace = Py_NewRef(make);
   g_raise = Py_NewRef(raise);
-  PyObject** to[7] = {&g_cache_cls, &g_ring_cls, &g_norm_cls, &g_recurrent_cls, &g_attention_cls, &g_mlp_cls,
-                      &g_residual_cls};
-  for (int i = 0; i < 7; ++i) *to[i] = Py_NewRef(cls[i]);
+  PyObject** to[11] = {&g_cache_cls, &g_ring_cls, &g_norm_cls, &g_recurrent_cls, &g_attention_cls, &g_mlp_cls,
+                       &g_residual_cls, &g_conv_cls, &g_lru_cls, &g_einsum_cls, &g_linear_cls};
+  for (int i = 0; i < 11; ++i) *to[i] = Py_NewRef(cls[i]);
   g_hooks = Py_NewRef(hooks);
   g_pre_hooks = Py_NewRef(pre_hooks);
   g_ready = true;

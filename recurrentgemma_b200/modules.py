@@ -52,6 +52,8 @@ def recurrent_path(
                                     inplace)
   if done is not NotImplemented:
     return done
+  if not (layers.as_built(conv_1d, layers.Conv1D) and layers.as_built(rg_lru, layers.RGLRU)):
+    return _composed_path(xb, yb, segment_pos, conv_1d, rg_lru, cache, return_cache, out, inplace)
   bs, l, e = xb.shape
   dev = _lib.require_cuda(xb, yb, segment_pos, conv_1d.w, rg_lru.a_param)
   layers._same_dtype(xb, conv_1d.w, conv_1d.b, rg_lru.a_param, rg_lru.input_gate.w,
@@ -101,6 +103,22 @@ def recurrent_path(
   if not return_cache:
     return out, None
   return out, RecurrentBlockCache(rg_lru_state=h_last, conv1d_state=conv_state)
+
+
+def _composed_path(xb, yb, segment_pos, conv_1d, rg_lru, cache, return_cache, out, inplace):
+  """`recurrent_path` by calling the two modules: they have hooks or a forward of their own."""
+  conv_state, h = (None, None) if cache is None else (cache.conv1d_state, cache.rg_lru_state)
+  want = return_cache or (cache is not None and inplace)
+  c, conv_state = conv_1d(xb, segment_pos, conv_state, want)
+  z, h = rg_lru(c, segment_pos, h, want)
+  if yb is not None:
+    z = z * torch.nn.functional.gelu(yb, approximate="tanh")
+  z = z if out is None else out.copy_(z)
+  if cache is not None and inplace:
+    cache.conv1d_state.copy_(conv_state)
+    cache.rg_lru_state.copy_(h)
+    return z, cache if return_cache else None
+  return z, RecurrentBlockCache(rg_lru_state=h, conv1d_state=conv_state) if return_cache else None
 
 
 @torch.no_grad()
@@ -177,7 +195,8 @@ def linear_pair(x: torch.Tensor, lin_a: nn.Linear, lin_b: nn.Linear
                 ) -> Tuple[torch.Tensor, torch.Tensor]:
   """(lin_a(x), lin_b(x)): one launch of the few-row kernel where it applies, else two `linear`."""
   rows = x.numel() // x.shape[-1]
-  if (rows < SMALL_M and _small_ok(x, lin_a.weight) and _small_ok(x, lin_b.weight)
+  if (rows < SMALL_M and layers.as_built(lin_a, nn.Linear) and layers.as_built(lin_b, nn.Linear)
+      and _small_ok(x, lin_a.weight) and _small_ok(x, lin_b.weight)
       and lin_a.weight.shape[0] % 128 == 0
       and all(l.bias is None or l.bias.is_contiguous() for l in (lin_a, lin_b))):
     return small_linear_pair(x, lin_a, lin_b)
@@ -192,9 +211,11 @@ def _small_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 def linear(x: torch.Tensor, lin: nn.Linear, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
   """lin(x) (+ residual): the prefill GEMM from SMALL_M rows on, the few-row kernel up to
-  SMALL_ROWS rows, torch in between and for float32."""
+  SMALL_ROWS rows, torch in between, for float32 and where `lin` is more than its parameters."""
   rows = x.numel() // x.shape[-1]
-  if x.dtype == torch.bfloat16 and rows >= SMALL_M:
+  if not layers.as_built(lin, nn.Linear):
+    y = lin(x)
+  elif x.dtype == torch.bfloat16 and rows >= SMALL_M:
     y = dense_linear(x, lin.weight, lin.bias)
   elif _small_ok(x, lin.weight):
     layers._same_dtype(x, lin.weight, *([lin.bias] if lin.bias is not None else []))
@@ -311,7 +332,11 @@ class RecurrentBlock(nn.Module):
   def _fusable(self, x: torch.Tensor, cache) -> bool:
     return (cache is None and x.dtype == torch.bfloat16
             and self.lru_width // self.num_heads == 256 and self.conv1d_temporal_width == 4
-            and self.width % 8 == 0 and self.rg_lru.gates_impl != _lib.GATES_SIMT)
+            and self.width % 8 == 0 and layers.as_built(self.conv_1d, layers.Conv1D)
+            and layers.as_built(self.rg_lru, layers.RGLRU)
+            and self.rg_lru.gates_impl != _lib.GATES_SIMT
+            and all(layers.as_built(lin, nn.Linear)
+                    for lin in (self.linear_y, self.linear_x, self.linear_out)))
 
   @classmethod
   def init_cache(cls, batch_size: int, lru_width: int, dtype: torch.dtype,
@@ -338,7 +363,9 @@ def recurrent_residual(
   the block's kernels, residual add in the epilogue of linear_out); other cases compose the
   modules."""
   dev = _lib.require_cuda(x, segment_pos, recurrent_block.linear_x.weight)
-  if recurrent_block._fusable(x, cache) and temporal_pre_norm.width == recurrent_block.width:
+  if (recurrent_block._fusable(x, cache) and temporal_pre_norm.width == recurrent_block.width
+      and layers.as_built(recurrent_block, RecurrentBlock)
+      and layers.as_built(temporal_pre_norm, layers.RMSNorm)):
     return recurrent_block._forward_fused(x, segment_pos, return_cache, dev, norm=temporal_pre_norm)
   y, new_cache = recurrent_block(temporal_pre_norm(x), segment_pos, cache, return_cache,
                                  inplace=inplace)
@@ -374,7 +401,11 @@ class MLPBlock(nn.Module):
     # below SMALL_M rows the 128 x 256 tiles of the GEMM leave most SMs without a tile (a decode
     # step has M = batch): library contractions, which split K, are used there
     return (x.dtype == torch.bfloat16 and self.width % 8 == 0 and self.expanded_width % 64 == 0
-            and x.numel() // x.shape[-1] >= SMALL_M)
+            and x.numel() // x.shape[-1] >= SMALL_M and self._as_built())
+
+  def _as_built(self) -> bool:
+    """Both contractions are their parameters and nothing else."""
+    return layers.as_built(self.ffw_up, layers.Einsum) and layers.as_built(self.ffw_down, nn.Linear)
 
   def invalidate_packed(self) -> None:
     """Drops the packed copy of ffw_up; the next forward rebuilds it.  Needed after a write that
@@ -412,6 +443,8 @@ class MLPBlock(nn.Module):
     """ffw_down(gelu(up_0) * up_1).  The two optional arguments (not in the reference) select the
     channel half of a residual block as one call: with `pre_norm` the MLP reads pre_norm(x) and
     x is added to the result; with `residual` alone that tensor is added."""
+    if pre_norm is not None and not layers.as_built(pre_norm, layers.RMSNorm):
+      residual, x, pre_norm = x, pre_norm(x), None
     dev = _lib.require_cuda(x, self.ffw_up.w)
     params = [self.ffw_up.w, self.ffw_up.b, self.ffw_down.weight, self.ffw_down.bias]
     if pre_norm is not None:
@@ -420,7 +453,8 @@ class MLPBlock(nn.Module):
     assert x.shape[-1] == self.width
     rows = x.numel() // x.shape[-1]
     if (x.dtype == torch.bfloat16 and rows <= SMALL_ROWS_MLP and rows < SMALL_M and self.width % 8 == 0
-        and self.expanded_width % 64 == 0 and self.ffw_down.weight.is_contiguous()):
+        and self.expanded_width % 64 == 0 and self.ffw_down.weight.is_contiguous()
+        and self._as_built()):
       # a decode step: both contractions on the few-row kernel, GeGLU and the residual add in
       # their epilogues
       xin = x if pre_norm is None else pre_norm(x)
@@ -433,20 +467,24 @@ class MLPBlock(nn.Module):
       return small_linear(hidden, self.ffw_down.weight, self.ffw_down.bias, residual=res)
     if not self._fusable(x):
       xin = x if pre_norm is None else pre_norm(x)
-      # ffw_up as two plain contractions (the einsum of layers.Einsum would first make a permuted
-      # copy of the weights): the contraction and the bias add are two tensor operations
-      w, bias = self.ffw_up.w, self.ffw_up.b.reshape(2, -1)
       xw = self.expanded_width
-      up = torch.matmul(xin.reshape(1, -1, self.width), w)          # [2, M, X], one batched call
-      if (xw * x.element_size()) % 16 == 0:
-        hidden = torch.empty((*x.shape[:-1], xw), dtype=x.dtype, device=dev)
-        with torch.cuda.device(dev):
-          _lib.check(_lib.load().rgk_geglu_bias(
-              up.data_ptr(), bias.contiguous().data_ptr(), up.shape[1], xw,
-              _lib.dtype_code(x.dtype), hidden.data_ptr(), _lib.stream_ptr(dev)))
+      if not layers.as_built(self.ffw_up, layers.Einsum):
+        gate, value = self.ffw_up(xin)
+        hidden = torch.nn.functional.gelu(gate, approximate="tanh") * value
       else:
-        gate, value = up[0] + bias[0], up[1] + bias[1]
-        hidden = (torch.nn.functional.gelu(gate, approximate="tanh") * value).reshape(*x.shape[:-1], xw)
+        # ffw_up as two plain contractions (the einsum of layers.Einsum would first make a permuted
+        # copy of the weights): the contraction and the bias add are two tensor operations
+        w, bias = self.ffw_up.w, self.ffw_up.b.reshape(2, -1)
+        up = torch.matmul(xin.reshape(1, -1, self.width), w)          # [2, M, X], one batched call
+        if (xw * x.element_size()) % 16 == 0:
+          hidden = torch.empty((*x.shape[:-1], xw), dtype=x.dtype, device=dev)
+          with torch.cuda.device(dev):
+            _lib.check(_lib.load().rgk_geglu_bias(
+                up.data_ptr(), bias.contiguous().data_ptr(), up.shape[1], xw,
+                _lib.dtype_code(x.dtype), hidden.data_ptr(), _lib.stream_ptr(dev)))
+        else:
+          gate, value = up[0] + bias[0], up[1] + bias[1]
+          hidden = (torch.nn.functional.gelu(gate, approximate="tanh") * value).reshape(*x.shape[:-1], xw)
       y = self.ffw_down(hidden)
       if pre_norm is not None:
         return y + x
@@ -495,14 +533,20 @@ def residual_block(
   if done is not NotImplemented:
     return done
   if (isinstance(temporal_block, RecurrentBlock) and temporal_block._fusable(x, cache)
-      and temporal_pre_norm.width == temporal_block.width):
+      and temporal_pre_norm.width == temporal_block.width
+      and layers.as_built(temporal_block, RecurrentBlock)
+      and layers.as_built(temporal_pre_norm, layers.RMSNorm)):
     # bfloat16 prefill of the recurrent kind: each half is one library call
     r, new_cache = recurrent_residual(x, segment_pos, temporal_pre_norm, temporal_block, cache,
                                       return_cache, inplace)
     return mlp_block(r, pre_norm=channel_pre_norm), new_cache
   y, new_cache = temporal_block(temporal_pre_norm(x), segment_pos, cache, return_cache,
                                 inplace=inplace)
-  r, normed = channel_pre_norm.add_norm(y, x)        # the residual add rides in the norm kernel
+  if layers.as_built(channel_pre_norm, layers.RMSNorm):
+    r, normed = channel_pre_norm.add_norm(y, x)      # the residual add rides in the norm kernel
+  else:
+    r = y + x
+    normed = channel_pre_norm(r)
   return mlp_block(normed, residual=r), new_cache
 
 
