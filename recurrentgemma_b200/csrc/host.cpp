@@ -7,7 +7,7 @@
 // device), so that every small call was bound by its host code.  Here they take a few microseconds.
 //
 // Every function returns NotImplemented for arguments it does not handle - a CPU tensor, a dtype
-// mismatch, a strided input, and wherever a module's parameters stand for a
+// mismatch, a strided input, parameters of another size, and wherever a module's parameters stand for a
 // call of the module, one of another class, with hooks or with a forward of its own (`plain`) - and the
 // Python form of the same forward then runs, which also raises the errors.  Nothing is cached here:
 // parameters are looked up in the modules on every call.
@@ -101,21 +101,21 @@ PyObject* entry(PyObject* module, PyObject* dict_name, PyObject* name) {
 }
 PyObject* submodule(PyObject* module, PyObject* name) { return entry(module, s__modules, name); }
 
-// A parameter of the activations' dtype on their device.
+// A parameter of the activations' dtype and the given sizes on their device.
 struct Params {
   at::ScalarType dtype;
   c10::Device device;
   bool ok = true;
-  const at::Tensor* get(PyObject* module, PyObject* name) {
+  const at::Tensor* get(PyObject* module, PyObject* name, at::IntArrayRef sizes) {
     const at::Tensor* t = module == nullptr ? nullptr : dense(entry(module, s__parameters, name));
-    if (t == nullptr || t->scalar_type() != dtype || t->device() != device) {
+    if (t == nullptr || t->scalar_type() != dtype || t->device() != device || t->sizes() != sizes) {
       ok = false;
       return nullptr;
     }
     return t;
   }
-  const void* ptr(PyObject* module, PyObject* name) {
-    const at::Tensor* t = get(module, name);
+  const void* ptr(PyObject* module, PyObject* name, at::IntArrayRef sizes) {
+    const at::Tensor* t = get(module, name, sizes);
     return t == nullptr ? nullptr : t->const_data_ptr();
   }
 };
@@ -245,15 +245,15 @@ Found path_params(PyObject* conv, PyObject* lru, Params& pr, int dt, long width,
   const long bw = width / *heads;
   PyObject* gx = submodule(lru, s_input_gate);
   PyObject* ga = submodule(lru, s_a_gate);
-  const at::Tensor* wx = pr.get(gx, s_w);
-  const at::Tensor* wa = pr.get(ga, s_w);
-  p->gate_x_b = pr.ptr(gx, s_b);
-  p->gate_a_b = pr.ptr(ga, s_b);
-  p->a_param = pr.ptr(lru, s_a_param);
+  const at::Tensor* wx = pr.get(gx, s_w, {*heads, bw, bw});
+  const at::Tensor* wa = pr.get(ga, s_w, {*heads, bw, bw});
+  p->gate_x_b = pr.ptr(gx, s_b, {*heads, bw});
+  p->gate_a_b = pr.ptr(ga, s_b, {*heads, bw});
+  p->a_param = pr.ptr(lru, s_a_param, {width});
   if (conv != nullptr) {
     long tw = 0;
-    p->conv_w = pr.ptr(conv, s_w);
-    p->conv_b = pr.ptr(conv, s_b);
+    p->conv_w = pr.ptr(conv, s_w, {4, width});
+    p->conv_b = pr.ptr(conv, s_b, {width});
     if (!int_attr(conv, s_temporal_width, &tw) || tw != 4) return Found::no;
   }
   if (!pr.ok) return Found::no;
@@ -418,9 +418,9 @@ Found recurrent_params(PyObject* block, Params& pr, long D, long E, rgk_block_pa
   if (!plain(ly, g_linear_cls) || !plain(lx, g_linear_cls) || !plain(lo, g_linear_cls) ||
       !plain(conv, g_conv_cls) || !plain(lru, g_lru_cls))
     return Found::no;
-  p->linear_y_w = pr.ptr(ly, s_weight); p->linear_y_b = pr.ptr(ly, s_bias);
-  p->linear_x_w = pr.ptr(lx, s_weight); p->linear_x_b = pr.ptr(lx, s_bias);
-  p->linear_out_w = pr.ptr(lo, s_weight); p->linear_out_b = pr.ptr(lo, s_bias);
+  p->linear_y_w = pr.ptr(ly, s_weight, {E, D}); p->linear_y_b = pr.ptr(ly, s_bias, {E});
+  p->linear_x_w = pr.ptr(lx, s_weight, {E, D}); p->linear_x_b = pr.ptr(lx, s_bias, {E});
+  p->linear_out_w = pr.ptr(lo, s_weight, {D, E}); p->linear_out_b = pr.ptr(lo, s_bias, {D});
   if (!pr.ok) return Found::no;
   return path_params(conv, lru, pr, RGK_BF16, E, &p->path, heads, impl, made);
 }
@@ -432,11 +432,11 @@ rgk_attention_params attention_params(PyObject* block, Params& pr, long D) {
            *f = submodule(block, s_proj_final);
   for (PyObject* m : {q, k, v, f}) pr.ok = pr.ok && plain(m, g_linear_cls);
   if (!pr.ok) return p;
-  p.q_w = pr.ptr(q, s_weight);
-  p.k_w = pr.ptr(k, s_weight);
-  p.v_w = pr.ptr(v, s_weight);
-  p.final_w = pr.ptr(f, s_weight);
-  p.final_b = pr.ptr(f, s_bias);
+  p.q_w = pr.ptr(q, s_weight, {D, D});
+  p.k_w = pr.ptr(k, s_weight, {256, D});
+  p.v_w = pr.ptr(v, s_weight, {256, D});
+  p.final_w = pr.ptr(f, s_weight, {D, D});
+  p.final_b = pr.ptr(f, s_bias, {D});
   return p;
 }
 
@@ -455,11 +455,11 @@ bool channel_params(PyObject* norm, PyObject* mlp, Params& pr, long D, Channel* 
     return false;
   PyObject *up = submodule(mlp, s_ffw_up), *down = submodule(mlp, s_ffw_down);
   if (!plain(up, g_einsum_cls) || !plain(down, g_linear_cls)) return false;
-  c->up_w = pr.get(up, s_w);
-  c->up_b = pr.get(up, s_b);
-  c->scale = pr.ptr(norm, s_scale);
-  c->down_w = pr.ptr(down, s_weight);
-  c->down_b = pr.ptr(down, s_bias);
+  c->up_w = pr.get(up, s_w, {2, D, c->X});
+  c->up_b = pr.get(up, s_b, {2, 1, 1, c->X});
+  c->scale = pr.ptr(norm, s_scale, {D});
+  c->down_w = pr.ptr(down, s_weight, {D, c->X});
+  c->down_b = pr.ptr(down, s_bias, {D});
   return pr.ok;
 }
 
@@ -491,7 +491,7 @@ PyObject* step(PyObject* x_arg, PyObject* pos_arg, PyObject* norm1, PyObject* bl
   c.down_w = ch.down_w;
   c.down_b = ch.down_b;
   c.eps = ch.eps;
-  const void* scale1 = pr.ptr(norm1, s_scale);
+  const void* scale1 = pr.ptr(norm1, s_scale, {D});
   if (!pr.ok) return not_here();
   const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const int pc = pos_code(*pos);
@@ -584,7 +584,7 @@ Found temporal_prefill(const at::Tensor& x, const at::Tensor& pos, PyObject* nor
   long w1 = 0, width = 0;
   if (norm != nullptr) {
     if (!plain(norm, g_norm_cls) || !plain(block, recurrent ? g_recurrent_cls : g_attention_cls)) return Found::no;
-    scale = pr.ptr(norm, s_scale);
+    scale = pr.ptr(norm, s_scale, {D});
     if (!pr.ok || !int_attr(norm, s_width, &w1) || w1 != D || !float_attr(norm, s_eps, &eps)) return Found::no;
   }
   if (!int_attr(block, s_width, &width) || width != D || D % 8 != 0) return Found::no;

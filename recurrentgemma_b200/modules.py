@@ -55,6 +55,7 @@ def recurrent_path(
   if not (layers.as_built(conv_1d, layers.Conv1D) and layers.as_built(rg_lru, layers.RGLRU)):
     return _composed_path(xb, yb, segment_pos, conv_1d, rg_lru, cache, return_cache, out, inplace)
   bs, l, e = xb.shape
+  assert e == conv_1d.width == rg_lru.width, (e, conv_1d.width, rg_lru.width)
   dev = _lib.require_cuda(xb, yb, segment_pos, conv_1d.w, rg_lru.a_param)
   layers._same_dtype(xb, conv_1d.w, conv_1d.b, rg_lru.a_param, rg_lru.input_gate.w,
                      rg_lru.input_gate.b, rg_lru.a_gate.w, rg_lru.a_gate.b)
@@ -130,7 +131,7 @@ def dense_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
   dev = _lib.require_cuda(x, weight, bias)
   layers._same_dtype(x, weight, *([bias] if bias is not None else []))
   n, k = weight.shape
-  assert x.shape[-1] == k
+  assert x.shape[-1] == k and (bias is None or bias.shape == (n,))
   xc, wc = x.contiguous(), weight.contiguous()
   bc = None if bias is None else bias.contiguous()
   out = torch.empty((*x.shape[:-1], n), dtype=x.dtype, device=dev)
@@ -157,6 +158,8 @@ def small_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
   m = xc.numel() // k
   n_out = n // 2 if act == _lib.ACT_GEGLU else n
   out = torch.empty((*x.shape[:-1], n_out), dtype=x.dtype, device=dev)
+  assert residual is None or residual.shape == out.shape
+  assert bias is None or bias.shape == (n,)
   rc = None if residual is None else residual.contiguous()
   bc = None if bias is None else bias.contiguous()
   lib = _lib.load()
@@ -335,8 +338,11 @@ class RecurrentBlock(nn.Module):
             and self.width % 8 == 0 and layers.as_built(self.conv_1d, layers.Conv1D)
             and layers.as_built(self.rg_lru, layers.RGLRU)
             and self.rg_lru.gates_impl != _lib.GATES_SIMT
-            and all(layers.as_built(lin, nn.Linear)
-                    for lin in (self.linear_y, self.linear_x, self.linear_out)))
+            and self.lru_width == self.conv_1d.width == self.rg_lru.width
+            and all(layers.as_built(lin, nn.Linear) and lin.weight.shape == (n, k) for lin, n, k in (
+                (self.linear_y, self.lru_width, self.width),
+                (self.linear_x, self.lru_width, self.width),
+                (self.linear_out, self.width, self.lru_width))))
 
   @classmethod
   def init_cache(cls, batch_size: int, lru_width: int, dtype: torch.dtype,
@@ -404,8 +410,10 @@ class MLPBlock(nn.Module):
             and x.numel() // x.shape[-1] >= SMALL_M and self._as_built())
 
   def _as_built(self) -> bool:
-    """Both contractions are their parameters and nothing else."""
-    return layers.as_built(self.ffw_up, layers.Einsum) and layers.as_built(self.ffw_down, nn.Linear)
+    """Both contractions are their parameters and nothing else, in the block's sizes."""
+    d, e = self.width, self.expanded_width
+    return (layers.as_built(self.ffw_up, layers.Einsum) and self.ffw_up.w.shape == (2, d, e)
+            and layers.as_built(self.ffw_down, nn.Linear) and self.ffw_down.weight.shape == (d, e))
 
   def invalidate_packed(self) -> None:
     """Drops the packed copy of ffw_up; the next forward rebuilds it.  Needed after a write that

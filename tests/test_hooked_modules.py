@@ -1,5 +1,6 @@
 """Fused calls read the parameters of a block's modules instead of calling them; a module with hooks, a
-forward of its own or of another class is called all the same.  The calls on blocks need a B200."""
+forward of its own or of another class is called all the same, and parameters of another size than the
+block's are refused.  The calls on blocks need a B200."""
 import pytest
 import torch
 
@@ -70,6 +71,20 @@ def test_module_is_called(kind, name, batch, seq, how):
   got = _call(block, kind, batch, seq)
   assert calls, f"{name} was passed by"
   _close(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,seq", CALLS)
+@pytest.mark.parametrize("kind,name,n_in,n_out", [
+    ("recurrent", "linear_x", WIDTH, 2 * WIDTH), ("recurrent", "linear_out", WIDTH, 2 * WIDTH),
+    ("attention", "proj_k", WIDTH, 512), ("attention", "proj_final", WIDTH, 2 * WIDTH),
+    ("recurrent", "ffw_down", EXPANDED, 2 * WIDTH)])
+def test_other_sizes_are_refused(kind, name, n_in, n_out, batch, seq):
+  block = _block(kind)
+  owner = block.mlp_block if name == "ffw_down" else block.temporal_block
+  setattr(owner, name, torch.nn.Linear(n_in, n_out, bias=name != "proj_k", device=DEV, dtype=BF16))
+  with pytest.raises((AssertionError, RuntimeError)):
+    _call(block, kind, batch, seq)
 
 
 def test_as_built():
