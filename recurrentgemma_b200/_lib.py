@@ -5,9 +5,11 @@ the tensors are not on a CUDA device of compute capability 10.x, the call raises
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import threading
+import weakref
 from typing import Optional
 
 import torch
@@ -254,6 +256,31 @@ def workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
   return buf
 
 
+# Buffers that have left the table below with the CUDA graph that holds their addresses (weak: the graph's
+# owner keeps them).
+_owned = []
+
+
+@contextlib.contextmanager
+def own_workspace(dev: torch.device):
+  """Within, the calls on the current stream have scratch buffers of their own, which nothing uses
+  afterwards: they belong to a CUDA graph captured here, which may be replayed on any stream while
+  others run.  Yields the list that holds them in the end; keep it as long as the graph."""
+  key = (dev.index if dev.index is not None else torch.cuda.current_device(),
+         torch.cuda.current_stream(dev).cuda_stream)
+  before = [table.pop(key, None) for table in (_workspaces, _retired)]
+  held = []
+  try:
+    yield held
+  finally:
+    held += [_workspaces.pop(key, None), *_retired.pop(key, [])]
+    held[:] = [b for b in held if b is not None]
+    _owned[:] = [r for r in _owned if r() is not None] + [weakref.ref(b) for b in held]
+    for table, entry in zip((_workspaces, _retired), before):
+      if entry is not None:
+        table[key] = entry
+
+
 def workspace_bytes(b: int, t: int, e: int, dt: torch.dtype) -> int:
   return int(load().rgk_workspace_bytes(b, t, e, dtype_code(dt)))
 
@@ -275,7 +302,8 @@ def check_status(device: Optional[torch.device] = None) -> None:
   """Raises RgkError(RGK_ETIMEOUT) if any kernel launched through this package on `device` (every
   stream that has a workspace) gave up on a bounded wait since the last check.  The kernels finish
   on their own after such an expiry, but what they computed is invalid, and nothing else reports
-  it: call this wherever the host synchronises anyway (it synchronises those streams)."""
+  it: call this wherever the host synchronises anyway (it synchronises those streams, and the device
+  where captured graphs have scratch of their own)."""
   index = None
   if device is not None:
     device = torch.device(device)
@@ -285,3 +313,8 @@ def check_status(device: Optional[torch.device] = None) -> None:
       with torch.cuda.device(dev_index):
         for b in [buf, *_retired.get((dev_index, stream), [])]:
           workspace_status(b, stream)
+  for buf in [r() for r in list(_owned)]:
+    if buf is not None and (index is None or buf.device.index == index):
+      with torch.cuda.device(buf.device):
+        torch.cuda.synchronize(buf.device)
+        workspace_status(buf)

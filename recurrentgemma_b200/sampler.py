@@ -12,6 +12,7 @@ the reference `Sampler`, which can drive a `recurrentgemma_b200.Griffin` unchang
 from __future__ import annotations
 
 import gc
+import threading
 from typing import NamedTuple, Optional
 
 import torch
@@ -62,34 +63,46 @@ class GreedySampler:
       state = {"last_token": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "positions": torch.zeros((b, 1), dtype=torch.int32, device=dev),
                "cache": _own(cache), "logits": None}
-      # one eager step on the capture stream creates every lazily made buffer of a decode step (the
-      # stream's workspace among them, which must not come from the graph's own memory pool: it
-      # outlives this graph); capturing then records the launches without running them
+      graph = self._capture(state)
+      self._state, self._graph, self._graph_key = state, graph, (b, dev)
+    # the buffers were made on another stream than they are used on from here
+    stream = torch.cuda.current_stream(dev)
+    for t in [*self._state["scratch"], self._state["last_token"], self._state["positions"],
+              *[t for c in self._state["cache"].values() for t in c]]:
+      t.record_stream(stream)
+    for name, c in cache.items():
+      for dst, src in zip(self._state["cache"][name], c):
+        dst.copy_(src)
+    return self._state, self._graph
+
+  def _capture(self, state) -> torch.cuda.CUDAGraph:
+    """The CUDA graph of one step on `state`, whose scratch buffers become part of `state`: replays of
+    several samplers may overlap, on whatever streams they are called."""
+    dev = self.device
+    with _capture_lock:
       stream = _capture_stream(dev)
       stream.wait_stream(torch.cuda.current_stream(dev))
-      with torch.cuda.stream(stream):
+      with torch.cuda.stream(stream), _lib.own_workspace(dev) as scratch:
+        # one eager step on the capture stream creates every lazily made buffer of a decode step (the
+        # scratch among them); capturing then records the launches without running them
         self._step(state)
-      graph = torch.cuda.CUDAGraph()
-      torch.cuda.synchronize(dev)
-      # without the emptied allocator cache that `with torch.cuda.graph(...)` begins with: in a
-      # program that holds gigabytes of cached blocks freeing and allocating them again took up to 1.4 s
-      collecting = gc.isenabled()
-      gc.disable()                       # nothing of another graph is to be destroyed meanwhile
-      try:
-        with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize(dev)
+        # without the emptied allocator cache that `with torch.cuda.graph(...)` begins with: in a program
+        # that holds gigabytes of cached blocks freeing and allocating them again took up to 1.4 s
+        collecting = gc.isenabled()
+        gc.disable()                     # nothing of another graph is to be destroyed meanwhile
+        try:
           graph.capture_begin()
           try:
             self._step(state)
           finally:
             graph.capture_end()
-      finally:
-        if collecting:
-          gc.enable()
-      self._state, self._graph, self._graph_key = state, graph, (b, dev)
-    for name, c in cache.items():
-      for dst, src in zip(self._state["cache"][name], c):
-        dst.copy_(src)
-    return self._state, self._graph
+        finally:
+          if collecting:
+            gc.enable()
+      state["scratch"] = scratch
+    return graph
 
   def _step(self, state) -> None:
     """One sampling step (recurrentgemma/torch/sampler.py:137-187) on static buffers: reads
@@ -164,10 +177,11 @@ class GreedySampler:
 
 
 _capture_streams = {}
+_capture_lock = threading.Lock()
 
 
 def _capture_stream(dev: torch.device) -> torch.cuda.Stream:
-  """The one stream per device that samplers capture their graphs on."""
+  """The one stream per device that samplers capture their graphs on, one after the other."""
   index = dev.index if dev.index is not None else torch.cuda.current_device()
   if index not in _capture_streams:
     _capture_streams[index] = torch.cuda.Stream(index)
