@@ -233,26 +233,32 @@ def stream_ptr(dev: torch.device) -> int:
 
 
 # One growing scratch buffer per (device, stream): calls on one stream are ordered, so they can
-# share it; different streams get different buffers.  A buffer that has become too small is retired,
-# not freed: a CUDA graph captured while it was current holds its address.  Buffers at least double,
-# so the retired ones of a stream together are no larger than its current one.
+# share it; different streams get different buffers.  A buffer that has become too small goes back to
+# the allocator, unless a call under capture has used it: a CUDA graph may hold its address then, and it
+# is kept as long as the process.
 _workspaces = {}
 _retired = {}
+_in_graphs = set()             # keys whose current buffer a capture has used
 
 
 def workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
   key = (dev.index if dev.index is not None else torch.cuda.current_device(),
          torch.cuda.current_stream(dev).cuda_stream)
-  buf = _workspaces.get(key)
-  if buf is None or buf.numel() < nbytes:
-    size = max(nbytes, 1 << 20) if buf is None else max(nbytes, 2 * buf.numel())
-    with torch.cuda.device(dev):
-      new = torch.empty(size, dtype=torch.uint8, device=dev)
+  with torch.cuda.device(dev):
+    buf = _workspaces.get(key)
+    if buf is None or buf.numel() < nbytes:
+      new = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
       # the status word (first int): kernels only ever raise it, nobody but its reader clears it
-      new[:4].zero_()
-    if buf is not None:
-      _retired.setdefault(key, []).append(buf)
-    _workspaces[key] = buf = new
+      if buf is None or key in _in_graphs:
+        new[:4].zero_()
+      else:
+        new[:4].copy_(buf[:4])
+      if key in _in_graphs:
+        _retired.setdefault(key, []).append(buf)
+        _in_graphs.remove(key)
+      _workspaces[key] = buf = new
+    if torch.cuda.is_current_stream_capturing():
+      _in_graphs.add(key)
   return buf
 
 
@@ -269,6 +275,8 @@ def own_workspace(dev: torch.device):
   key = (dev.index if dev.index is not None else torch.cuda.current_device(),
          torch.cuda.current_stream(dev).cuda_stream)
   before = [table.pop(key, None) for table in (_workspaces, _retired)]
+  captured = key in _in_graphs
+  _in_graphs.discard(key)
   held = []
   try:
     yield held
@@ -279,6 +287,9 @@ def own_workspace(dev: torch.device):
     for table, entry in zip((_workspaces, _retired), before):
       if entry is not None:
         table[key] = entry
+    _in_graphs.discard(key)
+    if captured:
+      _in_graphs.add(key)
 
 
 def workspace_bytes(b: int, t: int, e: int, dt: torch.dtype) -> int:

@@ -14,6 +14,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
@@ -167,7 +168,8 @@ at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, c10::Device dev) {
 }
 PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
-// The scratch buffer of (device, stream), shared with the Python side, of at least `bytes` bytes.
+// The scratch buffer of (device, stream), shared with the Python side, of at least `bytes` bytes.  (The Python
+// side is asked for it under capture too: it keeps what a graph may hold the address of.)
 struct Workspace {
   void* ptr = nullptr;
   size_t bytes = 0;
@@ -177,8 +179,8 @@ bool workspace(const at::Tensor& on, cudaStream_t stream, size_t bytes, Workspac
   if (key.p == nullptr) return false;
   PyObject* buf = PyDict_GetItemWithError(g_workspaces, key.p);
   Ref made(nullptr);
-  if (buf == nullptr || !THPVariable_Check(buf) ||
-      (size_t)THPVariable_Unpack(buf).numel() < bytes) {
+  if (buf == nullptr || !THPVariable_Check(buf) || (size_t)THPVariable_Unpack(buf).numel() < bytes ||
+      c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
     if (PyErr_Occurred()) return false;
     Ref dev(THPDevice_New(on.device()));
     Ref n(PyLong_FromSize_t(bytes));
