@@ -285,7 +285,7 @@ constexpr float kSlack = 8.0f / kLogitScale;         // logits a row may exceed 
 
 __global__ void __launch_bounds__(kThreadsA, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                    const __grid_constant__ CUtensorMap map_vt, const int* __restrict__ lo_all, int B,
+                    const __grid_constant__ CUtensorMap map_vt, const int* lo_all, int B,
                     int T_, int N, int window, int n_units, __nv_bfloat16* __restrict__ out,
                     int* status) {
   extern __shared__ uint8_t smem_raw[];

@@ -67,7 +67,7 @@ template <> struct PackOps<__nv_bfloat16> {
 
 template <typename T>
 __global__ void __launch_bounds__(kConvThreads)
-conv1d_prefill_kernel(const T* __restrict__ x, const void* __restrict__ pos, int pos64,
+conv1d_prefill_kernel(const T* x, const void* pos, int pos64,
                       const T* __restrict__ w, const T* __restrict__ bias, int T_, int E,
                       T* __restrict__ out, T* __restrict__ cache_out, const ChanPrep prep) {
   constexpr int kPack = Traits<T>::kPack;

@@ -59,8 +59,8 @@ __device__ __forceinline__ uint4 add4(const uint4& a, const uint4& b) {
 // a = exp(log_a) and the input multiplier from a shared-memory table, built in the prologue.
 template <bool kMul, int kMath>
 __global__ void __launch_bounds__(kThreadsDec, 1)
-decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* __restrict__ xb,
-                 const __nv_bfloat16* __restrict__ yb, const void* __restrict__ pos, int pos64,
+decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* xb,
+                 const __nv_bfloat16* yb, const void* pos, int pos64,
                  const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ conv_b,
                  const __nv_bfloat16* __restrict__ a_param, const __nv_bfloat16* __restrict__ bias_x,
                  const __nv_bfloat16* __restrict__ bias_a, const float* h_in,

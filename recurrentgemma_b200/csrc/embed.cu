@@ -45,7 +45,7 @@ __global__ void embed_kernel(const void* __restrict__ tokens, int tokens64, cons
 // between threads go to the smaller index.
 constexpr int kArgmaxCluster = 8;
 template <typename T>
-__global__ void argmax_kernel(const T* __restrict__ x, int64_t M, int64_t V, int parts, int* __restrict__ out) {
+__global__ void argmax_kernel(const T* x, int64_t M, int64_t V, int parts, int* __restrict__ out) {
   constexpr int kPer = 16 / (int)sizeof(T);
   __shared__ float s_val[32];
   __shared__ int s_idx[32];

@@ -81,8 +81,8 @@ __device__ __forceinline__ float tf32_low_part(float v) { return v - tf32_high_p
 template <int kTN, int kPerSm>
 __global__ void __launch_bounds__((Cfg<kTN, kPerSm>::kThreads), kPerSm)
 gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wh,
-                  const __grid_constant__ CUtensorMap map_wl, const float* __restrict__ x,
-                  const void* __restrict__ pos, int pos64, const float* __restrict__ a_param,
+                  const __grid_constant__ CUtensorMap map_wl, const float* x,
+                  const void* pos, int pos64, const float* __restrict__ a_param,
                   const float* __restrict__ bias_x, const float* __restrict__ bias_a, int64_t M,
                   int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr, const ScanPrep prep) {
   using C = Cfg<kTN, kPerSm>;
@@ -230,7 +230,7 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       for (int k = 0; k < 8; ++k) {
         const int r = cr + 4 * k;
         cin[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row0 + r < M) cin[k] = __ldg(reinterpret_cast<const float4*>(x + (row0 + r) * E + e0 + cp * 4));
+        if (row0 + r < M) cin[k] = *reinterpret_cast<const float4*>(x + (row0 + r) * E + e0 + cp * 4);
       }
       if (ok) ok = mbar_wait(bar_acc, 0, s_abort);             // every MMA has read the ring by now
       __syncwarp();

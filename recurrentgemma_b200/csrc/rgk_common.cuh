@@ -88,10 +88,11 @@ template <> __device__ __forceinline__ uint4 pack<__nv_bfloat16>(const float* f)
                     pack_bf16x2(f[6], f[7]));
 }
 
-// Streaming 16-byte global access: activations are touched once, keep them out of L1.
+// Streaming 16-byte global access: activations are touched once, keep them out of L1.  (Ordinary loads, not
+// .nc: a kernel launched as a dependent may have started before the data were written, see launch_dependent.)
 __device__ __forceinline__ uint4 ld_stream(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }

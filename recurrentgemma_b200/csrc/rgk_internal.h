@@ -42,7 +42,8 @@ class PerDeviceOnce {
 
 // A launch that may be placed while the kernel in front still runs (programmatic dependent launch): every
 // CTA of `kernel` executes griddepcontrol.wait before it touches memory that a kernel may have written
-// or still reads.
+// or still reads.  Such a kernel promises of nothing but weights that it does not change while it runs: no
+// __restrict__ on other pointers that it reads, no __ldg, no ld.global.nc.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchAttribute attr[1];

@@ -271,9 +271,9 @@ template <int kJoin, int kMath, bool kConv>
 __global__ void __launch_bounds__(kConv ? kThreadsConv : kThreads, 1)
 rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_w,
                   const __grid_constant__ CUtensorMap map_ct, const __grid_constant__ CUtensorMap map_yt,
-                  const __grid_constant__ CUtensorMap map_ot, const void* __restrict__ pos, int pos64,
+                  const __grid_constant__ CUtensorMap map_ot, const void* pos, int pos64,
                   const __nv_bfloat16* __restrict__ bias_x, const __nv_bfloat16* __restrict__ bias_a,
-                  const __nv_bfloat16* m8sp, const float* __restrict__ h0, int B, int T_,
+                  const __nv_bfloat16* m8sp, const float* h0, int B, int T_,
                   int E, int groups, int n_units, float* __restrict__ h_last, WsHeader* hdr,
                   unsigned long long* agg, unsigned long long* incl, int use_agg,
                   const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ conv_b) {

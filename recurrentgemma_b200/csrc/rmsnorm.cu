@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t bf2add(uint32_t a, uint32_t b) {
 
 template <typename T, int kPacks>   // kPacks: packs per lane this instantiation can hold
 __global__ void __launch_bounds__(kNormWarps * 32)
-rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ addend, const T* __restrict__ scale,
+rmsnorm_kernel(const T* x, const T* addend, const T* __restrict__ scale,
                int64_t M, int D, float eps, T* __restrict__ sum_out, T* __restrict__ out) {
   constexpr int kPack = Traits<T>::kPack;
   constexpr bool kBf16 = Traits<T>::kBf16;
@@ -119,7 +119,7 @@ constexpr int kRowThreads = 128;
 
 template <int kPacks>
 __global__ void __launch_bounds__(kRowThreads)
-rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ scale, int D,
+rmsnorm_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ scale, int D,
                    float eps, int early, __nv_bfloat16* __restrict__ out) {
   __shared__ float s_sum[kRowThreads / 32];
   const int packs = D / 8, tid = threadIdx.x;

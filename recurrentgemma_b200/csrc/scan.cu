@@ -100,8 +100,8 @@ template <typename T> struct ScanSmem {
 template <typename T, int kJoin>   // 0: no join, 1: y * gelu_tanh(y_mul), 2: y * y_mul
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4)
 scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_a,
-            const uint8_t* __restrict__ reset, const void* __restrict__ pos, int pos64,
-            const float* __restrict__ h0, const T* __restrict__ y_mul, int B, int T_, int E,
+            const uint8_t* reset, const void* pos, int pos64,
+            const float* h0, const T* y_mul, int B, int T_, int E,
             int tiles_t, int groups, T* __restrict__ y, float* __restrict__ h_last, WsHeader* hdr,
             unsigned* flags, float2* agg, float* incl, unsigned ticket_base, unsigned spin_limit) {
   using Cfg = ScanCfg<T>;
