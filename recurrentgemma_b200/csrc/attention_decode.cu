@@ -455,8 +455,10 @@ attn_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
     }
     if (lane == 0) {
-      s_m[h] = with_new ? round_bf16(round_bf16(dot) * 0.0625f) : kMasked;
-      s_l[h] = with_new ? 1.0f : 0.0f;
+      // (the maximum stays a number, and above -inf; a logit that is neither leaves its mark in the sum)
+      const float x = round_bf16(round_bf16(dot) * 0.0625f), m = with_new ? fmaxf(x, kMasked) : kMasked;
+      s_m[h] = m;
+      s_l[h] = with_new ? __expf(x - m) : 0.0f;
     }
   }
   if (with_new) {
@@ -479,6 +481,14 @@ attn_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int m_row = (lane & 7) + ((lane >> 3) & 1) * 8;      // row of an 8 x 8 matrix pair this lane names
   const int m_piece = lane >> 4;
   __syncthreads();
+  if (with_new) {                                  // (times one, unless the new logit is infinite or no number)
+    const float f0 = s_l[g], f1 = s_l[g + 8];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      acc[n][0] *= f0; acc[n][1] *= f0;
+      acc[n][2] *= f1; acc[n][3] *= f1;
+    }
+  }
 
   bool ok = true;
   for (int i = 0; i < n_st; ++i) {
@@ -522,14 +532,15 @@ attn_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         // two tensor operations in the reference: the contraction, then the scaling by 256^-1/2
         float x = round_bf16(round_bf16(l0[0] + l1[0]) * 0.0625f);
         float y = round_bf16(round_bf16(l0[kLogPitch] + l1[kLogPitch]) * 0.0625f);
-        if (e >= lim) x = kMasked;
-        if (e + 1 >= lim) y = kMasked;
+        if (e >= lim) x = -INFINITY;
+        if (e + 1 >= lim) y = -INFINITY;
         float mx = fmaxf(x, y);
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_old = s_m[h], l_old = s_l[h];
         const float m = fmaxf(mx, m_old);
-        const float p0 = x > kMasked ? __expf(x - m) : 0.0f, p1 = y > kMasked ? __expf(y - m) : 0.0f;
+        // (0 where nothing is visible: m is at least kMasked; what is no number stays none)
+        const float p0 = __expf(x - m), p1 = __expf(y - m);
         float sum = p0 + p1;
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

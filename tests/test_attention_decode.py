@@ -70,3 +70,36 @@ def test_decode(batch, heads, window):
   assert torch.equal(ring.keys.view(torch.int16), new.keys.view(torch.int16))
   assert torch.equal(ring.values.view(torch.int16), new.values.view(torch.int16))
   assert torch.equal(ring.num_tokens, new.num_tokens)
+
+
+# what a key or the new key holds; whether torch's softmax over such logits is a number
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("where", ["ring", "new"])
+@pytest.mark.parametrize("batch,window", [(2, 100), (1, 2048)])
+def test_logits_that_are_no_numbers(value, where, batch, window):
+  """Through the attention proper: every head of the sequence is what softmax makes of its logits - NaN for
+  a NaN or +inf logit, weight zero for -inf - and the other sequence is left alone."""
+  from recurrentgemma_b200 import _lib
+  torch.manual_seed(window)
+  heads, lib = 2, _lib.load()
+  q = torch.randn(batch, heads, 256, device=DEV).to(BF16)
+  k, v = (torch.randn(batch, 256, device=DEV).to(BF16) for _ in range(2))
+  keys, values = (torch.randn(batch, window, 256, device=DEV).to(BF16) for _ in range(2))
+  q[0, :, 0] = 2.0                                 # the sign of an infinite logit
+  (keys[0, 37] if where == "ring" else k[0])[0] = value
+  seen = torch.full((batch,), 2 * window, device=DEV, dtype=torch.int32)
+  ks, vs = torch.cat([keys, k[:, None]], 1).float(), torch.cat([values, v[:, None]], 1).float()
+  logits = (torch.einsum("bnh,bsh->bns", q.float(), ks).to(BF16) * 0.0625).float()
+  want = torch.einsum("bns,bsh->bnh", torch.softmax(logits, -1), vs).reshape(batch, -1)
+  out = torch.empty(batch, heads * 256, device=DEV, dtype=BF16)
+  ws = torch.zeros(lib.rgk_attention_decode_workspace_bytes(batch, heads, window), dtype=torch.uint8,
+                   device=DEV)
+  _lib.check(lib.rgk_local_attention_decode(
+      q.data_ptr(), k.data_ptr(), v.data_ptr(), keys.data_ptr(), values.data_ptr(), seen.data_ptr(),
+      batch, heads, 256, window, _lib.RGK_BF16, 0, out.data_ptr(), ws.data_ptr(), ws.numel(),
+      _lib.stream_ptr(q.device)))
+  assert torch.equal(torch.isnan(out), torch.isnan(want))
+  assert torch.isnan(want[0]).all().item() == (value != -float("inf"))
+  fine = ~torch.isnan(want)
+  if fine.any():                                   # weights rounded to 2^-9, the output to 2^-9
+    assert ((out[fine].float() - want[fine]).norm() / want[fine].norm()).item() <= 2.0 ** -7
