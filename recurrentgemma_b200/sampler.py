@@ -65,10 +65,14 @@ class GreedySampler:
                "cache": _own(cache), "logits": None}
       graph = self._capture(state)
       self._state, self._graph, self._graph_key = state, graph, (b, dev)
-    # the buffers were made on another stream than they are used on from here
+    # what was made on another stream than it is used on from here: the scratch always, the rest if the
+    # caller has changed streams
     stream = torch.cuda.current_stream(dev)
-    for t in [*self._state["scratch"], self._state["last_token"], self._state["positions"],
-              *[t for c in self._state["cache"].values() for t in c]]:
+    used = list(self._state["scratch"])
+    if stream != self._state["stream"]:
+      used += [self._state["last_token"], self._state["positions"],
+               *[t for c in self._state["cache"].values() for t in c]]
+    for t in used:
       t.record_stream(stream)
     for name, c in cache.items():
       for dst, src in zip(self._state["cache"][name], c):
@@ -101,7 +105,7 @@ class GreedySampler:
         finally:
           if collecting:
             gc.enable()
-      state["scratch"] = scratch
+      state["scratch"], state["stream"] = scratch, torch.cuda.current_stream(dev)
     return graph
 
   def _step(self, state) -> None:
