@@ -276,6 +276,8 @@ class RGLRU(nn.Module):
       with torch.cuda.device(wx.device):
         _lib.check(lib.rgk_pack_gate_weights(ctypes.byref(p), self.num_heads, 256, dt,
                                              buf.data_ptr(), _lib.stream_ptr(wx.device)))
+        if torch.cuda.is_current_stream_capturing():
+          key = None               # nothing has been packed yet: the graph will, for itself
       self._pack_buf, self._pack_key = buf, key
     return self._pack_buf.data_ptr()
 

@@ -442,6 +442,8 @@ class MLPBlock(nn.Module):
       with torch.cuda.device(w.device):
         _lib.check(lib.rgk_pack_mlp_up(w.data_ptr(), b.data_ptr(), self.width, self.expanded_width,
                                        _lib.RGK_BF16, buf.data_ptr(), _lib.stream_ptr(w.device)))
+        if torch.cuda.is_current_stream_capturing():
+          key = None               # nothing has been packed yet: the graph will, for itself
       self._pack_buf, self._pack_key = buf, key
     return self._pack_buf.data_ptr()
 
