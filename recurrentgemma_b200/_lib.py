@@ -244,21 +244,21 @@ _in_graphs = set()             # keys whose current buffer a capture has used
 def workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
   key = (dev.index if dev.index is not None else torch.cuda.current_device(),
          torch.cuda.current_stream(dev).cuda_stream)
-  with torch.cuda.device(dev):
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
+  buf = _workspaces.get(key)
+  if buf is None or buf.numel() < nbytes:
+    with torch.cuda.device(dev):
       new = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
       # the status word (first int): kernels only ever raise it, nobody but its reader clears it
       if buf is None or key in _in_graphs:
         new[:4].zero_()
       else:
         new[:4].copy_(buf[:4])
-      if key in _in_graphs:
-        _retired.setdefault(key, []).append(buf)
-        _in_graphs.remove(key)
-      _workspaces[key] = buf = new
-    if torch.cuda.is_current_stream_capturing():
-      _in_graphs.add(key)
+    if key in _in_graphs:
+      _retired.setdefault(key, []).append(buf)
+      _in_graphs.remove(key)
+    _workspaces[key] = buf = new
+  if torch.cuda.is_current_stream_capturing():      # (dev is the current device where kernels are launched)
+    _in_graphs.add(key)
   return buf
 
 

@@ -730,6 +730,22 @@ PyObject* block_step(PyObject* const* args, Py_ssize_t n) {
               PyObject_IsTrue(args[5]) == 1, PyObject_IsTrue(args[6]) == 1);
 }
 
+// as_built(module, class): `plain`, for the Python forms, which also take a subclass that keeps the forward.
+PyObject* as_built(PyObject* const* args, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "as_built(module, class)");
+    return nullptr;
+  }
+  if (g_hooks == nullptr || !no_global_hooks()) Py_RETURN_FALSE;
+  PyObject *module = args[0], *cls = args[1], *type = (PyObject*)Py_TYPE(module);
+  if (type != cls) {
+    Ref own(PyObject_GetAttr(type, s_forward)), theirs(PyObject_GetAttr(cls, s_forward));
+    if (own.p == nullptr || theirs.p == nullptr) PyErr_Clear();
+    if (own.p != theirs.p || own.p == nullptr) Py_RETURN_FALSE;
+  }
+  return PyBool_FromLong(plain(module, type));
+}
+
 // ---- set-up --------------------------------------------------------------------------------------
 // init(librgk path, _workspaces, workspace, check, (RecurrentBlockCache, AttentionBlockCache, RMSNorm,
 // RecurrentBlock, LocalAttentionBlock, MLPBlock, ResidualBlock, Conv1D, RGLRU, Einsum, nn.Linear), torch's
@@ -804,6 +820,7 @@ PyMethodDef methods[] = {
     FAST(block_step),
     FAST(prefill),
     FAST(residual_prefill),
+    FAST(as_built),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr,
                           nullptr};

@@ -34,10 +34,7 @@ def _same_dtype(x: torch.Tensor, *params: torch.Tensor) -> None:
 def as_built(module: nn.Module, cls: type) -> bool:
   """Whether calling `module` is running `cls.forward` on its parameters and nothing else: no hooks, no
   forward of its own.  Only then may its parameters stand for the call in a fused one."""
-  hooks = torch.nn.modules.module
-  return (getattr(type(module), "forward", None) is cls.forward and "forward" not in module.__dict__
-          and not module._forward_hooks and not module._forward_pre_hooks
-          and not hooks._global_forward_hooks and not hooks._global_forward_pre_hooks)
+  return _lib.host().as_built(module, cls)
 
 
 def _pos(segment_pos: torch.Tensor, bs: int, l: int) -> torch.Tensor:
