@@ -495,24 +495,30 @@ int rgk_dense_linear(const void* x, const void* weight, const void* bias, int64_
   return RGK_OK;
 }
 
+static constexpr int kRowsGemm = 8;                // rows that the kernel that streams weights into registers takes
+
 // Up to how many rows the few-row kernels take a projection.  Every SM has weights to stream there, where
 // a pair of CTAs of the GEMM walks all of K for its tile: at 128 rows 9.2 us against 11.2 for 2560 x
 // 2560 and 14.9 against 24.1 for 7680 -> 2560, at 199 12.8 / 11.4 and 17.9 / 25.4, at 300 21.3 / 27.0 for
 // the latter; wide outputs fill the chip sooner (2560 -> 15360: 16.6 / 19.0 at 48 rows, 21.7 / 20.3 at 128).
-static bool few_rows(int64_t M, int64_t K, int64_t N) {
+// From two tiles of 128 features an SM on (logits) the persistent form of the GEMM has its epilogues under the
+// loads of the next tile and the few-row kernel has not: 2560 -> 256000 at 9, 33 and 64 rows 307 / 226,
+// 421 / 229 and 360 / 226, 2560 -> 64000 86 / 76, 111 / 77 and 106 / 74; plain: nothing but the cap follows.
+static bool few_rows(int64_t M, int64_t K, int64_t N, bool plain = false) {
+  if (plain && N >= 2 * 128 * 148) return false;
   return M <= (N >= 4 * K ? 96 : (K >= 2 * N ? 352 : 160));
 }
 
 // Projections of few rows on the kernel for their number: up to kRowsGemm rows the one that streams
 // weights into registers, above that the one with 128-feature tensor-core tiles, and the GEMM of many rows
 // where that is faster (its epilogues have gelu or a residual, not both).
-static constexpr int kRowsGemm = 8;
 static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats,
                                    const void* residual, int64_t M, int K, int act, float cap, int* status,
                                    bool early, bool wide, cudaStream_t s) {
   if (M <= kRowsGemm)
     return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
-  if (!few_rows(M, K, mats[0].n) && (act == 0 || residual == nullptr))
+  const bool plain = n_mats == 1 && act == 0 && residual == nullptr;
+  if (!few_rows(M, K, mats[0].n, plain) && (act == 0 || residual == nullptr))
     return rgk::launch_dense_tc(x, mats, n_mats, residual, M, K, act, status, s, cap);
   return rgk::launch_dense_small(x, mats, n_mats, residual, M, K, act, cap, status, early, wide, s);
 }

@@ -2,7 +2,8 @@
 // torch/modules.py:531-548, 627-631, 647) on the 5th-generation tensor cores, bfloat16 in and out,
 // float32 accumulation, optional gelu_tanh epilogue (the y branch, torch/modules.py:628).
 //
-// x [M, K] and W [N, K] are both K-contiguous, i.e. K-major operands as they are.  Two CTAs of a
+// x [M, K] and W [N, K] are both K-contiguous, i.e. K-major operands as they are.  (Up to 128 rows of the
+// logits go to single CTAs, see launch_dense_tc.)  Two CTAs of a
 // cluster share one tile of 256 rows x BN columns (tcgen05.mma.cta_group::2, M 256): each brings its
 // 128 rows of x and its HALF of the tile's columns of W (128 x 64 and BN/2 x 64 boxes, 128-byte
 // swizzle) into a ring of its own and keeps the accumulator of its rows, so an SM reads 32 KB per K
@@ -67,10 +68,12 @@ struct DenseArgs {
   const __nv_bfloat16* residual;
   int64_t M;
   int k_blocks, m_tiles, n_tiles, group, bn;
+  int load_bytes;                      // what a CTA's loads of a stage bring
   float cap;
 };
 
-template <int kMode>
+// kCtas = 1: a CTA by itself, tiles of 128 rows.
+template <int kMode, int kCtas>
 __global__ void __launch_bounds__(kThreadsG, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
                const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2,
@@ -89,29 +92,37 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbortG);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)cluster_rank();            // cluster = (2, 1, 1)
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int rank = kCtas == 2 ? (int)cluster_rank() : 0;   // cluster = (2, 1, 1)
+  const int pair = blockIdx.x / kCtas, pairs = gridDim.x / kCtas;
   const int k_blocks = a.k_blocks, m_tiles = a.m_tiles, n_tiles = a.n_tiles, group = a.group, bn = a.bn;
   const int64_t M = a.M;
   const int n_my = (m_tiles * n_tiles - pair + pairs - 1) / pairs;
-  const uint32_t stage_bytes = kABytes + (uint32_t)bn * (BK * 2 / 2);
+  const uint32_t stage_bytes = kABytes + (uint32_t)bn * (BK * 2 / kCtas);
   const int n_stages = min(kMaxStages, kRingBytes / (int)stage_bytes);
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
     for (int s = 0; s < n_stages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), 2 * kEpi); }
+    for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), kCtas * kEpi); }
     mbar_fence_init();
   }
   if (warp == kEpi + 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                 :: "r"(s_base + kOffTmemG), "r"(512) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    if constexpr (kCtas == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                   :: "r"(s_base + kOffTmemG), "r"(512) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                   :: "r"(s_base + kOffTmemG), "r"(512) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
-  cluster_wait();                                  // the peer's barriers are set up, its TMEM is there
+  if constexpr (kCtas == 2) {
+    cluster_arrive();
+    cluster_wait();                                // the peer's barriers are set up, its TMEM is there
+  }
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
   // everything up to here overlaps the kernel in front
@@ -122,7 +133,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     // ------------------------------ TMA producers -------------------------------------------------
     // Two, for even and odd K blocks: a turn of this loop takes one 340 cycles, as long as the MMAs of a
     // narrow tile's K blocks.  The whole warp runs it and one elected lane issues (see mma_ring).
-    const uint32_t full0 = peer_smem(bar_full(0), 0);  // the loads of both CTAs report to the even one
+    const uint32_t full0 = kCtas == 2 ? peer_smem(bar_full(0), 0) : bar_full(0);   // the loads of both report to the even one
     int kb = warp == kEpi ? 0 : 1, s = kb;
     uint32_t phase = 1;
     bool ok = true, ready = false;       // ready: the stage was already free when last asked
@@ -131,8 +142,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       tile_at(pair + t * pairs, m_tiles, n_tiles, group, &m0, &n0);
       const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
       const CUtensorMap* map_w = mi == 0 ? &map_w0 : (mi == 1 ? &map_w1 : &map_w2);
-      m0 = m0 * (2 * BM) + rank * BM;
-      n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn + rank * (bn / 2);
+      m0 = m0 * (kCtas * BM) + rank * BM;
+      n0 = (n0 - (mi == 0 ? 0 : (mi == 1 ? a.mat[1].tile0 : a.mat[2].tile0))) * bn + rank * (bn / kCtas);
       for (; kb < k_blocks; kb += 2) {
         if (!ready) {
           ok = __all_sync(0xffffffffu, mbar_wait(bar_empty(s), phase, s_abort));
@@ -143,10 +154,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         if (next >= n_stages) { next -= n_stages; next_phase ^= 1; }
         const bool free_next = mbar_test(bar_empty(next), next_phase);   // looked at behind the loads
         if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(bar_full(s), 2 * stage_bytes);
+          if (rank == 0) mbar_expect_tx(bar_full(s), kCtas * a.load_bytes);
           const uint32_t st = s_base + kOffRing + s * stage_bytes;
-          tma_load_2d_pair(st, &map_x, kb * BK, m0, full0 + 8u * s);
-          tma_load_2d_pair(st + kABytes, map_w, kb * BK, n0, full0 + 8u * s);
+          if constexpr (kCtas == 2) {
+            tma_load_2d_pair(st, &map_x, kb * BK, m0, full0 + 8u * s);
+            tma_load_2d_pair(st + kABytes, map_w, kb * BK, n0, full0 + 8u * s);
+          } else {
+            tma_load_2d(st, &map_x, kb * BK, m0, full0 + 8u * s);
+            tma_load_2d(st + kABytes, map_w, kb * BK, n0, full0 + 8u * s);
+          }
         }
         __syncwarp();
         ready = __all_sync(0xffffffffu, free_next);
@@ -162,15 +178,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       bool ok = true;
       for (int t = 0; t < n_my; ++t) {
         const int as = t & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait_cluster(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+        const uint32_t parity = ((t >> 1) & 1) ^ 1;
+        ok = __all_sync(0xffffffffu, kCtas == 2 ? mbar_wait_cluster(bar_acc_empty(as), parity, s_abort)
+                                                : mbar_wait(bar_acc_empty(as), parity, s_abort));
         if (!ok) break;
         tc_fence_after();
-        ok = mma_ring<BK / 16, 2>(tmem_base + as * kBnMax, smem_desc_sw128(s_base + kOffRing),
+        ok = mma_ring<BK / 16, kCtas>(tmem_base + as * kBnMax, smem_desc_sw128(s_base + kOffRing),
                                   smem_desc_sw128(s_base + kOffRing + kABytes), stage_bytes >> 4,
-                                  tc_idesc_bf16(2 * BM, bn), k_blocks, n_stages, bar_full(0), bar_empty(0),
+                                  tc_idesc_bf16(kCtas * BM, bn), k_blocks, n_stages, bar_full(0), bar_empty(0),
                                   at, s_abort);
         if (!ok) break;
-        if (elect_one()) tc_commit_pair(bar_acc_full(as));
+        if (elect_one()) {
+          if constexpr (kCtas == 2) tc_commit_pair(bar_acc_full(as));
+          else tc_commit(bar_acc_full(as));
+        }
         __syncwarp();
       }
     }
@@ -185,7 +206,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const int as = t & 1;                  // accumulator
       int mt, n0;
       tile_at(pair + t * pairs, m_tiles, n_tiles, group, &mt, &n0);
-      const int64_t m0 = (int64_t)mt * (2 * BM) + rank * BM;
+      const int64_t m0 = (int64_t)mt * (kCtas * BM) + rank * BM;
       // (copies, so that nothing indexes the parameters dynamically)
       const int mi = (n0 >= a.mat[1].tile0) + (n0 >= a.mat[2].tile0);
       const __nv_bfloat16* bias = mi == 0 ? a.mat[0].bias : (mi == 1 ? a.mat[1].bias : a.mat[2].bias);
@@ -324,19 +345,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(peer_smem(bar_acc_empty(as), 0));
+      if (lane == 0) {
+        if constexpr (kCtas == 2) mbar_arrive_cluster(peer_smem(bar_acc_empty(as), 0));
+        else mbar_arrive(bar_acc_empty(as));
+      }
     }
   }
 
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *s_abort && status != nullptr) atomicExch(status, kStatusTimeout);
-  cluster_arrive();
-  cluster_wait();                                  // the peer signals this CTA no more
+  if constexpr (kCtas == 2) {
+    cluster_arrive();
+    cluster_wait();                                // the peer signals this CTA no more
+  }
   if (warp == kEpi + 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
-                 : "memory");
+    if constexpr (kCtas == 2)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
+                   : "memory");
   }
 }
 
@@ -412,25 +442,36 @@ cudaError_t launch_dense_tc(const void* x, const RowsMatrix* mats, int n_mats, c
       if (r == cudaSuccess)
         r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemG);
     };
-    set(gemm_tc_kernel<0>);
-    set(gemm_tc_kernel<1>);
-    set(gemm_tc_kernel<2>);
-    set(gemm_tc_kernel<3>);
-    set(gemm_tc_kernel<4>);
+    set(gemm_tc_kernel<0, 2>);
+    set(gemm_tc_kernel<1, 2>);
+    set(gemm_tc_kernel<2, 2>);
+    set(gemm_tc_kernel<3, 2>);
+    set(gemm_tc_kernel<4, 2>);
+    set(gemm_tc_kernel<0, 1>);
+    set(gemm_tc_kernel<4, 1>);
     return r;
   }, &num_sms);
   if (e != cudaSuccess) return e;
-  const int64_t m_tiles = (M + 2 * BM - 1) / (2 * BM);
+  // One tile of 128 rows is left to single CTAs where nothing but the cap follows the contraction: half of a
+  // pair would work on rows that do not exist, and a pair has 96 KB of weights in flight an SM where a CTA
+  // by itself has 128 (logits of 64 rows over 256000 tokens 306 -> 226 us, over 32000 53 -> 42).
+  const int ctas = M <= BM && n_mats == 1 && act == 0 && residual == nullptr ? 1 : 2;
+  const int64_t m_tiles = (M + ctas * BM - 1) / (ctas * BM);
   DenseArgs a = {};
-  a.bn = tile_columns(m_tiles, mats, n_mats, num_sms / 2, act == 2 ? 64 : 32);
+  a.bn = tile_columns(m_tiles, mats, n_mats, num_sms / ctas, act == 2 ? 64 : 32);
   int64_t n_tiles = 0;
   CUtensorMap map_x, map_w[3];
-  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, BM, BK, true)) return cudaErrorInvalidValue;
+  // rows that do not exist are not asked for where there is one tile of rows: filling them with zeros slows
+  // the loads (16 rows of the above 298 -> 219 us), and what the instruction reads in their place reaches
+  // only rows that are not stored
+  const int box_m = ctas == 1 ? (int)M : BM;
+  a.load_bytes = (box_m + a.bn / ctas) * (BK * 2);
+  if (!tensor_map_2d(&map_x, x, (uint64_t)M, (uint64_t)K, (uint32_t)box_m, BK, true)) return cudaErrorInvalidValue;
   for (int i = 0; i < n_mats; ++i) {
     a.mat[i] = {static_cast<const __nv_bfloat16*>(mats[i].bias), static_cast<__nv_bfloat16*>(mats[i].out),
                 mats[i].n, (int)n_tiles};
     n_tiles += (mats[i].n + a.bn - 1) / a.bn;
-    if (!tensor_map_2d(&map_w[i], mats[i].w, (uint64_t)mats[i].n, (uint64_t)K, (uint32_t)(a.bn / 2), BK, true))
+    if (!tensor_map_2d(&map_w[i], mats[i].w, (uint64_t)mats[i].n, (uint64_t)K, (uint32_t)(a.bn / ctas), BK, true))
       return cudaErrorInvalidValue;
   }
   for (int i = n_mats; i < 3; ++i) {
@@ -447,22 +488,23 @@ cudaError_t launch_dense_tc(const void* x, const RowsMatrix* mats, int n_mats, c
   a.group = (int)((m_tiles + groups - 1) / groups);
   a.cap = cap;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2u * (unsigned)(total < num_sms / 2 ? total : num_sms / 2));
+  cfg.gridDim = dim3((unsigned)(ctas * (total < num_sms / ctas ? total : num_sms / ctas)));
   cfg.blockDim = dim3(kThreadsG);
   cfg.dynamicSmemBytes = kSmemG;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
-#define RGK_GEMM(MODE) \
-  cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MODE>, map_x, map_w[0], map_w[1], map_w[2], a, status)
-  e = cap != 0.0f ? RGK_GEMM(4) : act == 2 ? RGK_GEMM(3) : act == 1 ? RGK_GEMM(1)
-                  : residual != nullptr ? RGK_GEMM(2) : RGK_GEMM(0);
+  cfg.numAttrs = ctas;                             // (a CTA by itself has no cluster)
+#define RGK_GEMM(MODE, CTAS) \
+  cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MODE, CTAS>, map_x, map_w[0], map_w[1], map_w[2], a, status)
+  if (ctas == 1) e = cap != 0.0f ? RGK_GEMM(4, 1) : RGK_GEMM(0, 1);
+  else e = cap != 0.0f ? RGK_GEMM(4, 2) : act == 2 ? RGK_GEMM(3, 2) : act == 1 ? RGK_GEMM(1, 2)
+                       : residual != nullptr ? RGK_GEMM(2, 2) : RGK_GEMM(0, 2);
 #undef RGK_GEMM
   return e != cudaSuccess ? e : cudaGetLastError();
 }

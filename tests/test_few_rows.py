@@ -53,3 +53,36 @@ def test_gelu_and_residual_together(m, k, n):
   err = (got.float() - want.float()).abs().max() / want.float().abs().max()
   assert err.item() <= 3 * 2.0 ** -8
   assert (got != want).float().mean().item() <= 0.05
+
+
+def _close(got, want):
+  """Sums in another order move a value to its neighbour (2^-8 of its size, 2^-7 of the next power of two)
+  at each rounding, and few of them."""
+  err = (got.float() - want.float()).abs().max() / want.float().abs().max()
+  assert err.item() <= 3 * 2.0 ** -8
+  assert (got != want).float().mean().item() <= 0.05
+
+
+# 8 / 9: the change to the GEMM; 16, 100, 128: its single-CTA form, full and ragged; 129: a pair of CTAs.
+# 37888 is where a vocabulary takes it, 40008 leaves its last tile ragged
+@pytest.mark.parametrize("rows", [8, 9, 16, 100, 128, 129])
+@pytest.mark.parametrize("vocab", [37880, 37888, 40008])
+def test_logits_of_large_vocabularies(rows, vocab):
+  import recurrentgemma_b200 as rg
+  torch.manual_seed(rows)
+  emb = rg.Embedder(vocab, 328, True, device=DEV, dtype=BF16)
+  x = torch.randn(rows, 1, 328, device=DEV).to(BF16) * 8
+  z = (x.float() @ emb.input_embedding.float().t()).to(BF16)
+  _close(emb.decode(x), z)
+  _close(emb.decode(x, 30.0), torch.tanh((z.float() / 30.0).to(BF16).float()).to(BF16) * 30.0)
+
+
+# the GEMM for any number of rows: one to 128 by a CTA, 129 by a pair; K and N of one and of several tiles
+@pytest.mark.parametrize("rows", [1, 7, 127, 128, 129])
+@pytest.mark.parametrize("k,n", [(8, 8), (72, 264), (2560, 1000)])
+def test_dense_linear_of_few_rows(rows, k, n):
+  import recurrentgemma_b200 as rg
+  torch.manual_seed(rows + n)
+  x = torch.randn(rows, k, device=DEV).to(BF16)
+  w, b = (torch.randn(n, k, device=DEV) / k ** 0.5).to(BF16), (torch.randn(n, device=DEV) * 0.1).to(BF16)
+  _close(rg.dense_linear(x, w, b), (x.float() @ w.float().t() + b.float()).to(BF16))
