@@ -515,7 +515,7 @@ static bool few_rows(int64_t M, int64_t K, int64_t N, bool plain = false) {
 static cudaError_t few_rows_linear(const void* x, const rgk::RowsMatrix* mats, int n_mats,
                                    const void* residual, int64_t M, int K, int act, float cap, int* status,
                                    bool early, bool wide, cudaStream_t s) {
-  if (M <= kRowsGemm)
+  if (M <= kRowsGemm && rgk::rows_gemm_suits(M, K))
     return rgk::launch_rows_gemm(x, nullptr, 0.0f, mats, n_mats, residual, M, K, act, cap, early, s);
   const bool plain = n_mats == 1 && act == 0 && residual == nullptr;
   if (!few_rows(M, K, mats[0].n, plain) && (act == 0 || residual == nullptr))

@@ -35,6 +35,9 @@ constexpr int kU = 10;                    // 16-byte weight pieces in flight per
 constexpr int kCtasPerSm = 3;
 constexpr int kXBudget = 84 * 1024;       // staged x per CTA: 16 rows of 2560; up to 14 rows leave
 constexpr int kXThree = 71 * 1024;        // room for three CTAs per SM, above that two
+// Without a norm to apply, larger rows are better read from L2 as they are needed (four rows of 7680: 12.6 us
+// staged, while eight rows read from L2 take 10.4 us).
+constexpr int kXStage = 48 * 1024;
 
 struct RowsArgs {
   const __nv_bfloat16 *x, *scale, *residual;
@@ -297,6 +300,13 @@ int x_pitch(int K) { return (K * 2 + 127) / 128 * 128 + 64; }   // an odd half o
 
 }  // namespace
 
+// Rows read from L2 as they are needed cost the general form too much: its pieces have tests of their own and
+// its last chunk is partly empty (4096 -> 4096 18 us at 6 to 8 rows, 12288 -> 4096 39 us at two, where
+// gemm_small_tc.cu takes 9.5 and 20).
+bool rows_gemm_suits(int64_t M, int64_t K) {
+  return K % (kRowsWarps * kU * 32) == 0 || M * x_pitch((int)K) <= kXStage;
+}
+
 bool rows_gemm_supported(int dtype, int64_t M, int64_t K, int64_t N, bool norm) {
   return dtype == 1 && M >= 1 && M <= 16 && K >= 8 && N >= 8 && K % 8 == 0 && N % 8 == 0 &&
          K < (1 << 28) && N < (1 << 30) && (!norm || M * x_pitch((int)K) <= kXBudget);
@@ -342,9 +352,7 @@ cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, c
   a.chunks = (a.blocks_per_warp + kU - 1) / kU;
   a.pitch = x_pitch(K);
   a.eps = eps; a.cap = cap;
-  // without a norm to apply, large rows are better read from L2 as they are needed (four rows of
-  // 7680: 12.6 us staged, while eight rows read from L2 take 10.4 us)
-  const bool staged = (int64_t)M * a.pitch <= (norm_scale != nullptr ? kXBudget : 48 * 1024);
+  const bool staged = (int64_t)M * a.pitch <= (norm_scale != nullptr ? kXBudget : kXStage);
   if (norm_scale != nullptr && !staged) return cudaErrorInvalidValue;
 
   cudaLaunchAttribute attr[2];

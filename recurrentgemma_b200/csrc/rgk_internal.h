@@ -190,6 +190,8 @@ struct RowsMatrix {
   void* out;
   int n;
 };
+// whether that kernel is the one for M <= 8 rows without a norm
+bool rows_gemm_suits(int64_t M, int64_t K);
 bool rows_gemm_supported(int dtype, int64_t M, int64_t K, int64_t N, bool norm);
 cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, const RowsMatrix* mats,
                              int n_mats, const void* residual, int64_t M, int K, int act, float cap,

@@ -86,3 +86,14 @@ def test_dense_linear_of_few_rows(rows, k, n):
   x = torch.randn(rows, k, device=DEV).to(BF16)
   w, b = (torch.randn(n, k, device=DEV) / k ** 0.5).to(BF16), (torch.randn(n, device=DEV) * 0.1).to(BF16)
   _close(rg.dense_linear(x, w, b), (x.float() @ w.float().t() + b.float()).to(BF16))
+
+
+# 5 / 6 rows of 4096: as many as are staged, and the change of kernel; 12288: one row and two
+@pytest.mark.parametrize("m,k", [(5, 4096), (6, 4096), (8, 4096), (1, 12288), (2, 12288), (8, 7680)])
+def test_few_rows_of_long_contractions(m, k):
+  from recurrentgemma_b200 import modules
+  torch.manual_seed(m + k)
+  x, w = torch.randn(m, k, device=DEV).to(BF16), (torch.randn(264, k, device=DEV) / k ** 0.5).to(BF16)
+  b, res = (torch.randn(264, device=DEV) * 0.1).to(BF16), torch.randn(m, 264, device=DEV).to(BF16)
+  y = (x.float() @ w.float().t() + b.float()).to(BF16)
+  _close(modules.small_linear(x, w, b, residual=res), (y.float() + res.float()).to(BF16))
