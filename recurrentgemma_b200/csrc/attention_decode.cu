@@ -27,20 +27,15 @@ constexpr int kSplits = 16;                // CTAs per sequence in the logits an
 constexpr int kHeadPad = 16;               // heads of a logits row, padded
 constexpr int kWarps = 8;                  // warps per CTA
 
-// The 16-byte packs of this lane's 8 elements of a row: one for bfloat16, two for float32.
-template <typename T> struct RowPack { uint4 v[sizeof(T) == 2 ? 1 : 2]; };
+// The 16-byte packs of this lane's 8 elements of a row.
+struct RowPack { uint4 v[2]; };
 
-template <typename T>
-__device__ __forceinline__ RowPack<T> load_pack(const T* row, int lane) {
-  RowPack<T> r;
-  r.v[0] = ld_stream(row + lane * kPerLane);
-  if constexpr (sizeof(T) == 4) r.v[1] = ld_stream(row + lane * kPerLane + 4);
-  return r;
+__device__ __forceinline__ RowPack load_pack(const float* row, int lane) {
+  return {{ld_stream(row + lane * kPerLane), ld_stream(row + lane * kPerLane + 4)}};
 }
-template <typename T>
-__device__ __forceinline__ void unpack_row(const RowPack<T>& r, float (&f)[kPerLane]) {
-  unpack<T>(r.v[0], f);
-  if constexpr (sizeof(T) == 4) unpack<T>(r.v[1], f + 4);
+__device__ __forceinline__ void unpack_row(const RowPack& r, float (&f)[kPerLane]) {
+  unpack<float>(r.v[0], f);
+  unpack<float>(r.v[1], f + 4);
 }
 
 // Ring slot j holds the latest position congruent to j (mod W) that is below nt, the number of
@@ -57,13 +52,12 @@ __device__ __forceinline__ int chunk_of(int total) { return (total + kSplits - 1
 // grid (B, kSplits).  logits: float [B, W + 1, 16] (head-minor; row e = visible entry e);
 // stats: float2 [B, kSplits, kN] = the maximum of the CTA's logits of a head and the sum of
 // exp(logit - maximum) over them.
-template <typename T, int kN>
+template <int kN>
 __global__ void __launch_bounds__(kWarps * 32)
-attn_decode_logits_kernel(const T* __restrict__ q, const T* __restrict__ k_new,
-                          const T* __restrict__ keys, const int* __restrict__ num_tokens, int W,
+attn_decode_logits_kernel(const float* __restrict__ q, const float* __restrict__ k_new,
+                          const float* __restrict__ keys, const int* __restrict__ num_tokens, int W,
                           float* __restrict__ logits, float2* __restrict__ stats) {
-  constexpr bool kBf16 = Traits<T>::kBf16;
-  constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;   // rows whose loads are in flight together
+  constexpr int kBatch = 4;   // rows whose loads are in flight together
   __shared__ float2 s_part[kWarps][kN];
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nt = num_tokens[b];
@@ -75,26 +69,26 @@ attn_decode_logits_kernel(const T* __restrict__ q, const T* __restrict__ k_new,
   float qf[kN][kPerLane];
 #pragma unroll
   for (int n = 0; n < kN; ++n) {
-    const RowPack<T> r = load_pack<T>(q + ((int64_t)b * kN + n) * kHdD, lane);
-    unpack_row<T>(r, qf[n]);
+    const RowPack r = load_pack(q + ((int64_t)b * kN + n) * kHdD, lane);
+    unpack_row(r, qf[n]);
   }
   float* lg = logits + (int64_t)b * (W + 1) * kHeadPad;
   float m_run = kMasked, l_run = 0.0f;             // lanes < kN: this warp's statistics of head `lane`
   for (int e0 = e_begin + warp; e0 < e_end; e0 += kWarps * kBatch) {
-    RowPack<T> raw[kBatch];
+    RowPack raw[kBatch];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
       const int e = e0 + u * kWarps;
       if (e < e_end)
-        raw[u] = load_pack<T>(e == n_vis ? k_new + (int64_t)b * kHdD
-                                         : keys + ((int64_t)b * W + e) * kHdD, lane);
+        raw[u] = load_pack(e == n_vis ? k_new + (int64_t)b * kHdD
+                                      : keys + ((int64_t)b * W + e) * kHdD, lane);
     }
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
       const int e = e0 + u * kWarps;
       if (e < e_end) {                             // (the same for every lane of the warp)
         float kf[kPerLane];
-        unpack_row<T>(raw[u], kf);
+        unpack_row(raw[u], kf);
         float part[kN];
 #pragma unroll
         for (int n = 0; n < kN; ++n) {
@@ -108,11 +102,10 @@ attn_decode_logits_kernel(const T* __restrict__ q, const T* __restrict__ k_new,
 #pragma unroll
           for (int n = 0; n < kN; ++n) part[n] += __shfl_xor_sync(0xffffffffu, part[n], o);
         }
-        // two tensor operations in the reference: the contraction, then the scaling
         float mine = 0.0f;
 #pragma unroll
         for (int n = 0; n < kN; ++n)
-          if (lane == n) mine = rnd<kBf16>(rnd<kBf16>(part[n]) * scale);
+          if (lane == n) mine = part[n] * scale;
         if (lane < kN) {
           lg[(int64_t)e * kHeadPad + lane] = mine;
           const float m_new = fmaxf(m_run, mine);
@@ -137,13 +130,12 @@ attn_decode_logits_kernel(const T* __restrict__ q, const T* __restrict__ k_new,
 
 // grid (B, kSplits): CTA (b, c) multiplies the probabilities of its entries with their value rows,
 // all 256 columns (a lane holds 8 of them), for the kN heads.  partial: float [B, kSplits, kN, 256].
-template <typename T, int kN>
+template <int kN>
 __global__ void __launch_bounds__(kWarps * 32)
 attn_decode_values_kernel(const float* __restrict__ logits, const float2* __restrict__ stats,
-                          const T* __restrict__ v_new, const T* __restrict__ values,
+                          const float* __restrict__ v_new, const float* __restrict__ values,
                           const int* __restrict__ num_tokens, int W, float* __restrict__ partial) {
-  constexpr bool kBf16 = Traits<T>::kBf16;
-  constexpr int kBatch = sizeof(T) == 2 ? 8 : 4;
+  constexpr int kBatch = 4;
   static_assert(kN <= kHeadPad, "a logits row holds 16 heads");
   __shared__ float s_acc[kWarps / 2][kN][kHdD];    // 40 KiB at 10 heads
   __shared__ float s_stat[2][kHeadPad];            // maximum and 1 / sum of every head
@@ -175,15 +167,15 @@ attn_decode_values_kernel(const float* __restrict__ logits, const float2* __rest
 #pragma unroll
     for (int i = 0; i < kPerLane; ++i) acc[n][i] = 0.0f;
   for (int e0 = e_begin + warp; e0 < e_end; e0 += kWarps * kBatch) {
-    RowPack<T> raw[kBatch];
+    RowPack raw[kBatch];
     float lgv[kBatch];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
       const int e = e0 + u * kWarps;
       lgv[u] = kMasked;
       if (e < e_end) {
-        raw[u] = load_pack<T>(e == n_vis ? v_new + (int64_t)b * kHdD
-                                         : values + ((int64_t)b * W + e) * kHdD, lane);
+        raw[u] = load_pack(e == n_vis ? v_new + (int64_t)b * kHdD
+                                      : values + ((int64_t)b * W + e) * kHdD, lane);
         if (lane < kN) lgv[u] = lg[(int64_t)e * kHeadPad + lane];
       }
     }
@@ -192,9 +184,9 @@ attn_decode_values_kernel(const float* __restrict__ logits, const float2* __rest
       const int e = e0 + u * kWarps;
       if (e < e_end) {                             // (the same for every lane of the warp)
         float vf[kPerLane];
-        unpack_row<T>(raw[u], vf);
-        // lane n < kN: the normalised probability of head n, rounded as the reference casts it
-        const float p_mine = lgv[u] > kMasked ? rnd<kBf16>(__expf(lgv[u] - my_m) * my_inv) : 0.0f;
+        unpack_row(raw[u], vf);
+        // lane n < kN: the normalised probability of head n
+        const float p_mine = lgv[u] > kMasked ? __expf(lgv[u] - my_m) * my_inv : 0.0f;
 #pragma unroll
         for (int n = 0; n < kN; ++n) {
           const float p = __shfl_sync(0xffffffffu, p_mine, n);
@@ -249,14 +241,6 @@ attn_decode_values_kernel(const float* __restrict__ logits, const float2* __rest
 // The logits are rounded to bfloat16 twice as the reference does; weights 2^(s - m) are rounded to
 // bfloat16 before the division by their sum instead of behind it.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                          uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -665,16 +649,16 @@ cudaError_t launch_ring(RingArgs a, const void* keys_in, const void* values_in, 
 // grid (B, kN), 256 threads = the 256 columns: out [B, kN, 256] = the rounded sum of the partials;
 // then (update != 0; the CTAs of head 0) the new key and value take ring slot num_tokens % W and
 // num_tokens grows by one.
-template <typename T, int kN>
+template <int kN>
 __global__ void __launch_bounds__(kHdD)
-attn_decode_finish_kernel(const float* __restrict__ partial, const T* __restrict__ k_new,
-                          const T* __restrict__ v_new, T* __restrict__ keys, T* __restrict__ values,
-                          int* __restrict__ num_tokens, int W, int update, T* __restrict__ out) {
+attn_decode_finish_kernel(const float* __restrict__ partial, const float* __restrict__ k_new,
+                          const float* __restrict__ v_new, float* __restrict__ keys, float* __restrict__ values,
+                          int* __restrict__ num_tokens, int W, int update, float* __restrict__ out) {
   const int b = blockIdx.x, n = blockIdx.y, c = threadIdx.x;
   float a = 0.0f;
 #pragma unroll
   for (int s = 0; s < kSplits; ++s) a += partial[(((int64_t)b * kSplits + s) * kN + n) * kHdD + c];
-  out[((int64_t)b * kN + n) * kHdD + c] = static_cast<T>(a);
+  out[((int64_t)b * kN + n) * kHdD + c] = a;
   if (update && n == 0) {
     const int nt = num_tokens[b];
     const int slot = nt % W;
@@ -697,8 +681,8 @@ size_t partial_bytes(int64_t B, int N) {
   return (((size_t)B * kSplits * N * kHdD * sizeof(float)) + 255) & ~(size_t)255;
 }
 
-template <typename T, int kN>
-cudaError_t launch_decode_t(const void* q, const void* k_new, const void* v_new, void* keys,
+template <int kN>
+cudaError_t launch_decode_f32(const void* q, const void* k_new, const void* v_new, void* keys,
                             void* values, int* num_tokens, int64_t B, int W, int update, void* out,
                             void* ws, cudaStream_t s) {
   uint8_t* base = reinterpret_cast<uint8_t*>(ws) + 256;      // behind the status word
@@ -706,12 +690,12 @@ cudaError_t launch_decode_t(const void* q, const void* k_new, const void* v_new,
   float2* st = reinterpret_cast<float2*>(base + logits_bytes(B, W));
   float* part = reinterpret_cast<float*>(base + logits_bytes(B, W) + stats_bytes(B, kN));
   const dim3 grid((unsigned)B, kSplits);
-  attn_decode_logits_kernel<T, kN><<<grid, kWarps * 32, 0, s>>>(
-      (const T*)q, (const T*)k_new, (const T*)keys, num_tokens, W, lg, st);
-  attn_decode_values_kernel<T, kN><<<grid, kWarps * 32, 0, s>>>(
-      lg, st, (const T*)v_new, (const T*)values, num_tokens, W, part);
-  attn_decode_finish_kernel<T, kN><<<dim3((unsigned)B, kN), kHdD, 0, s>>>(
-      part, (const T*)k_new, (const T*)v_new, (T*)keys, (T*)values, num_tokens, W, update, (T*)out);
+  attn_decode_logits_kernel<kN><<<grid, kWarps * 32, 0, s>>>(
+      (const float*)q, (const float*)k_new, (const float*)keys, num_tokens, W, lg, st);
+  attn_decode_values_kernel<kN><<<grid, kWarps * 32, 0, s>>>(
+      lg, st, (const float*)v_new, (const float*)values, num_tokens, W, part);
+  attn_decode_finish_kernel<kN><<<dim3((unsigned)B, kN), kHdD, 0, s>>>(
+      part, (const float*)k_new, (const float*)v_new, (float*)keys, (float*)values, num_tokens, W, update, (float*)out);
   return cudaGetLastError();
 }
 
@@ -732,7 +716,7 @@ cudaError_t launch_attention_decode(const void* q, const void* k_new, const void
   if (B == 0) return cudaSuccess;
 #define RGK_DEC(NN)                                                                               \
   case NN:                                                                                        \
-    return launch_decode_t<float, NN>(q, k_new, v_new, keys, values, num_tokens, B, W, update, out, ws, s)
+    return launch_decode_f32<NN>(q, k_new, v_new, keys, values, num_tokens, B, W, update, out, ws, s)
   switch (N) {
     RGK_DEC(1); RGK_DEC(2); RGK_DEC(4); RGK_DEC(8); RGK_DEC(10);
     default: return cudaErrorInvalidValue;

@@ -25,14 +25,6 @@ constexpr int kHeadR = 256;
 constexpr int kRowsR = 16;                       // batch rows per CTA
 constexpr int kThreadsR = 512;
 constexpr int kPitchR = kHeadR * 2 + 64;         // conv rows in shared memory: conflict-free pieces
-__device__ __forceinline__ void mma_dec(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                        uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint4 mul4r(const uint4& a, const uint4& b) {
   return make_uint4(bmul2(a.x, b.x), bmul2(a.y, b.y), bmul2(a.z, b.z), bmul2(a.w, b.w));
 }
@@ -125,13 +117,13 @@ decode_rows_kernel(const DecodeRowsArgs a) {
   };
   if (a.early) {
     load_constants();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_launch_dependents();
+    grid_dependency_wait();
   } else {
     // the next kernel may fetch weights as soon as it starts: not before the kernel in front of
     // this one, which may have written them, has completed
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    grid_dependency_wait();
+    grid_launch_dependents();
     load_weights();
     load_constants();
   }
@@ -175,10 +167,10 @@ decode_rows_kernel(const DecodeRowsArgs a) {
     float zx[4] = {}, za[4] = {};
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      mma_dec(zx, lo[i].x, hi[i].x, lo[i].y, hi[i].y, wx[c][i].x, wx[c][i].y);
-      mma_dec(za, lo[i].x, hi[i].x, lo[i].y, hi[i].y, wa[c][i].x, wa[c][i].y);
-      mma_dec(zx, lo[i].z, hi[i].z, lo[i].w, hi[i].w, wx[c][i].z, wx[c][i].w);
-      mma_dec(za, lo[i].z, hi[i].z, lo[i].w, hi[i].w, wa[c][i].z, wa[c][i].w);
+      mma_16816(zx, lo[i].x, hi[i].x, lo[i].y, hi[i].y, wx[c][i].x, wx[c][i].y);
+      mma_16816(za, lo[i].x, hi[i].x, lo[i].y, hi[i].y, wa[c][i].x, wa[c][i].y);
+      mma_16816(zx, lo[i].z, hi[i].z, lo[i].w, hi[i].w, wx[c][i].z, wx[c][i].w);
+      mma_16816(za, lo[i].z, hi[i].z, lo[i].w, hi[i].w, wa[c][i].z, wa[c][i].w);
     }
     const int zc = (c * 4 + grp) * 8 + 2 * t;
     *reinterpret_cast<float2*>(&s_z[kq][0][g][zc]) = make_float2(zx[0], zx[1]);

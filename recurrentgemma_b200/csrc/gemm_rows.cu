@@ -1,4 +1,4 @@
-// Dense projections of a handful of rows (M <= 16: a decode step of a few sequences), with what
+// Dense projections of a handful of rows (M <= 8: a decode step of a few sequences), with what
 // surrounds them in the blocks: RMSNorm of the rows in front (torch/layers.py:65-73), bias, gelu,
 // GeGLU, residual add or the logits soft cap behind (recurrentgemma torch/modules.py:531-548,
 // 626-647, 749-752, 897-911, 1001-1003; torch/griffin.py:183-185).
@@ -10,18 +10,18 @@
 // registers - lane (g, t) of a warp holds 16-byte pieces of feature g - with K divided over the 8
 // warps of a CTA; at K = 2560 that is ten 16-byte loads per lane, all issued before the first use and
 // before the dependency wait of a programmatic dependent launch (the weights depend on no kernel
-// that signals early).  The rows of x are the 16-row A operand.  Against the 128-feature tcgen05
+// that signals early).  The rows of x are the A operand, its upper 8 rows empty.  Against the 128-feature tcgen05
 // tiles of gemm_small_tc.cu there is no tensor-memory or barrier set-up, no K split over CTAs and
-// no exchange of partial sums, and 8-feature units fill every SM evenly; a 128-row tile would also
-// be 7/8 padding.  The contraction index is permuted the same way in both operands, so that a lane
+// no exchange of partial sums, and 8-feature units fill every SM evenly.  The contraction index is permuted the same way in both operands, so that a lane
 // feeds two instructions from one 16-byte piece (elements 0-3, then 4-7).
 //
 // CTAs are persistent over units (three per SM), refilling each weight register as soon as its
 // value has been used.  x (normalised, if asked) is staged once per CTA in shared memory; where M x K
 // is too large for that, fragments of x are read from L2 as they are needed.
 //
-// From 17 rows on, the A operand would have to be read once per 8 features and the tcgen05 kernel,
-// whose 128-feature tile reads it once per 128, is the better one.
+// From 9 rows on the upper half of the A operand would have to be there too (its registers cost the weights
+// in flight) and x be read again for every 8 features, where the tcgen05 kernel reads it once per 128:
+// 2560 x 2560 at 9 rows 7.0 us this way, 6.5 that.
 #include "rgk_common.cuh"
 #include "rgk_internal.h"
 #include "tc_common.cuh"
@@ -33,8 +33,8 @@ constexpr int kRowsWarps = 8;
 constexpr int kRowsThreads = kRowsWarps * 32;
 constexpr int kU = 10;                    // 16-byte weight pieces in flight per lane
 constexpr int kCtasPerSm = 3;
-constexpr int kXBudget = 84 * 1024;       // staged x per CTA: 16 rows of 2560; up to 14 rows leave
-constexpr int kXThree = 71 * 1024;        // room for three CTAs per SM, above that two
+constexpr int kXBudget = 84 * 1024;       // staged x per CTA: 8 rows of 5120
+constexpr int kXThree = 71 * 1024;        // up to here there is room for three CTAs per SM, above that for two
 // Without a norm to apply, larger rows are better read from L2 as they are needed (four rows of 7680: 12.6 us
 // staged, while eight rows read from L2 take 10.4 us).
 constexpr int kXStage = 48 * 1024;
@@ -50,28 +50,20 @@ struct RowsArgs {
   int early;                              // the kernel in front does not write weights
 };
 
-__device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                         uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 // kMode: 0 bias, 1 gelu of the first matrix as well, residual if given; 2 GeGLU over the packed up-projection; 4 soft cap.
-// kTwo: rows 8-15 exist.  kStaged: x lies in shared memory (normalised if `scale` is given).
+// kStaged: x lies in shared memory (normalised if `scale` is given).
 // kFull: K is exactly 8 warps x chunks x kU blocks of 32 (2560, 7680), so no piece needs a test.
 enum { kPlain = 0, kGeluRows = 1, kGeglu = 2, kCap = 4 };
 
-template <int kMode, bool kTwo, bool kStaged, bool kFull>
+template <int kMode, bool kStaged, bool kFull>
 __global__ void __launch_bounds__(kRowsThreads, kCtasPerSm)
 gemm_rows_kernel(const RowsArgs a) {
   extern __shared__ __align__(16) uint8_t s_x[];
-  __shared__ float s_red[kRowsWarps][kTwo ? 16 : 8][8];
+  __shared__ float s_red[kRowsWarps][8][8];
   __shared__ float s_sum[kRowsWarps];
-  __shared__ uint32_t s_r[16];
+  __shared__ uint32_t s_r[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int M = a.M, K = a.K;
   const int kb0 = warp * a.blocks_per_warp;
@@ -98,8 +90,8 @@ gemm_rows_kernel(const RowsArgs a) {
   };
   if (a.early) {
     first_chunk();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_launch_dependents();
+    grid_dependency_wait();
   } else {
     // The kernel in front may have written the weights: until it has completed they are only asked
     // into L2 (the point of coherence), and the next kernel is not let loose on them either.
@@ -110,8 +102,8 @@ gemm_rows_kernel(const RowsArgs a) {
           asm volatile("prefetch.global.L2 [%0];" :: "l"(row + (kb0 + i) * 32));
       }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    grid_dependency_wait();
+    grid_launch_dependents();
     first_chunk();
   }
 
@@ -119,8 +111,8 @@ gemm_rows_kernel(const RowsArgs a) {
   if constexpr (kStaged) {
     const int packs = K / 8;
     if (a.scale != nullptr) {
-      // the sum over the bfloat16-rounded squares of a row, every rounding of the reference; up to 8
-      // rows at a time, all 8 warps at work whatever M is
+      // the sum over the bfloat16-rounded squares of a row, every rounding of the reference; all 8
+      // warps at work whatever M is
       constexpr int kS = 2;               // scale packs kept in registers while the sums are formed
       uint4 sc[kS];
 #pragma unroll
@@ -129,32 +121,30 @@ gemm_rows_kernel(const RowsArgs a) {
                     ? *reinterpret_cast<const uint4*>(a.scale + (tid + j * kRowsThreads) * 8)
                     : make_uint4(0u, 0u, 0u, 0u);
       const int wpr = M == 1 ? 8 : (M == 2 ? 4 : (M <= 4 ? 2 : 1));     // warps per row
-      for (int m0 = 0; m0 < M; m0 += kRowsWarps / wpr) {
-        const int m = m0 + warp / wpr;
-        float sum = 0.0f;
-        if (m < M) {
+      const int m = warp / wpr;
+      float sum = 0.0f;
+      if (m < M) {
 #pragma unroll 5
-          for (int p = (warp % wpr) * 32 + lane; p < packs; p += 32 * wpr) {
-            const uint4 v = *reinterpret_cast<const uint4*>(a.x + (int64_t)m * K + p * 8);
-            *reinterpret_cast<uint4*>(s_x + m * a.pitch + p * 16) = v;
-            const uint32_t q[4] = {bmul2(v.x, v.x), bmul2(v.y, v.y), bmul2(v.z, v.z), bmul2(v.w, v.w)};
+        for (int p = (warp % wpr) * 32 + lane; p < packs; p += 32 * wpr) {
+          const uint4 v = *reinterpret_cast<const uint4*>(a.x + (int64_t)m * K + p * 8);
+          *reinterpret_cast<uint4*>(s_x + m * a.pitch + p * 16) = v;
+          const uint32_t q[4] = {bmul2(v.x, v.x), bmul2(v.y, v.y), bmul2(v.z, v.z), bmul2(v.w, v.w)};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) sum += bf16_lo(q[k]) + bf16_hi(q[k]);
-          }
+          for (int k = 0; k < 4; ++k) sum += bf16_lo(q[k]) + bf16_hi(q[k]);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) s_sum[warp] = sum;
-        __syncthreads();
-        if (tid < kRowsWarps / wpr && m0 + tid < M) {
-          float total = 0.0f;
-          for (int i = 0; i < wpr; ++i) total += s_sum[tid * wpr + i];
-          const float var = round_bf16(total / (float)K);
-          const float r = round_bf16(1.0f / sqrtf(round_bf16(var + a.eps)));
-          s_r[m0 + tid] = pack_bf16x2(r, r);
-        }
-        __syncthreads();
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) s_sum[warp] = sum;
+      __syncthreads();
+      if (tid < M) {
+        float total = 0.0f;
+        for (int i = 0; i < wpr; ++i) total += s_sum[tid * wpr + i];
+        const float var = round_bf16(total / (float)K);
+        const float r = round_bf16(1.0f / sqrtf(round_bf16(var + a.eps)));
+        s_r[tid] = pack_bf16x2(r, r);
+      }
+      __syncthreads();
       constexpr uint32_t kOne = 0x3f803f80u;
       auto scale_pack = [&](int p, uint4 v) {
         const uint4 s1 = make_uint4(badd2(v.x, kOne), badd2(v.y, kOne), badd2(v.z, kOne), badd2(v.w, kOne));
@@ -217,20 +207,17 @@ gemm_rows_kernel(const RowsArgs a) {
       const int next_kb = last ? kb0 : kb + kU;
       const bool more = next_unit < a.units;
       if (last && more) row = weight_row(next_unit);
-      constexpr int kX = kStaged || kTwo ? 1 : 5;      // pieces of x in flight (registers)
+      constexpr int kX = kStaged ? 1 : 5;      // pieces of x in flight (registers)
 #pragma unroll
       for (int h = 0; h < kU; h += kX) {
-        uint4 xa[kX], xb[kX];
+        uint4 xa[kX];
 #pragma unroll
-        for (int i = 0; i < kX; ++i) {
-          xa[i] = x_piece(g, kb + h + i);
-          xb[i] = kTwo ? x_piece(g + 8, kb + h + i) : make_uint4(0u, 0u, 0u, 0u);
-        }
+        for (int i = 0; i < kX; ++i) xa[i] = x_piece(g, kb + h + i);
 #pragma unroll
         for (int i = 0; i < kX; ++i) {
           const uint4 b = w[h + i];
-          mma_rows(acc[0], xa[i].x, xb[i].x, xa[i].y, xb[i].y, b.x, b.y);
-          mma_rows(acc[1], xa[i].z, xb[i].z, xa[i].w, xb[i].w, b.z, b.w);
+          mma_16816(acc[0], xa[i].x, 0u, xa[i].y, 0u, b.x, b.y);
+          mma_16816(acc[1], xa[i].z, 0u, xa[i].w, 0u, b.z, b.w);
           if (more) w[h + i] = piece(row, next_kb + h + i);
         }
       }
@@ -238,9 +225,6 @@ gemm_rows_kernel(const RowsArgs a) {
     // ---- the warps' sums, then the epilogue ----------------------------------------------------------
     *reinterpret_cast<float2*>(&s_red[warp][g][2 * t]) =
         make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
-    if constexpr (kTwo)
-      *reinterpret_cast<float2*>(&s_red[warp][g + 8][2 * t]) =
-          make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
     __syncthreads();
     {
       if constexpr (!kStaged) epilogue_operands();
@@ -273,13 +257,13 @@ gemm_rows_kernel(const RowsArgs a) {
   }
 }
 
-template <int kMode, bool kTwo>
+template <int kMode>
 cudaError_t launch_rows_t(const cudaLaunchConfig_t& cfg, bool staged, const RowsArgs& a) {
   if (a.K == kRowsWarps * a.chunks * kU * 32)
-    return staged ? cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, kTwo, true, true>, a)
-                  : cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, kTwo, false, true>, a);
-  return staged ? cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, kTwo, true, false>, a)
-                : cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, kTwo, false, false>, a);
+    return staged ? cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, true, true>, a)
+                  : cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, false, true>, a);
+  return staged ? cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, true, false>, a)
+                : cudaLaunchKernelEx(&cfg, gemm_rows_kernel<kMode, false, false>, a);
 }
 
 template <int kMode>
@@ -289,10 +273,8 @@ cudaError_t set_smem() {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXBudget);
   };
-  set(gemm_rows_kernel<kMode, false, true, true>);
-  set(gemm_rows_kernel<kMode, true, true, true>);
-  set(gemm_rows_kernel<kMode, false, true, false>);
-  set(gemm_rows_kernel<kMode, true, true, false>);
+  set(gemm_rows_kernel<kMode, true, true>);
+  set(gemm_rows_kernel<kMode, true, false>);
   return e;
 }
 
@@ -308,7 +290,7 @@ bool rows_gemm_suits(int64_t M, int64_t K) {
 }
 
 bool rows_gemm_supported(int dtype, int64_t M, int64_t K, int64_t N, bool norm) {
-  return dtype == 1 && M >= 1 && M <= 16 && K >= 8 && N >= 8 && K % 8 == 0 && N % 8 == 0 &&
+  return dtype == 1 && M >= 1 && M <= 8 && K >= 8 && N >= 8 && K % 8 == 0 && N % 8 == 0 &&
          K < (1 << 28) && N < (1 << 30) && (!norm || M * x_pitch((int)K) <= kXBudget);
 }
 
@@ -325,7 +307,7 @@ cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, c
     return e;
   }, &num_sms);
   if (e0 != cudaSuccess) return e0;
-  if (n_mats < 1 || n_mats > 3) return cudaErrorInvalidValue;
+  if (n_mats < 1 || n_mats > 3 || M < 1 || M > 8) return cudaErrorInvalidValue;
   RowsArgs a;
   a.x = (const __nv_bfloat16*)x;
   a.scale = (const __nv_bfloat16*)norm_scale;
@@ -368,8 +350,7 @@ cudaError_t launch_rows_gemm(const void* x, const void* norm_scale, float eps, c
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const bool two = M > 8;
-#define RGK_ROWS(MODE) (two ? launch_rows_t<MODE, true>(cfg, staged, a) : launch_rows_t<MODE, false>(cfg, staged, a))
+#define RGK_ROWS(MODE) launch_rows_t<MODE>(cfg, staged, a)
   cudaError_t e;
   if (cap != 0.0f) e = RGK_ROWS(kCap);
   else if (act == 2) e = RGK_ROWS(kGeglu);

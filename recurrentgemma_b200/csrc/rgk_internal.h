@@ -178,7 +178,7 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
                               const void* conv_w = nullptr, const void* conv_b = nullptr,
                               bool prepared = false);
 
-// gemm_rows.cu: up to three projections (matrices) of the same M <= 16 rows in one launch, with
+// gemm_rows.cu: up to three projections (matrices) of the same M <= 8 rows in one launch, with
 // RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as below behind (act 1 on the
 // first matrix only); one
 // residual for a single matrix.  early: no kernel in front of this one on the stream that could still be

@@ -135,10 +135,10 @@ rmsnorm_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ sca
   __shared__ float s_sum[kRowThreads / 32];
   const int packs = D / 8, tid = threadIdx.x;
   const int64_t row = blockIdx.x;
-  if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (early) grid_launch_dependents();
+  grid_dependency_wait();
   // (the kernel behind may fetch weights as soon as it starts, see launch_rows_gemm)
-  if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!early) grid_launch_dependents();
   uint4 v[kPacks], sc[kPacks];
 #pragma unroll
   for (int i = 0; i < kPacks; ++i) {

@@ -254,6 +254,16 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   return false;
 }
 
+// Warp-level matrix instruction for tiles too small for tcgen05: c += A (16 x 16, rows) B (16 x 8, columns).
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // packed bfloat16x2 arithmetic, each lane rounded to nearest even (what torch does per element)
 __device__ __forceinline__ uint32_t bmul2(uint32_t a, uint32_t b) {
   uint32_t r;
