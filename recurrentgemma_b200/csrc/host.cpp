@@ -14,7 +14,6 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
@@ -92,13 +91,19 @@ const at::Tensor* dense(PyObject* o) {
   return &t;
 }
 
-// module.<dict>[name], borrowed (the module keeps it alive for the call); null if absent.
-PyObject* entry(PyObject* module, PyObject* dict_name, PyObject* name) {
-  PyObject* d = PyObject_GetAttr(module, dict_name);
+// module.__dict__[name], borrowed (the module keeps it alive for the call); null if absent.  Modules hold
+// all that is asked for here as instance attributes, and looking there is cheaper than PyObject_GetAttr.
+PyObject* field(PyObject* module, PyObject* name) {
+  PyObject* d = PyObject_GenericGetDict(module, nullptr);
   if (d == nullptr) return nullptr;
-  PyObject* v = PyDict_Check(d) ? PyDict_GetItemWithError(d, name) : nullptr;
+  PyObject* v = PyDict_GetItemWithError(d, name);
   Py_DECREF(d);
   return v;
+}
+// module.<dict>[name], borrowed; null if absent.
+PyObject* entry(PyObject* module, PyObject* dict_name, PyObject* name) {
+  PyObject* d = field(module, dict_name);
+  return d != nullptr && PyDict_Check(d) ? PyDict_GetItemWithError(d, name) : nullptr;
 }
 PyObject* submodule(PyObject* module, PyObject* name) { return entry(module, s__modules, name); }
 
@@ -123,11 +128,9 @@ struct Params {
 
 // Whether calling `module` is running cls.forward on its parameters and nothing else.
 bool plain(PyObject* module, PyObject* cls) {
-  if (module == nullptr || (PyObject*)Py_TYPE(module) != cls) return false;
-  Ref d(PyObject_GenericGetDict(module, nullptr));
-  if (d.p == nullptr || !PyDict_Check(d.p) || PyDict_GetItemWithError(d.p, s_forward) != nullptr) return false;
+  if (module == nullptr || (PyObject*)Py_TYPE(module) != cls || field(module, s_forward) != nullptr) return false;
   for (PyObject* name : {s__forward_hooks, s__forward_pre_hooks}) {
-    PyObject* hooks = PyDict_GetItemWithError(d.p, name);
+    PyObject* hooks = field(module, name);
     if (hooks == nullptr || !PyDict_Check(hooks) || PyDict_Size(hooks) != 0) return false;
   }
   return true;
@@ -135,9 +138,9 @@ bool plain(PyObject* module, PyObject* cls) {
 bool no_global_hooks() { return PyDict_Size(g_hooks) == 0 && PyDict_Size(g_pre_hooks) == 0; }
 
 bool int_attr(PyObject* o, PyObject* name, long* v) {
-  Ref a(PyObject_GetAttr(o, name));
-  if (a.p == nullptr || !PyLong_Check(a.p)) return false;
-  *v = PyLong_AsLong(a.p);
+  PyObject* a = field(o, name);
+  if (a == nullptr || !PyLong_Check(a)) return false;
+  *v = PyLong_AsLong(a);
   return !(*v == -1 && PyErr_Occurred());
 }
 
@@ -174,13 +177,20 @@ struct Workspace {
   void* ptr = nullptr;
   size_t bytes = 0;
 };
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+  return status != cudaStreamCaptureStatusNone;
+}
 bool workspace(const at::Tensor& on, cudaStream_t stream, size_t bytes, Workspace* ws) {
-  Ref key(Py_BuildValue("(iK)", (int)on.device().index(), (unsigned long long)(uintptr_t)stream));
+  Ref index(PyLong_FromLong(on.device().index())), address(PyLong_FromUnsignedLongLong((uintptr_t)stream));
+  if (index.p == nullptr || address.p == nullptr) return false;
+  Ref key(PyTuple_Pack(2, index.p, address.p));
   if (key.p == nullptr) return false;
   PyObject* buf = PyDict_GetItemWithError(g_workspaces, key.p);
   Ref made(nullptr);
   if (buf == nullptr || !THPVariable_Check(buf) || (size_t)THPVariable_Unpack(buf).numel() < bytes ||
-      c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+      capturing(stream)) {
     if (PyErr_Occurred()) return false;
     Ref dev(THPDevice_New(on.device()));
     Ref n(PyLong_FromSize_t(bytes));
@@ -208,25 +218,23 @@ bool succeeded(int rc) {
 // (address, version) of both and, for the gates, the dtype.  *made: a packing kernel was enqueued.  False: a Python error is set.
 bool packed(PyObject* module, const at::Tensor& p0, const at::Tensor& p1, int dt, PyObject* method,
             const void** out, bool* made = nullptr) {
-  Ref key(PyObject_GetAttr(module, s__pack_key));
-  if (key.p == nullptr) PyErr_Clear();
+  PyObject* key = field(module, s__pack_key);
   const Py_ssize_t n = dt >= 0 ? 5 : 4;
-  if (key.p != nullptr && PyTuple_Check(key.p) && PyTuple_GET_SIZE(key.p) == n) {
+  if (key != nullptr && PyTuple_Check(key) && PyTuple_GET_SIZE(key) == n) {
     const unsigned long long want[5] = {(unsigned long long)(uintptr_t)p0.const_data_ptr(),
                                         (unsigned long long)p0._version(),
                                         (unsigned long long)(uintptr_t)p1.const_data_ptr(),
                                         (unsigned long long)p1._version(), (unsigned long long)dt};
     bool same = true;
     for (Py_ssize_t i = 0; i < n && same; ++i)
-      same = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(key.p, i)) == want[i];
+      same = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(key, i)) == want[i];
     if (PyErr_Occurred()) PyErr_Clear();
     if (same) {
-      Ref buf(PyObject_GetAttr(module, s__pack_buf));
-      if (buf.p != nullptr && THPVariable_Check(buf.p)) {
-        *out = THPVariable_Unpack(buf.p).const_data_ptr();
+      PyObject* buf = field(module, s__pack_buf);
+      if (buf != nullptr && THPVariable_Check(buf)) {
+        *out = THPVariable_Unpack(buf).const_data_ptr();
         return true;
       }
-      PyErr_Clear();
     }
   }
   if (made != nullptr) *made = true;
@@ -401,9 +409,9 @@ PyObject* rglru(PyObject* const* args, Py_ssize_t n) {
 
 bool exactly(PyObject* module, PyObject* cls) { return (PyObject*)Py_TYPE(module) == cls; }
 bool float_attr(PyObject* o, PyObject* name, float* v) {
-  Ref a(PyObject_GetAttr(o, name));
-  if (a.p == nullptr) return false;
-  *v = (float)PyFloat_AsDouble(a.p);
+  PyObject* a = field(o, name);
+  if (a == nullptr) return false;
+  *v = (float)PyFloat_AsDouble(a);
   return !PyErr_Occurred();
 }
 // An activation-sized tensor of one token per sequence: [B, 1, width] or the ring's tensors.

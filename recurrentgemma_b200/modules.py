@@ -2,8 +2,9 @@
 
 Same constructor, parameter names (`linear_y`, `linear_x`, `linear_out`, `conv_1d`, `rg_lru`),
 forward signature and cache type as the reference, so it slots into the reference `Griffin` model
-and `Sampler` unchanged.  The RG-LRU + Conv1D sub-path between the projections runs as one
-composed call into librgk.so; the three dense projections are plain library GEMMs.
+and `Sampler` unchanged.  A prompt, and a decode step inside a residual block, is one call into
+librgk.so, the three dense projections included; called on its own a decode step runs the RG-LRU +
+Conv1D sub-path as one call between projections that `linear` places.
 """
 from __future__ import annotations
 
@@ -20,15 +21,17 @@ from recurrentgemma_b200 import layers
 
 # Fewest rows for which the prefill GEMM of the library is used (see MLPBlock._fusable), and most
 # rows for which the few-row (weight-streaming, split-K) kernel is used; torch's contractions in
-# between.  The few-row kernel takes up to 256 rows, but the exchange of its K-split partial sums
-# grows with the row count: measured on a B200 at 2560 x 2560 it is ahead of the library GEMM up
-# to 32 rows (two projections in one launch: 9.7 against 12.6 us at 16 rows) and behind it from 64.
+# between, for calls of a module on its own (a residual block's step and a prompt are native calls with
+# their own rule).  The few-row kernels take up to 256 rows, but the exchange of K-split partial sums
+# grows with the row count: at 2560 x 2560, chained over distinct weights, 5.9 us against 7.8 of the
+# library GEMM at 8 rows, 6.5 / 6.3 at 16 (two projections in one launch 8.0), 7.2 / 6.4 at 32,
+# 7.5 / 6.6 at 64 and 11.0 / 7.2 at 256.
 SMALL_M = 1024
 SMALL_ROWS = 32
-# The MLP's contractions (2560 -> 2 x 7680 -> 2560) stay on the library below SMALL_M: with 120
-# feature tiles there is nothing to split, and the library's kernel streams those weights faster
-# (15.5 against 21 us).  Raise to SMALL_ROWS to route them through the few-row kernel as well
-# (GeGLU and the residual add then run in its epilogues).
+# The MLP's contractions (2560 -> 2 x 7680 -> 2560) stay on the library below SMALL_M, where the first
+# version of the few-row kernel streamed their weights more slowly (21 us against 15.5).  Raise to
+# SMALL_ROWS to route them through the few-row kernels as well (GeGLU and the residual add then run in
+# their epilogues, as they do in a residual block's step).
 SMALL_ROWS_MLP = 0
 
 
@@ -131,7 +134,7 @@ def dense_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
   dev = _lib.require_cuda(x, weight, bias)
   layers._same_dtype(x, weight, *([bias] if bias is not None else []))
   n, k = weight.shape
-  assert x.shape[-1] == k and (bias is None or bias.shape == (n,))
+  assert x.shape[-1] == k and (bias is None or bias.numel() == n)
   xc, wc = x.contiguous(), weight.contiguous()
   bc = None if bias is None else bias.contiguous()
   out = torch.empty((*x.shape[:-1], n), dtype=x.dtype, device=dev)
@@ -159,7 +162,7 @@ def small_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
   n_out = n // 2 if act == _lib.ACT_GEGLU else n
   out = torch.empty((*x.shape[:-1], n_out), dtype=x.dtype, device=dev)
   assert residual is None or residual.shape == out.shape
-  assert bias is None or bias.shape == (n,)
+  assert bias is None or bias.numel() == n
   rc = None if residual is None else residual.contiguous()
   bc = None if bias is None else bias.contiguous()
   lib = _lib.load()
@@ -602,10 +605,11 @@ def _cache_from_prompt(keys: torch.Tensor, values: torch.Tensor, segment_pos: to
 class LocalAttentionBlock(nn.Module):
   """Local multi-query attention (recurrentgemma/torch/modules.py:293-493): same constructor,
   parameter names (`proj_q/k/v.weight`, `proj_final.weight/.bias`), forward and cache.  bfloat16
-  prefill with head dimension 256 runs on the library (projections on the tcgen05 GEMM, rotary
-  kernel, the tcgen05 attention kernel), and so does the decode step with head dimension
-  256 (rotary kernel, the two ring kernels; projections of a handful of rows are library GEMMs);
-  other shapes compose the rotary kernel with library contractions."""
+  prefill with head dimension 256 is one call into librgk.so (projections on its GEMMs, rotary
+  embedding, ring cache and transposed values in one kernel, the tcgen05 attention kernel).  The decode
+  step with head dimension 256 and 1, 2, 4, 8 or 10 heads runs rotary kernel and ring attention there,
+  its projections where `linear` places them (a residual block's step is one call); other shapes compose
+  the rotary kernel with library contractions."""
 
   def __init__(self, width: int, num_heads: int, window_size: int,
                final_w_init_variance_scale: float = 1.0, device=None, dtype=None):
