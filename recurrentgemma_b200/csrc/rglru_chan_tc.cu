@@ -25,12 +25,23 @@
 //             every global access of the kernel is a bulk tensor copy, every shared-memory access
 //             of the tiles a 16-byte one.
 // Per unit an epilogue thread: tcgen05.ld of 2 x 16 columns -> gate arithmetic on token pairs in
-// packed bfloat16 with the reference's roundings -> (a, x) kept packed in 32 registers while the
-// 32-token map (P, H): h -> P h + H is accumulated -> the four token quarters of a channel quarter
-// meet at a 128-thread named barrier; the last one publishes the tile's map, resolves the incoming
-// state (decoupled look-back over earlier time tiles, normally one already inclusive record) and
-// publishes the inclusive state -> second named barrier -> replay from registers with the true
-// incoming state, join, 16-byte stores into the output tile.
+// packed bfloat16 with the reference's roundings -> (a, x) kept packed in 32 registers -> the state that
+// enters the thread's tokens, in one of two ways (chan_uses_maps says when):
+//   chains  the state itself goes through the token quarters one after the other, from tile to tile
+//           through one record a chain;
+//   maps    the 32-token map (P, H): h -> P h + H is accumulated with the gates; the four token quarters
+//           of a channel quarter meet at a 128-thread named barrier; the last one resolves the incoming
+//           state (decoupled look-back over the maps of earlier time tiles, normally one already inclusive
+//           record) and publishes the tile's own; second named barrier unless the state was known
+// -> recurrence in registers, join, 16-byte stores into the output tile.
+//
+// What bounds it is instruction issue: 42 warp instructions an element (35 without a join) with four
+// epilogue warps a scheduler; stripped of every memory access the arithmetic alone takes 105 of 124 us at
+// 8 x 4096 tokens without a join.  There: 151 us as look-back over maps for every call -> 136 without maps where
+// chains are many -> 134 with the MMA loop on a whole warp -> 129 with 112 instead of 96 registers for the
+// epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with table addresses in one
+// instruction and waits that are asked once ahead of their loop.  The recurrent path 243 -> 209 us,
+// 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a tile).
 // All waits (mbarriers, look-back flags) are bounded; on expiry WsHeader::status is raised, the
 // affected values are taken as zero and the kernel runs to completion.
 #include <cuda.h>
@@ -52,12 +63,16 @@ constexpr int kCBytes = kUT * kKB * 2;         // 16 KiB: conv-output slice (ope
 constexpr int kWBytes = 2 * kUC * kKB * 2;     // 32 KiB: x-gate rows then a-gate rows (operand A)
 constexpr int kStage = kCBytes + kWBytes;
 constexpr int kEpi = 16;
-constexpr int kThreads = (kEpi + 2) * 32;
+// The producer, MMA and two idle warps are a warpgroup of their own, which hands registers to the
+// epilogue warps: launched with 96 a thread, 112 x 4 + 32 = 5 x 96.
+constexpr int kThreads = (kEpi + 4) * 32;
+constexpr int kRegsEpilogue = 112, kRegsOther = 32;
+static_assert(4 * kRegsEpilogue + kRegsOther <= 5 * 96, "more registers than the CTA is launched with");
 // With the Conv1D fused (kConv): two more warps turn the block input into the conv-output operand.
 // The ring then has two stages; the room of the third holds two staging buffers for the input rows
 // of a K-slice (the unit's 128 tokens and the three before them, 64 channels).
 constexpr int kConvWarps = 2;
-constexpr int kThreadsConv = (kEpi + 2 + kConvWarps) * 32;
+static_assert(kThreads == (kEpi + 2 + kConvWarps) * 32, "the conv warps are the two idle ones");
 constexpr int kRingConv = 2;
 constexpr int kXRows = kUT + 3;
 constexpr int kXBytes = kXRows * kKB * 2;      // 16768
@@ -73,7 +88,13 @@ constexpr int kOffHin = kOffQmap + 2 * 4 * 3 * 32 * 8;         // float  [2 pari
 constexpr int kOffKnown = kOffHin + 2 * 4 * 32 * 4;              // int    [2 parity][4 chq]
 constexpr int kOffBar = kOffKnown + 2 * 4 * 4;
 constexpr int kNumBar = 2 * kRing + 4 + 2 * kEpi + 5;        // + staging full[2], empty[2], conv tiles free
-constexpr int kOffTmem = kOffBar + kNumBar * 8;
+// Without maps the state goes from token quarter to token quarter through shared memory: a float a channel
+// and a barrier for each of three hand-overs, four units deep (see the hand-over below).
+constexpr int kSlots = 4;
+constexpr int kCarryBars = kSlots * 4 * 3;
+constexpr int kOffCarry = kOffQmap;                            // float [slot][4 chq][3 tq][32]
+static_assert(kSlots * 4 * 3 * 32 * 4 <= kOffHin - kOffQmap, "the carries take the place of the maps");
+constexpr int kOffTmem = kOffBar + (kNumBar + kCarryBars) * 8;
 constexpr int kOffAbort = kOffTmem + 4;
 constexpr int kOffLut = (kOffAbort + 4 + 15) & ~15;            // {a, multiplier} by log_a, see tc_common.cuh
 constexpr int kSmem = kOffLut + kLutEntries * 4 + 1024;
@@ -141,11 +162,11 @@ __device__ __forceinline__ void sts_piece(uint32_t ld_base, int k, const uint4& 
 }
 
 // 16 tokens of one channel: gates from the accumulators, (a, x) packed per token pair, and the
-// running map (P, H) of the thread's tokens.  c holds the conv outputs of the 16 tokens as 8 token
+// running map (P, H) of the thread's tokens (kMaps).  c holds the conv outputs of the 16 tokens as 8 token
 // pairs; `rs` holds the reset bits of the 16 tokens, `inv` the bits of tokens past the end of the
 // sequence (the kResets variant handles both; the other one has no branch inside the unrolled loop,
 // so that the compiler interleaves the eight independent pairs).
-template <bool kResets, int kMath>
+template <bool kResets, int kMath, bool kMaps>
 __device__ __forceinline__ void gates_16(const uint32_t (&zx)[16], const uint32_t (&za)[16],
                                          const uint32_t (&c)[8], uint32_t bx2, uint32_t ba2, uint32_t hbx2,
                                          uint32_t m8sp2, uint32_t rs, uint32_t inv, uint32_t* a_out,
@@ -172,11 +193,13 @@ __device__ __forceinline__ void gates_16(const uint32_t (&zx)[16], const uint32_
     const uint32_t x2 = bmul2(bmul2(c[jp], gx2), mult2);
     a_out[jp] = a2;
     x_out[jp] = x2;
-    const float a0 = bf16_lo(a2), a1 = bf16_hi(a2);
-    // the pair as one map, then composed: keeps the dependent chain at one step per pair
-    const float p2 = a0 * a1, h2 = fmaf(a1, bf16_lo(x2), bf16_hi(x2));
-    H = fmaf(p2, H, h2);
-    P *= p2;
+    if constexpr (kMaps) {
+      const float a0 = bf16_lo(a2), a1 = bf16_hi(a2);
+      // the pair as one map, then composed: keeps the dependent chain at one step per pair
+      const float p2 = a0 * a1, h2 = fmaf(a1, bf16_lo(x2), bf16_hi(x2));
+      H = fmaf(p2, H, h2);
+      P *= p2;
+    }
   }
 }
 
@@ -185,7 +208,7 @@ __device__ __forceinline__ void gates_16(const uint32_t (&zx)[16], const uint32_
 // returns the state entering tile tt.
 __device__ __forceinline__ float look_back(const unsigned long long* agg, const unsigned long long* incl,
                                         const float* h0, int64_t rec, int tt, int per_tt, int b, int E,
-                                        int chan, int lane, int use_agg, bool* timed_out_p,
+                                        int chan, int lane, bool* timed_out_p,
                                         int64_t n_words, int64_t n_state, int* status) {
   float hin = 0.0f;
   bool timed_out = false;
@@ -194,28 +217,25 @@ __device__ __forceinline__ float look_back(const unsigned long long* agg, const 
     int pred = tt - 1;                 // the nearest tile not yet absorbed
     bool done = false;
     unsigned spins = 0;
-    const int depth = use_agg ? kLookback : 1;
     while (!done) {
       unsigned long long wi[kLookback], wp[kLookback], wh[kLookback];
 #pragma unroll
       for (int i = 0; i < kLookback; ++i) {
         const int pt = pred - i;
         wi[i] = 0ull; wp[i] = 0ull; wh[i] = 0ull;
-        if (i < depth && pt >= 0) {
+        if (pt >= 0) {
           const int64_t rp = (rec - (int64_t)(tt - pt) * per_tt * 4) * kSub + lane;
           if (RGK_IN_RANGE(rp, n_words, status)) {
             wi[i] = ld_relaxed_u64(incl + rp);
-            if (use_agg) {
-              wp[i] = ld_relaxed_u64(agg + rp * 2);
-              wh[i] = ld_relaxed_u64(agg + rp * 2 + 1);
-            }
+            wp[i] = ld_relaxed_u64(agg + rp * 2);
+            wh[i] = ld_relaxed_u64(agg + rp * 2 + 1);
           }
         }
       }
       bool progress = false;
 #pragma unroll
       for (int i = 0; i < kLookback; ++i) {
-        if (!done && pred >= 0 && i < depth) {
+        if (!done && pred >= 0) {
           // entries of this batch are consumed strictly in order: entry i belongs to `pred` only
           // while every earlier entry was absorbed
           if ((wi[i] >> 32) == 1ull) {
@@ -267,15 +287,15 @@ struct UnitStep {
 // kJoin 0: out = y, 1: out = y * gelu_tanh(yb), 2: out = y * yb;  kMath: see tc_common.cuh
 // kConv: map_c is a map of the block input xb (boxes of 131 rows x 64 channels, no swizzle) and the
 // kernel computes the Conv1D (conv_w [4, E], conv_b [E]) itself.
-template <int kJoin, int kMath, bool kConv>
-__global__ void __launch_bounds__(kConv ? kThreadsConv : kThreads, 1)
+template <int kJoin, int kMath, bool kConv, bool kMaps>
+__global__ void __launch_bounds__(kThreads, 1)
 rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_w,
                   const __grid_constant__ CUtensorMap map_ct, const __grid_constant__ CUtensorMap map_yt,
                   const __grid_constant__ CUtensorMap map_ot, const void* pos, int pos64,
                   const __nv_bfloat16* __restrict__ bias_x, const __nv_bfloat16* __restrict__ bias_a,
                   const __nv_bfloat16* m8sp, const float* h0, int B, int T_,
                   int E, int groups, int n_units, float* __restrict__ h_last, WsHeader* hdr,
-                  unsigned long long* agg, unsigned long long* incl, int use_agg,
+                  unsigned long long* agg, unsigned long long* incl,
                   const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ conv_b) {
   extern __shared__ uint8_t smem_raw[];
   // aligned by an offset into the shared array, so that the address space stays known to the
@@ -293,7 +313,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   auto bar_xs_empty = [&](int s) { return bar0 + 8u * (2 * kRing + 4 + 2 * kEpi + 2 + s); };
   const uint32_t bar_cfree = bar0 + 8u * (2 * kRing + 4 + 2 * kEpi + 4);
   constexpr int kR = kConv ? kRingConv : kRing;          // ring stages in use
-  constexpr int kAllThreads = kConv ? kThreadsConv : kThreads;
+  auto bar_carry = [&](int slot, int q, int tq) { return bar0 + 8u * (kNumBar + (slot * 4 + q) * 3 + tq); };
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
@@ -305,7 +325,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   // a = exp(log_a) and the input multiplier by log_a: computed once per CTA with the very
   // operations the gate arithmetic would use, so that looking them up changes no bit
   uint32_t* s_lut = reinterpret_cast<uint32_t*>(smem + kOffLut);
-  for (int i = threadIdx.x; i < kLutEntries; i += kAllThreads) s_lut[i] = a_mult_entry(i);
+  for (int i = threadIdx.x; i < kLutEntries; i += kThreads) s_lut[i] = a_mult_entry(i);
   if (threadIdx.x == 0) {
     *s_abort = 0;
     // with the conv fused a stage is full when the weights have landed AND the conv warps have
@@ -315,6 +335,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
     mbar_init(bar_cfree, kEpi);
     for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), kEpi); }
     for (int w = 0; w < kEpi; ++w) { mbar_init(bar_ct(w), 1); mbar_init(bar_yt(w), 1); }
+    for (int i = 0; i < kCarryBars; ++i) mbar_init(bar0 + 8u * (kNumBar + i), 1);
     mbar_fence_init();
   }
   if (warp == kEpi + 1) {
@@ -330,6 +351,8 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   // in before this one ends (its waiting warps cost this kernel, which is bound by issue, 6%)
   grid_dependency_wait();
 
+  if (warp >= kEpi) {
+  if constexpr (!kConv) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
   if (warp == kEpi) {
     // ------------------------------ TMA producer of the MMA operands ------------------------------
     if (lane == 0) {
@@ -367,31 +390,35 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
     }
   } else if (warp == kEpi + 1) {
     // ------------------------------ MMA issue -----------------------------------------------------
-    if (lane == 0) {
-      unsigned it = 0;
-      bool ok = true;
-      for (int t = 0; t < n_my && ok; ++t) {
-        const int as = t & 1;
-        ok = mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort);
+    // The whole warp runs the loop and one elected lane issues (see mma_ring): under `if (lane == 0)` a stage
+    // of eight instructions took a thousand cycles where they execute in 540.
+    const uint64_t desc_c = smem_desc_sw128(s_base + kOffRing), desc_w = smem_desc_sw128(s_base + kOffRing + kCBytes);
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = 0; t < n_my && ok; ++t) {
+      const int as = t & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_x = tmem_base + as * 2 * kUT;
+      for (int kb = 0; kb < kKBlocks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), phase, s_abort));
         if (!ok) break;
         tc_fence_after();
-        for (int kb = 0; kb < kKBlocks; ++kb, ++it) {
-          const int s = it % kR;
-          ok = mbar_wait(bar_full(s), (it / kR) & 1, s_abort);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t c0 = s_base + kOffRing + s * kStage, w0 = c0 + kCBytes;
+        if (elect_one()) {
+          const uint64_t dc = desc_c + (uint64_t)(s * (kStage >> 4)), dw = desc_w + (uint64_t)(s * (kStage >> 4));
 #pragma unroll
           for (int ks = 0; ks < kKB / 16; ++ks) {
             const uint32_t acc = (kb | ks) != 0 ? 1u : 0u;
-            const uint64_t bdesc = smem_desc_sw128(c0 + ks * 32);
-            tc_mma_bf16(tmem_base + as * 2 * kUT, smem_desc_sw128(w0 + ks * 32), bdesc, kIdesc, acc);
-            tc_mma_bf16(tmem_base + as * 2 * kUT + kUT, smem_desc_sw128(w0 + kUC * 128 + ks * 32), bdesc,
-                        kIdesc, acc);
+            tc_mma_bf16(d_x, dw + 2 * ks, dc + 2 * ks, kIdesc, acc);
+            tc_mma_bf16(d_x + kUT, dw + (kUC * 128 >> 4) + 2 * ks, dc + 2 * ks, kIdesc, acc);
           }
           tc_commit(bar_empty(s));
+          if (kb == kKBlocks - 1) tc_commit(bar_acc_full(as));
         }
-        if (ok) tc_commit(bar_acc_full(as));
+        __syncwarp();
+        if (++s == kR) { s = 0; phase ^= 1; }
       }
     }
   } else if (kConv && warp >= kEpi + 2) {
@@ -498,8 +525,13 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         }
       }
     }
+  }
   } else {
     // ------------------------------ epilogue ------------------------------------------------------
+    if constexpr (!kConv) {
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsEpilogue) : "memory");
+      named_bar_sync(6, kEpi * 32);
+    }
     const int chq = warp & 3;                // channel quarter = TMEM lane quarter of this warp
     const int tq = warp >> 2;                // token quarter: tokens 32 tq .. 32 tq + 31 of the unit
     const int set_id = 1 + chq;              // named barrier of the four token quarters
@@ -541,7 +573,10 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
     }
     // whether this lane's token of the next unit starts a document, and the constants of this
     // lane's channel in the next unit (gate biases, -8 softplus(a_param)): asked for a unit ahead
-    bool reset_next = n_my > 0 ? lane_reset(cur) : false;
+    // (an integer that the compiler may not turn back into a predicate: as a bool it arrived in the loop as
+    // false, on the first unit only, once the register counts were changed above)
+    int reset_next = n_my > 0 ? (int)lane_reset(cur) : 0;
+    asm volatile("" : "+r"(reset_next));
     uint32_t bxv = 0u, bav = 0u, spv = 0u;
     auto load_consts = [&](const UnitPos& u) {
       const int e = chan0(u) + lane;
@@ -556,31 +591,33 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
       const int tt = cur.tt, b = cur.b;
       const int e0 = chan0(cur);                                          // first channel of the warp
       const int tok0 = tt * kUT + tq * kSub;                              // first token of the warp
-      const int64_t rec = ((int64_t)(tt * per_tt + b * groups + cur.grp)) * 4 + chq;
+      // records: with maps one per tile and channel quarter, without one per chain and channel quarter
+      const int chain = b * groups + cur.grp;
+      const int64_t rec = ((int64_t)(kMaps ? tt * per_tt : 0) + chain) * 4 + chq;
+      const int64_t rec_in = kMaps ? rec - (int64_t)per_tt * 4 : rec;
+      const unsigned long long token = kMaps ? kToken : (unsigned long long)(unsigned)tt << 32;   // of the predecessor
       nxt = cur;
       step.advance(nxt);
-      float2* s_qmap = reinterpret_cast<float2*>(smem + kOffQmap) + ((par * 4 + chq) * 3) * 32;
-      float* s_hin = reinterpret_cast<float*>(smem + kOffHin) + (par * 4 + chq) * 32;
-      volatile int* s_known = reinterpret_cast<volatile int*>(smem + kOffKnown) + (par * 4 + chq);
 
-      const uint32_t resets = __ballot_sync(0xffffffffu, reset_next);
+      const uint32_t resets = __ballot_sync(0xffffffffu, reset_next != 0);
       // tokens of this warp past the end of the sequence (only in a sequence's last time tile)
       const int n_live = T_ - tok0;
       const uint32_t invalid = n_live >= 32 ? 0u : (n_live <= 0 ? 0xffffffffu : (0xffffffffu << n_live));
       const uint32_t bx2 = bxv | (bxv << 16), ba2 = bav | (bav << 16), m8sp2 = spv | (spv << 16);
       const uint32_t hbx2 = bmul2(bx2, 0x3f003f00u);
 
-      // the last token quarter asks for its predecessor's inclusive state now (normally published
-      // most of a round ago) and looks at the answer after the gate arithmetic
+      // the token quarter that needs it (the last one with maps, else the first) asks for its predecessor's
+      // inclusive state now (normally published most of a round ago) and looks at the answer after the
+      // gate arithmetic
       float hin_pref = 0.0f;
       bool have_hin = tt == 0;
       unsigned long long pre = 0ull;
-      if (tq == 3) {
+      if (tq == (kMaps ? 3 : 0)) {
         if (tt == 0) {
           if (h0 != nullptr && RGK_IN_RANGE((int64_t)b * E + e0 + lane, n_state, &hdr->status))
             hin_pref = h0[(int64_t)b * E + e0 + lane];
-        } else if (RGK_IN_RANGE((rec - (int64_t)per_tt * 4) * kSub + lane, n_words, &hdr->status)) {
-          pre = ld_relaxed_u64(incl + (rec - (int64_t)per_tt * 4) * kSub + lane);
+        } else if (RGK_IN_RANGE(rec_in * kSub + lane, n_words, &hdr->status)) {
+          pre = ld_relaxed_u64(incl + rec_in * kSub + lane);
         }
       }
 
@@ -629,10 +666,10 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         const uint32_t rs = (resets >> (half * 16)) & 0xffffu;
         const uint32_t inv = (invalid >> (half * 16)) & 0xffffu;
         if ((rs | inv) == 0u)
-          gates_16<false, kMath>(zx, za, c, bx2, ba2, hbx2, m8sp2, rs, inv, a_pk + half * 8,
+          gates_16<false, kMath, kMaps>(zx, za, c, bx2, ba2, hbx2, m8sp2, rs, inv, a_pk + half * 8,
                                  x_pk + half * 8, P, H, s_lut);
         else
-          gates_16<true, kMath>(zx, za, c, bx2, ba2, hbx2, m8sp2, rs, inv, a_pk + half * 8,
+          gates_16<true, kMath, kMaps>(zx, za, c, bx2, ba2, hbx2, m8sp2, rs, inv, a_pk + half * 8,
                                 x_pk + half * 8, P, H, s_lut);
         if (half == 0) {
           // the previous unit's output tile must have been read by its store before the buffer is
@@ -647,78 +684,138 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         }
       }
       if (t + 1 < n_my) load_consts(nxt);
-      if (t + 1 < n_my) reset_next = lane_reset(nxt);
+      if (t + 1 < n_my) reset_next = (int)lane_reset(nxt);
 
-      // The incoming state is normally known before the tile's own map is (the predecessor's
-      // inclusive record was there at the start of the unit): then the quarters need one barrier,
-      // to see each other's maps, and nothing waits for the record of this tile to be published.
-      if (tq == 3) {
-        if (tt > 0) {
-          bool all = __all_sync(0xffffffffu, (pre >> 32) == 1ull);
-          if (!all) {
-            // the predecessor's CTA runs a little behind: ask once more before taking the long way
-            pre = ld_relaxed_u64(incl + (rec - (int64_t)per_tt * 4) * kSub + lane);
-            all = __all_sync(0xffffffffu, (pre >> 32) == 1ull);
+      float h;                               // the state entering the thread's tokens
+      if constexpr (kMaps) {
+        float2* s_qmap = reinterpret_cast<float2*>(smem + kOffQmap) + ((par * 4 + chq) * 3) * 32;
+        float* s_hin = reinterpret_cast<float*>(smem + kOffHin) + (par * 4 + chq) * 32;
+        volatile int* s_known = reinterpret_cast<volatile int*>(smem + kOffKnown) + (par * 4 + chq);
+        // The incoming state is normally known before the tile's own map is (the predecessor's
+        // inclusive record was there at the start of the unit): then the quarters need one barrier,
+        // to see each other's maps, and nothing waits for the record of this tile to be published.
+        if (tq == 3) {
+          if (tt > 0) {
+            bool all = __all_sync(0xffffffffu, (pre >> 32) == 1ull);
+            if (!all) {
+              // the predecessor's CTA runs a little behind: ask once more before taking the long way
+              pre = ld_relaxed_u64(incl + rec_in * kSub + lane);
+              all = __all_sync(0xffffffffu, (pre >> 32) == 1ull);
+            }
+            if (all) {
+              hin_pref = __uint_as_float((uint32_t)pre);
+              have_hin = true;
+            }
           }
-          if (all) {
-            hin_pref = __uint_as_float((uint32_t)pre);
-            have_hin = true;
-          }
+          if (have_hin) s_hin[lane] = hin_pref;
+          if (lane == 0) *s_known = have_hin ? 1 : 0;
         }
-        if (have_hin) s_hin[lane] = hin_pref;
-        if (lane == 0) *s_known = have_hin ? 1 : 0;
-      }
-      if (tq < 3) s_qmap[tq * 32 + lane] = make_float2(P, H);   // the last quarter keeps its own
-      named_bar_sync(set_id, 128);
-      const bool known = *s_known != 0;
+        if (tq < 3) s_qmap[tq * 32 + lane] = make_float2(P, H);   // the last quarter keeps its own
+        named_bar_sync(set_id, 128);
+        const bool known = *s_known != 0;
 
-      // ---- the last token quarter: the tile's map, the incoming state, the records ---------------
-      if (tq == 3) {
-        float Pt = 1.0f, Ht = 0.0f;
+        // ---- the last token quarter: the tile's map, the incoming state, the records ---------------
+        if (tq == 3) {
+          float Pt = 1.0f, Ht = 0.0f;
 #pragma unroll
-        for (int qq = 0; qq < 3; ++qq) {
-          const float2 m = s_qmap[qq * 32 + lane];
-          Ht = fmaf(m.x, Ht, m.y);
-          Pt *= m.x;
-        }
-        Ht = fmaf(P, Ht, H);
-        Pt *= P;
-        float hin = hin_pref;
-        if (!known) {
-          // Decoupled look-back, one channel per lane.  With use_agg (fewer chains than CTAs: the
-          // earlier tiles of this chain are in flight on other SMs) the tile's own map is published
-          // first, and maps of earlier tiles are composed until a tile with a known state is met;
-          // otherwise only the predecessor's state is waited for (it was dealt out a round earlier).
-          if (use_agg && RGK_IN_RANGE(rec * kSub + lane, n_words, &hdr->status)) {
-            st_relaxed_u64(agg + (rec * kSub + lane) * 2, kToken | (unsigned long long)__float_as_uint(Pt));
-            st_relaxed_u64(agg + (rec * kSub + lane) * 2 + 1, kToken | (unsigned long long)__float_as_uint(Ht));
+          for (int qq = 0; qq < 3; ++qq) {
+            const float2 m = s_qmap[qq * 32 + lane];
+            Ht = fmaf(m.x, Ht, m.y);
+            Pt *= m.x;
           }
-          bool timed_out = false;
-          if (ok) hin = look_back(agg, incl, h0, rec, tt, per_tt, b, E, e0 + lane, lane, use_agg, &timed_out,
-                                 n_words, n_state, &hdr->status);
-          __syncwarp();
-          if (__any_sync(0xffffffffu, timed_out)) {
-            if (lane == 0) atomicExch(&hdr->status, kStatusTimeout);
-            hin = 0.0f;
+          Ht = fmaf(P, Ht, H);
+          Pt *= P;
+          float hin = hin_pref;
+          if (!known) {
+            // Decoupled look-back, one channel per lane: the tile's own map is published first, and maps of
+            // earlier tiles (in flight on other SMs) are composed until a tile with a known state is met.
+            if (RGK_IN_RANGE(rec * kSub + lane, n_words, &hdr->status)) {
+              st_relaxed_u64(agg + (rec * kSub + lane) * 2, kToken | (unsigned long long)__float_as_uint(Pt));
+              st_relaxed_u64(agg + (rec * kSub + lane) * 2 + 1, kToken | (unsigned long long)__float_as_uint(Ht));
+            }
+            bool timed_out = false;
+            if (ok) hin = look_back(agg, incl, h0, rec, tt, per_tt, b, E, e0 + lane, lane, &timed_out,
+                                   n_words, n_state, &hdr->status);
+            __syncwarp();
+            if (__any_sync(0xffffffffu, timed_out)) {
+              if (lane == 0) atomicExch(&hdr->status, kStatusTimeout);
+              hin = 0.0f;
+            }
+            if (!ok) hin = 0.0f;
+            s_hin[lane] = hin;
           }
-          if (!ok) hin = 0.0f;
-          s_hin[lane] = hin;
+          const float h_end = fmaf(Pt, hin, Ht);
+          if (RGK_IN_RANGE(rec * kSub + lane, n_words, &hdr->status))
+            st_relaxed_u64(incl + rec * kSub + lane, kToken | (unsigned long long)__float_as_uint(h_end));
+          if (h_last != nullptr && tt == tiles_t - 1 &&
+              RGK_IN_RANGE((int64_t)b * E + e0 + lane, n_state, &hdr->status))
+            h_last[(int64_t)b * E + e0 + lane] = h_end;
         }
-        const float h_end = fmaf(Pt, hin, Ht);
-        if (RGK_IN_RANGE(rec * kSub + lane, n_words, &hdr->status))
-          st_relaxed_u64(incl + rec * kSub + lane, kToken | (unsigned long long)__float_as_uint(h_end));
-        if (h_last != nullptr && tt == tiles_t - 1 &&
-            RGK_IN_RANGE((int64_t)b * E + e0 + lane, n_state, &hdr->status))
-          h_last[(int64_t)b * E + e0 + lane] = h_end;
-      }
-      if (!known) named_bar_sync(set_id, 128);
+        if (!known) named_bar_sync(set_id, 128);
 
-      // ---- replay with the true incoming state, join, output tile ---------------------------------
-      float h = s_hin[lane];
-      for (int qq = 0; qq < tq; ++qq) {
-        const float2 m = s_qmap[qq * 32 + lane];
-        h = fmaf(m.x, h, m.y);
+        // ---- replay with the true incoming state, join, output tile ---------------------------------
+        h = s_hin[lane];
+        for (int qq = 0; qq < tq; ++qq) {
+          const float2 m = s_qmap[qq * 32 + lane];
+          h = fmaf(m.x, h, m.y);
+        }
+      } else {
+        // Without maps the state itself goes through the token quarters, one after the other: the first
+        // has it from the predecessor's record, the last publishes it.  The four warps of a channel
+        // quarter share a scheduler and drift apart by what a hand-over takes, so that one's wait is
+        // covered by the others' gate arithmetic.  A warp is at most three units ahead of the one behind
+        // it (accumulator set t + 2 is written only when every warp has read set t), so with four slots
+        // no barrier phase and no carry is overtaken.  One record a chain: tile tt replaces the state it
+        // has read itself (its first quarter, before its last).
+        const int slot = t & (kSlots - 1);
+        float* s_carry = reinterpret_cast<float*>(smem + kOffCarry) + (slot * 4 + chq) * 3 * 32 + lane;
+        if (tq == 0) {
+          if (tt > 0) {
+            unsigned spins = 0;
+            while (ok && !__all_sync(0xffffffffu, (pre & ~0xffffffffull) == token)) {
+              if (++spins > kLookbackSpins) {
+                if (lane == 0) atomicExch(&hdr->status, kStatusTimeout);
+                pre = 0ull;
+                break;
+              }
+              if (spins > 16) __nanosleep(32);
+              pre = ld_relaxed_u64(incl + rec_in * kSub + lane);
+            }
+            hin_pref = ok ? __uint_as_float((uint32_t)pre) : 0.0f;
+          }
+          h = hin_pref;
+        } else {
+          if (ok) ok = mbar_wait(bar_carry(slot, chq, tq - 1), (t / kSlots) & 1, s_abort);
+          h = ok ? s_carry[(tq - 1) * 32] : 0.0f;
+        }
       }
+
+      // ---- the recurrence: x becomes y ------------------------------------------------------------
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const uint32_t a2 = a_pk[k], x2 = x_pk[k];
+        h = fmaf(bf16_lo(a2), h, bf16_lo(x2));
+        const float y0 = h;
+        h = fmaf(bf16_hi(a2), h, bf16_hi(x2));
+        x_pk[k] = pack_bf16x2(y0, h);
+      }
+      if constexpr (!kMaps) {
+        if (tq < 3) {
+          const int slot = t & (kSlots - 1);
+          reinterpret_cast<float*>(smem + kOffCarry)[((slot * 4 + chq) * 3 + tq) * 32 + lane] = h;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_carry(slot, chq, tq));
+        } else {
+          if (RGK_IN_RANGE(rec * kSub + lane, n_words, &hdr->status))
+            st_relaxed_u64(incl + rec * kSub + lane,
+                           (unsigned long long)(unsigned)(tt + 1) << 32 | (unsigned long long)__float_as_uint(h));
+          if (h_last != nullptr && tt == tiles_t - 1 &&
+              RGK_IN_RANGE((int64_t)b * E + e0 + lane, n_state, &hdr->status))
+            h_last[(int64_t)b * E + e0 + lane] = h;
+        }
+      }
+
+      // ---- join, output tile ----------------------------------------------------------------------
       if constexpr (kJoin != 0) {
         if (ok) ok = mbar_wait(bar_yt(warp), t & 1, s_abort);
         transpose_tile(tile_y_s + row_off, tile_y_s + st_off);
@@ -732,11 +829,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-          const uint32_t a2 = a_pk[4 * k + w], x2 = x_pk[4 * k + w];
-          h = fmaf(bf16_lo(a2), h, bf16_lo(x2));
-          const float y0 = h;
-          h = fmaf(bf16_hi(a2), h, bf16_hi(x2));
-          uint32_t y2 = pack_bf16x2(y0, h);
+          uint32_t y2 = x_pk[4 * k + w];
           if constexpr (kJoin == 1) y2 = join_gelu2<kMath>(y2, z[w]);
           else if constexpr (kJoin == 2) y2 = bmul2(y2, z[w]);
           o[w] = y2;
@@ -795,29 +888,42 @@ ChanLayout chan_layout(int64_t B, int64_t T, int64_t E) {
 
 // The kernel needs more dynamic shared memory than the default limit: the attribute is a property
 // of the function on ONE device, so it is set (and the SM count read) once per device.
-template <int kMath, bool kConv>
+template <int kMath, bool kConv, bool kMaps>
 cudaError_t chan_set_smem() {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<0, kMath, kConv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<1, kMath, kConv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)) != cudaSuccess) return e;
-  return cudaFuncSetAttribute(rglru_chan_kernel<2, kMath, kConv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<0, kMath, kConv, kMaps>, attr, kSmem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<1, kMath, kConv, kMaps>, attr, kSmem)) != cudaSuccess) return e;
+  return cudaFuncSetAttribute(rglru_chan_kernel<2, kMath, kConv, kMaps>, attr, kSmem);
+}
+template <bool kMaps>
+cudaError_t chan_set_smem_all() {
+  cudaError_t e;
+  if ((e = chan_set_smem<kMathExact, false, kMaps>()) != cudaSuccess) return e;
+  if ((e = chan_set_smem<kMathFast, false, kMaps>()) != cudaSuccess) return e;
+  if ((e = chan_set_smem<kMathExact, true, kMaps>()) != cudaSuccess) return e;
+  return chan_set_smem<kMathFast, true, kMaps>();
 }
 
 cudaError_t chan_device_setup(int* num_sms) {
   static PerDeviceOnce once;
   return once.run([] {
-    cudaError_t e;
-    if ((e = chan_set_smem<kMathExact, false>()) != cudaSuccess) return e;
-    if ((e = chan_set_smem<kMathFast, false>()) != cudaSuccess) return e;
-    if ((e = chan_set_smem<kMathExact, true>()) != cudaSuccess) return e;
-    return chan_set_smem<kMathFast, true>();
+    const cudaError_t e = chan_set_smem_all<false>();
+    return e != cudaSuccess ? e : chan_set_smem_all<true>();
   }, num_sms);
 }
 
-// With fewer units per time tile than CTAs, consecutive tiles of a chain are in flight at once
-// and carries are resolved from published maps; otherwise a tile's predecessor was dealt out a
-// round earlier and only its state is ever waited for.
-bool chan_uses_maps(int64_t B, int groups, int grid) { return B * groups < grid; }
+// How a tile's incoming state reaches it.  From tile to tile (kMaps false) a chain - one sequence, one half
+// head - moves on by one tile per hand-over, the four token quarters one after the other and a round trip to
+// the next SM, 2.3 us in all where a unit takes 3.3: fast enough as long as the SMs have a quarter as many
+// chains to share, and four instructions a token pair cheaper.  Below that, and where all of a call's units
+// are in flight at once, tiles publish their maps (P, H) and look back over several of them.  Recurrent path
+// of 2560 (20 chains a sequence) and RG-LRU of 4096 (32 chains) channels, us with maps / without: 20 chains
+// 2501 tokens 30.1 / 38.7, 32 chains 29.4 / 37.6, 40 chains 47.5 / 46.0, 64 chains 47.4 / 43.3, 128 chains
+// 82.6 / 66.5; 40 chains of 300 tokens (120 units) 16.5 / 17.5, 60 chains 20.0 / 19.2.
+bool chan_uses_maps(int64_t B, int groups, int64_t n_units, int num_sms) {
+  return n_units <= num_sms || B * groups * 4 < num_sms;
+}
 
 }  // namespace
 
@@ -830,7 +936,7 @@ size_t rglru_chan_workspace_bytes(int64_t B, int64_t T, int64_t E) {
   return chan_layout(B, T, E).total;
 }
 
-// State words (and map words, where used) start without their token; the status word in front of them
+// State words (and map words, where used) start without a token (0 is no tile's); the status word in front of them
 // belongs to the caller.
 ChanPrep rglru_chan_prep(void* ws, const void* a_param, int64_t B, int64_t T, int H) {
   ChanPrep p;
@@ -839,9 +945,8 @@ ChanPrep rglru_chan_prep(void* ws, const void* a_param, int64_t B, int64_t T, in
   const int E = H * kHW;
   const ChanLayout L = chan_layout(B, T, E);
   char* base = static_cast<char*>(ws);
-  const int grid = (int)(L.n_units < num_sms ? L.n_units : num_sms);
   p.zero = reinterpret_cast<uint4*>(base + L.incl_off);
-  p.n_zero = (int64_t)(((chan_uses_maps(B, 2 * H, grid) ? L.m8sp_off : L.agg_off) - L.incl_off) / 16);
+  p.n_zero = chan_uses_maps(B, 2 * H, L.n_units, num_sms) ? (int64_t)(L.m8sp_off - L.incl_off) / 16 : B * E * 8 / 16;
   p.a_param = static_cast<const __nv_bfloat16*>(a_param);
   p.m8sp = reinterpret_cast<__nv_bfloat16*>(base + L.m8sp_off);
   p.E = E;
@@ -864,7 +969,7 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
   const int groups = 2 * H;
   const int n_units = (int)L.n_units;
   const int grid = n_units < num_sms ? n_units : num_sms;   // all CTAs resident: look-back may spin
-  const int use_agg = chan_uses_maps(B, groups, grid) ? 1 : 0;
+  const bool maps = chan_uses_maps(B, groups, n_units, num_sms);
   const ChanPrep prep = rglru_chan_prep(ws, a_param, B, T, H);
   if (!prepared) {
     const int64_t n = prep.n_zero > prep.E ? prep.n_zero : prep.E, blocks = (n + 1023) / 1024;
@@ -883,16 +988,19 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
       !tensor_map_bte_sw64(&map_ot, out, Bu, Tu, Eu, kSub, kSub) ||
       !tensor_map_bte_sw64(&map_yt, yb != nullptr ? yb : out, Bu, Tu, Eu, kSub, kSub))
     return cudaErrorInvalidValue;
-#define RGK_CHAN_C(J, M, C, THREADS)                                                             \
-  err = launch_dependent(rglru_chan_kernel<J, M, C>, dim3(grid), dim3(THREADS), kSmem, s,        \
+#define RGK_CHAN_C(J, M, C, S)                                                                   \
+  err = launch_dependent(rglru_chan_kernel<J, M, C, S>, dim3(grid), dim3(kThreads), kSmem, s,    \
                          map_c, map_w, map_ct, map_yt, map_ot, pos, pos64, (const T_*)bx,        \
                          (const T_*)ba, m8sp, h0, (int)B, (int)T, E, groups, n_units, h_last,    \
                          reinterpret_cast<WsHeader*>(base),                                      \
                          reinterpret_cast<unsigned long long*>(base + L.agg_off),                \
-                         reinterpret_cast<unsigned long long*>(base + L.incl_off), use_agg,      \
+                         reinterpret_cast<unsigned long long*>(base + L.incl_off),               \
                          (const T_*)conv_w, (const T_*)conv_b)
 #define RGK_CHAN(J, M)                                                                           \
-  do { if (conv) RGK_CHAN_C(J, M, true, kThreadsConv); else RGK_CHAN_C(J, M, false, kThreads); } while (0)
+  do {                                                                                           \
+    if (conv) { if (maps) RGK_CHAN_C(J, M, true, true); else RGK_CHAN_C(J, M, true, false); }    \
+    else { if (maps) RGK_CHAN_C(J, M, false, true); else RGK_CHAN_C(J, M, false, false); }       \
+  } while (0)
 #define RGK_CHAN_J(M)                                                                            \
   if (join == 0) RGK_CHAN(0, M); else if (join == 1) RGK_CHAN(1, M); else RGK_CHAN(2, M)
   const int join = yb == nullptr ? 0 : (y_activated ? 2 : 1);

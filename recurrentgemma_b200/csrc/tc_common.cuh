@@ -8,18 +8,27 @@
 
 namespace rgk {
 
-// Waits ask the hardware to suspend the thread for up to kWaitHintNs per attempt (it wakes when the
-// barrier's phase completes), so a waiting thread issues an instruction only every so often; the
-// number of attempts bounds the wait at about a second.
-constexpr unsigned kWaitHintNs = 20000;
-constexpr unsigned kWaitLimit = 1u << 16;
+// A wait is bounded by kWaitNs: long behind anything a kernel here waits for, short enough to end by itself.
+constexpr unsigned long long kWaitNs = 2000000000ull;
+constexpr unsigned kWaitLimit = 1u << 26;                  // and by this many attempts, whatever the timer says
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 
 // Bounded wait.  Returns false (and raises the CTA's abort flag) when the limit is hit or another
-// role has already aborted.
+// role has already aborted.  The first attempt, which suspends the thread for as long as the hardware sees
+// fit, stands by itself, ahead of the loop (with a suspension time asked for, each attempt became a loop of
+// its own that slept and polled: 4 to 10 of 47 instructions an element of the RG-LRU kernel).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (unsigned i = 0; i < kWaitLimit; ++i) {
-    if (mbar_try_wait(bar, parity, kWaitHintNs)) return true;
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+#pragma unroll 1
+  for (unsigned i = 1; i < kWaitLimit; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
+    if ((i & 255u) == 0 && global_ns() - t0 > kWaitNs) break;
   }
   *abort_flag = 1;
   return false;
@@ -239,16 +248,23 @@ __device__ __forceinline__ void st_peer_u32(uint32_t addr, uint32_t v) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory");
 }
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (unsigned i = 0; i < kWaitLimit; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kWaitHintNs) : "memory");
-    if (ok) return true;
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+#pragma unroll 1
+  for (unsigned i = 1; i < kWaitLimit; ++i) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
     if (*abort_flag) return false;
+    if ((i & 255u) == 0 && global_ns() - t0 > kWaitNs) break;
   }
   *abort_flag = 1;
   return false;
@@ -414,8 +430,12 @@ __device__ __forceinline__ void a_mult_lookup(uint32_t la2, const uint32_t* lut,
   // directly, relative to the bits of -2^-11.
   uint32_t m;
   asm("min.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(la2), "r"(0x80008000u | kLutBase | (kLutBase << 16)));
-  const uint32_t* base = lut - (0x8000u | kLutBase);
-  const uint32_t e0 = base[m & 0xffffu], e1 = base[m >> 16];
+  // address = 4 x half + table, one instruction each (a dot product with 4 in the byte of the half meant)
+  const uint32_t base = smem_u32(lut) - 4u * (0x8000u | kLutBase);
+  const uint32_t p0 = __dp2a_lo(m, 0x0004u, base), p1 = __dp2a_lo(m, 0x0400u, base);
+  uint32_t e0, e1;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(e0) : "r"(p0));
+  asm("ld.shared.u32 %0, [%1];" : "=r"(e1) : "r"(p1));
   asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(a2) : "r"(e0), "r"(e1));
   asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(mult2) : "r"(e0), "r"(e1));
 }

@@ -25,16 +25,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
-// One attempt; the thread may be suspended by the hardware for up to `hint_ns` while it waits,
-// which keeps waiting warps from spending issue slots on polling.
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity,
-                                              uint32_t hint_ns = 1000u) {
+// One attempt; the hardware may suspend the thread for a while of its own choosing and wakes it when the
+// phase completes.
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar), "r"(parity), "r"(hint_ns) : "memory");
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
 // Non-blocking test of a phase; lets a caller ask early and look at the answer later.

@@ -515,6 +515,57 @@ def test_fused_rglru_kernel(rg, oracle, shape):
     m2(torch.zeros(1, 128, 256, device=DEV, dtype=dt), torch.arange(128, device=DEV)[None])
 
 
+@pytest.mark.parametrize("shape", [(18, 1, 1030), (19, 1, 1030), (74, 1, 257), (75, 1, 129), (74, 1, 129),
+                                   (5, 4, 640), (2, 16, 513)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("join", [False, True], ids=["plain", "join"])
+def test_fused_rglru_kernel_states_from_tile_to_tile(rg, oracle, shape, join):
+  """The two ways a tile's incoming state reaches it, on either side of where one takes over from the other
+  (36 / 38 chains, 148 / 150 units on 148 SMs), ragged last tiles, one to nine tiles a chain, an initial
+  state: against the oracle, and twice in a row on the same workspace (the records of the first call must
+  not be taken for the second's)."""
+  from recurrentgemma_b200 import _lib
+  b, h, t = shape
+  e = h * 256
+  dt = torch.bfloat16
+  case = C.Case(f"states_{b}_{t}_{e}", "rglru", "bfloat16", b, t, e, h, pos="multi")
+  p = C.make_params(case)
+  g = torch.Generator(device="cpu").manual_seed(b * 1000 + t)
+  x = torch.randn((b, t, e), generator=g).to(dt)
+  y = torch.randn((b, t, e), generator=g).to(dt)
+  pos = C.geometric_segment_pos(b, t, 100.0, 3)
+  pos[:, 0] = 5                      # the first token continues a document: the initial state counts
+  lru = rg.RGLRU(e, h, device=DEV, dtype=dt)
+  pr = {k[len("rg_lru."):]: v for k, v in p.items() if k.startswith("rg_lru.")}
+  lru.load_state_dict(pr)
+  rows = sorted({0, b - 1})
+  if join:
+    conv = rg.Conv1D(e, 4, device=DEV, dtype=dt)
+    conv.w.data.zero_()              # the identity
+    conv.w.data[3].fill_(1.0)
+    conv.b.data.zero_()
+    h0 = None
+  else:
+    h0 = torch.randn((b, e), generator=g) * 0.5
+  for scale in (1.0, 0.5):
+    xs = x * scale
+    if join:
+      out, cache = rg.recurrent_path(xs.to(DEV), y.to(DEV), pos.to(DEV), conv, lru)
+      h_last = cache.rg_lru_state
+    else:
+      out, h_last = lru(xs.to(DEV), pos.to(DEV), h0.to(DEV))
+    rg.check_status()
+    for row in rows:
+      o_r, h_r = oracle.rglru(xs[row:row + 1].contiguous(), pos[row:row + 1], pr["a_param"], pr["input_gate.w"],
+                              pr["input_gate.b"], pr["a_gate.w"], pr["a_gate.b"],
+                              None if h0 is None else h0[row:row + 1].contiguous())
+      if join:
+        o_r = o_r.to(dt) * torch.nn.functional.gelu(y[row:row + 1], approximate="tanh")
+      assert_close(out[row:row + 1], o_r, TOL[dt], f"row {row}")
+      assert_close(h_last[row:row + 1], h_r, TOL[dt], f"state of row {row}")
+
+
+
 def test_host_pipeline_matches_device_call(rg):
   """The host-buffer pipeline (rows streamed through copy-in / compute / copy-out streams) returns
   what the device-resident call returns."""
