@@ -72,6 +72,9 @@ __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, ui
       :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The place of a launch among those that share the tiles of a call.
+enum { kAlone = 0, kFirst = 1, kSecond = 2 };
+
 // v with the low 13 mantissa bits cleared (an exact TF32 value), and the rest of v (exact).
 __device__ __forceinline__ float tf32_high_part(float v) {
   return __uint_as_float(__float_as_uint(v) & 0xffffe000u);
@@ -84,7 +87,8 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                   const __grid_constant__ CUtensorMap map_wl, const float* x,
                   const void* pos, int pos64, const float* __restrict__ a_param,
                   const float* __restrict__ bias_x, const float* __restrict__ bias_a, int64_t M,
-                  int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr, const ScanPrep prep) {
+                  int E, float* __restrict__ a_out, float* __restrict__ xn_out, WsHeader* hdr, const ScanPrep prep,
+                  int first_tile, int order) {
   using C = Cfg<kTN, kPerSm>;
   constexpr int kEpi = C::kEpi;
   constexpr int kStages = C::kStages, kBBytes = C::kBBytes, kStageBytes = C::kStageBytes;
@@ -103,7 +107,8 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + C::kOffAbort);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = E / kChans, tile = blockIdx.x / n_tiles, chan0 = (blockIdx.x - tile * n_tiles) * kChans;
+  const int n_tiles = E / kChans, index = first_tile + blockIdx.x;
+  const int tile = index / n_tiles, chan0 = (index - tile * n_tiles) * kChans;
   const int head = chan0 / kHW;
   const int wrow = chan0 / kHalf * (2 * kHalf) + chan0 % kHalf;      // packed rows: x-gate, kHalf behind a-gate
 
@@ -122,7 +127,9 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                  :: "r"(s_base + C::kOffTmem), "r"(kTN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  grid_dependency_wait();
+  // (the second of two launches starts when every CTA of the first has passed its own wait)
+  if (order != kSecond) grid_dependency_wait();
+  if (order == kFirst) grid_launch_dependents();
   if (prep.ticket != nullptr) {                              // for the scan kernel behind
     if (blockIdx.x == 0 && threadIdx.x == 0) *prep.ticket = 0u;
     for (int64_t i = (int64_t)blockIdx.x * C::kThreads + threadIdx.x; i < prep.n_zero;
@@ -160,27 +167,31 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
   } else if (warp == kEpi + 1) {
     // ------------------------------ MMA issue -----------------------------------------------------
-    if (lane == 0) {
-      bool ok = true;
-      for (int kb = 0; kb < kSlices && ok; ++kb) {
-        const int s = kb % kStages;
-        ok = mbar_wait(bar_full(s), (kb / kStages) & 1, s_abort);
-        if (ok) ok = mbar_wait(bar_lo(s), (kb / kStages) & 1, s_abort);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t a_hi = s_base + s * kStageBytes, a_lo = a_hi + kABytes;
-        const uint32_t b_hi = a_hi + 2 * kABytes, b_lo = b_hi + kBBytes;
+    // (the whole warp runs the loop, one elected lane issues: see mma_ring)
+    const uint64_t desc_a = smem_desc_sw64(s_base), desc_b = smem_desc_sw64(s_base + 2 * kABytes);
+    bool ok = true;
+    int s = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < kSlices; ++kb) {
+      ok = mbar_wait(bar_full(s), phase, s_abort);
+      if (ok) ok = mbar_wait(bar_lo(s), phase, s_abort);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t st = (uint64_t)(s * (kStageBytes >> 4));
+        const uint64_t dah = desc_a + st, dal = dah + (kABytes >> 4), dbh = desc_b + st, dbl = dbh + (kBBytes >> 4);
 #pragma unroll
         for (int ks = 0; ks < kKS / 8; ++ks) {
-          const uint64_t dah = smem_desc_sw64(a_hi + ks * 32), dal = smem_desc_sw64(a_lo + ks * 32);
-          const uint64_t dbh = smem_desc_sw64(b_hi + ks * 32), dbl = smem_desc_sw64(b_lo + ks * 32);
-          tc_mma_tf32(tmem_base, dah, dbh, kIdescF, (kb | ks) != 0 ? 1u : 0u);
-          tc_mma_tf32(tmem_base, dal, dbh, kIdescF, 1u);
-          tc_mma_tf32(tmem_base, dah, dbl, kIdescF, 1u);
+          tc_mma_tf32(tmem_base, dah + 2 * ks, dbh + 2 * ks, kIdescF, (kb | ks) != 0 ? 1u : 0u);
+          tc_mma_tf32(tmem_base, dal + 2 * ks, dbh + 2 * ks, kIdescF, 1u);
+          tc_mma_tf32(tmem_base, dah + 2 * ks, dbl + 2 * ks, kIdescF, 1u);
         }
         tc_commit(bar_empty(s));
+        if (kb == kSlices - 1) tc_commit(bar_acc);
       }
-      if (ok) tc_commit(bar_acc);
+      __syncwarp();
+      if (++s == kStages) { s = 0; phase ^= 1; }
     }
   } else {
     // ------------------------------ helper, then epilogue ------------------------------------------
@@ -284,6 +295,7 @@ gates_tf32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 
   // ------------------------------ teardown --------------------------------------------------------
+  if (order == kSecond) grid_dependency_wait();            // whoever waits for this launch waits for the first too
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *s_abort) atomicExch(&hdr->status, kStatusTimeout);
@@ -303,17 +315,17 @@ cudaError_t set_smem() {
 template <int kTN, int kPerSm>
 cudaError_t launch_gates_t(const float* c, const void* pos, int pos64, const float* a_param, const float* bx,
                            const float* ba, int64_t M, int E, const float* hi, const float* lo, float* a_out,
-                           float* xn_out, WsHeader* hdr, cudaStream_t s, const ScanPrep& prep) {
+                           float* xn_out, WsHeader* hdr, cudaStream_t s, const ScanPrep& prep, int64_t first_tile,
+                           int64_t n_tiles, int order) {
   const uint64_t w_rows = (uint64_t)E / kHalf * (2 * kHalf);
   CUtensorMap map_x, map_wh, map_wl;
   if (!tensor_map_2d(&map_x, c, (uint64_t)M, (uint64_t)E, kTM, kKS, false, 4, true) ||
       !tensor_map_2d(&map_wh, hi, w_rows, kHW, kTN / 2, kKS, false, 4, true) ||
       !tensor_map_2d(&map_wl, lo, w_rows, kHW, kTN / 2, kKS, false, 4, true))
     return cudaErrorInvalidValue;
-  const int64_t tiles = (M + kTM - 1) / kTM * (E / (kTN / 2));
-  return launch_dependent(gates_tf32_kernel<kTN, kPerSm>, dim3((unsigned)tiles), dim3(Cfg<kTN, kPerSm>::kThreads),
+  return launch_dependent(gates_tf32_kernel<kTN, kPerSm>, dim3((unsigned)n_tiles), dim3(Cfg<kTN, kPerSm>::kThreads),
                           (size_t)Cfg<kTN, kPerSm>::kSmem, s, map_x, map_wh, map_wl, c, pos, pos64, a_param, bx, ba,
-                          M, E, a_out, xn_out, hdr, prep);
+                          M, E, a_out, xn_out, hdr, prep, (int)first_tile, order);
 }
 
 // Splits the two gate weights [H, 256 (k), 256 (n)] float32 into K-major groups
@@ -382,9 +394,20 @@ cudaError_t launch_gates_tf32(const void* c, const void* pos, int pos64, const v
   // 829 -> 737 us with the scan behind.  Few tiles are cut in half: 200 tokens 29 -> 25 us.
   const int64_t m_tiles = (M + kTM - 1) / kTM, tiles = m_tiles * (E / kHalf);
   if (2 * tiles > 0x7fffffff) return cudaErrorInvalidValue;
-  auto launch = tiles > num_sms ? launch_gates_t<256, 2> : (2 * tiles > num_sms ? launch_gates_t<256, 1> : launch_gates_t<128, 2>);
-  return launch((const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba, M, E, hi, lo,
-                (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header), s, prep);
+  auto run = [&](auto launch, int64_t first, int64_t n, int order) {
+    return launch((const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba, M, E, hi,
+                  lo, (float*)a_out, (float*)xn_out, reinterpret_cast<WsHeader*>(ws_header), s,
+                  order == kSecond ? ScanPrep() : prep, first, n, order);
+  };
+  if (2 * tiles <= num_sms) return run(launch_gates_t<128, 2>, 0, 2 * tiles, kAlone);
+  if (tiles <= num_sms) return run(launch_gates_t<256, 1>, 0, tiles, kAlone);
+  // A last wave that half tiles, one an SM, can carry becomes a second launch of those, whose CTAs start as
+  // the first's leave: 2048 tokens (24 of 320 tiles) 71 -> 66 us with the scan, 4096 (48 of 640) 131 -> 124;
+  // with 96 of 1280 tiles left over 234.5 -> 236, with 204 of 500 94 -> 98.
+  const int64_t slots = 2 * (int64_t)num_sms, rest = tiles > slots ? tiles % slots : 0;
+  if (rest == 0 || 2 * rest > num_sms) return run(launch_gates_t<256, 2>, 0, tiles, kAlone);
+  e0 = run(launch_gates_t<256, 2>, 0, tiles - rest, kFirst);
+  return e0 != cudaSuccess ? e0 : run(launch_gates_t<128, 2>, 2 * (tiles - rest), 2 * rest, kSecond);
 }
 
 }  // namespace rgk

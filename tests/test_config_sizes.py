@@ -54,6 +54,27 @@ def test_rglru_layer_float32_at_config_size(rg, oracle):
   assert float(y[:, 512].abs().max()) <= float(y_r[:, 512].abs().max()) * (1 + 1e-5) + 1e-6
 
 
+@pytest.mark.parametrize("tokens", [1793, 2301, 2309, 4097])
+def test_rglru_layer_float32_last_wave(rg, oracle, tokens):
+  """Tiles of the float32 gate kernel that a last wave holds: 4 and 64 of 300 and 360 (launched as half
+  tiles behind the others on 148 SMs), 84 of 380 (with the others), 68 of 660.  Heads at either end, the
+  last of which have their last tokens in the second launch, with an initial state."""
+  e, h = 2560, 10
+  g = torch.Generator(device="cpu").manual_seed(tokens)
+  p = synthetic.rglru_params(e, h, g, torch.float32)
+  x = torch.randn((1, tokens, e), generator=g)
+  h0 = torch.randn((1, e), generator=g) * 0.5
+  pos = synthetic.geometric_segment_pos(1, tokens, 300.0, 5)
+  pos[:, 0] = 1
+  y, h_last = _lru(rg, p, e, h, torch.float32)(x.to(DEV), pos.to(DEV), h0.to(DEV))
+  rg.check_status()
+  for head in (0, 7, 8, 9):
+    sl = slice(head * 256, (head + 1) * 256)
+    y_r, h_r = oracle.rglru(x[:, :, sl].contiguous(), pos, *_head_params(p, head), h0[:, sl].contiguous())
+    assert_close(y[:, :, sl], y_r, TOL[torch.float32], f"y of head {head}")
+    assert_close(h_last[:, sl], h_r, TOL[torch.float32], f"state of head {head}")
+
+
 @pytest.mark.parametrize("impl_name", ["GATES_FUSED", "GATES_FUSED_EXACT"])
 def test_long_scan_shard_vs_oracle(rg, oracle, impl_name):
   """What one of eight GPUs runs in the long head-sharded scan: bfloat16 RG-LRU, batch 4, 65536
