@@ -772,6 +772,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         if (tq == 0) {
           if (tt > 0) {
             unsigned spins = 0;
+            ok = __all_sync(0xffffffffu, ok);      // (uniform in the loop below whatever a wait gave)
             while (ok && !__all_sync(0xffffffffu, (pre & ~0xffffffffull) == token)) {
               if (++spins > kLookbackSpins) {
                 if (lane == 0) atomicExch(&hdr->status, kStatusTimeout);

@@ -30,6 +30,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kChan = 64;        // channels per tile
 constexpr unsigned kSpinLimit = 1u << 21;
+constexpr unsigned kTileWait = 1u << 18;         // attempts that the hardware suspends for up to 4 us each
 
 template <typename T> struct ScanCfg {
   static constexpr int kPack = Traits<T>::kPack;
@@ -175,7 +176,7 @@ scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
   // Bounded wait for the tiles.
   {
     bool ok = false;
-    for (unsigned i = 0; i < kSpinLimit; ++i) {
+    for (unsigned i = 0; i < kTileWait; ++i) {
       if (mbar_try_wait(bar, 0)) { ok = true; break; }
     }
     if (!ok) {

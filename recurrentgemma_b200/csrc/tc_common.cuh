@@ -8,30 +8,23 @@
 
 namespace rgk {
 
-// A wait is bounded by kWaitNs: long behind anything a kernel here waits for, short enough to end by itself.
-constexpr unsigned long long kWaitNs = 2000000000ull;
-constexpr unsigned kWaitLimit = 1u << 26;                  // and by this many attempts, whatever the timer says
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Bounded wait.  Returns false (and raises the CTA's abort flag) when the limit is hit or another
-// role has already aborted.  The first attempt, which suspends the thread for as long as the hardware sees
-// fit, stands by itself, ahead of the loop (with a suspension time asked for, each attempt became a loop of
-// its own that slept and polled: 4 to 10 of 47 instructions an element of the RG-LRU kernel).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
+// Bounded waits: return false (and raise the CTA's abort flag) when the limit is hit or another role has
+// already aborted.  An attempt suspends the thread until the phase completes, or for 7800 cycles: the number
+// of attempts bounds the wait at about a second.  (With a suspension time asked for, each attempt became a loop of its own that
+// slept and polled: 4 to 10 of 47 instructions an element of the RG-LRU kernel.)
+constexpr unsigned kWaitLimit = 1u << 18;
+__device__ __forceinline__ bool mbar_wait_brief(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
 #pragma unroll 1
-  for (unsigned i = 1; i < kWaitLimit; ++i) {
+  for (unsigned i = 0; i < kWaitLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
-    if ((i & 255u) == 0 && global_ns() - t0 > kWaitNs) break;
   }
   *abort_flag = 1;
   return false;
+}
+// The same with an attempt of its own ahead of the loop, for waits that mostly find the phase complete.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return mbar_try_wait(bar, parity) || mbar_wait_brief(bar, parity, abort_flag);
 }
 
 // One lane of a converged warp.  Code that the whole warp runs with only the tcgen05 / TMA
@@ -258,13 +251,10 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
 #pragma unroll 1
-  for (unsigned i = 1; i < kWaitLimit; ++i) {
+  for (unsigned i = 0; i < kWaitLimit; ++i) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     if (*abort_flag) return false;
-    if ((i & 255u) == 0 && global_ns() - t0 > kWaitNs) break;
   }
   *abort_flag = 1;
   return false;
