@@ -12,7 +12,7 @@
 // are numbered time-major and dealt out round-robin to persistent CTAs, one per SM, so the unit that
 // produces a carry has normally finished one round before the unit that consumes it starts.
 //
-// Roles in a CTA (18 warps):
+// Roles in a CTA (20 warps, two of them idle where the kernel does not convolve):
 //   producer  one thread: per K-slice of 64 the conv-output tile (128 tokens x 64, operand B) and the
 //             packed gate weights (256 gate rows x 64, operand A) by TMA into a 3-stage ring;
 //   MMA       one thread: per K-step two tcgen05.mma M128 N128 (x-gate rows, a-gate rows) into one
@@ -41,7 +41,8 @@
 // chains are many -> 134 with the MMA loop on a whole warp -> 129 with 112 instead of 96 registers for the
 // epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with table addresses in one
 // instruction and waits that are asked once ahead of their loop.  The recurrent path 243 -> 209 us,
-// 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a tile).
+// 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a tile).  Weights at
+// rest in tensor memory instead of streamed took as long a unit: loads are not the bound.
 // All waits (mbarriers, look-back flags) are bounded; on expiry WsHeader::status is raised, the
 // affected values are taken as zero and the kernel runs to completion.
 #include <cuda.h>
