@@ -529,10 +529,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   }
   } else {
     // ------------------------------ epilogue ------------------------------------------------------
-    if constexpr (!kConv) {
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsEpilogue) : "memory");
-      named_bar_sync(6, kEpi * 32);
-    }
+    if constexpr (!kConv) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsEpilogue) : "memory");
     const int chq = warp & 3;                // channel quarter = TMEM lane quarter of this warp
     const int tq = warp >> 2;                // token quarter: tokens 32 tq .. 32 tq + 31 of the unit
     const int set_id = 1 + chq;              // named barrier of the four token quarters
@@ -572,12 +569,12 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
       mbar_expect_tx(bar_ct(warp), kSubBytes);
       tma_load_3d(tile_c_s, &map_ct, chan0(cur), cur.tt * kUT + tq * kSub, cur.b, bar_ct(warp));
     }
-    // whether this lane's token of the next unit starts a document, and the constants of this
-    // lane's channel in the next unit (gate biases, -8 softplus(a_param)): asked for a unit ahead
-    // (an integer that the compiler may not turn back into a predicate: as a bool it arrived in the loop as
-    // false, on the first unit only, once the register counts were changed above)
-    int reset_next = n_my > 0 ? (int)lane_reset(cur) : 0;
-    asm volatile("" : "+r"(reset_next));
+    // which tokens of the warp start a document in the coming unit, and the constants of this lane's channel
+    // there (gate biases, -8 softplus(a_param)): asked for a unit ahead.  The document starts enter the loop as
+    // the warp's vote, a word: nothing of a lane's own that is computed here is carried in a predicate.  As a
+    // bool of each lane they arrived in the loop as false on every CTA's first unit, in each variant whose
+    // register counts are changed above and in none of the others.
+    uint32_t resets = __ballot_sync(0xffffffffu, n_my > 0 && lane_reset(cur));
     uint32_t bxv = 0u, bav = 0u, spv = 0u;
     auto load_consts = [&](const UnitPos& u) {
       const int e = chan0(u) + lane;
@@ -600,7 +597,6 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
       nxt = cur;
       step.advance(nxt);
 
-      const uint32_t resets = __ballot_sync(0xffffffffu, reset_next != 0);
       // tokens of this warp past the end of the sequence (only in a sequence's last time tile)
       const int n_live = T_ - tok0;
       const uint32_t invalid = n_live >= 32 ? 0u : (n_live <= 0 ? 0xffffffffu : (0xffffffffu << n_live));
@@ -685,7 +681,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         }
       }
       if (t + 1 < n_my) load_consts(nxt);
-      if (t + 1 < n_my) reset_next = (int)lane_reset(nxt);
+      const bool reset_next = t + 1 < n_my && lane_reset(nxt);
 
       float h;                               // the state entering the thread's tokens
       if constexpr (kMaps) {
@@ -847,6 +843,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         bulk_commit();
       }
       cur = nxt;
+      resets = __ballot_sync(0xffffffffu, reset_next);
     }
     if (lane == 0) bulk_wait_all();
   }

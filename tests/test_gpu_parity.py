@@ -515,6 +515,38 @@ def test_fused_rglru_kernel(rg, oracle, shape):
     m2(torch.zeros(1, 128, 256, device=DEV, dtype=dt), torch.arange(128, device=DEV)[None])
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 1500), (40, 2, 300)], ids=["maps", "states"])
+@pytest.mark.parametrize("impl", ["GATES_FUSED", "GATES_FUSED_EXACT"])
+def test_fused_rglru_kernel_document_starts_in_first_units(rg, shape, impl):
+  """Documents that start in every token quarter of every CTA's first unit (96 units in all, and 480 of which
+  the first round takes 148), in all three joins (none, gelu, y branch activated by its projection), against
+  the route of two kernels, which reads the positions token by token."""
+  from recurrentgemma_b200 import _lib
+  b, h, t = shape
+  e, dt = h * 256, torch.bfloat16
+  case = C.Case(f"first_{b}_{t}_{e}", "block", "bfloat16", b, t, e, h, width=e, pos="multi")
+  p = C.make_params(case)
+  m = rg.RecurrentBlock(e, h, e, device=DEV, dtype=dt)
+  m.load_state_dict(p)
+  g = torch.Generator(device="cpu").manual_seed(b)
+  x, y = (torch.randn((b, t, e), generator=g).to(dt).to(DEV) for _ in range(2))
+  pos = torch.where(torch.rand((b, t), generator=g) < 0.1, 0, 5)
+  assert all((pos[:, i:i + 32] == 0).any() for i in range(0, 128, 32))
+  pos = pos.to(DEV)
+  h0 = torch.randn((b, e), generator=g).to(DEV)
+  calls = {"none": lambda: m.rg_lru(x, pos, h0), "gelu": lambda: rg.recurrent_path(x, y, pos, m.conv_1d, m.rg_lru),
+           "activated": lambda: m(x, pos)}
+  for name, call in calls.items():
+    m.rg_lru.gates_impl = _lib.GATES_TCGEN05
+    y_u, c_u = call()
+    m.rg_lru.gates_impl = getattr(_lib, impl)
+    y_f, c_f = call()
+    rg.check_status()
+    assert_close(y_f, y_u, TOL[dt], name)
+    assert_close(c_f if name == "none" else c_f.rg_lru_state, c_u if name == "none" else c_u.rg_lru_state, TOL[dt],
+                 f"state, {name}")
+
+
 @pytest.mark.parametrize("shape", [(18, 1, 1030), (19, 1, 1030), (74, 1, 257), (75, 1, 129), (74, 1, 129),
                                    (5, 4, 640), (2, 16, 513)],
                          ids=lambda s: "x".join(map(str, s)))
