@@ -65,10 +65,13 @@ constexpr int kWBytes = 2 * kUC * kKB * 2;     // 32 KiB: x-gate rows then a-gat
 constexpr int kStage = kCBytes + kWBytes;
 constexpr int kEpi = 16;
 // The producer, MMA and two idle warps are a warpgroup of their own, which hands registers to the
-// epilogue warps: launched with 96 a thread, 112 x 4 + 32 = 5 x 96.
+// epilogue warps: compiled to 96 a thread, 112 x 4 + 32 = 5 x 96.  setmaxnreg.inc waits, without a limit, until
+// the CTA has that many to give: no variant is launched that was compiled to fewer (chan_set_attributes).
 constexpr int kThreads = (kEpi + 4) * 32;
 constexpr int kRegsEpilogue = 112, kRegsOther = 32;
-static_assert(4 * kRegsEpilogue + kRegsOther <= 5 * 96, "more registers than the CTA is launched with");
+constexpr bool registers_suffice(int per_thread) { return 5 * per_thread >= 4 * kRegsEpilogue + kRegsOther; }
+static_assert(kThreads == 5 * 128, "five warpgroups, four of them epilogue");
+static_assert(registers_suffice(96) && !registers_suffice(95), "the hand-over takes all of 96 a thread");
 // With the Conv1D fused (kConv): two more warps turn the block input into the conv-output operand.
 // The ring then has two stages; the room of the third holds two staging buffers for the input rows
 // of a K-slice (the unit's 128 tokens and the three before them, 64 channels).
@@ -887,28 +890,37 @@ ChanLayout chan_layout(int64_t B, int64_t T, int64_t E) {
 
 // The kernel needs more dynamic shared memory than the default limit: the attribute is a property
 // of the function on ONE device, so it is set (and the SM count read) once per device.
+template <int kJoin, int kMath, bool kConv, bool kMaps>
+cudaError_t chan_set_attributes() {
+  const auto kernel = rglru_chan_kernel<kJoin, kMath, kConv, kMaps>;
+  if (!kConv) {                                      // the variants that change their register counts
+    cudaFuncAttributes a;
+    if (const cudaError_t e = cudaFuncGetAttributes(&a, kernel); e != cudaSuccess) return e;
+    if (!registers_suffice(a.numRegs)) return cudaErrorLaunchOutOfResources;
+  }
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+}
 template <int kMath, bool kConv, bool kMaps>
-cudaError_t chan_set_smem() {
+cudaError_t chan_set_joins() {
   cudaError_t e;
-  constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<0, kMath, kConv, kMaps>, attr, kSmem)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(rglru_chan_kernel<1, kMath, kConv, kMaps>, attr, kSmem)) != cudaSuccess) return e;
-  return cudaFuncSetAttribute(rglru_chan_kernel<2, kMath, kConv, kMaps>, attr, kSmem);
+  if ((e = chan_set_attributes<0, kMath, kConv, kMaps>()) != cudaSuccess) return e;
+  if ((e = chan_set_attributes<1, kMath, kConv, kMaps>()) != cudaSuccess) return e;
+  return chan_set_attributes<2, kMath, kConv, kMaps>();
 }
 template <bool kMaps>
-cudaError_t chan_set_smem_all() {
+cudaError_t chan_set_all() {
   cudaError_t e;
-  if ((e = chan_set_smem<kMathExact, false, kMaps>()) != cudaSuccess) return e;
-  if ((e = chan_set_smem<kMathFast, false, kMaps>()) != cudaSuccess) return e;
-  if ((e = chan_set_smem<kMathExact, true, kMaps>()) != cudaSuccess) return e;
-  return chan_set_smem<kMathFast, true, kMaps>();
+  if ((e = chan_set_joins<kMathExact, false, kMaps>()) != cudaSuccess) return e;
+  if ((e = chan_set_joins<kMathFast, false, kMaps>()) != cudaSuccess) return e;
+  if ((e = chan_set_joins<kMathExact, true, kMaps>()) != cudaSuccess) return e;
+  return chan_set_joins<kMathFast, true, kMaps>();
 }
 
 cudaError_t chan_device_setup(int* num_sms) {
   static PerDeviceOnce once;
   return once.run([] {
-    const cudaError_t e = chan_set_smem_all<false>();
-    return e != cudaSuccess ? e : chan_set_smem_all<true>();
+    const cudaError_t e = chan_set_all<false>();
+    return e != cudaSuccess ? e : chan_set_all<true>();
   }, num_sms);
 }
 

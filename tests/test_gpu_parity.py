@@ -548,14 +548,15 @@ def test_fused_rglru_kernel_document_starts_in_first_units(rg, shape, impl):
 
 
 @pytest.mark.parametrize("shape", [(18, 1, 1030), (19, 1, 1030), (74, 1, 257), (75, 1, 129), (74, 1, 129),
-                                   (5, 4, 640), (2, 16, 513)],
+                                   (5, 4, 640), (2, 16, 513), (2, 10, 300), (37, 1, 129), (38, 1, 129)],
                          ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("join", [False, True], ids=["plain", "join"])
 def test_fused_rglru_kernel_states_from_tile_to_tile(rg, oracle, shape, join):
   """The two ways a tile's incoming state reaches it, on either side of where one takes over from the other
-  (36 / 38 chains, 148 / 150 units on 148 SMs), ragged last tiles, one to nine tiles a chain, an initial
-  state: against the oracle, and twice in a row on the same workspace (the records of the first call must
-  not be taken for the second's)."""
+  (36 / 38 chains; 40 chains of 120 units and 74 of 148, all in flight at once, / 76 of 152, on 148 SMs), ragged
+  last tiles, two to nine tiles a chain, an initial state: against the oracle.  The workspace has seen a call
+  of the same size and then one of two tiles, whose records are left where the compared call has its own, with
+  the marks that its tile 1 (records of a call with maps) or tile 2 (without) waits for."""
   from recurrentgemma_b200 import _lib
   b, h, t = shape
   e = h * 256
@@ -579,23 +580,27 @@ def test_fused_rglru_kernel_states_from_tile_to_tile(rg, oracle, shape, join):
     h0 = None
   else:
     h0 = torch.randn((b, e), generator=g) * 0.5
-  for scale in (1.0, 0.5):
-    xs = x * scale
+  def call(xs, n):
     if join:
-      out, cache = rg.recurrent_path(xs.to(DEV), y.to(DEV), pos.to(DEV), conv, lru)
+      out, cache = rg.recurrent_path(xs[:, :n].to(DEV), y[:, :n].to(DEV), pos[:, :n].to(DEV), conv, lru)
       h_last = cache.rg_lru_state
     else:
-      out, h_last = lru(xs.to(DEV), pos.to(DEV), h0.to(DEV))
+      out, h_last = lru(xs[:, :n].to(DEV), pos[:, :n].to(DEV), h0.to(DEV))
     rg.check_status()
-    for row in rows:
-      o_r, h_r = oracle.rglru(xs[row:row + 1].contiguous(), pos[row:row + 1], pr["a_param"], pr["input_gate.w"],
-                              pr["input_gate.b"], pr["a_gate.w"], pr["a_gate.b"],
-                              None if h0 is None else h0[row:row + 1].contiguous())
-      if join:
-        o_r = o_r.to(dt) * torch.nn.functional.gelu(y[row:row + 1], approximate="tanh")
-      assert_close(out[row:row + 1], o_r, TOL[dt], f"row {row}")
-      assert_close(h_last[row:row + 1], h_r, TOL[dt], f"state of row {row}")
-
+    return out, h_last
+  call(x * 0.5, t)
+  ws = _lib.workspace(torch.device(DEV), 1).data_ptr()
+  call(x * 0.25, min(t, 200))
+  out, h_last = call(x, t)
+  assert _lib.workspace(torch.device(DEV), 1).data_ptr() == ws
+  for row in rows:
+    o_r, h_r = oracle.rglru(x[row:row + 1].contiguous(), pos[row:row + 1], pr["a_param"], pr["input_gate.w"],
+                            pr["input_gate.b"], pr["a_gate.w"], pr["a_gate.b"],
+                            None if h0 is None else h0[row:row + 1].contiguous())
+    if join:
+      o_r = o_r.to(dt) * torch.nn.functional.gelu(y[row:row + 1], approximate="tanh")
+    assert_close(out[row:row + 1], o_r, TOL[dt], f"row {row}")
+    assert_close(h_last[row:row + 1], h_r, TOL[dt], f"state of row {row}")
 
 
 def test_host_pipeline_matches_device_call(rg):
