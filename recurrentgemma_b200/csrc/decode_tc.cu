@@ -17,6 +17,11 @@
 // row's 16 channels from global memory touches 32 rows per instruction, which took 4.6 us.
 // Per layer of 2560 channels at 256 rows: 11.2 -> 9.45 us in a chain of 26.
 //
+// A call of one row tile that is not full (kPart) asks only for rows that exist; where tiles are full, or
+// several, rows past the end repeat the last one and no load is conditional.  26 layers, us with conditional /
+// unconditional loads: width 2560, 100 and 112 rows 220 / 227 and 217 / 227, width 4096 225 / 230 and 222 / 228;
+// 256 rows 249 / 246 and 300 / 287.
+//
 // Every mbarrier wait is bounded; on expiry WsHeader::status is raised and the CTA leaves.
 #include <cuda.h>
 
@@ -57,7 +62,7 @@ __device__ __forceinline__ uint4 add4(const uint4& a, const uint4& b) {
 
 // kMath: how the gates and the gelu are evaluated (see rgk_internal.h); the fast variant takes
 // a = exp(log_a) and the input multiplier from a shared-memory table, built in the prologue.
-template <bool kMul, int kMath>
+template <bool kMul, int kMath, bool kPart>
 __global__ void __launch_bounds__(kThreadsDec, 1)
 decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* xb,
                  const __nv_bfloat16* yb, const void* pos, int pos64,
@@ -173,28 +178,33 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     // all loads before the first use: the windows of two rows per thread, then state and other branch
     constexpr int kPer = kRowsM * 8 / kThreadsDec;     // rows per thread: 2
     constexpr int kRowStep = kThreadsDec / 8;
+    auto row = [&](int r) { return kPart ? row0 + r : min(row0 + r, (int64_t)M - 1); };   // never read out of range
+    auto load = [&](const auto* p, int64_t m) {
+      if (kPart && m >= M) return make_uint4(0u, 0u, 0u, 0u);
+      return *reinterpret_cast<const uint4*>(p);
+    };
     uint4 xv[kPer][4];
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int64_t m = min(row0 + (tid >> 3) + kRowStep * i, (int64_t)M - 1);   // clamped: never out of range
+      const int64_t m = row((tid >> 3) + kRowStep * i);
       const __nv_bfloat16* cr = cache_in + m * 3 * E + e;
-      xv[i][0] = *reinterpret_cast<const uint4*>(cr);
-      xv[i][1] = *reinterpret_cast<const uint4*>(cr + E);
-      xv[i][2] = *reinterpret_cast<const uint4*>(cr + 2 * (int64_t)E);
-      xv[i][3] = *reinterpret_cast<const uint4*>(xb + m * E + e);
+      xv[i][0] = load(cr, m);
+      xv[i][1] = load(cr + E, m);
+      xv[i][2] = load(cr + 2 * (int64_t)E, m);
+      xv[i][3] = load(xb + m * E + e, m);
     }
     constexpr int kHPer = kRowsM * 16 / kThreadsDec, kYPer = kRowsM * 8 / kThreadsDec;   // packs per thread
     uint4 hp[kHPer], yp[kYPer];
 #pragma unroll
     for (int i = 0; i < kHPer; ++i) {
-      const int64_t m = min(row0 + (tid >> 4) + (kThreadsDec / 16) * i, (int64_t)M - 1);
-      hp[i] = *reinterpret_cast<const uint4*>(h_in + m * E + chan0 + (tid & 15) * 4);
+      const int64_t m = row((tid >> 4) + (kThreadsDec / 16) * i);
+      hp[i] = load(h_in + m * E + chan0 + (tid & 15) * 4, m);
     }
     if constexpr (kMul) {
 #pragma unroll
       for (int i = 0; i < kYPer; ++i) {
-        const int64_t m = min(row0 + (tid >> 3) + kRowStep * i, (int64_t)M - 1);
-        yp[i] = *reinterpret_cast<const uint4*>(yb + m * E + e);
+        const int64_t m = row((tid >> 3) + kRowStep * i);
+        yp[i] = load(yb + m * E + e, m);
       }
     }
 #pragma unroll
@@ -247,7 +257,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   // (The whole warp waits, one elected lane issues: see mma_ring.  A CTA runs through this code once, so it is
   // the short form of the wait: 250.8 -> 245.7 us at 256 rows for 26 layers, with the other 253.4.)
   if (warp == 0) {
-    const bool there = mbar_wait_brief(bar_b, 0, s_abort) && mbar_wait(bar_a, 0, s_abort);
+    const bool there = mbar_wait_brief(bar_b, 0, s_abort) &&
+                       (kPart ? mbar_wait_brief(bar_a, 0, s_abort) : mbar_wait(bar_a, 0, s_abort));
     if (__all_sync(0xffffffffu, there)) {
       tc_fence_after();
       const uint64_t desc_a = smem_desc_sw128(s_base + kOffA), desc_b = smem_desc_sw128(s_base + kOffB);
@@ -399,7 +410,9 @@ cudaError_t launch_path_decode_tc(const void* xb, const void* yb, const void* po
   cudaError_t e0 = once.run([] {
     cudaError_t e;
 #define RGK_DEC_ATTR(MUL, MATH)                                                                 \
-    if ((e = cudaFuncSetAttribute(decode_tc_kernel<MUL, MATH>,                                  \
+    if ((e = cudaFuncSetAttribute(decode_tc_kernel<MUL, MATH, false>,                           \
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)) != cudaSuccess) return e; \
+    if ((e = cudaFuncSetAttribute(decode_tc_kernel<MUL, MATH, true>,                            \
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)) != cudaSuccess) return e
     RGK_DEC_ATTR(true, kMathExact);
     RGK_DEC_ATTR(true, kMathFast);
@@ -427,11 +440,13 @@ cudaError_t launch_path_decode_tc(const void* xb, const void* yb, const void* po
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
+  const bool part = B < kRowsM;
 #define RGK_DEC(MUL, MATH)                                                                         \
-  cudaLaunchKernelEx(&cfg, decode_tc_kernel<MUL, MATH>, map_w, (const T_*)xb, (const T_*)yb, pos,  \
-                     pos64, (const T_*)conv_w, (const T_*)conv_b, (const T_*)a_param, (const T_*)bx, \
-                     (const T_*)ba, h_in, (const T_*)cache_in, packed_w, (int)B, E, (T_*)out,      \
-                     h_out, (T_*)cache_out, reinterpret_cast<WsHeader*>(ws_header))
+  cudaLaunchKernelEx(&cfg, part ? decode_tc_kernel<MUL, MATH, true> : decode_tc_kernel<MUL, MATH, false>, \
+                     map_w, (const T_*)xb, (const T_*)yb, pos, pos64, (const T_*)conv_w,           \
+                     (const T_*)conv_b, (const T_*)a_param, (const T_*)bx, (const T_*)ba, h_in,    \
+                     (const T_*)cache_in, packed_w, (int)B, E, (T_*)out, h_out, (T_*)cache_out,    \
+                     reinterpret_cast<WsHeader*>(ws_header))
   cudaError_t lerr;
   if (math == kMathExact) lerr = yb ? RGK_DEC(true, kMathExact) : RGK_DEC(false, kMathExact);
   else lerr = yb ? RGK_DEC(true, kMathFast) : RGK_DEC(false, kMathFast);

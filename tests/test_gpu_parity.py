@@ -354,7 +354,8 @@ def test_gates_tcgen05_matches_simt_and_oracle(rg, oracle, shape):
     assert_close(h_tc, h_ref, TOL[torch.bfloat16], "tcgen05 vs oracle h")
 
 
-@pytest.mark.parametrize("shape", [(256, 2560, 10), (5, 256, 1), (130, 512, 2)],
+@pytest.mark.parametrize("shape", [(256, 2560, 10), (5, 256, 1), (130, 512, 2), (97, 512, 2), (113, 256, 1),
+                                   (127, 512, 2), (128, 512, 2)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_fused_decode_step_matches_unfused_and_oracle(rg, oracle, shape):
   """The single-kernel decode step (conv step + tcgen05 gates + state update + join) against the
