@@ -8,7 +8,8 @@ namespace rgk {
 namespace {
 
 constexpr int kConvRows = 24;     // output rows per thread (16: 64 us at B8 T4096 E2560, 24: 60, 28: 65)
-constexpr int kConvThreads = 128; // packs (of 16 bytes) per block
+constexpr int kConvThreads = 128; // packs (of 16 bytes) per block, cache and decode form
+constexpr int kMaxChunks = 65535; // time chunks of one launch (grid.y)
 
 // One tap: acc <- round(acc + round(x * w)); the first tap initialises acc (the reference starts
 // from the Python float 0.0, torch/layers.py:483, 517).
@@ -65,10 +66,18 @@ template <> struct PackOps<__nv_bfloat16> {
   }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kConvThreads)
+// A block is 64 or 32 packs of one time chunk of one sequence: 64 where that divides the row, else 32, so that
+// few threads have nothing to do.  Rows of 320 packs (8 x 4096 tokens of 2560 bfloat16 channels) take 55.5 us,
+// 59 in blocks of 128 packs that run on from sequence to sequence (the sequence, and with it every address, is
+// then a thread's own), 60.6 in blocks of 128 of one sequence; rows of 640 (4 x 4000 tokens in float32) 51.7,
+// 62.7 and 53.4; 352 packs 59.8, 64 and 62 (blocks of 64: 62.4); 48 packs 50, 45.7 and 77.6.
+// kFar: chunks from chunk0 on, for sequences of more chunks than grid.y has room for.  A variant of its own,
+// because the loads of a thread are issued together only as long as the chunk is plainly blockIdx.y: with the
+// offset for every call the rows of 320 packs take 74 us.
+template <typename T, bool kFar>
+__global__ void __launch_bounds__(64)
 conv1d_prefill_kernel(const T* x, const void* pos, int pos64,
-                      const T* __restrict__ w, const T* __restrict__ bias, int B, int T_, int E,
+                      const T* __restrict__ w, const T* __restrict__ bias, int chunk0, int T_, int E,
                       T* __restrict__ out, T* __restrict__ cache_out, const ChanPrep prep) {
   constexpr int kPack = Traits<T>::kPack;
   using Ops = PackOps<T>;
@@ -77,17 +86,15 @@ conv1d_prefill_kernel(const T* x, const void* pos, int pos64,
   // of short documents 4% slower, nothing faster)
   grid_dependency_wait();
   if (prep.E > 0) {                              // for the RG-LRU kernel behind
-    const int64_t block = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
-    chan_prepare(prep, block * kConvThreads + threadIdx.x, (int64_t)gridDim.x * gridDim.y * kConvThreads);
+    const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    chan_prepare(prep, block * blockDim.x + threadIdx.x,
+                 (int64_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x);
   }
-  // a block is kConvThreads packs of one time chunk, sequence after sequence without a gap (with blocks of
-  // one sequence each, 320 packs a row left the third of three half empty: the path of 8 x 4096 tokens
-  // 209 -> 204 us; the last time chunks first, for the kernel behind to start with what was written last: 206)
-  const unsigned item = blockIdx.x * kConvThreads + threadIdx.x, packs = (unsigned)E / kPack;
-  const int b = (int)(item / packs);
-  if (b >= B) return;
-  const int e0 = (int)(item - (unsigned)b * packs) * kPack;
-  const int t_begin = blockIdx.y * kConvRows;
+  const int pack_idx = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e0 = pack_idx * kPack;
+  if (e0 >= E) return;
+  const int b = blockIdx.z;
+  const int t_begin = kFar ? (chunk0 + (int)blockIdx.y) * kConvRows : blockIdx.y * kConvRows;
   const int64_t row0 = (int64_t)b * T_;
 
   // All rows this thread touches (3 halo rows + kConvRows), loaded back to back; rows outside the
@@ -234,18 +241,22 @@ cudaError_t launch_conv1d_prefill(const void* x, const void* pos, int pos64, con
                                   const void* b, int64_t B, int64_t T, int64_t E, int dtype,
                                   void* out, void* cache_out, cudaStream_t s, const ChanPrep& prep) {
   if (B == 0 || T == 0 || E == 0) return cudaSuccess;
-  const int pack = dtype ? 8 : 4;
-  const int64_t items = E / pack * B;
-  if (items > 0x7fffffff - kConvThreads) return cudaErrorInvalidValue;
-  dim3 grid((unsigned)((items + kConvThreads - 1) / kConvThreads), (unsigned)((T + kConvRows - 1) / kConvRows));
-  if (dtype) {
-    using T_ = __nv_bfloat16;
-    return launch_dependent(conv1d_prefill_kernel<T_>, grid, dim3(kConvThreads), 0, s, (const T_*)x, pos, pos64,
-                            (const T_*)w, (const T_*)b, (int)B, (int)T, (int)E, (T_*)out, (T_*)cache_out, prep);
+  const unsigned packs = (unsigned)(E / (dtype ? 8 : 4)), threads = packs % 64 == 0 ? 64 : 32;
+  const int chunks = (int)((T + kConvRows - 1) / kConvRows);
+  cudaError_t e = cudaSuccess;
+  for (int c0 = 0; c0 < chunks && e == cudaSuccess; c0 += kMaxChunks) {
+    const dim3 grid((packs + threads - 1) / threads, (unsigned)min(chunks - c0, kMaxChunks), (unsigned)B);
+    auto run = [&](auto* kernel, auto* t) {
+      using P = decltype(t);
+      return launch_dependent(kernel, grid, dim3(threads), 0, s, (const P)x, pos, pos64, (const P)w, (const P)b, c0,
+                              (int)T, (int)E, (P)out, (P)cache_out, c0 == 0 ? prep : ChanPrep());
+    };
+    const bool far = chunks > kMaxChunks;
+    if (dtype) e = run(far ? conv1d_prefill_kernel<__nv_bfloat16, true> : conv1d_prefill_kernel<__nv_bfloat16, false>,
+                       (__nv_bfloat16*)nullptr);
+    else e = run(far ? conv1d_prefill_kernel<float, true> : conv1d_prefill_kernel<float, false>, (float*)nullptr);
   }
-  return launch_dependent(conv1d_prefill_kernel<float>, grid, dim3(kConvThreads), 0, s, (const float*)x, pos,
-                          pos64, (const float*)w, (const float*)b, (int)B, (int)T, (int)E, (float*)out,
-                          (float*)cache_out, prep);
+  return e;
 }
 
 cudaError_t launch_conv1d_cache(const void* x, const void* pos, int pos64, int64_t B, int64_t T,

@@ -516,6 +516,33 @@ def test_fused_rglru_kernel(rg, oracle, shape):
     m2(torch.zeros(1, 128, 256, device=DEV, dtype=dt), torch.arange(128, device=DEV)[None])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(3, 25, 8), (2, 49, 264), (5, 72, 512), (2, 100, 1280), (1, 24 * 65535 + 50, 16)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_conv1d_blocks(rg, dtype, shape):
+  """Blocks of 64 and 32 packs, rows that leave the last one partly idle, and a sequence of more time chunks
+  than one launch covers: every product and sum is rounded to the tensor's type where torch's are, so the
+  results are the same bits."""
+  b, t, e = shape
+  g = torch.Generator().manual_seed(t)
+  conv = rg.Conv1D(e, 4, device=DEV, dtype=dtype)
+  conv.w.data.copy_(torch.randn((4, e), generator=g))
+  conv.b.data.copy_(torch.randn((e,), generator=g))
+  x = torch.randn((b, t, e), generator=g).to(dtype).to(DEV)
+  pos = torch.where(torch.rand((b, t), generator=g) < 0.05, 0, 7).to(DEV)
+  out, cache = conv(x, pos)
+  ref = x * conv.w[3]
+  kept = torch.ones((b, t, 1), dtype=dtype, device=DEV)
+  window = [x]
+  for s in (1, 2, 3):                # the tap s tokens back, if no document has started since
+    kept = kept * torch.nn.functional.pad(pos != 0, (s - 1, 0))[:, :t, None]
+    back = torch.nn.functional.pad(x, (0, 0, s, 0))[:, :t] * kept
+    ref = ref + back * conv.w[3 - s]
+    window.append(back)
+  assert torch.equal(out, ref + conv.b)
+  assert torch.equal(cache, torch.stack([window[s][:, -1] for s in (2, 1, 0)], dim=1))
+
+
 @pytest.mark.parametrize("shape", [(2, 2, 1500), (40, 2, 300)], ids=["maps", "states"])
 @pytest.mark.parametrize("impl", ["GATES_FUSED", "GATES_FUSED_EXACT"])
 def test_fused_rglru_kernel_document_starts_in_first_units(rg, shape, impl):
