@@ -19,8 +19,8 @@
 //
 // A call of one row tile that is not full (kPart) asks only for rows that exist; where tiles are full, or
 // several, rows past the end repeat the last one and no load is conditional.  26 layers, us with conditional /
-// unconditional loads: width 2560, 100 and 112 rows 220 / 227 and 217 / 227, width 4096 225 / 230 and 222 / 228;
-// 256 rows 249 / 246 and 300 / 287.
+// unconditional loads: width 2560, 97, 100 and 112 rows 223 / 227, 217 / 227 and 218 / 228, width 4096 225 / 230,
+// 219 / 230 and 221 / 228; 256 rows 249 / 246 and 300 / 287.
 //
 // Every mbarrier wait is bounded; on expiry WsHeader::status is raised and the CTA leaves.
 #include <cuda.h>

@@ -16,8 +16,8 @@
 // arrives in sixteen slices of 16 (64-byte rows, 64-byte swizzle) through a ring: activations 8 KiB, their
 // low part 8 KiB (written by the helper warps), weights hi and lo 16 KiB each (kTN = 256) - the
 // per-slice hand-offs (copy engine -> split -> tensor core -> release) of a CTA are serial, so more and
-// smaller stages in flight hide them.  A single thread issues three tcgen05.mma.cta_group::1.kind::tf32
-// (M 128, N kTN, K 8) per K step.  The epilogue (TMEM lane quarter x 32-channel chunks per warp) reads the
+// smaller stages in flight hide them.  One warp runs the MMA loop, an elected lane issues three
+// tcgen05.mma.cta_group::1.kind::tf32 (M 128, N kTN, K 8) per K step.  The epilogue (TMEM lane quarter x 32-channel chunks per warp) reads the
 // accumulators, applies the float32-accurate gate arithmetic and writes a and the normalised input for
 // the scan kernel.
 //

@@ -15,8 +15,8 @@
 // Roles in a CTA (20 warps, two of them idle where the kernel does not convolve):
 //   producer  one thread: per K-slice of 64 the conv-output tile (128 tokens x 64, operand B) and the
 //             packed gate weights (256 gate rows x 64, operand A) by TMA into a 3-stage ring;
-//   MMA       one thread: per K-step two tcgen05.mma M128 N128 (x-gate rows, a-gate rows) into one
-//             of two TMEM accumulator sets (2 x 128 columns each);
+//   MMA       one warp, an elected lane of which issues: per K-step two tcgen05.mma M128 N128 (x-gate
+//             rows, a-gate rows) into one of two TMEM accumulator sets (2 x 128 columns each);
 //   epilogue  16 warps = 4 channel quarters (the warp's TMEM lane quarter) x 4 token quarters.
 //             A warp fetches its own 32 x 32 tiles of the conv output and of the other branch by
 //             TMA (64-byte swizzle) into 2 KiB buffers, transposes each in place (ldmatrix.trans +
@@ -684,7 +684,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         }
       }
       if (t + 1 < n_my) load_consts(nxt);
-      const bool reset_next = t + 1 < n_my && lane_reset(nxt);
+      const uint32_t resets_next = __ballot_sync(0xffffffffu, t + 1 < n_my && lane_reset(nxt));
 
       float h;                               // the state entering the thread's tokens
       if constexpr (kMaps) {
@@ -846,7 +846,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         bulk_commit();
       }
       cur = nxt;
-      resets = __ballot_sync(0xffffffffu, reset_next);
+      resets = resets_next;
     }
     if (lane == 0) bulk_wait_all();
   }
@@ -925,13 +925,14 @@ cudaError_t chan_device_setup(int* num_sms) {
 }
 
 // How a tile's incoming state reaches it.  From tile to tile (kMaps false) a chain - one sequence, one half
-// head - moves on by one tile per hand-over, the four token quarters one after the other and a round trip to
-// the next SM, 2.3 us in all where a unit takes 3.3: fast enough as long as the SMs have a quarter as many
-// chains to share, and four instructions a token pair cheaper.  Below that, and where all of a call's units
-// are in flight at once, tiles publish their maps (P, H) and look back over several of them.  Recurrent path
-// of 2560 (20 chains a sequence) and RG-LRU of 4096 (32 chains) channels, us with maps / without: 20 chains
-// 2501 tokens 30.1 / 38.7, 32 chains 29.4 / 37.6, 40 chains 47.5 / 46.0, 64 chains 47.4 / 43.3, 128 chains
-// 82.6 / 66.5; 40 chains of 300 tokens (120 units) 16.5 / 17.5, 60 chains 20.0 / 19.2.
+// head - moves on by one tile per hand-over: the four token quarters one after the other and a round trip to
+// the next SM, 1.2 us a tile (40 chains: 20 tiles 33.9 us, 47 tiles 67.3).  The SMs could take 148 units every
+// 3.3 us, 1.2 us' worth of which are some 55 chains: with fewer the hand-over is what bounds the call.  With
+// maps, which cost four instructions a token pair, tiles look back over several others.  The line is where the
+// two were measured to cross; calls whose units are all in flight at once gain from maps with any number of
+// chains.  Recurrent path of 2560 (20 chains a sequence) and RG-LRU of 4096 (32 chains) channels, us with maps /
+// without: 20 chains 2501 tokens 30.1 / 38.7, 32 chains 29.4 / 37.6, 40 chains 47.5 / 46.0, 64 chains 47.4 /
+// 43.3, 128 chains 82.6 / 66.5; 40 chains of 300 tokens (120 units) 16.5 / 17.5, 60 chains 20.0 / 19.2.
 bool chan_uses_maps(int64_t B, int groups, int64_t n_units, int num_sms) {
   return n_units <= num_sms || B * groups * 4 < num_sms;
 }
