@@ -35,14 +35,14 @@
 //           record) and publishes the tile's own; second named barrier unless the state was known
 // -> recurrence in registers, join, 16-byte stores into the output tile.
 //
-// What bounds it is instruction issue: 42 warp instructions an element (35 without a join) with four
-// epilogue warps a scheduler; stripped of every memory access the arithmetic alone takes 105 of 124 us at
-// 8 x 4096 tokens without a join.  There: 151 us as look-back over maps for every call -> 136 without maps where
-// chains are many -> 134 with the MMA loop on a whole warp -> 129 with 112 instead of 96 registers for the
-// epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with table addresses in one
-// instruction and waits that are asked once ahead of their loop.  The recurrent path 243 -> 209 us,
-// 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a tile).  Weights at
-// rest in tensor memory instead of streamed took as long a unit: loads are not the bound.
+// What bounds it is instruction issue: 38 warp instructions for 32 elements (32 without a join, 48 with maps and
+// a join), 68 % of the issue slots, with four epilogue warps a scheduler.  Stripped of every memory access the
+// arithmetic alone takes 105 of 124 us at 8 x 4096 tokens without a join.  There: 151 us as look-back over maps
+// for every call -> 136 without maps where chains are many -> 134 with the MMA loop on a whole warp -> 129 with
+// 112 instead of 96 registers for the epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with
+// table addresses in one instruction and waits that are asked once ahead of their loop.  The recurrent path
+// 243 -> 209 us, 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a
+// tile).  Weights at rest in tensor memory instead of streamed took as long a unit: loads are not the bound.
 // All waits (mbarriers, look-back flags) are bounded; on expiry WsHeader::status is raised, the
 // affected values are taken as zero and the kernel runs to completion.
 #include <cuda.h>

@@ -30,7 +30,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kChan = 64;        // channels per tile
 constexpr unsigned kSpinLimit = 1u << 21;
-constexpr unsigned kTileWait = 1u << 18;         // attempts, suspended for up to 4 us each as measured (see mbar_wait_brief)
+constexpr unsigned kTileWait = 1u << 18;         // attempts, suspended for up to 4 us each (see mbar_wait_brief)
 
 template <typename T> struct ScanCfg {
   static constexpr int kPack = Traits<T>::kPack;

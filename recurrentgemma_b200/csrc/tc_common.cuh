@@ -12,7 +12,7 @@ namespace rgk {
 // already aborted.  What bounds a wait is its number of attempts.  An attempt suspends the thread until the
 // phase completes, or for a time that PTX leaves to the hardware: 7800 cycles as measured on a B200, which makes
 // about a second of them.  (With a suspension time asked for, each attempt became a loop of its own that slept
-// and polled: 4 to 10 of 47 instructions an element of the RG-LRU kernel.  A look at the clock every 4096
+// and polled: 4 to 10 of then 47 instructions for 32 elements in the RG-LRU kernel.  A look at the clock every 4096
 // attempts: 256 rows of a decode step, 26 layers, 245.5 -> 248.3 us, RG-LRU and float32 gates 0 to 2 % slower.)
 constexpr unsigned kWaitLimit = 1u << 18;
 __device__ __forceinline__ bool mbar_wait_brief(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
