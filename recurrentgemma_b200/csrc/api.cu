@@ -148,14 +148,33 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
   const bool chan_route = rgk::rglru_chan_supported(dtype, bw, B, T) &&
                           (gates_impl == RGK_GATES_AUTO || gates_impl >= RGK_GATES_FUSED);
   const bool fuse_conv = xb != nullptr && chan_route && out != xb && conv_fusion_enabled();
+  // float32 in one kernel: a unit reads the head's other channels of its tokens while they are being written
+  // elsewhere, so not where the output lies over the input
+  const size_t act = static_cast<size_t>(B) * T * E * elem_size(dtype);
+  const uintptr_t c0 = reinterpret_cast<uintptr_t>(c), out0 = reinterpret_cast<uintptr_t>(out);
+  const bool f32_route = gates_impl == RGK_GATES_AUTO && rgk::rglru_f32_supported(dtype, bw, B, T, H) &&
+                         (c0 + act <= out0 || out0 + act <= c0);
   if (xb != nullptr) {
     cudaError_t e = fuse_conv
         ? rgk::launch_conv1d_cache(xb, pos, pos64, B, T, E, dtype, conv_cache_out, s)
         : rgk::launch_conv1d_prefill(xb, pos, pos64, p->conv_w, p->conv_b, B, T, E, dtype,
                                      const_cast<void*>(c), conv_cache_out, s,
                                     chan_route ? rgk::rglru_chan_prep(scan_ws, p->a_param, B, T, H)
-                                               : rgk::ChanPrep());
+                                    : f32_route ? rgk::rglru_f32_prep(scan_ws, B, T, H) : rgk::ChanPrep());
     if (e != cudaSuccess) return cuda_fail(e, "conv1d launch");
+  }
+  if (f32_route) {
+    const void* packed = wpack;
+    if (p->gates_packed != nullptr) {                  // behind the TF32 copy
+      packed = static_cast<const char*>(p->gates_packed) + rgk::gates_tf32_packed_bytes(H);
+    } else {
+      cudaError_t e = rgk::launch_pack_gate_weights_f16(p->gate_x_w, p->gate_a_w, H, wpack, s);
+      if (e != cudaSuccess) return cuda_fail(e, "pack_gate_weights launch");
+    }
+    cudaError_t e = rgk::launch_rglru_f32(c, pos, pos64, p->a_param, p->gate_x_b, p->gate_a_b, packed, h0, yb,
+                                          y_activated, B, T, H, out, h_last, scan_ws, s, xb != nullptr);
+    if (e != cudaSuccess) return cuda_fail(e, "float32 RG-LRU launch");
+    return RGK_OK;
   }
   const bool fused_ok = rgk::rglru_chan_supported(dtype, bw, B, T);
   const bool want_fused = gates_impl >= RGK_GATES_FUSED;
@@ -202,7 +221,8 @@ struct PathWs {
 PathWs carve(void* ws, int64_t B, int64_t T, int64_t E, int dtype) {
   PathWs w;
   size_t scan_bytes = rgk::scan_workspace_bytes(B, T, E, dtype);
-  const size_t fused_bytes = dtype == RGK_BF16 ? rgk::rglru_chan_workspace_bytes(B, T, E) : 0;
+  const size_t fused_bytes = dtype == RGK_BF16 ? rgk::rglru_chan_workspace_bytes(B, T, E)
+                                               : rgk::rglru_f32_workspace_bytes(B, T, E);
   if (fused_bytes > scan_bytes) scan_bytes = fused_bytes;
   const size_t act = up256(static_cast<size_t>(B) * T * E * elem_size(dtype));
   char* base = static_cast<char*>(ws);
@@ -334,7 +354,7 @@ size_t rgk_gate_pack_bytes(int H) { return H > 0 ? rgk::gates_tc_packed_bytes(H)
 size_t rgk_gate_pack_bytes_for(int H, int dtype) {
   if (H <= 0) return 0;
   if (dtype == RGK_BF16) return rgk::gates_tc_packed_bytes(H);
-  if (dtype == RGK_F32) return rgk::gates_tf32_packed_bytes(H);
+  if (dtype == RGK_F32) return rgk::gates_tf32_packed_bytes(H) + rgk::rglru_f32_packed_bytes(H);
   return 0;
 }
 
@@ -351,6 +371,10 @@ int rgk_pack_gate_weights(const rgk_params* p, int H, int bw, int dtype, void* p
     RGK_CUDA(rgk::launch_pack_gate_weights_tf32(p->gate_x_w, p->gate_a_w, H, packed_out,
                                                 static_cast<cudaStream_t>(stream)),
              "pack_gate_weights (TF32 split) launch");
+    RGK_CUDA(rgk::launch_pack_gate_weights_f16(p->gate_x_w, p->gate_a_w, H,
+                                               static_cast<char*>(packed_out) + rgk::gates_tf32_packed_bytes(H),
+                                               static_cast<cudaStream_t>(stream)),
+             "pack_gate_weights (float16 split) launch");
     return RGK_OK;
   }
   RGK_CUDA(rgk::launch_pack_gate_weights(p->gate_x_w, p->gate_a_w, H, packed_out,

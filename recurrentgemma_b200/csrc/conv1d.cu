@@ -85,7 +85,7 @@ conv1d_prefill_kernel(const T* x, const void* pos, int pos64,
   // kernel would sit on the SMs in another order, neighbours of a chain farther apart: 4 x 8000 tokens
   // of short documents 4% slower, nothing faster)
   grid_dependency_wait();
-  if (prep.E > 0) {                              // for the RG-LRU kernel behind
+  if (prep.n_zero > 0) {                         // for the RG-LRU kernel behind
     const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     chan_prepare(prep, block * blockDim.x + threadIdx.x,
                  (int64_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x);

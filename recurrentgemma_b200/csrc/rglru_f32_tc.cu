@@ -1,0 +1,778 @@
+// RG-LRU forward in float32 as ONE kernel: the block-diagonal gate projections, the gate arithmetic, the linear
+// recurrence and the join with the other branch (recurrentgemma torch/layers.py:127-137, 313-365, 140-191; join of
+// torch/modules.py:627-628, 646), heads of width 256.  a and the normalised input never reach memory.
+//
+// The contraction runs on the tensor cores as three products of float16 halves: with x scaled by a power of two
+// of its token (over the 256 channels of the head) and w by one of its output channel, so that the largest
+// magnitude lies in [2^14, 2^15),
+//     x w  ~  x1 w1 + x2 w1 + x1 w2,      v1 = fp16(v),  v2 = fp16(v - v1)
+// with float32 accumulation.  What is dropped is 2^-22 of a product (2^-40 of the largest one where a factor is
+// below 2^-18 of its row's largest); the scales are exact and undone in the epilogue.  As three TF32 products
+// (gates_tf32.cu) the dropped part is up to 2^-20, an operand twice the bytes, and an instruction half as fast.
+//
+// Accumulators are channel-major, D[channel, token] = W[channel, k] . X[token, k]^T: a TMEM lane is a channel, its
+// columns are tokens, and a thread walks its channel's tokens in time order.  A global access of a warp is one
+// token of 32 consecutive channels: 128 contiguous bytes.
+//
+// Work: 128 tokens of one sequence x one head, as two units of 128 channels each that share the split activations;
+// jobs are numbered time-major and dealt out round-robin to persistent CTAs, one per SM.  A last round that leaves
+// half of the CTAs without a job is dealt out as units.
+//
+// Roles in a CTA (24 warps, two of them idle):
+//   split     4 warps: the scale of each token (a pass over the head's 256 channels), then per K-slice of 64 the two
+//             halves of the activations into the operand tiles (128-byte swizzle), as the tensor core releases them;
+//   producer  one thread: packed weights, per K-slice and gate the two halves (128 rows x 64, 16 KiB each) by TMA
+//             through a ring of five;
+//   MMA       one warp, an elected lane of which issues tcgen05.mma kind::f16 M128 N128 into one of two accumulator
+//             sets (x-gate and a-gate columns, 2 x 128 each);
+//   epilogue  two groups of 8 warps, a group an accumulator set, so that one's waits lie under the other's arithmetic;
+//             8 warps = 4 channel quarters (TMEM lane quarters) x 2 token halves.  Pass one: gates, (a, x) of each
+//             token back into the accumulator's own columns, the map (P, H): h -> P h + H of the thread's 64
+//             tokens.  Then the state that enters the tile, by look-back over the maps of earlier tiles (records of
+//             64-bit words {value, token}: no flags, no fences).  Pass two: the recurrence from tensor memory, join,
+//             stores.
+//
+// What bounds it: the epilogue, 67 warp instructions for 32 elements without a join at 54 % of the issue slots, which
+// wait for loads and tensor memory (tensor pipe 39 %, special functions 39 %).  Width 2560, float32, us as gate and
+// scan kernels with a and the normalised input through memory / this: 2 x 1024 tokens 64 / 34, 5001 tokens 150 / 61,
+// 8 x 4096 730 / 329, 16 tokens 19 / 12; with Conv1D and join 1500 tokens 64 / 36, 4 x 4000 458 / 286.  With one
+// epilogue group of eight warps 2 x 1024 tokens took 42.  Distance of the 2-norm from a 64-bit evaluation: 9.5e-7 /
+// 5.6e-7 at 2 x 1024 tokens, and the smaller one at every size and magnitude compared.
+//
+// All waits are bounded; on expiry WsHeader::status is raised, the affected values are taken as zero and the
+// kernel runs to completion.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include "rgk_common.cuh"
+#include "rgk_internal.h"
+#include "tc_common.cuh"
+
+namespace rgk {
+namespace {
+
+constexpr int kHW = 256;                 // head width = K
+constexpr int kUT = 128;                 // tokens of a unit (MMA N)
+constexpr int kUC = 128;                 // channels of a unit (MMA M)
+constexpr int kKB = 64;                  // K of a slice: 128-byte rows of float16
+constexpr int kKBlocks = kHW / kKB;
+constexpr int kRing = 5;
+constexpr int kXPart = kUT * kKB * 2;    // 16 KiB: one half of the activations of a slice
+constexpr int kWPart = kUC * kKB * 2;    // 16 KiB: one half of one gate's weights of a slice
+constexpr int kGroup = 8, kEpi = 2 * kGroup, kSplit = 4;
+// Six warpgroups: four of epilogue warps, one of split warps, one of the producer, MMA and two idle warps, which
+// hands registers to the split warps (loads in flight).  setmaxnreg.inc waits, without a limit, until the CTA has
+// that many to give: no variant is launched that was compiled to fewer (set_attributes).
+constexpr int kThreads = (kEpi + kSplit + 4) * 32;
+constexpr int kRegsEpilogue = 80, kRegsSplit = 120, kRegsOther = 40;
+constexpr bool registers_suffice(int per_thread) {
+  return 6 * per_thread >= 4 * kRegsEpilogue + kRegsSplit + kRegsOther;
+}
+static_assert(kThreads == 6 * 128, "six warpgroups, four of them epilogue");
+static_assert(registers_suffice(80) && !registers_suffice(79), "the hand-over takes all of 80 a thread");
+constexpr int kTokHalf = kUT / 2;        // tokens of an epilogue thread
+constexpr int kBarFirst = 9;             // named barrier behind the first job's activations (1-8: the epilogue's)
+constexpr int kBatch = 8;                // tokens between two loads from tensor memory
+constexpr int kOffX = 0;                                         // [slice][half]
+constexpr int kOffRing = kOffX + kKBlocks * 2 * kXPart;
+constexpr int kScaleBufs = 4;
+constexpr int kOffScale = kOffRing + kRing * kWPart;             // float [job & 3][token]: 1 / scale
+constexpr int kOffMap = kOffScale + kScaleBufs * kUT * 4;        // float2 [group][channel]: map of the first half
+constexpr int kOffBar = kOffMap + 2 * kUC * 8;                   // ring full, empty; slice full, empty; sets full, empty
+constexpr int kNumBar = 2 * kRing + 2 * kKBlocks + 4;
+constexpr int kOffTmem = kOffBar + kNumBar * 8;
+constexpr int kOffAbort = kOffTmem + 4;
+constexpr int kSmem = kOffAbort + 4 + 1024;
+static_assert(kSmem <= 232448, "exceeds the 227 KiB of shared memory a CTA may use");
+
+// kind::f16, D float32, A and B float16, both K-major
+constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kUT >> 3) << 17) | ((uint32_t)(kUC >> 4) << 24);
+
+constexpr unsigned kLookbackSpins = 1u << 20;
+constexpr int kLookback = 4;             // earlier tiles asked for per round trip
+constexpr unsigned long long kToken = 1ull << 32;
+
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_word(unsigned long long* p, float v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(kToken | (unsigned long long)__float_as_uint(v))
+               : "memory");
+}
+
+// The power of two that brings a largest magnitude (its bits) into [2^14, 2^15), and its inverse, both normal.
+// (Infinity and NaN: any power, the halves carry them on.)
+__device__ __forceinline__ float scale_of(uint32_t max_bits) {
+  const int e = max((int)(max_bits >> 23), 15);
+  return __uint_as_float((uint32_t)(268 - e) << 23);
+}
+__device__ __forceinline__ float inverse_scale_of(uint32_t max_bits) {
+  const int e = max((int)(max_bits >> 23), 15);
+  return __uint_as_float((uint32_t)(e - 14) << 23);
+}
+
+// Two scaled values -> their float16 halves, packed.
+__device__ __forceinline__ void split_pair(float v0, float v1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(v0, v1);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(v0 - f.x, v1 - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// Bits of the largest magnitude among the 256 values that a warp holds, 8 a lane.  (A value that is no number does
+// not count: it reaches the products whatever the scale.)
+__device__ __forceinline__ uint32_t largest(const float4& a, const float4& b) {
+  const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
+                        fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
+  return __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+}
+
+// gelu_tanh(z) = z sigmoid(2 u), u = sqrt(2 / pi) (z + 0.044715 z^3), on the hardware exponential and reciprocal: no
+// cancellation at negative z, where 1 + tanh(u) has some, so nearer to a 64-bit evaluation than the float32 tanh.
+__device__ __forceinline__ float gelu_f32(float z) {
+  constexpr float k0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
+  const float w = z * fmaf(z * z, k0 * 0.044715f, k0);
+  return z * rcpf(1.0f + ex2f(w));
+}
+
+// The jobs of a CTA: whole heads (two units) round-robin, then a unit of the last round where that was cut.
+struct Jobs {
+  int n_full, n_units, cut;                // whole jobs of this CTA, its units, its unit of the cut round (or -1)
+  int per_tt, heads, first_cut;
+  __device__ __forceinline__ Jobs(int n_jobs, int per_tt_, int heads_) : per_tt(per_tt_), heads(heads_) {
+    const int grid = (int)gridDim.x, id = (int)blockIdx.x;
+    const int rounds = n_jobs / grid, rest = n_jobs - rounds * grid;
+    const bool cuts = 2 * rest <= grid;
+    n_full = rounds + (!cuts && id < rest ? 1 : 0);
+    first_cut = rounds * grid;
+    cut = cuts && id < 2 * rest ? id : -1;
+    n_units = 2 * n_full + (cut >= 0 ? 1 : 0);
+  }
+  __device__ __forceinline__ int count() const { return n_full + (cut >= 0 ? 1 : 0); }
+  // (time tile, sequence, head) of job j; its units are `half` .. `half` + n - 1
+  __device__ __forceinline__ void get(int j, int& tt, int& b, int& head, int& half, int& n) const {
+    int i;
+    if (j < n_full) {
+      i = (int)blockIdx.x + j * (int)gridDim.x;
+      half = 0;
+      n = 2;
+    } else {
+      i = first_cut + (cut >> 1);
+      half = cut & 1;
+      n = 1;
+    }
+    tt = i / per_tt;
+    const int r = i - tt * per_tt;
+    b = r / heads;
+    head = r - b * heads;
+  }
+};
+
+// The state entering tile tt of a chain, one channel per lane: composes the published maps of earlier tiles,
+// nearest first, until a tile with a known state or the start of the sequence is met.
+__device__ __forceinline__ float look_back(const unsigned long long* agg, const unsigned long long* incl, float hs,
+                                           int64_t word, int tt, int64_t tile_words, bool* timed_out_p,
+                                           int64_t n_words, int* status) {
+  float Pc = 1.0f, Hc = 0.0f;
+  int pred = tt - 1;
+  unsigned spins = 0;
+  *timed_out_p = false;
+  while (pred >= 0) {
+    unsigned long long wi[kLookback], wp[kLookback], wh[kLookback];
+#pragma unroll
+    for (int i = 0; i < kLookback; ++i) {
+      wi[i] = 0ull; wp[i] = 0ull; wh[i] = 0ull;
+      const int64_t w = word - (int64_t)(tt - pred + i) * tile_words;
+      if (pred - i >= 0 && RGK_IN_RANGE(w, n_words, status)) {
+        wi[i] = ld_word(incl + w);
+        wp[i] = ld_word(agg + 2 * w);
+        wh[i] = ld_word(agg + 2 * w + 1);
+      }
+    }
+    const int before = pred;
+#pragma unroll
+    for (int i = 0; i < kLookback; ++i) {
+      // entry i belongs to `pred` only while every entry in front of it was absorbed
+      if (pred >= 0 && pred == before - i) {
+        if ((wi[i] >> 32) == 1ull) return fmaf(Pc, __uint_as_float((uint32_t)wi[i]), Hc);
+        if ((wp[i] >> 32) == 1ull && (wh[i] >> 32) == 1ull) {
+          Hc = fmaf(Pc, __uint_as_float((uint32_t)wh[i]), Hc);
+          Pc *= __uint_as_float((uint32_t)wp[i]);
+          --pred;
+        }
+      }
+    }
+    if (pred == before) {
+      if (++spins > kLookbackSpins) {
+        *timed_out_p = true;
+        return 0.0f;
+      }
+      __nanosleep(32);
+    }
+  }
+  return fmaf(Pc, hs, Hc);
+}
+
+// kJoin 0: out = y, 1: out = y * gelu_tanh(yb), 2: out = y * yb
+template <int kJoin>
+__global__ void __launch_bounds__(kThreads, 1)
+rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl,
+                 const float* __restrict__ scale, const float* c, const void* pos, int pos64,
+                 const float* __restrict__ a_param, const float* __restrict__ bias_x,
+                 const float* __restrict__ bias_a, const float* h0, const float* yb, int B, int T_, int E, int heads,
+                 int n_jobs, float* out, float* h_last, WsHeader* hdr, unsigned long long* agg,
+                 unsigned long long* incl) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t s_base = smem_u32(smem);
+  const uint32_t bar0 = s_base + kOffBar;
+  auto bar_w_full = [&](int s) { return bar0 + 8u * s; };
+  auto bar_w_empty = [&](int s) { return bar0 + 8u * (kRing + s); };
+  auto bar_x_full = [&](int kb) { return bar0 + 8u * (2 * kRing + kb); };
+  auto bar_x_empty = [&](int kb) { return bar0 + 8u * (2 * kRing + kKBlocks + kb); };
+  auto bar_acc_full = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + s); };
+  auto bar_acc_empty = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + 2 + s); };
+  float* s_scale = reinterpret_cast<float*>(smem + kOffScale);
+  volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_t = (T_ + kUT - 1) / kUT;
+  const Jobs jobs(n_jobs, B * heads, heads);
+  const int n_my = jobs.count();
+
+  if (threadIdx.x == 0) {
+    *s_abort = 0;
+    for (int s = 0; s < kRing; ++s) { mbar_init(bar_w_full(s), 1); mbar_init(bar_w_empty(s), 1); }
+    for (int kb = 0; kb < kKBlocks; ++kb) { mbar_init(bar_x_full(kb), kSplit); mbar_init(bar_x_empty(kb), 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), kGroup); }
+    mbar_fence_init();
+  }
+  if (warp == kEpi + kSplit + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(s_base + kOffTmem), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *s_tmem;
+  grid_dependency_wait();
+
+  if (warp >= kEpi && warp < kEpi + kSplit) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsSplit) : "memory");
+    // ------------------------------ activations: scales and halves ----------------------------------
+    const int w0 = (warp - kEpi) * 32;                   // first of the warp's 32 tokens
+    bool ok = true;
+    // (the first job's activations are the epilogue warps' work, who have nothing else to do yet)
+    named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
+    if (lane == 0 && n_my > 0)
+      for (int kb = 0; kb < kKBlocks; ++kb) mbar_arrive(bar_x_full(kb));
+    for (int j = 1; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      const int tok0 = tt * kUT + w0;
+      const int live = T_ - tok0;                        // tokens of the warp inside the sequence (may be < 1)
+      const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW;
+      uint32_t top = 0u;                                 // bits of the largest magnitude of token `lane`
+#pragma unroll 1
+      for (int i0 = 0; i0 < 32; i0 += 8) {
+        float4 v[8][2];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i0 + i < live)
+              v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(i0 + i) * E + q * 128 + lane * 4);
+          }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t all = largest(v[i][0], v[i][1]);
+          if (lane == i0 + i) top = all;
+        }
+      }
+      // (four buffers: the job whose scales were here has passed the epilogue.  Its last unit's accumulators
+      // were read before the set could be written for the unit two behind, of a job at most two behind, whose
+      // slices were released before this job's scales are looked for.)
+      s_scale[(j & (kScaleBufs - 1)) * kUT + w0 + lane] = inverse_scale_of(top);
+      const float factor = scale_of(top);
+      const int r = lane >> 3, p = lane & 7;
+#pragma unroll 1
+      for (int kb = 0; kb < kKBlocks; ++kb) {
+        float4 v[8][2];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (4 * i + r < live)
+              v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(4 * i + r) * E + kb * kKB + p * 8 + q * 4);
+          }
+        ok = mbar_wait(bar_x_empty(kb), (j & 1) ^ 1, s_abort);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        uint8_t* hi_tile = smem + kOffX + kb * 2 * kXPart;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = w0 + 4 * i + r;
+          const float s = __shfl_sync(0xffffffffu, factor, 4 * i + r);
+          uint4 hi, lo;
+          split_pair(v[i][0].x * s, v[i][0].y * s, hi.x, lo.x);
+          split_pair(v[i][0].z * s, v[i][0].w * s, hi.y, lo.y);
+          split_pair(v[i][1].x * s, v[i][1].y * s, hi.z, lo.z);
+          split_pair(v[i][1].z * s, v[i][1].w * s, hi.w, lo.w);
+          const int at = row * 128 + ((p ^ (row & 7)) << 4);
+          *reinterpret_cast<uint4*>(hi_tile + at) = hi;
+          *reinterpret_cast<uint4*>(hi_tile + kXPart + at) = lo;
+        }
+        fence_proxy_async();                             // the tensor core reads this through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_x_full(kb));
+      }
+    }
+  } else if (warp >= kEpi + kSplit) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
+    if (warp == kEpi + kSplit) {
+    // ------------------------------ weights ---------------------------------------------------------
+    if (lane == 0) {
+      bool ok = true;
+      int s = 0;
+      uint32_t phase = 1;
+      for (int j = 0; j < n_my && ok; ++j) {
+        int tt, b, head, half, n;
+        jobs.get(j, tt, b, head, half, n);
+        for (int u = 0; u < n && ok; ++u) {
+          const int row = (head * 2 + half + u) * 2 * kUC;
+          for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
+            ok = mbar_wait(bar_w_empty(s), phase, s_abort);
+            if (!ok) break;
+            mbar_expect_tx(bar_w_full(s), kWPart);
+            tma_load_2d(s_base + kOffRing + s * kWPart, (i & 1) ? &map_wl : &map_wh, (i >> 2) * kKB,
+                        row + ((i >> 1) & 1) * kUC, bar_w_full(s));
+            if (++s == kRing) { s = 0; phase ^= 1; }
+          }
+        }
+      }
+    }
+  } else if (warp == kEpi + kSplit + 1) {
+    // ------------------------------ MMA issue -------------------------------------------------------
+    // (the whole warp runs the loop, one elected lane issues: see mma_ring)
+    const uint64_t desc_x = smem_desc_sw128(s_base + kOffX), desc_w = smem_desc_sw128(s_base + kOffRing);
+    bool ok = true;
+    int s = 0, t = 0;
+    uint32_t phase = 0;
+    for (int j = 0; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      for (int u = 0; u < n && ok; ++u, ++t) {
+        const int as = t & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+        if (!ok) break;
+        tc_fence_after();
+        for (int kb = 0; kb < kKBlocks && ok; ++kb) {
+          if (u == 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_x_full(kb), j & 1, s_abort));
+            if (!ok) break;
+          }
+          const uint64_t x1 = desc_x + (uint64_t)(kb * (2 * kXPart >> 4)), x2 = x1 + (kXPart >> 4);
+          for (int g = 0; g < 2 && ok; ++g) {
+            const uint32_t d = tmem_base + (as * 2 + g) * kUT;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar_w_full(s), phase, s_abort));
+              if (!ok) break;
+              tc_fence_after();
+              if (elect_one()) {
+                const uint64_t w = desc_w + (uint64_t)(s * (kWPart >> 4));
+#pragma unroll
+                for (int ks = 0; ks < kKB / 16; ++ks) {
+                  tc_mma_bf16(d, w + 2 * ks, x1 + 2 * ks, kIdesc, (part | kb | ks) != 0 ? 1u : 0u);
+                  if (part == 0) tc_mma_bf16(d, w + 2 * ks, x2 + 2 * ks, kIdesc, 1u);
+                }
+                tc_commit(bar_w_empty(s));
+                if (part == 1 && g == 1) {
+                  if (u == n - 1) tc_commit(bar_x_empty(kb));
+                  if (kb == kKBlocks - 1) tc_commit(bar_acc_full(as));
+                }
+              }
+              __syncwarp();
+              if (++s == kRing) { s = 0; phase ^= 1; }
+            }
+          }
+        }
+      }
+    }
+    }
+  } else {
+    // ------------------------------ epilogue --------------------------------------------------------
+    const int chq = warp & 3, th = (warp >> 2) & 1, group = warp >> 3;
+    const int64_t n_state = (int64_t)B * E;
+    const int64_t n_words = (int64_t)tiles_t * B * E, tile_words = (int64_t)B * E;
+    (void)n_state; (void)n_words;
+    // (a, x) of a batch of tokens, from its accumulators
+    constexpr float kNegLog2e = -1.4426950408889634f;
+    bool ok = true;
+    // ---- the first job's activations, a warp eight tokens, read once: 4 us less until the first MMA than by the
+    // split warps, which read them twice ----
+    if (n_my > 0) {
+      int tt, b, head, half, n;
+      jobs.get(0, tt, b, head, half, n);
+      const int w0 = warp * (kUT / kEpi), tok0 = tt * kUT + w0;
+      const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW + lane * 4;
+#pragma unroll 1
+      for (int i0 = 0; i0 < kUT / kEpi; i0 += 4) {
+        float4 v[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            v[i][q] = tok0 + i0 + i < T_ ? *reinterpret_cast<const float4*>(x0 + (int64_t)(i0 + i) * E + q * 128)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t top = largest(v[i][0], v[i][1]);
+          const float s = scale_of(top);
+          const int row = w0 + i0 + i;
+          if (lane == 0) s_scale[row] = inverse_scale_of(top);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            uint2 hi, lo;
+            split_pair(v[i][q].x * s, v[i][q].y * s, hi.x, lo.x);
+            split_pair(v[i][q].z * s, v[i][q].w * s, hi.y, lo.y);
+            const int k = q * 128 + lane * 4;            // the lane's first channel of the head
+            uint8_t* at = smem + kOffX + (k >> 6) * 2 * kXPart + row * 128 +
+                          ((((k & 63) >> 3) ^ (row & 7)) << 4) + (k & 4) * 2;
+            *reinterpret_cast<uint2*>(at) = hi;
+            *reinterpret_cast<uint2*>(at + kXPart) = lo;
+          }
+        }
+      }
+      fence_proxy_async();
+    }
+    named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
+    int t = 0;
+    for (int j = 0; j < n_my; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      const int u = (t ^ group) & 1;                     // the group's unit of this job, if it has one
+      const int tu = t + u;
+      t += n;
+      if (u >= n) continue;
+      const int as = group;
+      const int tok0 = tt * kUT + th * kTokHalf;
+      const int live = T_ - tok0;                        // tokens of the thread inside the sequence
+      // tokens that start a document, and tokens past the end of the sequence (the identity map)
+      uint32_t rs[2], inv[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int k = q * 32 + lane;
+        rs[q] = __ballot_sync(0xffffffffu, k < live && pos_is_zero(pos, pos64, (int64_t)b * T_ + tok0 + k));
+        inv[q] = __ballot_sync(0xffffffffu, k >= live);
+      }
+      const float* st_row = s_scale + (j & (kScaleBufs - 1)) * kUT + th * kTokHalf;
+      const int grp = head * 2 + half + u;
+      const int e = grp * kUC + chq * 32 + lane;
+      const int64_t at0 = ((int64_t)b * T_ + tok0) * E + e;
+      // z log2(e) with the sign turned: the sigmoid is 1 / (1 + 2^that)
+      const int wrow = grp * 2 * kUC + chq * 32 + lane;
+      const float kx = kNegLog2e * scale[wrow], ka = kNegLog2e * scale[wrow + kUC];
+      const float bx = kNegLog2e * bias_x[e], ba = kNegLog2e * bias_a[e];
+      const float m8sp = -8.0f * softplus_(a_param[e]);
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(chq * 32) << 16) + as * 2 * kUT + th * kTokHalf;
+      auto load_rows = [&](const float* src, int k0, float (&v)[kBatch], bool whole) {
+        const float* p = src + at0 + (int64_t)k0 * E;
+        if (whole) {
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) v[k] = p[(int64_t)k * E];
+        } else {
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) v[k] = k0 + k < live ? p[(int64_t)k * E] : 0.0f;
+        }
+      };
+      const bool whole = live >= kTokHalf;
+      if constexpr (kJoin != 0) {                        // the other branch into L2: pass two has little to hide it under
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int k = q * 32 + lane;
+          if (k < live) asm volatile("prefetch.global.L2 [%0];" :: "l"(yb + (at0 - lane) + (int64_t)k * E));
+        }
+      }
+      const int end = min(kTokHalf, live);               // batches past the end of the sequence are left out
+      float P = 1.0f, H = 0.0f;
+      {
+        float cn[kBatch];
+        load_rows(c, 0, cn, whole);
+        if (ok) ok = mbar_wait(bar_acc_full(as), (tu >> 1) & 1, s_abort);
+        __syncwarp();
+        tc_fence_after();
+#pragma unroll 1
+        for (int k0 = 0; k0 < end; k0 += kBatch) {
+          uint32_t zx[kBatch], za[kBatch];
+          tc_ld_32x8(t_row + k0, zx);
+          tc_ld_32x8(t_row + kUT + k0, za);
+          float cv[kBatch], st[kBatch];
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) cv[k] = cn[k];
+#pragma unroll
+          for (int k = 0; k < kBatch; k += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(st_row + k0 + k);
+            st[k] = s4.x; st[k + 1] = s4.y; st[k + 2] = s4.z; st[k + 3] = s4.w;
+          }
+          if (k0 + kBatch < end) load_rows(c, k0 + kBatch, cn, whole);
+          const uint32_t rs8 = ((k0 < 32 ? rs[0] : rs[1]) >> (k0 & 31)) & 0xffu;
+          const uint32_t inv8 = ((k0 < 32 ? inv[0] : inv[1]) >> (k0 & 31)) & 0xffu;
+          tc_wait_ld();
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) {
+            const float ex = ex2f(fmaf(__uint_as_float(zx[k]) * st[k], kx, bx));
+            const float ea = ex2f(fmaf(__uint_as_float(za[k]) * st[k], ka, ba));
+            const float gate_x = rcpf(1.0f + ex), gate_a = rcpf(1.0f + ea);
+            // exp(log_a) on the accurate function: a slow channel multiplies a into its state a thousand times
+            const float a = expf(gate_a * m8sp);
+            cv[k] *= gate_x;
+            zx[k] = __float_as_uint(cv[k] * sqrtf_approx(fmaf(-a, a, 1.0f)));
+            za[k] = __float_as_uint(a);
+          }
+          if ((rs8 | inv8) != 0u) {
+            // a token that starts a document: a = 0, multiplier = 1; one past the end: a = 1, x = 0
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+              if ((rs8 >> k) & 1u) { zx[k] = __float_as_uint(cv[k]); za[k] = 0u; }
+              if ((inv8 >> k) & 1u) { zx[k] = 0u; za[k] = 0x3f800000u; }
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) {
+            P *= __uint_as_float(za[k]);
+            H = fmaf(__uint_as_float(za[k]), H, __uint_as_float(zx[k]));
+          }
+          tc_st_32x8(t_row + k0, zx);
+          tc_st_32x8(t_row + kUT + k0, za);
+        }
+        tc_wait_st();
+      }
+
+      // ---- the state that enters the thread's tokens -----------------------------------------------
+      // (in front of the barrier, and so of all records of the tile: h_last may be h0)
+      const float hs = (h0 != nullptr && RGK_IN_RANGE((int64_t)b * E + e, n_state, &hdr->status))
+                           ? h0[(int64_t)b * E + e] : 0.0f;
+      float2* s_map = reinterpret_cast<float2*>(smem + kOffMap) + group * kUC + chq * 32 + lane;
+      if (th == 0) *s_map = make_float2(P, H);
+      named_bar_sync(1 + group * 4 + chq, 64);
+      const float2 first = *s_map;
+      const int64_t word = (int64_t)tt * tile_words + (int64_t)b * E + e;
+      const bool owner = th == 1;
+      const float Pt = P * first.x, Ht = fmaf(P, first.y, H);     // of the whole tile, in the second half's threads
+      if (owner && tt > 0 && tt < tiles_t - 1 && RGK_IN_RANGE(word, n_words, &hdr->status)) {
+        st_word(agg + 2 * word, Pt);
+        st_word(agg + 2 * word + 1, Ht);
+      }
+      float yn[kBatch];
+      if constexpr (kJoin != 0) load_rows(yb, 0, yn, whole);      // in flight during the look-back
+      bool timed_out = !ok;
+      float hin = 0.0f;
+      if (ok) hin = look_back(agg, incl, hs, word, tt, tile_words, &timed_out, n_words, &hdr->status);
+      __syncwarp();
+      if (__any_sync(0xffffffffu, timed_out)) {
+        if (lane == 0) atomicExch(&hdr->status, kStatusTimeout);
+        hin = 0.0f;
+      }
+      if (owner && tt < tiles_t - 1 && RGK_IN_RANGE(word, n_words, &hdr->status))
+        st_word(incl + word, fmaf(Pt, hin, Ht));
+      float h = owner ? fmaf(first.x, hin, first.y) : hin;
+
+      auto release = [&] {                                 // the set has been read: it may be written again
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_acc_empty(as));
+      };
+      if (end <= 0) release();
+
+      // ---- the recurrence, join, stores ------------------------------------------------------------
+#pragma unroll 1
+      for (int k0 = 0; k0 < end; k0 += kBatch) {
+        uint32_t xn[kBatch], av[kBatch];
+        tc_ld_32x8(t_row + k0, xn);
+        tc_ld_32x8(t_row + kUT + k0, av);
+        float yv[kBatch];
+        if constexpr (kJoin != 0) {
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) yv[k] = kJoin == 1 ? gelu_f32(yn[k]) : yn[k];
+          if (k0 + kBatch < end) load_rows(yb, k0 + kBatch, yn, whole);
+        }
+        tc_wait_ld();
+        if (k0 + kBatch >= end) release();
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          h = fmaf(__uint_as_float(av[k]), h, __uint_as_float(xn[k]));
+          xn[k] = __float_as_uint(kJoin != 0 ? h * yv[k] : h);
+        }
+        float* o = out + at0 + (int64_t)k0 * E;
+        if (whole) {
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k) o[(int64_t)k * E] = __uint_as_float(xn[k]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k)
+            if (k0 + k < live) o[(int64_t)k * E] = __uint_as_float(xn[k]);
+        }
+      }
+      if (owner && h_last != nullptr && tt == tiles_t - 1 &&
+          RGK_IN_RANGE((int64_t)b * E + e, n_state, &hdr->status))
+        h_last[(int64_t)b * E + e] = h;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *s_abort) atomicExch(&hdr->status, kStatusTimeout);
+  if (warp == kEpi + kSplit + 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
+                 : "memory");
+  }
+}
+
+// Gate weights [H, 256 (k), 256 (n)] float32 -> [H, 2, 256 (n'), 256 (k)] float16, first and second halves of the
+// scaled values (rows 0-127 of a group: the x-gate columns of its 128 channels, rows 128-255 the a-gate ones), and
+// 1 / scale of each row.
+__global__ void pack_gate_weights_f16_kernel(const float* __restrict__ wx, const float* __restrict__ wa,
+                                             __half* __restrict__ hi, __half* __restrict__ lo,
+                                             float* __restrict__ scale) {
+  __shared__ float tile[kHW][33];                                  // [k][n']
+  const int group = blockIdx.y, head = group >> 1, half = group & 1;
+  const int n0 = blockIdx.x * 32;                                  // n' in [0, 256)
+  const float* src = (n0 < kUC ? wx : wa) + (int64_t)head * kHW * kHW + half * kUC + (n0 % kUC);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = warp; k < kHW; k += 8) tile[k][lane] = src[(int64_t)k * kHW + lane];
+  __syncthreads();
+  for (int r = warp; r < 32; r += 8) {
+    uint32_t m = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(tile[lane * 8 + i][r]) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    const float s = scale_of(m);
+    const int64_t row = (int64_t)group * 2 * kUC + n0 + r;
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      split_pair(tile[lane * 8 + 2 * i][r] * s, tile[lane * 8 + 2 * i + 1][r] * s, h[i], l[i]);
+    *reinterpret_cast<uint4*>(hi + row * kHW + lane * 8) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(lo + row * kHW + lane * 8) = make_uint4(l[0], l[1], l[2], l[3]);
+    if (lane == 0) scale[row] = inverse_scale_of(m);
+  }
+}
+
+// early: the kernel behind is let in at once (its own wait is for this one's end).  One token 18.6 -> 11.4 us; where
+// there are several rounds of units its CTAs, placed as this one's leave, sit on the SMs in another order,
+// neighbours of a chain farther apart: 8 x 4096 tokens 327 -> 340.
+__global__ void rglru_f32_prepare_kernel(uint4* zero, int64_t n, int early) {
+  if (early) grid_launch_dependents();
+  grid_dependency_wait();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    zero[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+struct Layout {
+  int64_t n_words;
+  size_t incl_off, agg_off, total;
+};
+Layout layout(int64_t B, int64_t T, int64_t E) {
+  Layout L;
+  L.n_words = (T + kUT - 1) / kUT * B * E;
+  L.incl_off = sizeof(WsHeader);
+  L.agg_off = L.incl_off + (size_t)L.n_words * 8;
+  L.total = (L.agg_off + (size_t)L.n_words * 16 + 255) & ~(size_t)255;
+  return L;
+}
+
+template <int kJoin>
+cudaError_t set_attributes() {
+  cudaFuncAttributes a;
+  if (const cudaError_t e = cudaFuncGetAttributes(&a, rglru_f32_kernel<kJoin>); e != cudaSuccess) return e;
+  if (!registers_suffice(a.numRegs)) return cudaErrorLaunchOutOfResources;
+  return cudaFuncSetAttribute(rglru_f32_kernel<kJoin>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+}
+
+constexpr int64_t packed_rows(int H) { return (int64_t)H * 2 * 2 * kUC; }
+
+}  // namespace
+
+// Every sequence begins a tile of its own, where the kernels of gates_tf32.cu and scan.cu cut the tokens of all
+// sequences into tiles together.  Width 2560, us those / this: 6 x 50 tokens 20.3 / 17.0, 64 x 50 95 / 73, 20 x 43
+// 27.8 / 28.8; few jobs run at once however empty their tiles: 8 x 1 token 19.7 / 16.5, 8 x 16 20.8 / 17.6.
+bool rglru_f32_supported(int dtype, int bw, int64_t B, int64_t T, int H) {
+  if (dtype != 0 || bw != kHW || B < 1 || T < 1) return false;
+  const int64_t tiles = (T + kUT - 1) / kUT * B;
+  return tiles < ((int64_t)1 << 17) && (5 * tiles * kUT <= 13 * B * T || tiles * H <= 128);
+}
+
+size_t rglru_f32_workspace_bytes(int64_t B, int64_t T, int64_t E) { return T < 1 ? 0 : layout(B, T, E).total; }
+
+size_t rglru_f32_packed_bytes(int H) { return (size_t)packed_rows(H) * (kHW * 2 * 2 + 4); }
+
+cudaError_t launch_pack_gate_weights_f16(const void* wx, const void* wa, int H, void* packed_w, cudaStream_t s) {
+  __half* hi = static_cast<__half*>(packed_w);
+  __half* lo = hi + packed_rows(H) * kHW;
+  pack_gate_weights_f16_kernel<<<dim3(2 * kUC / 32, 2 * H), 256, 0, s>>>(
+      (const float*)wx, (const float*)wa, hi, lo, reinterpret_cast<float*>(lo + packed_rows(H) * kHW));
+  return cudaGetLastError();
+}
+
+ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H) {
+  const Layout L = layout(B, T, (int64_t)H * kHW);
+  ChanPrep p;
+  p.zero = reinterpret_cast<uint4*>(static_cast<char*>(ws) + L.incl_off);
+  p.n_zero = L.n_words * 24 / 16;
+  return p;
+}
+
+cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const void* a_param, const void* bx,
+                             const void* ba, const void* packed_w, const float* h0, const void* yb, int y_activated,
+                             int64_t B, int64_t T, int H, void* out, float* h_last, void* ws, cudaStream_t s,
+                             bool prepared) {
+  const int E = H * kHW;
+  const Layout L = layout(B, T, E);
+  static PerDeviceOnce once;
+  int num_sms = 0;
+  cudaError_t err = once.run([] {
+    cudaError_t e = set_attributes<0>();
+    if (e == cudaSuccess) e = set_attributes<1>();
+    if (e == cudaSuccess) e = set_attributes<2>();
+    return e;
+  }, &num_sms);
+  if (err != cudaSuccess) return err;
+  const int64_t n_jobs = (T + kUT - 1) / kUT * B * H;     // below 2^29
+  if (!prepared) {
+    const ChanPrep prep = rglru_f32_prep(ws, B, T, H);
+    const int64_t blocks = (prep.n_zero + 1023) / 1024;
+    err = launch_dependent(rglru_f32_prepare_kernel, dim3((unsigned)(blocks < 8 * num_sms ? blocks : 8 * num_sms)),
+                           dim3(256), 0, s, prep.zero, prep.n_zero, (int)(2 * n_jobs <= num_sms));
+    if (err != cudaSuccess) return err;
+  }
+  const __half* hi = static_cast<const __half*>(packed_w);
+  const __half* lo = hi + packed_rows(H) * kHW;
+  const float* scale = reinterpret_cast<const float*>(lo + packed_rows(H) * kHW);
+  CUtensorMap map_wh, map_wl;
+  if (!tensor_map_2d(&map_wh, hi, (uint64_t)packed_rows(H), kHW, kUC, kKB, true) ||
+      !tensor_map_2d(&map_wl, lo, (uint64_t)packed_rows(H), kHW, kUC, kKB, true))
+    return cudaErrorInvalidValue;
+  // all CTAs resident (look-back may spin), and as many as there are units
+  const int grid = 2 * n_jobs < num_sms ? (int)(2 * n_jobs) : num_sms;
+  auto run = [&](auto kernel) {
+    return launch_dependent(kernel, dim3(grid), dim3(kThreads), (size_t)kSmem, s, map_wh, map_wl, scale,
+                            (const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba,
+                            h0, (const float*)yb, (int)B, (int)T, E, H, (int)n_jobs, (float*)out, h_last,
+                            reinterpret_cast<WsHeader*>(ws),
+                            reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.agg_off),
+                            reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.incl_off));
+  };
+  if (yb == nullptr) return run(rglru_f32_kernel<0>);
+  return y_activated ? run(rglru_f32_kernel<2>) : run(rglru_f32_kernel<1>);
+}
+
+}  // namespace rgk

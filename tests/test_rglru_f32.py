@@ -1,0 +1,111 @@
+"""The float32 RG-LRU as one kernel (tiles of 128 tokens, units of 128 channels) against float64, at the edges of
+its tiles and of its last round of work (recurrentgemma/torch/layers.py:140-191, 338-376; join of
+torch/modules.py:627-628, 646).  Needs a B200."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _layer(heads, seed):
+  import recurrentgemma_b200 as rg
+  torch.manual_seed(seed)
+  e = heads * 256
+  lru = rg.RGLRU(e, heads, device=DEV, dtype=torch.float32)
+  conv = rg.Conv1D(e, 4, device=DEV, dtype=torch.float32)
+  for b in (lru.input_gate.b, lru.a_gate.b, conv.b):
+    b.data.normal_(0, 0.1)
+  conv.w.data.normal_(0, 0.5)
+  return rg, lru, conv
+
+
+def _float64(lru, x, pos, h0, yb=None):
+  b, t, e = x.shape
+  xd = x.double().view(b, t, e // 256, 256)
+  gate = lambda g: torch.sigmoid(torch.einsum("bthi,hij->bthj", xd, g.w.double()) + g.b.double()).reshape(b, t, e)
+  log_a = -8.0 * gate(lru.a_gate) * torch.nn.functional.softplus(lru.a_param.double())
+  reset = (pos == 0)[..., None]
+  a = torch.where(reset, torch.zeros_like(log_a), torch.exp(log_a))
+  xn = x.double() * gate(lru.input_gate) * torch.where(reset, torch.ones_like(a), torch.sqrt(1 - torch.exp(2 * log_a)))
+  h = torch.zeros(b, e, dtype=torch.float64, device=DEV) if h0 is None else h0.double()
+  y = []
+  for i in range(t):
+    h = a[:, i] * h + xn[:, i]
+    y.append(h)
+  y = torch.stack(y, 1)
+  if yb is not None:
+    z = yb.double()
+    y = y * 0.5 * z * (1 + torch.tanh(math.sqrt(2 / math.pi) * (z + 0.044715 * z ** 3)))
+  return y, h
+
+
+def _close(got, want, t):
+  # a handful of roundings of 2^-24 a token, carried along by a <= 1 and independent of one another, and a
+  # contraction good to 2^-22 of its terms
+  tol = 2.0 ** -21 * math.sqrt(t)
+  err = float((got.double() - want).norm() / want.norm())
+  assert err <= tol, (err, tol)
+
+
+# one token; a tile less one, whole, and one more; whole heads and units in the last round (148 SMs: 75 jobs are dealt
+# out whole, 74 as units, 160 leave 12 to be cut); tiles of many chains
+@pytest.mark.parametrize("b,t,heads", [(1, 1, 1), (2, 127, 2), (1, 128, 3), (3, 129, 1), (1, 385, 2), (75, 43, 1),
+                                       (74, 50, 1), (16, 100, 10), (5, 300, 16), (2, 1024, 10)])
+@pytest.mark.parametrize("state", [False, True])
+def test_forward(b, t, heads, state):
+  rg, lru, _ = _layer(heads, b + t)
+  x = torch.randn(b, t, heads * 256, device=DEV)
+  # documents that begin at the edges of tiles and of halves of tiles, and short ones
+  pos = torch.arange(1, t + 1, device=DEV).repeat(b, 1)
+  pos[torch.rand(b, t, device=DEV) < 0.02] = 0
+  pos[:, [i for i in (63, 64, 127, 128) if i < t]] = 0
+  h0 = torch.randn(b, heads * 256, device=DEV) if state else None
+  y, h = lru(x, pos, h0)
+  want, want_h = _float64(lru, x, pos, h0)
+  _close(y, want, t)
+  _close(h, want_h, t)
+
+
+@pytest.mark.parametrize("b,t,heads", [(2, 200, 3), (1, 1500, 10)])
+def test_path(b, t, heads):
+  rg, lru, conv = _layer(heads, t)
+  x, yb = (torch.randn(b, t, heads * 256, device=DEV) for _ in range(2))
+  pos = torch.arange(t, device=DEV).repeat(b, 1)
+  out, cache = rg.recurrent_path(x, yb, pos, conv, lru)
+  want, want_h = _float64(lru, conv(x, pos)[0], pos, None, yb)
+  _close(out, want, t)
+  _close(cache.rg_lru_state, want_h, t)
+
+
+@pytest.mark.parametrize("scale_x,scale_w", [(1e30, 1.0), (1e-30, 1.0), (1.0, 1e30), (3e4, 1e-4)])
+def test_magnitudes(scale_x, scale_w):
+  """Far outside float16: the scales of tokens and channels carry it."""
+  rg, lru, _ = _layer(1, 5)
+  for g in (lru.input_gate, lru.a_gate):
+    g.w.data.mul_(scale_w)
+    g.w.data[:, :, ::3].mul_(1e-3)                     # channels of very different magnitude
+  x = torch.randn(2, 200, 256, device=DEV) * scale_x
+  x[:, ::2] *= 1e-4
+  pos = torch.arange(200, device=DEV).repeat(2, 1)
+  y, h = lru(x, pos)
+  want, want_h = _float64(lru, x, pos, None)
+  # (gates of arguments far above 1 turn a relative error of 2^-22 of an argument into as much of themselves
+  # times the argument, of which sigmoids that are not yet 0 or 1 leave some ten)
+  _close(y, want, 200 * 100)
+  _close(h, want_h, 200 * 100)
+
+
+def test_not_numbers():
+  """A token with a value that is no number reaches its own head's later states and nothing else."""
+  rg, lru, _ = _layer(2, 6)
+  x = torch.randn(2, 200, 512, device=DEV)
+  pos = torch.arange(200, device=DEV).repeat(2, 1)
+  clean, _ = lru(x, pos)
+  x[1, 70, 300] = float("nan")
+  y, _ = lru(x, pos)
+  assert torch.equal(y[1, :, :256], clean[1, :, :256]) and torch.equal(y[0], clean[0])
+  assert torch.equal(y[:, :70], clean[:, :70])
+  assert bool(torch.isnan(y[1, 70:, 256:]).all())
