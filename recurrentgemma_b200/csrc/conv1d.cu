@@ -81,9 +81,11 @@ conv1d_prefill_kernel(const T* x, const void* pos, int pos64,
                       T* __restrict__ out, T* __restrict__ cache_out, const ChanPrep prep) {
   constexpr int kPack = Traits<T>::kPack;
   using Ops = PackOps<T>;
-  // (no early launch of the kernel behind: placed as this one's blocks drain, the CTAs of the RG-LRU
-  // kernel would sit on the SMs in another order, neighbours of a chain farther apart: 4 x 8000 tokens
-  // of short documents 4% slower, nothing faster)
+  // (early launch of the kernel behind only in float32, where it has a unit a CTA at most: placed as this one's blocks
+  // drain, the CTAs of the RG-LRU kernel would sit on the SMs in another order, neighbours of a chain farther apart: 4 x
+  // 8000 tokens of short documents 4% slower; and in the chain of a prompt's kernels in bfloat16 the projection behind
+  // lands worse on the SMs: prompts of 38 tokens 1.85 -> 2.01 ms)
+  if (prep.early) grid_launch_dependents();
   grid_dependency_wait();
   if (prep.n_zero > 0) {                         // for the RG-LRU kernel behind
     const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;

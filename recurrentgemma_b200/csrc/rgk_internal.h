@@ -69,6 +69,7 @@ struct ChanPrep {
   const __nv_bfloat16* a_param = nullptr;
   __nv_bfloat16* m8sp = nullptr;
   int E = 0;
+  int early = 0;                         // the kernel behind is let in at once: it has a unit a CTA at most
 };
 
 // What scan_kernel finds cleared: its ticket and its flags.  The gate kernel in front does it on the side

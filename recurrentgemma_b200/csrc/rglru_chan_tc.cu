@@ -864,8 +864,10 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
 // The preparation where no kernel in front does it on the side.
 __global__ void chan_prepare_kernel(const ChanPrep p) {
   static_assert(kLogAFloor == -127.5f, "the clamp of chan_prepare");
-  // (no early launch of the kernel behind: its CTAs, placed as this one's drain, would sit on the SMs in
-  // another order, and neighbours of a chain farther apart: 4 x 28741 tokens 542 -> 586 us)
+  // (early launch of the kernel behind only where it has a unit a CTA at most: its CTAs, placed as this one's drain,
+  // would sit on the SMs in another order, and neighbours of a chain farther apart: 4 x 28741 tokens 542 -> 586 us; 16
+  // tokens 10.7 -> 9.6)
+  if (p.early) grid_launch_dependents();
   grid_dependency_wait();
   chan_prepare(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
@@ -982,8 +984,9 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
   const int n_units = (int)L.n_units;
   const int grid = n_units < num_sms ? n_units : num_sms;   // all CTAs resident: look-back may spin
   const bool maps = chan_uses_maps(B, groups, n_units, num_sms);
-  const ChanPrep prep = rglru_chan_prep(ws, a_param, B, T, H);
+  ChanPrep prep = rglru_chan_prep(ws, a_param, B, T, H);
   if (!prepared) {
+    prep.early = n_units <= num_sms;
     const int64_t n = prep.n_zero > prep.E ? prep.n_zero : prep.E, blocks = (n + 1023) / 1024;
     err = launch_dependent(chan_prepare_kernel, dim3((unsigned)(blocks < 8 * num_sms ? blocks : 8 * num_sms)),
                            dim3(256), 0, s, prep);

@@ -89,7 +89,7 @@ static_assert(kSmem <= 232448, "exceeds the 227 KiB of shared memory a CTA may u
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kUT >> 3) << 17) | ((uint32_t)(kUC >> 4) << 24);
 
 constexpr unsigned kLookbackSpins = 1u << 20;
-constexpr int kLookback = 4;             // earlier tiles asked for per round trip
+constexpr int kLookback = 2;             // earlier tiles asked for per round trip (four: 8 x 4096 tokens 341 against 329 us)
 constexpr unsigned long long kToken = 1ull << 32;
 
 __device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
@@ -667,14 +667,12 @@ __global__ void pack_gate_weights_f16_kernel(const float* __restrict__ wx, const
   }
 }
 
-// early: the kernel behind is let in at once (its own wait is for this one's end).  One token 18.6 -> 11.4 us; where
-// there are several rounds of units its CTAs, placed as this one's leave, sit on the SMs in another order,
-// neighbours of a chain farther apart: 8 x 4096 tokens 327 -> 340.
-__global__ void rglru_f32_prepare_kernel(uint4* zero, int64_t n, int early) {
-  if (early) grid_launch_dependents();
+// (early launch of the kernel behind only where no CTA has a second unit: its CTAs, placed as this one's leave, would sit
+// on the SMs in another order, neighbours of a chain farther apart: 8 x 4096 tokens 327 -> 340 us)
+__global__ void rglru_f32_prepare_kernel(const ChanPrep p) {
+  if (p.early) grid_launch_dependents();
   grid_dependency_wait();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    zero[i] = make_uint4(0u, 0u, 0u, 0u);
+  chan_prepare(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 struct Layout {
@@ -696,6 +694,16 @@ cudaError_t set_attributes() {
   if (const cudaError_t e = cudaFuncGetAttributes(&a, rglru_f32_kernel<kJoin>); e != cudaSuccess) return e;
   if (!registers_suffice(a.numRegs)) return cudaErrorLaunchOutOfResources;
   return cudaFuncSetAttribute(rglru_f32_kernel<kJoin>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+}
+
+cudaError_t device_setup(int* num_sms) {
+  static PerDeviceOnce once;
+  return once.run([] {
+    cudaError_t e = set_attributes<0>();
+    if (e == cudaSuccess) e = set_attributes<1>();
+    if (e == cudaSuccess) e = set_attributes<2>();
+    return e;
+  }, num_sms);
 }
 
 constexpr int64_t packed_rows(int H) { return (int64_t)H * 2 * 2 * kUC; }
@@ -726,8 +734,11 @@ cudaError_t launch_pack_gate_weights_f16(const void* wx, const void* wa, int H, 
 ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H) {
   const Layout L = layout(B, T, (int64_t)H * kHW);
   ChanPrep p;
+  int num_sms = 0;
+  if (device_setup(&num_sms) != cudaSuccess) return p;
   p.zero = reinterpret_cast<uint4*>(static_cast<char*>(ws) + L.incl_off);
   p.n_zero = L.n_words * 24 / 16;
+  p.early = 2 * ((T + kUT - 1) / kUT * B * H) <= num_sms;
   return p;
 }
 
@@ -737,21 +748,15 @@ cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const vo
                              bool prepared) {
   const int E = H * kHW;
   const Layout L = layout(B, T, E);
-  static PerDeviceOnce once;
   int num_sms = 0;
-  cudaError_t err = once.run([] {
-    cudaError_t e = set_attributes<0>();
-    if (e == cudaSuccess) e = set_attributes<1>();
-    if (e == cudaSuccess) e = set_attributes<2>();
-    return e;
-  }, &num_sms);
+  cudaError_t err = device_setup(&num_sms);
   if (err != cudaSuccess) return err;
   const int64_t n_jobs = (T + kUT - 1) / kUT * B * H;     // below 2^29
   if (!prepared) {
     const ChanPrep prep = rglru_f32_prep(ws, B, T, H);
     const int64_t blocks = (prep.n_zero + 1023) / 1024;
     err = launch_dependent(rglru_f32_prepare_kernel, dim3((unsigned)(blocks < 8 * num_sms ? blocks : 8 * num_sms)),
-                           dim3(256), 0, s, prep.zero, prep.n_zero, (int)(2 * n_jobs <= num_sms));
+                           dim3(256), 0, s, prep);
     if (err != cudaSuccess) return err;
   }
   const __half* hi = static_cast<const __half*>(packed_w);
