@@ -54,7 +54,8 @@ enum { RGK_I32 = 0, RGK_I64 = 1 };
 
 /* Which kernels a composed call may use for the block-diagonal gate projections. */
 enum {
-  RGK_GATES_AUTO = 0,    /* the fastest kernel that covers the shape (see below) */
+  RGK_GATES_AUTO = 0,    /* the fastest kernel that covers the shape (see below; float32 with head width 256: gates,
+                            gate arithmetic and scan in one kernel on three float16 products) */
   RGK_GATES_SIMT = 1,    /* CUDA-core gate kernel, then the scan kernel (any head width that is a
                             multiple of 16; float32 or bfloat16) */
   RGK_GATES_TCGEN05 = 2, /* tensor-core gate kernel, then the scan kernel (head width 256: bfloat16,
@@ -164,7 +165,7 @@ typedef struct rgk_params {
 
 /* ------------------------------------------------------------------------------------------------
  * K-major copy of the two gate weights for the tcgen05 kernels (head width 256 only; for float32
- * the hi and lo halves of the 3xTF32 split): rgk_gate_pack_bytes_for(H, dtype) bytes
+ * the halves of the 3xTF32 split and those of the float16 one): rgk_gate_pack_bytes_for(H, dtype) bytes
  * (rgk_gate_pack_bytes(H) = the bfloat16 size), written once per weight update and passed as
  * rgk_params.gates_packed afterwards, with parameters of the same dtype (saves a repack per call;
  * matters for decode steps and short sequences).

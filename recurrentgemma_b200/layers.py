@@ -253,7 +253,7 @@ class RGLRU(nn.Module):
 
   def _packed_gates(self) -> Optional[int]:
     """Device pointer of the K-major copy of the gate weights the tcgen05 kernels read (bfloat16,
-    or the hi / lo halves of the float32 weights for the 3xTF32 kernel), rebuilt
+    or the halves of the float32 weights for the TF32 and float16 kernels), rebuilt
     whenever either weight tensor is replaced or modified in place (a derived, non-persistent
     buffer: it never enters the state_dict).  Writes through `.data` bypass the version counter:
     call `invalidate_packed()` after them."""
