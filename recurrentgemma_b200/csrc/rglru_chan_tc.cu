@@ -13,8 +13,9 @@
 // produces a carry has normally finished one round before the unit that consumes it starts.
 //
 // Roles in a CTA (20 warps, two of them idle where the kernel does not convolve):
-//   producer  one thread: per K-slice of 64 the conv-output tile (128 tokens x 64, operand B) and the
-//             packed gate weights (256 gate rows x 64, operand A) by TMA into a 3-stage ring;
+//   producer  one warp, an elected lane of which issues: per K-slice of 64 the conv-output tile (128
+//             tokens x 64, operand B) and the packed gate weights (256 gate rows x 64, operand A) by
+//             TMA into a 3-stage ring;
 //   MMA       one warp, an elected lane of which issues: per K-step two tcgen05.mma M128 N128 (x-gate
 //             rows, a-gate rows) into one of two TMEM accumulator sets (2 x 128 columns each);
 //   epilogue  16 warps = 4 channel quarters (the warp's TMEM lane quarter) x 4 token quarters.
@@ -35,12 +36,13 @@
 //           record) and publishes the tile's own; second named barrier unless the state was known
 // -> recurrence in registers, join, 16-byte stores into the output tile.
 //
-// What bounds it is instruction issue: 38 warp instructions for 32 elements (32 without a join, 48 with maps and
-// a join), 68 % of the issue slots, with four epilogue warps a scheduler.  Stripped of every memory access the
-// arithmetic alone takes 105 of 124 us at 8 x 4096 tokens without a join.  There: 151 us as look-back over maps
+// What bounds it is instruction issue, with four epilogue warps a scheduler: 38 warp instructions for 32 elements
+// (32 without a join, 48 with maps and a join) and 68 % of the issue slots before the last step below.  Stripped of
+// every memory access the arithmetic alone takes 105 us at 8 x 4096 tokens without a join.  There: 151 us as look-back over maps
 // for every call -> 136 without maps where chains are many -> 134 with the MMA loop on a whole warp -> 129 with
 // 112 instead of 96 registers for the epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with
-// table addresses in one instruction and waits that are asked once ahead of their loop.  The recurrent path
+// table addresses in one instruction and waits that are asked once ahead of their loop -> 121 with the warp's own
+// coordinates and barriers in uniform registers (8 x 4096 tokens with a join and the conv 232 -> 226).  The path
 // 243 -> 209 us, 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a
 // tile).  Weights at rest in tensor memory instead of streamed took as long a unit: loads are not the bound.
 // All waits (mbarriers, look-back flags) are bounded; on expiry WsHeader::status is raised, the
@@ -321,7 +323,11 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // The warp's number comes from a lane, so that the compiler knows it to be the same in all of them: barriers,
+  // addresses and coordinates are then in uniform registers, and the copies are issued under elect_one, which keeps
+  // them there, instead of by a lane in a branch of its own.  8 x 4096 tokens without a join, us: elect_one alone
+  // 124.9 -> 123.3, with the shuffle 120.7.
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tiles_t = (T_ + kUT - 1) / kUT;
   const int per_tt = B * groups;                         // units per time tile
   const int n_my = (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -359,27 +365,30 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
   if constexpr (!kConv) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
   if (warp == kEpi) {
     // ------------------------------ TMA producer of the MMA operands ------------------------------
-    if (lane == 0) {
-      unsigned it = 0;
-      bool ok = true;
-      for (int t = 0; t < n_my && ok; ++t) {
-        const int u = blockIdx.x + t * gridDim.x;
-        const int tt = u / per_tt, rem = u - tt * per_tt;
-        const int b = rem / groups, grp = rem - b * groups;
-        for (int kb = 0; kb < kKBlocks; ++kb, ++it) {
-          if constexpr (kConv) {
-            // the input rows of this K-slice for the conv warps (rows before the sequence and past
-            // its end read as zero: the first coordinate may be negative)
-            const int xs = it & 1;
-            ok = mbar_wait(bar_xs_empty(xs), ((it >> 1) & 1) ^ 1, s_abort);
-            if (!ok) break;
+    // (the whole warp runs the loop, one elected lane issues: as the MMA warp)
+    unsigned it = 0;
+    bool ok = true;
+    for (int t = 0; t < n_my && ok; ++t) {
+      const int u = blockIdx.x + t * gridDim.x;
+      const int tt = u / per_tt, rem = u - tt * per_tt;
+      const int b = rem / groups, grp = rem - b * groups;
+      for (int kb = 0; kb < kKBlocks; ++kb, ++it) {
+        if constexpr (kConv) {
+          // the input rows of this K-slice for the conv warps (rows before the sequence and past
+          // its end read as zero: the first coordinate may be negative)
+          const int xs = it & 1;
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_xs_empty(xs), ((it >> 1) & 1) ^ 1, s_abort));
+          if (!ok) break;
+          if (elect_one()) {
             mbar_expect_tx(bar_xs_full(xs), kXBytes);
             tma_load_3d(s_base + kOffXs + xs * kXStage, &map_c, (grp >> 1) * kHW + kb * kKB, tt * kUT - 3,
                         b, bar_xs_full(xs));
           }
-          const int s = it % kR;
-          ok = mbar_wait(bar_empty(s), ((it / kR) & 1) ^ 1, s_abort);
-          if (!ok) break;
+        }
+        const int s = it % kR;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_empty(s), ((it / kR) & 1) ^ 1, s_abort));
+        if (!ok) break;
+        if (elect_one()) {
           if constexpr (kConv) {
             mbar_expect_tx(bar_full(s), kWBytes);
           } else {
@@ -390,6 +399,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
           tma_load_2d(s_base + kOffRing + s * kStage + kCBytes, &map_w, kb * kKB, grp * 2 * kUC,
                       bar_full(s));
         }
+        __syncwarp();
       }
     }
   } else if (warp == kEpi + 1) {
@@ -658,7 +668,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
           __syncwarp();
           if constexpr (kConv) {
             if (lane == 0) mbar_arrive(bar_cfree);   // the conv warps may write the next unit's tile
-          } else if (lane == 0 && t + 1 < n_my) {
+          } else if (t + 1 < n_my && elect_one()) {
             mbar_expect_tx(bar_ct(warp), kSubBytes);
             tma_load_3d(tile_c_s, &map_ct, chan0(nxt), nxt.tt * kUT + tq * kSub, nxt.b, bar_ct(warp));
           }
@@ -674,7 +684,7 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
         if (half == 0) {
           // the previous unit's output tile must have been read by its store before the buffer is
           // written again; then the other branch's tile of this unit is fetched into it
-          if (lane == 0) {
+          if (elect_one()) {
             bulk_wait_read();
             if constexpr (kJoin != 0) {
               mbar_expect_tx(bar_yt(warp), kSubBytes);
@@ -841,14 +851,14 @@ rglru_chan_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_consta
       transpose_tile(tile_y_s + row_off, tile_y_s + st_off);
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         tma_store_3d(&map_ot, e0, tok0, b, tile_y_s);
         bulk_commit();
       }
       cur = nxt;
       resets = resets_next;
     }
-    if (lane == 0) bulk_wait_all();
+    if (elect_one()) bulk_wait_all();
   }
 
   tc_fence_before();
