@@ -21,8 +21,8 @@
 // Roles in a CTA (24 warps, two of them idle):
 //   split     4 warps: the scale of each token (a pass over the head's 256 channels), then per K-slice of 64 the two
 //             halves of the activations into the operand tiles (128-byte swizzle), as the tensor core releases them;
-//   producer  one thread: packed weights, per K-slice and gate the two halves (128 rows x 64, 16 KiB each) by TMA
-//             through a ring of five;
+//   producer  one warp, an elected lane of which issues: packed weights, per K-slice and gate the two halves (128
+//             rows x 64, 16 KiB each) by TMA through a ring of five;
 //   MMA       one warp, an elected lane of which issues tcgen05.mma kind::f16 M128 N128 into one of two accumulator
 //             sets (x-gate and a-gate columns, 2 x 128 each);
 //   epilogue  two groups of 8 warps, a group an accumulator set, so that one's waits lie under the other's arithmetic;
@@ -36,8 +36,8 @@
 // weights and halves share the shared memory's bandwidth) and then to its epilogue group for 18,000 (12,500 in pass one,
 // 2,500 to 4,000 until the state is there, 3,500 in pass two), and there is room for two sets: 15,500 a unit.  67 warp
 // instructions for 32 elements without a join, 54 % of the issue slots.  Width 2560, float32, us as gate and
-// scan kernels with a and the normalised input through memory / this: 2 x 1024 tokens 64 / 34, 5001 tokens 150 / 61,
-// 8 x 4096 730 / 329, 16 tokens 19 / 12; with Conv1D and join 1500 tokens 64 / 36, 4 x 4000 458 / 286.  With one
+// scan kernels with a and the normalised input through memory / this: 2 x 1024 tokens 64 / 32, 5001 tokens 150 / 57,
+// 8 x 4096 730 / 329, 16 tokens 19 / 12; with Conv1D and join 1500 tokens 64 / 36, 4 x 4000 458 / 276.  With one
 // epilogue group of eight warps 2 x 1024 tokens took 42.  Distance of the 2-norm from a 64-bit evaluation: 9.5e-7 /
 // 5.6e-7 at 2 x 1024 tokens, and the smaller one at every size and magnitude compared.
 //
@@ -241,7 +241,10 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (from a lane, so that the compiler knows it to be the same in the whole warp: barriers, addresses and what the
+  // loops run over are then in uniform registers.  With the weights' loop on its whole warp, us: 2 x 1024 tokens 33.9
+  // -> 31.7, 8 x 4096 tokens 348..358 -> 332..355, 1 x 300 tokens 18.2 -> 16.8)
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tiles_t = (T_ + kUT - 1) / kUT;
   const Jobs jobs(n_jobs, B * heads, heads);
   const int n_my = jobs.count();
@@ -340,23 +343,25 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
     if (warp == kEpi + kSplit) {
     // ------------------------------ weights ---------------------------------------------------------
-    if (lane == 0) {
-      bool ok = true;
-      int s = 0;
-      uint32_t phase = 1;
-      for (int j = 0; j < n_my && ok; ++j) {
-        int tt, b, head, half, n;
-        jobs.get(j, tt, b, head, half, n);
-        for (int u = 0; u < n && ok; ++u) {
-          const int row = (head * 2 + half + u) * 2 * kUC;
-          for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
-            ok = mbar_wait(bar_w_empty(s), phase, s_abort);
-            if (!ok) break;
+    // (the whole warp runs the loop, one elected lane issues: as the MMA warp)
+    bool ok = true;
+    int s = 0;
+    uint32_t phase = 1;
+    for (int j = 0; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      for (int u = 0; u < n && ok; ++u) {
+        const int row = (head * 2 + half + u) * 2 * kUC;
+        for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_w_empty(s), phase, s_abort));
+          if (!ok) break;
+          if (elect_one()) {
             mbar_expect_tx(bar_w_full(s), kWPart);
             tma_load_2d(s_base + kOffRing + s * kWPart, (i & 1) ? &map_wl : &map_wh, (i >> 2) * kKB,
                         row + ((i >> 1) & 1) * kUC, bar_w_full(s));
-            if (++s == kRing) { s = 0; phase ^= 1; }
           }
+          __syncwarp();
+          if (++s == kRing) { s = 0; phase ^= 1; }
         }
       }
     }
