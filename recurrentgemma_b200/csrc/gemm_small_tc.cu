@@ -123,7 +123,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + a.bar_off + kOffTmemS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + a.bar_off + kOffAbortS);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (from a lane, so that the compiler knows it to be the same in the whole warp; with it the first copies, too, are
+  // issued under elect_one: a block's decode step of 64 rows 106.1 -> 105.1 us)
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int F = a.F, R = a.R, splits = a.splits, n_stages = a.n_stages;
   const int split = splits > 1 ? (int)cluster_rank() : 0;   // cluster = (1, splits, 1)
   // the matrix this feature tile belongs to, its first feature there, the rows of x of this CTA
@@ -142,7 +144,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const int rpr = a.rows_per_rank, stride = a.row_stride;
   const uint32_t block_bytes = (uint32_t)(F * stride) * 4;   // partial sums of one rank's rows
 
-  if (warp == kEpiS && lane == 0) {
+  if (warp == kEpiS && elect_one()) {
     *s_abort = 0;
     for (int s = 0; s < n_stages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
     mbar_init(bar_acc, 1);
@@ -186,7 +188,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
   if (warp == kEpiS) {
     // ------------------------------ TMA producer --------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       for (int i = 0; i < pre; ++i) {
         if (!a.early) {
           mbar_expect_tx(bar_full(i), stage_bytes);
