@@ -36,9 +36,9 @@
 //           record) and publishes the tile's own; second named barrier unless the state was known
 // -> recurrence in registers, join, 16-byte stores into the output tile.
 //
-// What bounds it is instruction issue, with four epilogue warps a scheduler: 38 warp instructions for 32 elements
-// (32 without a join, 48 with maps and a join) and 68 % of the issue slots before the last step below.  Stripped of
-// every memory access the arithmetic alone takes 105 us at 8 x 4096 tokens without a join.  There: 151 us as look-back over maps
+// What bounds it is instruction issue, with four epilogue warps a scheduler: 36 warp instructions for 32 elements (30
+// without a join), 68 % of the issue slots.  Stripped of every memory access the arithmetic alone took 105 us of 124
+// at 8 x 4096 tokens without a join.  There: 151 us as look-back over maps
 // for every call -> 136 without maps where chains are many -> 134 with the MMA loop on a whole warp -> 129 with
 // 112 instead of 96 registers for the epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with
 // table addresses in one instruction and waits that are asked once ahead of their loop -> 121 with the warp's own

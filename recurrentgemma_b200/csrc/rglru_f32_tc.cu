@@ -35,7 +35,8 @@
 // What bounds it: an accumulator set belongs to the tensor core for 11,000 cycles (6,144 of instructions: operands,
 // weights and halves share the shared memory's bandwidth) and then to its epilogue group for 18,000 (12,500 in pass one,
 // 2,500 to 4,000 until the state is there, 3,500 in pass two), and there is room for two sets: 15,500 a unit.  67 warp
-// instructions for 32 elements without a join, 54 % of the issue slots.  Width 2560, float32, us as gate and
+// instructions for 32 elements without a join, 54 % of the issue slots.  (Cycles and instructions before the warp's
+// number was uniform, which took 5 to 7 % off the calls up to 5001 tokens.)  Width 2560, float32, us as gate and
 // scan kernels with a and the normalised input through memory / this: 2 x 1024 tokens 64 / 32, 5001 tokens 150 / 57,
 // 8 x 4096 730 / 329, 16 tokens 19 / 12; with Conv1D and join 1500 tokens 64 / 36, 4 x 4000 458 / 276.  With one
 // epilogue group of eight warps 2 x 1024 tokens took 42.  Distance of the 2-norm from a 64-bit evaluation: 9.5e-7 /
