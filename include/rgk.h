@@ -55,7 +55,8 @@ enum { RGK_I32 = 0, RGK_I64 = 1 };
 /* Which kernels a composed call may use for the block-diagonal gate projections. */
 enum {
   RGK_GATES_AUTO = 0,    /* the fastest kernel that covers the shape (see below; float32 with head width 256: gates,
-                            gate arithmetic and scan in one kernel on three float16 products) */
+                            gate arithmetic and scan in one kernel on three float16 products, where a token's values
+                            span too wide a range for those float32 dot products, which are slow) */
   RGK_GATES_SIMT = 1,    /* CUDA-core gate kernel, then the scan kernel (any head width that is a
                             multiple of 16; float32 or bfloat16) */
   RGK_GATES_TCGEN05 = 2, /* tensor-core gate kernel, then the scan kernel (head width 256: bfloat16,

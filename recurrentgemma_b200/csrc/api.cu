@@ -171,8 +171,10 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
       cudaError_t e = rgk::launch_pack_gate_weights_f16(p->gate_x_w, p->gate_a_w, H, wpack, s);
       if (e != cudaSuccess) return cuda_fail(e, "pack_gate_weights launch");
     }
-    cudaError_t e = rgk::launch_rglru_f32(c, pos, pos64, p->a_param, p->gate_x_b, p->gate_a_b, packed, h0, yb,
-                                          y_activated, B, T, H, out, h_last, scan_ws, s, xb != nullptr);
+    cudaError_t e = rgk::launch_rglru_f32(c, pos, pos64, p->a_param, p->gate_x_w, p->gate_x_b, p->gate_a_w,
+                                          p->gate_a_b, packed, h0, yb, y_activated, B, T, H,
+                                          static_cast<float*>(a_buf), static_cast<float*>(xn_buf), out, h_last,
+                                          scan_ws, s, xb != nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "float32 RG-LRU launch");
     return RGK_OK;
   }

@@ -6,9 +6,15 @@
 // of its token (over the 256 channels of the head) and w by one of its output channel, so that the largest
 // magnitude lies in [2^14, 2^15),
 //     x w  ~  x1 w1 + x2 w1 + x1 w2,      v1 = fp16(v),  v2 = fp16(v - v1)
-// with float32 accumulation.  What is dropped is 2^-22 of a product (2^-40 of the largest one where a factor is
-// below 2^-18 of its row's largest); the scales are exact and undone in the epilogue.  As three TF32 products
+// with float32 accumulation.  What is dropped is 2^-22 of a product, and 2^-39 of the row's largest factor where a
+// factor is below 2^-17 of that; the scales are exact and undone in the epilogue.  As three TF32 products
 // (gates_tf32.cu) the dropped part is up to 2^-20, an operand twice the bytes, and an instruction half as fast.
+// TF32 keeps an exponent for each value, though, and halves under a common scale do not.  Where what they drop beyond
+// 2^-22 could move the argument of any gate of the head by more than 2^-23, and by more than 2^-22 of the sum of its
+// terms' magnitudes, the token's gates are float32 dot products on the CUDA cores instead (wide_tokens, exact_tokens).
+// With N(0, 1/256) weights no token is looked at below a magnitude of some thousand, and normal data of any magnitude
+// stay on the tensor cores: 2 x 1024 tokens of width 2560 33 us, 43 where all are looked at.  Where all are recomputed,
+// one input channel 1e8 times the others and its weights as much smaller, they take 1.2 ms.
 //
 // Accumulators are channel-major, D[channel, token] = W[channel, k] . X[token, k]^T: a TMEM lane is a channel, its
 // columns are tokens, and a thread walks its channel's tokens in time order.  A global access of a warp is one
@@ -20,7 +26,8 @@
 //
 // Roles in a CTA (24 warps, two of them idle):
 //   split     4 warps: the scale of each token (a pass over the head's 256 channels), then per K-slice of 64 the two
-//             halves of the activations into the operand tiles (128-byte swizzle), as the tensor core releases them;
+//             halves of the activations into the operand tiles (128-byte swizzle), as the tensor core releases them, and
+//             ahead of the last slice's release the gates of tokens that are not left to the halves;
 //   producer  one warp, an elected lane of which issues: packed weights, per K-slice and gate the two halves (128
 //             rows x 64, 16 KiB each) by TMA through a ring of five;
 //   MMA       one warp, an elected lane of which issues tcgen05.mma kind::f16 M128 N128 into one of two accumulator
@@ -79,8 +86,9 @@ constexpr int kBatch = 8;                // tokens between two loads from tensor
 constexpr int kOffX = 0;                                         // [slice][half]
 constexpr int kOffRing = kOffX + kKBlocks * 2 * kXPart;
 constexpr int kScaleBufs = 4;
-constexpr int kOffScale = kOffRing + kRing * kWPart;             // float [job & 3][token]: 1 / scale
-constexpr int kOffMap = kOffScale + kScaleBufs * kUT * 4;        // float2 [group][channel]: map of the first half
+constexpr int kOffScale = kOffRing + kRing * kWPart;             // float [job & 3][token]: 1 / scale, < 0: not trusted
+constexpr int kOffWide = kOffScale + kScaleBufs * kUT * 4;       // bit [job & 3][token]: gates not left to the halves
+constexpr int kOffMap = kOffWide + kScaleBufs * kUT / 8;         // float2 [group][channel]: map of the first half
 constexpr int kOffBar = kOffMap + 2 * kUC * 8;                   // ring full, empty; slice full, empty; sets full, empty
 constexpr int kNumBar = 2 * kRing + 2 * kKBlocks + 4;
 constexpr int kOffTmem = kOffBar + kNumBar * 8;
@@ -131,6 +139,187 @@ __device__ __forceinline__ uint32_t largest(const float4& a, const float4& b) {
   const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
                         fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
   return __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+}
+
+// How far the halves of activations and weights may move a gate's argument, beyond 2^-22 of its terms.
+constexpr float kAllowed = 0x1p-23f;
+
+// What the halves of a value under its row's scale drop, beyond 2^-22 of it.
+__device__ __forceinline__ float dropped(float v) {
+  const float hi = __half2float(__float2half_rn(v));
+  const float rest = v - hi;
+  return fmaxf(fabsf(rest - __half2float(__float2half_rn(rest))) - 0x1p-22f * fabsf(v), 0.0f);
+}
+
+// What the packing kernel says of 32 rows of weights, as bits.
+struct WeightRange {
+  uint32_t limit;                          // smallest over the rows: a token's largest magnitude up to which it is trusted
+  uint32_t lost;                           // largest over the rows: sum of what the halves drop
+  uint32_t largest;
+  uint32_t pad;
+};
+constexpr int kRangesHead = 2 * 2 * kUC / 32;
+// (from 2^113 on the products overflow before the scales are undone)
+constexpr float kTopLimit = 0x1p100f;
+
+// Which of the tokens in `tokens` (bit i: token i behind x0, of stride E) really lose too much, by themselves and against
+// the least that |x| . |w| can be.  x0: the lane's first four values of the first token, the other four 128 behind;
+// least: the smallest weight of each of these channels, by blocks of 32 rows.
+__device__ __forceinline__ uint32_t wide_tokens(const float* x0, int E, uint32_t tokens, const WeightRange* range,
+                                                const float* least, int lane) {
+  const WeightRange r = range[lane & (kRangesHead - 1)];
+  const float lost = __uint_as_float(__reduce_max_sync(0xffffffffu, r.lost));
+  const float weight = __uint_as_float(__reduce_max_sync(0xffffffffu, r.largest));
+  float4 m[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    m[q] = *reinterpret_cast<const float4*>(least + q * 128);
+#pragma unroll 5
+    for (int i = 1; i < kRangesHead; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(least + i * kHW + q * 128);
+      m[q] = make_float4(fminf(m[q].x, v.x), fminf(m[q].y, v.y), fminf(m[q].z, v.z), fminf(m[q].w, v.w));
+    }
+  }
+  uint32_t wide = 0u;
+#pragma unroll 1
+  while (tokens != 0u) {
+    int at[4];                                           // (the last one again where fewer are left)
+    float moved[4], product[4], top[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      at[i] = tokens != 0u ? __ffs(tokens) - 1 : at[i > 0 ? i - 1 : 0];
+      tokens &= tokens - 1u;
+      const float* p = x0 + (int64_t)at[i] * E;
+      const float4 v[2] = {*reinterpret_cast<const float4*>(p), *reinterpret_cast<const float4*>(p + 128)};
+      const uint32_t t = largest(v[0], v[1]);
+      const float s = scale_of(t);
+      top[i] = __uint_as_float(t);
+      moved[i] = product[i] = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        moved[i] += dropped(v[q].x * s) + dropped(v[q].y * s) + dropped(v[q].z * s) + dropped(v[q].w * s);
+        product[i] += fabsf(v[q].x) * m[q].x + fabsf(v[q].y) * m[q].y + fabsf(v[q].z) * m[q].z + fabsf(v[q].w) * m[q].w;
+      }
+      moved[i] *= inverse_scale_of(t) * weight;
+    }
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        moved[i] += __shfl_xor_sync(0xffffffffu, moved[i], j);
+        product[i] += __shfl_xor_sync(0xffffffffu, product[i], j);
+      }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (!(fmaf(top[i], lost, moved[i]) <= fmaxf(kAllowed, 0x1p-22f * product[i])) || !(top[i] <= kTopLimit))
+        wide |= 1u << at[i];
+  }
+  return wide;
+}
+
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 c, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// The gates' arguments (without bias) of the tokens of `wide`, as float32 dot products with the weights as they are
+// given, to zx and za (stride E as x; all three at token 0's values of the head).  A lane has eight channels of a gate at
+// a time, four tokens share the weights' loads, and sums are added up by quarters, which rounds less.  (mine: of a head
+// that two CTAs share, the lanes of each with its own channels write.)  A call, and with the roles in the order in
+// which a short call needs their instructions: inlined between them 16 tokens with Conv1D took 15.0 us, not 13.9.
+__device__ __noinline__ void exact_tokens(const float* x, int E, uint32_t wide, const float* wx, const float* wa,
+                                          float* zx, float* za, bool mine, int lane) {
+  constexpr int kTokens = 4, kQuarter = kHW / 4;
+#pragma unroll 1
+  while (wide != 0u) {
+    int at[kTokens];
+    const int n = __popc(wide);
+#pragma unroll
+    for (int i = 0; i < kTokens; ++i) {                  // (the last one again where fewer are left)
+      at[i] = wide != 0u ? (__ffs(wide) - 1) * E : at[i > 0 ? i - 1 : 0];
+      wide &= wide - 1u;
+    }
+#pragma unroll 1
+    for (int pass = 0; pass < 8; ++pass) {               // gate, quarter
+      const int k0 = (pass & 3) * kQuarter;
+      const float* w = (pass < 4 ? wx : wa) + (int64_t)k0 * kHW + lane * 8;
+      float* z = (pass < 4 ? zx : za) + lane * 8;
+      float2 sum[kTokens][4];
+#pragma unroll
+      for (int i = 0; i < kTokens; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum[i][q] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+      for (int k = 0; k < kQuarter; k += 32) {
+        float v[kTokens];
+#pragma unroll
+        for (int i = 0; i < kTokens; ++i) v[i] = x[at[i] + k0 + k + lane];
+#pragma unroll 4
+        for (int kk = 0; kk < 32; ++kk) {
+          const float4 w0 = *reinterpret_cast<const float4*>(w + (k + kk) * kHW);
+          const float4 w1 = *reinterpret_cast<const float4*>(w + (k + kk) * kHW + 4);
+#pragma unroll
+          for (int i = 0; i < kTokens; ++i) {
+            const float xv = __shfl_sync(0xffffffffu, v[i], kk);
+            const float2 x2 = make_float2(xv, xv);
+            sum[i][0] = fma2(x2, make_float2(w0.x, w0.y), sum[i][0]);
+            sum[i][1] = fma2(x2, make_float2(w0.z, w0.w), sum[i][1]);
+            sum[i][2] = fma2(x2, make_float2(w1.x, w1.y), sum[i][2]);
+            sum[i][3] = fma2(x2, make_float2(w1.z, w1.w), sum[i][3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kTokens; ++i) {
+        if (i >= n || !mine) break;
+        float4* p = reinterpret_cast<float4*>(z + at[i]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float4 v = make_float4(sum[i][2 * q].x, sum[i][2 * q].y, sum[i][2 * q + 1].x, sum[i][2 * q + 1].y);
+          if ((pass & 3) != 0) {
+            const float4 before = p[q];
+            v = make_float4(before.x + v.x, before.y + v.y, before.z + v.z, before.w + v.w);
+          }
+          p[q] = v;
+        }
+      }
+    }
+  }
+}
+
+// v / (s0 s1), powers of two whose product or quotients may be out of range.
+__device__ __forceinline__ uint32_t unscaled(float v, float s0, float s1) {
+  return __float_as_uint(scalbnf(v, -(ilogbf(s0) + ilogbf(s1))));
+}
+
+// These arguments of a channel per lane (zx, za: at token 0) into the accumulators, under the scales (token_scale, and
+// the channel's two rows) that the epilogue undoes.  (A call, so that nothing of it is in the way of the other tokens.)
+__device__ __noinline__ void place_tokens(const float* zx, const float* za, int E, uint32_t wide,
+                                          const float* token_scale, float scale_x, float scale_a, uint32_t taddr) {
+#pragma unroll 1
+  while (wide != 0u) {
+    int at[4];                                           // (the last one again where fewer are left)
+    float vx[4], va[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      at[i] = wide != 0u ? __ffs(wide) - 1 : at[i > 0 ? i - 1 : 0];
+      wide &= wide - 1u;
+      vx[i] = zx[(int64_t)at[i] * E];
+      va[i] = za[(int64_t)at[i] * E];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float s = token_scale[at[i]];
+      tc_st_32x1(taddr + at[i], unscaled(vx[i], s, scale_x));
+      tc_st_32x1(taddr + kUT + at[i], unscaled(va[i], s, scale_a));
+    }
+  }
+  tc_wait_st();
 }
 
 // gelu_tanh(z) = z sigmoid(2 u), u = sqrt(2 / pi) (z + 0.044715 z^3), on the hardware exponential and reciprocal: no
@@ -223,8 +412,9 @@ __device__ __forceinline__ float look_back(const unsigned long long* agg, const 
 template <int kJoin>
 __global__ void __launch_bounds__(kThreads, 1)
 rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl,
-                 const float* __restrict__ scale, const float* c, const void* pos, int pos64,
-                 const float* __restrict__ a_param, const float* __restrict__ bias_x,
+                 const float* __restrict__ scale, const WeightRange* ranges, const float* least,
+                 const float* wx, const float* wa, float* zx_wide, float* za_wide, const float* c, const void* pos,
+                 int pos64, const float* __restrict__ a_param, const float* __restrict__ bias_x,
                  const float* __restrict__ bias_a, const float* h0, const float* yb, int B, int T_, int E, int heads,
                  int n_jobs, float* out, float* h_last, WsHeader* hdr, unsigned long long* agg,
                  unsigned long long* incl) {
@@ -239,6 +429,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   auto bar_acc_full = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + s); };
   auto bar_acc_empty = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + 2 + s); };
   float* s_scale = reinterpret_cast<float*>(smem + kOffScale);
+  uint32_t* s_wide = reinterpret_cast<uint32_t*>(smem + kOffWide);
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
@@ -268,160 +459,12 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   const uint32_t tmem_base = *s_tmem;
   grid_dependency_wait();
 
-  if (warp >= kEpi && warp < kEpi + kSplit) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsSplit) : "memory");
-    // ------------------------------ activations: scales and halves ----------------------------------
-    const int w0 = (warp - kEpi) * 32;                   // first of the warp's 32 tokens
-    bool ok = true;
-    // (the first job's activations are the epilogue warps' work, who have nothing else to do yet)
-    named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
-    if (lane == 0 && n_my > 0)
-      for (int kb = 0; kb < kKBlocks; ++kb) mbar_arrive(bar_x_full(kb));
-    for (int j = 1; j < n_my && ok; ++j) {
-      int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
-      const int tok0 = tt * kUT + w0;
-      const int live = T_ - tok0;                        // tokens of the warp inside the sequence (may be < 1)
-      const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW;
-      uint32_t top = 0u;                                 // bits of the largest magnitude of token `lane`
-#pragma unroll 1
-      for (int i0 = 0; i0 < 32; i0 += 8) {
-        float4 v[8][2];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i0 + i < live)
-              v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(i0 + i) * E + q * 128 + lane * 4);
-          }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t all = largest(v[i][0], v[i][1]);
-          if (lane == i0 + i) top = all;
-        }
-      }
-      // (four buffers: the job whose scales were here has passed the epilogue.  Its last unit's accumulators
-      // were read before the set could be written for the unit two behind, of a job at most two behind, whose
-      // slices were released before this job's scales are looked for.)
-      s_scale[(j & (kScaleBufs - 1)) * kUT + w0 + lane] = inverse_scale_of(top);
-      const float factor = scale_of(top);
-      const int r = lane >> 3, p = lane & 7;
-#pragma unroll 1
-      for (int kb = 0; kb < kKBlocks; ++kb) {
-        float4 v[8][2];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (4 * i + r < live)
-              v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(4 * i + r) * E + kb * kKB + p * 8 + q * 4);
-          }
-        ok = mbar_wait(bar_x_empty(kb), (j & 1) ^ 1, s_abort);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        uint8_t* hi_tile = smem + kOffX + kb * 2 * kXPart;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = w0 + 4 * i + r;
-          const float s = __shfl_sync(0xffffffffu, factor, 4 * i + r);
-          uint4 hi, lo;
-          split_pair(v[i][0].x * s, v[i][0].y * s, hi.x, lo.x);
-          split_pair(v[i][0].z * s, v[i][0].w * s, hi.y, lo.y);
-          split_pair(v[i][1].x * s, v[i][1].y * s, hi.z, lo.z);
-          split_pair(v[i][1].z * s, v[i][1].w * s, hi.w, lo.w);
-          const int at = row * 128 + ((p ^ (row & 7)) << 4);
-          *reinterpret_cast<uint4*>(hi_tile + at) = hi;
-          *reinterpret_cast<uint4*>(hi_tile + kXPart + at) = lo;
-        }
-        fence_proxy_async();                             // the tensor core reads this through the async proxy
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_x_full(kb));
-      }
-    }
-  } else if (warp >= kEpi + kSplit) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
-    if (warp == kEpi + kSplit) {
-    // ------------------------------ weights ---------------------------------------------------------
-    // (the whole warp runs the loop, one elected lane issues: as the MMA warp)
-    bool ok = true;
-    int s = 0;
-    uint32_t phase = 1;
-    for (int j = 0; j < n_my && ok; ++j) {
-      int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
-      for (int u = 0; u < n && ok; ++u) {
-        const int row = (head * 2 + half + u) * 2 * kUC;
-        for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
-          ok = __all_sync(0xffffffffu, mbar_wait(bar_w_empty(s), phase, s_abort));
-          if (!ok) break;
-          if (elect_one()) {
-            mbar_expect_tx(bar_w_full(s), kWPart);
-            tma_load_2d(s_base + kOffRing + s * kWPart, (i & 1) ? &map_wl : &map_wh, (i >> 2) * kKB,
-                        row + ((i >> 1) & 1) * kUC, bar_w_full(s));
-          }
-          __syncwarp();
-          if (++s == kRing) { s = 0; phase ^= 1; }
-        }
-      }
-    }
-  } else if (warp == kEpi + kSplit + 1) {
-    // ------------------------------ MMA issue -------------------------------------------------------
-    // (the whole warp runs the loop, one elected lane issues: see mma_ring)
-    const uint64_t desc_x = smem_desc_sw128(s_base + kOffX), desc_w = smem_desc_sw128(s_base + kOffRing);
-    bool ok = true;
-    int s = 0, t = 0;
-    uint32_t phase = 0;
-    for (int j = 0; j < n_my && ok; ++j) {
-      int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
-      for (int u = 0; u < n && ok; ++u, ++t) {
-        const int as = t & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
-        if (!ok) break;
-        tc_fence_after();
-        for (int kb = 0; kb < kKBlocks && ok; ++kb) {
-          if (u == 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_x_full(kb), j & 1, s_abort));
-            if (!ok) break;
-          }
-          const uint64_t x1 = desc_x + (uint64_t)(kb * (2 * kXPart >> 4)), x2 = x1 + (kXPart >> 4);
-          for (int g = 0; g < 2 && ok; ++g) {
-            const uint32_t d = tmem_base + (as * 2 + g) * kUT;
-#pragma unroll
-            for (int part = 0; part < 2; ++part) {
-              ok = __all_sync(0xffffffffu, mbar_wait(bar_w_full(s), phase, s_abort));
-              if (!ok) break;
-              tc_fence_after();
-              if (elect_one()) {
-                const uint64_t w = desc_w + (uint64_t)(s * (kWPart >> 4));
-#pragma unroll
-                for (int ks = 0; ks < kKB / 16; ++ks) {
-                  tc_mma_bf16(d, w + 2 * ks, x1 + 2 * ks, kIdesc, (part | kb | ks) != 0 ? 1u : 0u);
-                  if (part == 0) tc_mma_bf16(d, w + 2 * ks, x2 + 2 * ks, kIdesc, 1u);
-                }
-                tc_commit(bar_w_empty(s));
-                if (part == 1 && g == 1) {
-                  if (u == n - 1) tc_commit(bar_x_empty(kb));
-                  if (kb == kKBlocks - 1) tc_commit(bar_acc_full(as));
-                }
-              }
-              __syncwarp();
-              if (++s == kRing) { s = 0; phase ^= 1; }
-            }
-          }
-        }
-      }
-    }
-    }
-  } else {
+  if (warp < kEpi) {
     // ------------------------------ epilogue --------------------------------------------------------
     const int chq = warp & 3, th = (warp >> 2) & 1, group = warp >> 3;
     const int64_t n_state = (int64_t)B * E;
     const int64_t n_words = (int64_t)tiles_t * B * E, tile_words = (int64_t)B * E;
     (void)n_state; (void)n_words;
-    // (a, x) of a batch of tokens, from its accumulators
     constexpr float kNegLog2e = -1.4426950408889634f;
     bool ok = true;
     // ---- the first job's activations, a warp eight tokens, read once: 4 us less until the first MMA than by the
@@ -431,6 +474,9 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
       jobs.get(0, tt, b, head, half, n);
       const int w0 = warp * (kUT / kEpi), tok0 = tt * kUT + w0;
       const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW + lane * 4;
+      const WeightRange* range = ranges + head * kRangesHead;
+      const uint32_t limits = range[lane & (kRangesHead - 1)].limit;
+      uint32_t tops = 0u;                                // bits of the largest magnitude of token `lane`
 #pragma unroll 1
       for (int i0 = 0; i0 < kUT / kEpi; i0 += 4) {
         float4 v[4][2];
@@ -445,7 +491,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
           const uint32_t top = largest(v[i][0], v[i][1]);
           const float s = scale_of(top);
           const int row = w0 + i0 + i;
-          if (lane == 0) s_scale[row] = inverse_scale_of(top);
+          if (lane == i0 + i) tops = top;
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             uint2 hi, lo;
@@ -460,6 +506,10 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
         }
       }
       fence_proxy_async();
+      if (lane < kUT / kEpi) s_scale[w0 + lane] = inverse_scale_of(tops);
+      const uint32_t limit = __reduce_min_sync(0xffffffffu, limits);
+      const uint32_t wide = __ballot_sync(0xffffffffu, tops > limit && tok0 + lane < T_ && lane < kUT / kEpi);
+      if (lane == 0) reinterpret_cast<uint8_t*>(s_wide)[warp] = (uint8_t)wide;
     }
     named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
     int t = 0;
@@ -517,6 +567,13 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
         if (ok) ok = mbar_wait(bar_acc_full(as), (tu >> 1) & 1, s_abort);
         __syncwarp();
         tc_fence_after();
+        const uint2 wide = *reinterpret_cast<const uint2*>(s_wide + (j & (kScaleBufs - 1)) * (kUT / 32) + th * 2);
+        if (__builtin_expect((wide.x | wide.y) != 0u, 0)) {
+#pragma unroll 1
+          for (int q = 0; q < 2; ++q)
+            place_tokens(zx_wide + at0 + (int64_t)q * 32 * E, za_wide + at0 + (int64_t)q * 32 * E, E,
+                         q == 0 ? wide.x : wide.y, st_row + q * 32, scale[wrow], scale[wrow + kUC], t_row + q * 32);
+        }
 #pragma unroll 1
         for (int k0 = 0; k0 < end; k0 += kBatch) {
           uint32_t zx[kBatch], za[kBatch];
@@ -633,6 +690,174 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
           RGK_IN_RANGE((int64_t)b * E + e, n_state, &hdr->status))
         h_last[(int64_t)b * E + e] = h;
     }
+  } else if (warp >= kEpi + kSplit) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kRegsOther) : "memory");
+    if (warp == kEpi + kSplit) {
+    // ------------------------------ weights ---------------------------------------------------------
+    // (the whole warp runs the loop, one elected lane issues: as the MMA warp)
+    bool ok = true;
+    int s = 0;
+    uint32_t phase = 1;
+    for (int j = 0; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      for (int u = 0; u < n && ok; ++u) {
+        const int row = (head * 2 + half + u) * 2 * kUC;
+        for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_w_empty(s), phase, s_abort));
+          if (!ok) break;
+          if (elect_one()) {
+            mbar_expect_tx(bar_w_full(s), kWPart);
+            tma_load_2d(s_base + kOffRing + s * kWPart, (i & 1) ? &map_wl : &map_wh, (i >> 2) * kKB,
+                        row + ((i >> 1) & 1) * kUC, bar_w_full(s));
+          }
+          __syncwarp();
+          if (++s == kRing) { s = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == kEpi + kSplit + 1) {
+    // ------------------------------ MMA issue -------------------------------------------------------
+    // (the whole warp runs the loop, one elected lane issues: see mma_ring)
+    const uint64_t desc_x = smem_desc_sw128(s_base + kOffX), desc_w = smem_desc_sw128(s_base + kOffRing);
+    bool ok = true;
+    int s = 0, t = 0;
+    uint32_t phase = 0;
+    for (int j = 0; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      for (int u = 0; u < n && ok; ++u, ++t) {
+        const int as = t & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
+        if (!ok) break;
+        tc_fence_after();
+        for (int kb = 0; kb < kKBlocks && ok; ++kb) {
+          if (u == 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_x_full(kb), j & 1, s_abort));
+            if (!ok) break;
+          }
+          const uint64_t x1 = desc_x + (uint64_t)(kb * (2 * kXPart >> 4)), x2 = x1 + (kXPart >> 4);
+          for (int g = 0; g < 2 && ok; ++g) {
+            const uint32_t d = tmem_base + (as * 2 + g) * kUT;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar_w_full(s), phase, s_abort));
+              if (!ok) break;
+              tc_fence_after();
+              if (elect_one()) {
+                const uint64_t w = desc_w + (uint64_t)(s * (kWPart >> 4));
+#pragma unroll
+                for (int ks = 0; ks < kKB / 16; ++ks) {
+                  tc_mma_bf16(d, w + 2 * ks, x1 + 2 * ks, kIdesc, (part | kb | ks) != 0 ? 1u : 0u);
+                  if (part == 0) tc_mma_bf16(d, w + 2 * ks, x2 + 2 * ks, kIdesc, 1u);
+                }
+                tc_commit(bar_w_empty(s));
+                if (part == 1 && g == 1) {
+                  if (u == n - 1) tc_commit(bar_x_empty(kb));
+                  if (kb == kKBlocks - 1) tc_commit(bar_acc_full(as));
+                }
+              }
+              __syncwarp();
+              if (++s == kRing) { s = 0; phase ^= 1; }
+            }
+          }
+        }
+      }
+    }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsSplit) : "memory");
+    // ------------------------------ activations: scales and halves ----------------------------------
+    const int w0 = (warp - kEpi) * 32;                   // first of the warp's 32 tokens
+    bool ok = true;
+    // (the first job's activations are the epilogue warps' work, who have nothing else to do yet)
+    named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
+    const uint32_t first_wide = n_my > 0 ? s_wide[w0 >> 5] : 0u;
+    if (lane == 0 && n_my > 0)
+      for (int kb = 0; kb < kKBlocks - (first_wide != 0u ? 1 : 0); ++kb) mbar_arrive(bar_x_full(kb));
+    for (int j = first_wide != 0u ? 0 : 1; j < n_my && ok; ++j) {
+      int tt, b, head, half, n;
+      jobs.get(j, tt, b, head, half, n);
+      const int tok0 = tt * kUT + w0;
+      const int live = T_ - tok0;                        // tokens of the warp inside the sequence (may be < 1)
+      const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW;
+      const WeightRange* range = ranges + head * kRangesHead;
+      uint32_t* wide_at = s_wide + (j & (kScaleBufs - 1)) * (kUT / 32) + (w0 >> 5);
+      uint32_t wide = first_wide;                        // tokens whose gates may not be left to the halves
+      if (j > 0) {
+        const uint32_t limits = range[lane & (kRangesHead - 1)].limit;
+        uint32_t top = 0u;                               // bits of the largest magnitude of token `lane`
+#pragma unroll 1
+        for (int i0 = 0; i0 < 32; i0 += 8) {
+          float4 v[8][2];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (i0 + i < live)
+                v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(i0 + i) * E + q * 128 + lane * 4);
+            }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t all = largest(v[i][0], v[i][1]);
+            if (lane == i0 + i) top = all;
+          }
+        }
+        wide = __ballot_sync(0xffffffffu, top > __reduce_min_sync(0xffffffffu, limits) && lane < live);
+        // (four buffers: the job whose scales were here has passed the epilogue.  Its last unit's accumulators
+        // were read before the set could be written for the unit two behind, of a job at most two behind, whose
+        // slices were released before this job's scales are looked for.)
+        s_scale[(j & (kScaleBufs - 1)) * kUT + w0 + lane] = inverse_scale_of(top);
+        const float factor = scale_of(top);
+        const int r = lane >> 3, p = lane & 7;
+#pragma unroll 1
+        for (int kb = 0; kb < kKBlocks; ++kb) {
+          float4 v[8][2];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (4 * i + r < live)
+                v[i][q] = *reinterpret_cast<const float4*>(x0 + (int64_t)(4 * i + r) * E + kb * kKB + p * 8 + q * 4);
+            }
+          ok = mbar_wait(bar_x_empty(kb), (j & 1) ^ 1, s_abort);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          uint8_t* hi_tile = smem + kOffX + kb * 2 * kXPart;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int row = w0 + 4 * i + r;
+            const float s = __shfl_sync(0xffffffffu, factor, 4 * i + r);
+            uint4 hi, lo;
+            split_pair(v[i][0].x * s, v[i][0].y * s, hi.x, lo.x);
+            split_pair(v[i][0].z * s, v[i][0].w * s, hi.y, lo.y);
+            split_pair(v[i][1].x * s, v[i][1].y * s, hi.z, lo.z);
+            split_pair(v[i][1].z * s, v[i][1].w * s, hi.w, lo.w);
+            const int at = row * 128 + ((p ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(hi_tile + at) = hi;
+            *reinterpret_cast<uint4*>(hi_tile + kXPart + at) = lo;
+          }
+          fence_proxy_async();                           // the tensor core reads this through the async proxy
+          __syncwarp();
+          if (lane == 0 && kb < kKBlocks - 1) mbar_arrive(bar_x_full(kb));
+        }
+        if (!ok) break;
+      }
+      if (__builtin_expect(wide != 0u, 0)) {             // in front of the last slice, and so of the epilogue
+        const int64_t col = (int64_t)head * kHW * kHW, row0 = ((int64_t)b * T_ + tok0) * E + head * kHW;
+        wide = wide_tokens(x0 + lane * 4, E, wide, range, least + head * kRangesHead * kHW + lane * 4, lane);
+        exact_tokens(x0, E, wide, wx + col, wa + col, zx_wide + row0, za_wide + row0, n == 2 || (lane >> 4) == half,
+                     lane);
+        __threadfence_block();
+        __syncwarp();
+      }
+      if (lane == 0) {
+        *wide_at = wide;
+        mbar_arrive(bar_x_full(kKBlocks - 1));
+      }
+    }
   }
 
   tc_fence_before();
@@ -646,12 +871,15 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
 }
 
 // Gate weights [H, 256 (k), 256 (n)] float32 -> [H, 2, 256 (n'), 256 (k)] float16, first and second halves of the
-// scaled values (rows 0-127 of a group: the x-gate columns of its 128 channels, rows 128-255 the a-gate ones), and
-// 1 / scale of each row.
+// scaled values (rows 0-127 of a group: the x-gate columns of its 128 channels, rows 128-255 the a-gate ones),
+// 1 / scale of each row, and of each 32 rows the range, and the smallest weight by input channel.
 __global__ void pack_gate_weights_f16_kernel(const float* __restrict__ wx, const float* __restrict__ wa,
                                              __half* __restrict__ hi, __half* __restrict__ lo,
-                                             float* __restrict__ scale) {
+                                             float* __restrict__ scale, WeightRange* __restrict__ ranges,
+                                             float* __restrict__ least) {
   __shared__ float tile[kHW][33];                                  // [k][n']
+  __shared__ WeightRange range;
+  if (threadIdx.x == 0) range = WeightRange{__float_as_uint(kTopLimit), 0u, 0u, 0u};
   const int group = blockIdx.y, head = group >> 1, half = group & 1;
   const int n0 = blockIdx.x * 32;                                  // n' in [0, 256)
   const float* src = (n0 < kUC ? wx : wa) + (int64_t)head * kHW * kHW + half * kUC + (n0 % kUC);
@@ -665,14 +893,38 @@ __global__ void pack_gate_weights_f16_kernel(const float* __restrict__ wx, const
     m = __reduce_max_sync(0xffffffffu, m);
     const float s = scale_of(m);
     const int64_t row = (int64_t)group * 2 * kUC + n0 + r;
+    float sum = 0.0f, lost = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      sum += fabsf(tile[lane * 8 + i][r]);
+      lost += dropped(tile[lane * 8 + i][r] * s);
+    }
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, i);
+      lost += __shfl_xor_sync(0xffffffffu, lost, i);
+    }
     uint32_t h[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       split_pair(tile[lane * 8 + 2 * i][r] * s, tile[lane * 8 + 2 * i + 1][r] * s, h[i], l[i]);
     *reinterpret_cast<uint4*>(hi + row * kHW + lane * 8) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(lo + row * kHW + lane * 8) = make_uint4(l[0], l[1], l[2], l[3]);
-    if (lane == 0) scale[row] = inverse_scale_of(m);
+    if (lane == 0) {
+      scale[row] = inverse_scale_of(m);
+      // (sum and m may be no number or infinite: no token is trusted)
+      lost *= inverse_scale_of(m);
+      const float limit = kAllowed / fmaf(0x1p-39f, sum, lost);
+      atomicMin(&range.limit, limit > 0.0f ? __float_as_uint(limit) : 0u);
+      atomicMax(&range.lost, __float_as_uint(lost));
+      atomicMax(&range.largest, m);
+    }
   }
+  __syncthreads();
+  if (threadIdx.x == 0) ranges[group * (2 * kUC / 32) + blockIdx.x] = range;
+  float smallest = fabsf(tile[threadIdx.x][0]);
+  for (int r = 1; r < 32; ++r) smallest = fminf(smallest, fabsf(tile[threadIdx.x][r]));
+  least[(int64_t)(group * (2 * kUC / 32) + blockIdx.x) * kHW + threadIdx.x] = smallest;
 }
 
 // (early launch of the kernel behind only where no CTA has a second unit: its CTAs, placed as this one's leave, would sit
@@ -729,13 +981,30 @@ bool rglru_f32_supported(int dtype, int bw, int64_t B, int64_t T, int H) {
 
 size_t rglru_f32_workspace_bytes(int64_t B, int64_t T, int64_t E) { return T < 1 ? 0 : layout(B, T, E).total; }
 
-size_t rglru_f32_packed_bytes(int H) { return (size_t)packed_rows(H) * (kHW * 2 * 2 + 4); }
+size_t rglru_f32_packed_bytes(int H) {
+  return (size_t)packed_rows(H) * (kHW * 2 * 2 + 4) + (size_t)H * kRangesHead * (sizeof(WeightRange) + kHW * 4);
+}
+
+namespace {
+struct Packed {
+  __half *hi, *lo;
+  float* scale;
+  WeightRange* ranges;
+  float* least;
+  Packed(void* p, int H) {
+    hi = static_cast<__half*>(p);
+    lo = hi + packed_rows(H) * kHW;
+    scale = reinterpret_cast<float*>(lo + packed_rows(H) * kHW);
+    ranges = reinterpret_cast<WeightRange*>(scale + packed_rows(H));
+    least = reinterpret_cast<float*>(ranges + H * kRangesHead);
+  }
+};
+}  // namespace
 
 cudaError_t launch_pack_gate_weights_f16(const void* wx, const void* wa, int H, void* packed_w, cudaStream_t s) {
-  __half* hi = static_cast<__half*>(packed_w);
-  __half* lo = hi + packed_rows(H) * kHW;
+  const Packed p(packed_w, H);
   pack_gate_weights_f16_kernel<<<dim3(2 * kUC / 32, 2 * H), 256, 0, s>>>(
-      (const float*)wx, (const float*)wa, hi, lo, reinterpret_cast<float*>(lo + packed_rows(H) * kHW));
+      (const float*)wx, (const float*)wa, p.hi, p.lo, p.scale, p.ranges, p.least);
   return cudaGetLastError();
 }
 
@@ -750,10 +1019,10 @@ ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H) {
   return p;
 }
 
-cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const void* a_param, const void* bx,
-                             const void* ba, const void* packed_w, const float* h0, const void* yb, int y_activated,
-                             int64_t B, int64_t T, int H, void* out, float* h_last, void* ws, cudaStream_t s,
-                             bool prepared) {
+cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const void* a_param, const void* wx,
+                             const void* bx, const void* wa, const void* ba, const void* packed_w, const float* h0,
+                             const void* yb, int y_activated, int64_t B, int64_t T, int H, float* zx, float* za,
+                             void* out, float* h_last, void* ws, cudaStream_t s, bool prepared) {
   const int E = H * kHW;
   const Layout L = layout(B, T, E);
   int num_sms = 0;
@@ -767,19 +1036,18 @@ cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const vo
                            dim3(256), 0, s, prep);
     if (err != cudaSuccess) return err;
   }
-  const __half* hi = static_cast<const __half*>(packed_w);
-  const __half* lo = hi + packed_rows(H) * kHW;
-  const float* scale = reinterpret_cast<const float*>(lo + packed_rows(H) * kHW);
+  const Packed w(const_cast<void*>(packed_w), H);
   CUtensorMap map_wh, map_wl;
-  if (!tensor_map_2d(&map_wh, hi, (uint64_t)packed_rows(H), kHW, kUC, kKB, true) ||
-      !tensor_map_2d(&map_wl, lo, (uint64_t)packed_rows(H), kHW, kUC, kKB, true))
+  if (!tensor_map_2d(&map_wh, w.hi, (uint64_t)packed_rows(H), kHW, kUC, kKB, true) ||
+      !tensor_map_2d(&map_wl, w.lo, (uint64_t)packed_rows(H), kHW, kUC, kKB, true))
     return cudaErrorInvalidValue;
   // all CTAs resident (look-back may spin), and as many as there are units
   const int grid = 2 * n_jobs < num_sms ? (int)(2 * n_jobs) : num_sms;
   auto run = [&](auto kernel) {
-    return launch_dependent(kernel, dim3(grid), dim3(kThreads), (size_t)kSmem, s, map_wh, map_wl, scale,
-                            (const float*)c, pos, pos64, (const float*)a_param, (const float*)bx, (const float*)ba,
-                            h0, (const float*)yb, (int)B, (int)T, E, H, (int)n_jobs, (float*)out, h_last,
+    return launch_dependent(kernel, dim3(grid), dim3(kThreads), (size_t)kSmem, s, map_wh, map_wl, w.scale,
+                            w.ranges, w.least, (const float*)wx, (const float*)wa, zx, za, (const float*)c, pos,
+                            pos64, (const float*)a_param, (const float*)bx, (const float*)ba, h0,
+                            (const float*)yb, (int)B, (int)T, E, H, (int)n_jobs, (float*)out, h_last,
                             reinterpret_cast<WsHeader*>(ws),
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.agg_off),
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.incl_off));

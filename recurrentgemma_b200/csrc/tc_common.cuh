@@ -93,6 +93,10 @@ __device__ __forceinline__ void tc_st_32x16(uint32_t taddr, const uint32_t (&v)[
          "r"(v[14]), "r"(v[15])
       : "memory");
 }
+// the same for one column
+__device__ __forceinline__ void tc_st_32x1(uint32_t taddr, uint32_t v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" :: "r"(taddr), "r"(v) : "memory");
+}
 // the same for 8 columns, and back
 __device__ __forceinline__ void tc_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"

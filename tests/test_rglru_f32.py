@@ -22,22 +22,24 @@ def _layer(heads, seed):
   return rg, lru, conv
 
 
-def _float64(lru, x, pos, h0, yb=None):
+@torch.no_grad()
+def _evaluate(lru, x, pos, h0, yb=None, dt=torch.float64):
   b, t, e = x.shape
-  xd = x.double().view(b, t, e // 256, 256)
-  gate = lambda g: torch.sigmoid(torch.einsum("bthi,hij->bthj", xd, g.w.double()) + g.b.double()).reshape(b, t, e)
-  log_a = -8.0 * gate(lru.a_gate) * torch.nn.functional.softplus(lru.a_param.double())
+  xd = x.to(dt)
+  gate = lambda g: torch.sigmoid(torch.einsum("bthi,hij->bthj", xd.view(b, t, e // 256, 256), g.w.to(dt))
+                                 + g.b.to(dt)).reshape(b, t, e)
+  log_a = -8.0 * gate(lru.a_gate) * torch.nn.functional.softplus(lru.a_param.to(dt))
   reset = (pos == 0)[..., None]
   a = torch.where(reset, torch.zeros_like(log_a), torch.exp(log_a))
-  xn = x.double() * gate(lru.input_gate) * torch.where(reset, torch.ones_like(a), torch.sqrt(1 - torch.exp(2 * log_a)))
-  h = torch.zeros(b, e, dtype=torch.float64, device=DEV) if h0 is None else h0.double()
+  xn = xd * gate(lru.input_gate) * torch.where(reset, torch.ones_like(a), torch.sqrt(1 - torch.exp(2 * log_a)))
+  h = torch.zeros(b, e, dtype=dt, device=DEV) if h0 is None else h0.to(dt)
   y = []
   for i in range(t):
     h = a[:, i] * h + xn[:, i]
     y.append(h)
   y = torch.stack(y, 1)
   if yb is not None:
-    z = yb.double()
+    z = yb.to(dt)
     y = y * 0.5 * z * (1 + torch.tanh(math.sqrt(2 / math.pi) * (z + 0.044715 * z ** 3)))
   return y, h
 
@@ -64,7 +66,7 @@ def test_forward(b, t, heads, state):
   pos[:, [i for i in (63, 64, 127, 128) if i < t]] = 0
   h0 = torch.randn(b, heads * 256, device=DEV) if state else None
   y, h = lru(x, pos, h0)
-  want, want_h = _float64(lru, x, pos, h0)
+  want, want_h = _evaluate(lru, x, pos, h0)
   _close(y, want, t)
   _close(h, want_h, t)
 
@@ -75,7 +77,7 @@ def test_path(b, t, heads):
   x, yb = (torch.randn(b, t, heads * 256, device=DEV) for _ in range(2))
   pos = torch.arange(t, device=DEV).repeat(b, 1)
   out, cache = rg.recurrent_path(x, yb, pos, conv, lru)
-  want, want_h = _float64(lru, conv(x, pos)[0], pos, None, yb)
+  want, want_h = _evaluate(lru, conv(x, pos)[0], pos, None, yb)
   _close(out, want, t)
   _close(cache.rg_lru_state, want_h, t)
 
@@ -91,11 +93,55 @@ def test_magnitudes(scale_x, scale_w):
   x[:, ::2] *= 1e-4
   pos = torch.arange(200, device=DEV).repeat(2, 1)
   y, h = lru(x, pos)
-  want, want_h = _float64(lru, x, pos, None)
+  want, want_h = _evaluate(lru, x, pos, None)
   # (gates of arguments far above 1 turn a relative error of 2^-22 of an argument into as much of themselves
   # times the argument, of which sigmoids that are not yet 0 or 1 leave some ten)
   _close(y, want, 200 * 100)
   _close(h, want_h, 200 * 100)
+
+
+def _stretch(kind, r, x, gates):
+  """Ranges along the contraction, which a scale of the token and one of the output channel cannot follow."""
+  if kind == "input":                                  # one input channel larger, its weights smaller
+    x[..., 5::256] *= r
+    for g in gates:
+      g.w.data[:, 5] /= r
+  elif kind == "weights":                              # the other way round
+    x[..., 5::256] /= r
+    for g in gates:
+      g.w.data[:, 5] *= r
+  elif kind == "unused":                               # a large channel that half of the outputs have no weight on
+    x[..., 5::256] *= r
+    for g in gates:
+      g.w.data[:, 5, ::2] = 0.0
+  else:                                                # every input channel at a magnitude of its own
+    f = r ** torch.rand(x.shape[-1], device=DEV)
+    x *= f
+    for g in gates:
+      g.w.data /= f.view(-1, 256)[..., None]
+
+
+@pytest.mark.parametrize("r", [1.0, 1e3, 1e5, 1e7, 1e9, 1e20])
+@pytest.mark.parametrize("kind", ["input", "weights", "unused", "all"])
+def test_ranges_within_a_token(kind, r):
+  """Every output channel is as near to float64 as a plain float32 evaluation of the same inputs is, but that a^2, of
+  which 1 - a^2 leaves little, carries the rounding of a twice instead of one of its own, and that the tensor core adds
+  up 48 partial sums of arguments of order 1 with up to 2^-23 of them dropped each, of which a gate keeps a quarter:
+  2^-20 where all of it points one way."""
+  rg, lru, _ = _layer(2, 9)
+  # (150 heads of sequences, three tiles each: the first by other warps than the rest, the last with tokens past the end)
+  x = torch.randn(75, 300, 512, device=DEV)
+  pos = torch.arange(300, device=DEV).repeat(75, 1)
+  _stretch(kind, r, x, (lru.input_gate, lru.a_gate))
+  y, h = lru(x, pos)
+  want, want_h = _evaluate(lru, x, pos, None)
+  plain, plain_h = _evaluate(lru, x, pos, None, dt=torch.float32)
+  far = lambda v, w, d: (v.double() - w).norm(dim=d) / w.norm(dim=d)
+  # ("unused": the gates of the other half are 0 or 1 to the last bit, and 1 - a^2 is nothing but rounding)
+  keep = slice(0, None, 2 if kind == "unused" else 1)
+  for got, p, w, d in ((y, plain, want, (0, 1)), (h, plain_h, want_h, (0,))):
+    worst = float((far(got, w, d) / (2 * far(p, w, d) + 2.0 ** -20))[keep].max())
+    assert worst <= 1.0, worst
 
 
 def test_not_numbers():
