@@ -175,9 +175,8 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
                                           p->gate_a_b, packed, h0, yb, y_activated, B, T, H,
                                           static_cast<float*>(a_buf), static_cast<float*>(xn_buf), out, h_last,
                                           scan_ws, s, xb != nullptr);
-    // (a context with fewer SMs than the device, where its CTAs could not wait for one another: the kernels below)
-    if (e != cudaErrorCooperativeLaunchTooLarge)
-      return e != cudaSuccess ? cuda_fail(e, "float32 RG-LRU launch") : RGK_OK;
+    if (e != cudaSuccess) return cuda_fail(e, "float32 RG-LRU launch");
+    return RGK_OK;
   }
   const bool fused_ok = rgk::rglru_chan_supported(dtype, bw, B, T);
   const bool want_fused = gates_impl >= RGK_GATES_FUSED;

@@ -40,38 +40,24 @@ class PerDeviceOnce {
   int sms_[kMaxDevices] = {};
 };
 
-template <typename... P, typename... A>
-cudaError_t launch_with(bool resident, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                        A... args) {
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeCooperative;
-  attr[1].val.cooperative = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = resident ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-  return e != cudaSuccess ? e : cudaGetLastError();
-}
 // A launch that may be placed while the kernel in front still runs (programmatic dependent launch): every
 // CTA of `kernel` executes griddepcontrol.wait before it touches memory that a kernel may have written
 // or still reads.  Such a kernel promises of nothing but weights that it does not change while it runs: no
 // __restrict__ on other pointers that it reads, no __ldg, no ld.global.nc.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  return launch_with(false, kernel, grid, block, smem, s, args...);
-}
-// The same for a kernel whose CTAs wait for one another without drawing their work by a ticket: all of them are on the
-// device at once or none is (a cooperative launch), whatever other streams have there.  Where that cannot be:
-// cudaErrorCooperativeLaunchTooLarge.
-template <typename... P, typename... A>
-cudaError_t launch_resident(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  return launch_with(true, kernel, grid, block, smem, s, args...);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // What rglru_chan_kernel finds prepared: the words that states (and maps) arrive in without their tokens,

@@ -21,10 +21,21 @@
 // token of 32 consecutive channels: 128 contiguous bytes.
 //
 // Work: 128 tokens of one sequence x one head, as two units of 128 channels each that share the split activations;
-// jobs are numbered time-major and dealt out round-robin to persistent CTAs, one per SM.  A last round that leaves
-// half of the CTAs without a job is dealt out as units.
+// jobs are numbered time-major, for persistent CTAs, one per SM.  A last round that leaves half of the CTAs without a
+// job goes as units.  A tile waits for the state of earlier ones, so no CTA may wait for one that work of other streams
+// keeps off the device:
+//   - the first round is dealt out by the CTAs' numbers.  Grids are placed in that order (what any look-back by block
+//     number rests on), so a CTA waits for ones that have started;
+//   - where there is more than a round, and tiles that wait (kDrawn), the rest is drawn by an atomic ticket, and only
+//     once all CTAs have started: what a tile waits for was drawn before it, by a CTA that runs.  A CTA that finds some
+//     missing for 20 us leaves when its job is done, which makes room; the last one to start finds none missing.
+// All dealt out / drawn, us, inputs from memory: 2 x 1024 tokens 33.2 / 34.6, 5001 60.4 / 60.7 (coordinates that do not
+// come from the CTA's number are in no uniform registers), 3 x 2000 of width 4096 99.1 / 96.5, with Conv1D and join 2 x
+// 1024 48.7 / 48.8, 4 x 4000 302 / 280.  A cooperative launch of all dealt out: as that in a graph, 2 us more elsewhere.
 //
-// Roles in a CTA (24 warps, two of them idle):
+// Roles in a CTA (24 warps, one or two of them idle):
+//   tickets   one warp, if jobs are drawn: the next one as the tensor core begins the one before (with a join its last
+//             unit: 3 x 2000 tokens of width 4096 169 -> 166 us, without 96.5 -> 98.1);
 //   split     4 warps: the scale of each token (a pass over the head's 256 channels), then per K-slice of 64 the two
 //             halves of the activations into the operand tiles (128-byte swizzle), as the tensor core releases them, and
 //             ahead of the last slice's release the gates of tokens that are not left to the halves;
@@ -53,6 +64,7 @@
 // kernel runs to completion.
 #include <cuda.h>
 #include <cuda_fp16.h>
+#include <limits.h>
 
 #include "rgk_common.cuh"
 #include "rgk_internal.h"
@@ -89,17 +101,21 @@ constexpr int kScaleBufs = 4;
 constexpr int kOffScale = kOffRing + kRing * kWPart;             // float [job & 3][token]: 1 / scale, < 0: not trusted
 constexpr int kOffWide = kOffScale + kScaleBufs * kUT * 4;       // bit [job & 3][token]: gates not left to the halves
 constexpr int kOffMap = kOffWide + kScaleBufs * kUT / 8;         // float2 [group][channel]: map of the first half
-constexpr int kOffBar = kOffMap + 2 * kUC * 8;                   // ring full, empty; slice full, empty; sets full, empty
-constexpr int kNumBar = 2 * kRing + 2 * kKBlocks + 4;
-constexpr int kOffTmem = kOffBar + kNumBar * 8;
-constexpr int kOffAbort = kOffTmem + 4;
-constexpr int kSmem = kOffAbort + 4 + 1024;
+constexpr int kDraws = 4;                                        // jobs between their draw and the last warp that reads it
+constexpr int kDrawReaders = kEpi + kSplit + 2;                  // warps
+constexpr int kOffBar = kOffMap + 2 * kUC * 8;  // ring full, empty; slice full, empty; sets full, empty; draw full, empty; go
+constexpr int kNumBar = 2 * kRing + 2 * kKBlocks + 4 + 2 * kDraws + 1;
+constexpr int kOffDraw = kOffBar + kNumBar * 8;
+constexpr int kOffTmem = kOffDraw + kDraws * 4;
+constexpr int kOffAbort = kOffTmem + 4;                          // two: the second of the waits for draws
+constexpr int kSmem = kOffAbort + 8 + 1024;
 static_assert(kSmem <= 232448, "exceeds the 227 KiB of shared memory a CTA may use");
 
 // kind::f16, D float32, A and B float16, both K-major
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kUT >> 3) << 17) | ((uint32_t)(kUC >> 4) << 24);
 
 constexpr unsigned kLookbackSpins = 1u << 20;
+constexpr int kStartPolls = 40;          // looks at how many CTAs have started, half a microsecond apart
 constexpr int kLookback = 2;             // earlier tiles asked for per round trip (four: 8 x 4096 tokens 341 against 329 us)
 constexpr unsigned long long kToken = 1ull << 32;
 
@@ -332,7 +348,7 @@ __device__ __forceinline__ float gelu_f32(float z) {
 
 // The jobs of a CTA: whole heads (two units) round-robin, then a unit of the last round where that was cut.
 struct Jobs {
-  int n_full, n_units, cut;                // whole jobs of this CTA, its units, its unit of the cut round (or -1)
+  int n_full, cut;                         // whole jobs of this CTA, its unit of the cut round (or -1)
   int per_tt, heads, first_cut;
   __device__ __forceinline__ Jobs(int n_jobs, int per_tt_, int heads_) : per_tt(per_tt_), heads(heads_) {
     const int grid = (int)gridDim.x, id = (int)blockIdx.x;
@@ -341,7 +357,6 @@ struct Jobs {
     n_full = rounds + (!cuts && id < rest ? 1 : 0);
     first_cut = rounds * grid;
     cut = cuts && id < 2 * rest ? id : -1;
-    n_units = 2 * n_full + (cut >= 0 ? 1 : 0);
   }
   __device__ __forceinline__ int count() const { return n_full + (cut >= 0 ? 1 : 0); }
   // (time tile, sequence, head) of job j; its units are `half` .. `half` + n - 1
@@ -356,11 +371,38 @@ struct Jobs {
       half = cut & 1;
       n = 1;
     }
+    place(i, tt, b, head);
+  }
+  __device__ __forceinline__ void place(int i, int& tt, int& b, int& head) const {
     tt = i / per_tt;
     const int r = i - tt * per_tt;
     b = r / heads;
     head = r - b * heads;
   }
+};
+
+// The same jobs by ticket: whole heads, then the units of a last round that is cut.
+struct Tickets {
+  int n, n_whole;
+  __device__ __forceinline__ explicit Tickets(int n_jobs) {
+    const int grid = (int)gridDim.x, rest = n_jobs % grid;
+    const bool cuts = 2 * rest <= grid;
+    n_whole = cuts ? n_jobs - rest : n_jobs;
+    n = cuts ? n_jobs + rest : n_jobs;
+  }
+  __device__ __forceinline__ void get(const Jobs& jobs, int ticket, int& tt, int& b, int& head, int& half,
+                                      int& units) const {
+    const int c = ticket - n_whole;
+    half = c >= 0 ? c & 1 : 0;
+    units = c >= 0 ? 1 : 2;
+    jobs.place(c >= 0 ? n_whole + (c >> 1) : ticket, tt, b, head);
+  }
+};
+
+// What the CTAs of a call share, cleared in front of it.
+struct Shared {
+  int started, drawn;
+  int pad[2];
 };
 
 // The state entering tile tt of a chain, one channel per lane: composes the published maps of earlier tiles,
@@ -409,14 +451,14 @@ __device__ __forceinline__ float look_back(const unsigned long long* agg, const 
 }
 
 // kJoin 0: out = y, 1: out = y * gelu_tanh(yb), 2: out = y * yb
-template <int kJoin>
+template <int kJoin, bool kDrawn>
 __global__ void __launch_bounds__(kThreads, 1)
 rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl,
                  const float* __restrict__ scale, const WeightRange* ranges, const float* least,
                  const float* wx, const float* wa, float* zx_wide, float* za_wide, const float* c, const void* pos,
                  int pos64, const float* __restrict__ a_param, const float* __restrict__ bias_x,
                  const float* __restrict__ bias_a, const float* h0, const float* yb, int B, int T_, int E, int heads,
-                 int n_jobs, float* out, float* h_last, WsHeader* hdr, unsigned long long* agg,
+                 int n_jobs, float* out, float* h_last, WsHeader* hdr, Shared* shared, unsigned long long* agg,
                  unsigned long long* incl) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -428,6 +470,10 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   auto bar_x_empty = [&](int kb) { return bar0 + 8u * (2 * kRing + kKBlocks + kb); };
   auto bar_acc_full = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + s); };
   auto bar_acc_empty = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + 2 + s); };
+  auto bar_draw_full = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + 4 + s); };
+  auto bar_draw_empty = [&](int s) { return bar0 + 8u * (2 * kRing + 2 * kKBlocks + 4 + kDraws + s); };
+  const uint32_t bar_draw_go = bar0 + 8u * (2 * kRing + 2 * kKBlocks + 4 + 2 * kDraws);
+  int* s_draw = reinterpret_cast<int*>(smem + kOffDraw);
   float* s_scale = reinterpret_cast<float*>(smem + kOffScale);
   uint32_t* s_wide = reinterpret_cast<uint32_t*>(smem + kOffWide);
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + kOffTmem);
@@ -440,12 +486,35 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   const int tiles_t = (T_ + kUT - 1) / kUT;
   const Jobs jobs(n_jobs, B * heads, heads);
   const int n_my = jobs.count();
+  // whether there is a job j for this CTA, and which (for a warp of the roles that work on it)
+  int ticket = (int)blockIdx.x;
+  auto next = [&](int j) -> bool {
+    if constexpr (!kDrawn) {
+      return j < n_my;
+    } else {
+      if (j > 0) {
+        const int s = (j - 1) & (kDraws - 1);
+        const bool got = __all_sync(0xffffffffu, mbar_wait(bar_draw_full(s), ((j - 1) / kDraws) & 1, s_abort + 1));
+        ticket = __shfl_sync(0xffffffffu, got ? s_draw[s] : INT_MAX, 0);
+        if (lane == 0) mbar_arrive(bar_draw_empty(s));
+      }
+      return ticket < Tickets(n_jobs).n;
+    }
+  };
+  auto get = [&](int j, int& tt, int& b, int& head, int& half, int& n) {
+    if constexpr (kDrawn) Tickets(n_jobs).get(jobs, ticket, tt, b, head, half, n);
+    else jobs.get(j, tt, b, head, half, n);
+  };
 
   if (threadIdx.x == 0) {
-    *s_abort = 0;
+    s_abort[0] = s_abort[1] = 0;
     for (int s = 0; s < kRing; ++s) { mbar_init(bar_w_full(s), 1); mbar_init(bar_w_empty(s), 1); }
     for (int kb = 0; kb < kKBlocks; ++kb) { mbar_init(bar_x_full(kb), kSplit); mbar_init(bar_x_empty(kb), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(bar_acc_full(s), 1); mbar_init(bar_acc_empty(s), kGroup); }
+    if constexpr (kDrawn) {
+      for (int s = 0; s < kDraws; ++s) { mbar_init(bar_draw_full(s), 1); mbar_init(bar_draw_empty(s), kDrawReaders); }
+      mbar_init(bar_draw_go, 1);
+    }
     mbar_fence_init();
   }
   if (warp == kEpi + kSplit + 1) {
@@ -469,9 +538,9 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     bool ok = true;
     // ---- the first job's activations, a warp eight tokens, read once: 4 us less until the first MMA than by the
     // split warps, which read them twice ----
-    if (n_my > 0) {
+    if (next(0)) {
       int tt, b, head, half, n;
-      jobs.get(0, tt, b, head, half, n);
+      get(0, tt, b, head, half, n);
       const int w0 = warp * (kUT / kEpi), tok0 = tt * kUT + w0;
       const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW + lane * 4;
       const WeightRange* range = ranges + head * kRangesHead;
@@ -513,9 +582,9 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     }
     named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
     int t = 0;
-    for (int j = 0; j < n_my; ++j) {
+    for (int j = 0; next(j); ++j) {
       int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
+      get(j, tt, b, head, half, n);
       const int u = (t ^ group) & 1;                     // the group's unit of this job, if it has one
       const int tu = t + u;
       t += n;
@@ -698,9 +767,9 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     bool ok = true;
     int s = 0;
     uint32_t phase = 1;
-    for (int j = 0; j < n_my && ok; ++j) {
+    for (int j = 0; (kDrawn || ok) && next(j); ++j) {
       int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
+      get(j, tt, b, head, half, n);
       for (int u = 0; u < n && ok; ++u) {
         const int row = (head * 2 + half + u) * 2 * kUC;
         for (int i = 0; i < kKBlocks * 4; ++i) {       // slice, gate, half
@@ -723,13 +792,14 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     bool ok = true;
     int s = 0, t = 0;
     uint32_t phase = 0;
-    for (int j = 0; j < n_my && ok; ++j) {
+    for (int j = 0; (kDrawn || ok) && next(j); ++j) {
       int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
+      get(j, tt, b, head, half, n);
       for (int u = 0; u < n && ok; ++u, ++t) {
         const int as = t & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(as), ((t >> 1) & 1) ^ 1, s_abort));
         if (!ok) break;
+        if (kDrawn && u == (kJoin == 0 ? 0 : n - 1) && lane == 0) mbar_arrive(bar_draw_go);
         tc_fence_after();
         for (int kb = 0; kb < kKBlocks && ok; ++kb) {
           if (u == 0) {
@@ -764,6 +834,30 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
         }
       }
     }
+  } else if (kDrawn && warp == kEpi + kSplit + 2) {
+    // ------------------------------ tickets ---------------------------------------------------------
+    // (with an expired wait somewhere jobs are drawn all the same: the other roles go on without work, and the
+    // epilogue publishes the records that other CTAs wait for)
+    if (lane == 0) atomicAdd(&shared->started, 1);
+    const Tickets tickets(n_jobs);
+    const volatile int* started = &shared->started;
+    bool all = false;
+    int i = ticket;
+    for (int j = 0; i < tickets.n; ++j) {
+      const int s = j & (kDraws - 1);
+      mbar_wait(bar_draw_go, j & 1, s_abort);
+      const bool free = j < kDraws || mbar_wait(bar_draw_empty(s), ((j / kDraws) & 1) ^ 1, s_abort + 1);
+      if (!__all_sync(0xffffffffu, free)) break;
+      if (lane == 0) {
+        if (!all) {
+          for (int k = 0; !(all = *started == (int)gridDim.x) && k < kStartPolls; ++k) __nanosleep(500);
+        }
+        i = all ? (int)gridDim.x + atomicAdd(&shared->drawn, 1) : tickets.n;
+        s_draw[s] = i;
+        mbar_arrive(bar_draw_full(s));
+      }
+      i = __shfl_sync(0xffffffffu, i, 0);
+    }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(kRegsSplit) : "memory");
@@ -772,12 +866,14 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
     bool ok = true;
     // (the first job's activations are the epilogue warps' work, who have nothing else to do yet)
     named_bar_sync(kBarFirst, (kEpi + kSplit) * 32);
-    const uint32_t first_wide = n_my > 0 ? s_wide[w0 >> 5] : 0u;
-    if (lane == 0 && n_my > 0)
+    const bool any = next(0);
+    const uint32_t first_wide = any ? s_wide[w0 >> 5] : 0u;
+    if (lane == 0 && any)
       for (int kb = 0; kb < kKBlocks - (first_wide != 0u ? 1 : 0); ++kb) mbar_arrive(bar_x_full(kb));
-    for (int j = first_wide != 0u ? 0 : 1; j < n_my && ok; ++j) {
+    for (int j = first_wide != 0u ? 0 : 1; (kDrawn || ok) && next(j); ++j) {
+      if (kDrawn && !ok) continue;
       int tt, b, head, half, n;
-      jobs.get(j, tt, b, head, half, n);
+      get(j, tt, b, head, half, n);
       const int tok0 = tt * kUT + w0;
       const int live = T_ - tok0;                        // tokens of the warp inside the sequence (may be < 1)
       const float* x0 = c + ((int64_t)b * T_ + tok0) * E + head * kHW;
@@ -843,7 +939,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
           __syncwarp();
           if (lane == 0 && kb < kKBlocks - 1) mbar_arrive(bar_x_full(kb));
         }
-        if (!ok) break;
+        if (!ok) continue;
       }
       if (__builtin_expect(wide != 0u, 0)) {             // in front of the last slice, and so of the epilogue
         const int64_t col = (int64_t)head * kHW * kHW, row0 = ((int64_t)b * T_ + tok0) * E + head * kHW;
@@ -862,7 +958,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
 
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort) atomicExch(&hdr->status, kStatusTimeout);
+  if (threadIdx.x == 0 && (s_abort[0] | (kDrawn ? s_abort[1] : 0)) != 0) atomicExch(&hdr->status, kStatusTimeout);
   if (warp == kEpi + kSplit + 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(512)
@@ -937,31 +1033,35 @@ __global__ void rglru_f32_prepare_kernel(const ChanPrep p) {
 
 struct Layout {
   int64_t n_words;
-  size_t incl_off, agg_off, total;
+  size_t shared_off, incl_off, agg_off, total;
 };
 Layout layout(int64_t B, int64_t T, int64_t E) {
   Layout L;
   L.n_words = (T + kUT - 1) / kUT * B * E;
-  L.incl_off = sizeof(WsHeader);
+  L.shared_off = sizeof(WsHeader);
+  L.incl_off = L.shared_off + 256;                       // (whole lines of records for a warp)
   L.agg_off = L.incl_off + (size_t)L.n_words * 8;
   L.total = (L.agg_off + (size_t)L.n_words * 16 + 255) & ~(size_t)255;
   return L;
 }
 
-template <int kJoin>
+template <int kJoin, bool kDrawn>
 cudaError_t set_attributes() {
   cudaFuncAttributes a;
-  if (const cudaError_t e = cudaFuncGetAttributes(&a, rglru_f32_kernel<kJoin>); e != cudaSuccess) return e;
+  if (const cudaError_t e = cudaFuncGetAttributes(&a, rglru_f32_kernel<kJoin, kDrawn>); e != cudaSuccess) return e;
   if (!registers_suffice(a.numRegs)) return cudaErrorLaunchOutOfResources;
-  return cudaFuncSetAttribute(rglru_f32_kernel<kJoin>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  return cudaFuncSetAttribute(rglru_f32_kernel<kJoin, kDrawn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
 }
 
 cudaError_t device_setup(int* num_sms) {
   static PerDeviceOnce once;
   return once.run([] {
-    cudaError_t e = set_attributes<0>();
-    if (e == cudaSuccess) e = set_attributes<1>();
-    if (e == cudaSuccess) e = set_attributes<2>();
+    cudaError_t e = set_attributes<0, false>();
+    if (e == cudaSuccess) e = set_attributes<1, false>();
+    if (e == cudaSuccess) e = set_attributes<2, false>();
+    if (e == cudaSuccess) e = set_attributes<0, true>();
+    if (e == cudaSuccess) e = set_attributes<1, true>();
+    if (e == cudaSuccess) e = set_attributes<2, true>();
     return e;
   }, num_sms);
 }
@@ -1013,8 +1113,8 @@ ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H) {
   ChanPrep p;
   int num_sms = 0;
   if (device_setup(&num_sms) != cudaSuccess) return p;
-  p.zero = reinterpret_cast<uint4*>(static_cast<char*>(ws) + L.incl_off);
-  p.n_zero = L.n_words * 24 / 16;
+  p.zero = reinterpret_cast<uint4*>(static_cast<char*>(ws) + L.shared_off);
+  p.n_zero = (256 + L.n_words * 24) / 16;
   p.early = 2 * ((T + kUT - 1) / kUT * B * H) <= num_sms;
   return p;
 }
@@ -1041,21 +1141,24 @@ cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const vo
   if (!tensor_map_2d(&map_wh, w.hi, (uint64_t)packed_rows(H), kHW, kUC, kKB, true) ||
       !tensor_map_2d(&map_wl, w.lo, (uint64_t)packed_rows(H), kHW, kUC, kKB, true))
     return cudaErrorInvalidValue;
-  // All CTAs resident, since look-back waits for tiles of others, and as many as there are units.  (Jobs drawn by an
-  // atomic ticket instead, for all roles of a CTA: 2 x 1024 tokens 30.6 -> 32.5 us, 700 tokens 17.6 -> 18.6, 8 x 4096
-  // 360 -> 340; the cooperative launch costs nothing.)
+  // as many CTAs as SMs, or as there are units
   const int grid = 2 * n_jobs < num_sms ? (int)(2 * n_jobs) : num_sms;
   auto run = [&](auto kernel) {
-    return launch_resident(kernel, dim3(grid), dim3(kThreads), (size_t)kSmem, s, map_wh, map_wl, w.scale,
+    return launch_dependent(kernel, dim3(grid), dim3(kThreads), (size_t)kSmem, s, map_wh, map_wl, w.scale,
                             w.ranges, w.least, (const float*)wx, (const float*)wa, zx, za, (const float*)c, pos,
                             pos64, (const float*)a_param, (const float*)bx, (const float*)ba, h0,
                             (const float*)yb, (int)B, (int)T, E, H, (int)n_jobs, (float*)out, h_last,
                             reinterpret_cast<WsHeader*>(ws),
+                            reinterpret_cast<Shared*>(static_cast<char*>(ws) + L.shared_off),
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.agg_off),
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.incl_off));
   };
-  if (yb == nullptr) return run(rglru_f32_kernel<0>);
-  return y_activated ? run(rglru_f32_kernel<2>) : run(rglru_f32_kernel<1>);
+  if (n_jobs > grid && T > kUT) {
+    if (yb == nullptr) return run(rglru_f32_kernel<0, true>);
+    return y_activated ? run(rglru_f32_kernel<2, true>) : run(rglru_f32_kernel<1, true>);
+  }
+  if (yb == nullptr) return run(rglru_f32_kernel<0, false>);
+  return y_activated ? run(rglru_f32_kernel<2, false>) : run(rglru_f32_kernel<1, false>);
 }
 
 }  // namespace rgk
