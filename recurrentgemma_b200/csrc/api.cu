@@ -153,7 +153,7 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
   const size_t act = static_cast<size_t>(B) * T * E * elem_size(dtype);
   const uintptr_t c0 = reinterpret_cast<uintptr_t>(c), out0 = reinterpret_cast<uintptr_t>(out);
   const bool f32_route = gates_impl == RGK_GATES_AUTO && rgk::rglru_f32_supported(dtype, bw, B, T, H) &&
-                         (c0 + act <= out0 || out0 + act <= c0);
+                         !y_activated && (c0 + act <= out0 || out0 + act <= c0);
   if (xb != nullptr) {
     cudaError_t e = fuse_conv
         ? rgk::launch_conv1d_cache(xb, pos, pos64, B, T, E, dtype, conv_cache_out, s)
@@ -172,9 +172,8 @@ int run_rglru(const void* c, const void* pos, int pos64, const rgk_params* p, co
       if (e != cudaSuccess) return cuda_fail(e, "pack_gate_weights launch");
     }
     cudaError_t e = rgk::launch_rglru_f32(c, pos, pos64, p->a_param, p->gate_x_w, p->gate_x_b, p->gate_a_w,
-                                          p->gate_a_b, packed, h0, yb, y_activated, B, T, H,
-                                          static_cast<float*>(a_buf), static_cast<float*>(xn_buf), out, h_last,
-                                          scan_ws, s, xb != nullptr);
+                                          p->gate_a_b, packed, h0, yb, B, T, H, static_cast<float*>(a_buf),
+                                          static_cast<float*>(xn_buf), out, h_last, scan_ws, s, xb != nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "float32 RG-LRU launch");
     return RGK_OK;
   }

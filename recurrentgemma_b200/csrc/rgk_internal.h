@@ -180,7 +180,7 @@ cudaError_t launch_rglru_chan(const void* c, const void* pos, int pos64, const v
                               bool prepared = false);
 
 // rglru_f32_tc.cu: the same in float32 (gates on three float16 products per float32 product).  Supported where
-// the tiles of 128 tokens a sequence is cut into are not mostly empty.  out must not overlap c.
+// the tiles of 128 tokens a sequence is cut into are not mostly empty.  out must not overlap c; the join is the gelu one.
 // zx, za: float32 [B, T, E] of scratch for the gates' arguments of tokens that are not left to the halves.
 // ws: rglru_f32_workspace_bytes(B, T, E) bytes whose first word is the caller's status word.
 bool rglru_f32_supported(int dtype, int bw, int64_t B, int64_t T, int H);
@@ -191,8 +191,8 @@ cudaError_t launch_pack_gate_weights_f16(const void* wx, const void* wa, int H, 
 ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H);
 cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const void* a_param, const void* wx,
                              const void* bx, const void* wa, const void* ba, const void* packed_w, const float* h0,
-                             const void* yb, int y_activated, int64_t B, int64_t T, int H, float* zx, float* za,
-                             void* out, float* h_last, void* ws, cudaStream_t s, bool prepared);
+                             const void* yb, int64_t B, int64_t T, int H, float* zx, float* za, void* out,
+                             float* h_last, void* ws, cudaStream_t s, bool prepared);
 
 // gemm_rows.cu: up to three projections (matrices) of the same M <= 8 rows in one launch, with
 // RMSNorm of the rows in front (norm_scale, or NULL) and act 0 / 1 / 2 or cap as below behind (act 1 on the

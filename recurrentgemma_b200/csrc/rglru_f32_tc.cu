@@ -450,7 +450,7 @@ __device__ __forceinline__ float look_back(const unsigned long long* agg, const 
   return fmaf(Pc, hs, Hc);
 }
 
-// kJoin 0: out = y, 1: out = y * gelu_tanh(yb), 2: out = y * yb
+// kJoin 0: out = y, 1: out = y * gelu_tanh(yb)
 template <int kJoin, bool kDrawn>
 __global__ void __launch_bounds__(kThreads, 1)
 rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl,
@@ -735,7 +735,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
         float yv[kBatch];
         if constexpr (kJoin != 0) {
 #pragma unroll
-          for (int k = 0; k < kBatch; ++k) yv[k] = kJoin == 1 ? gelu_f32(yn[k]) : yn[k];
+          for (int k = 0; k < kBatch; ++k) yv[k] = gelu_f32(yn[k]);
           if (k0 + kBatch < end) load_rows(yb, k0 + kBatch, yn, whole);
         }
         tc_wait_ld();
@@ -1058,10 +1058,8 @@ cudaError_t device_setup(int* num_sms) {
   return once.run([] {
     cudaError_t e = set_attributes<0, false>();
     if (e == cudaSuccess) e = set_attributes<1, false>();
-    if (e == cudaSuccess) e = set_attributes<2, false>();
     if (e == cudaSuccess) e = set_attributes<0, true>();
     if (e == cudaSuccess) e = set_attributes<1, true>();
-    if (e == cudaSuccess) e = set_attributes<2, true>();
     return e;
   }, num_sms);
 }
@@ -1121,8 +1119,8 @@ ChanPrep rglru_f32_prep(void* ws, int64_t B, int64_t T, int H) {
 
 cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const void* a_param, const void* wx,
                              const void* bx, const void* wa, const void* ba, const void* packed_w, const float* h0,
-                             const void* yb, int y_activated, int64_t B, int64_t T, int H, float* zx, float* za,
-                             void* out, float* h_last, void* ws, cudaStream_t s, bool prepared) {
+                             const void* yb, int64_t B, int64_t T, int H, float* zx, float* za, void* out,
+                             float* h_last, void* ws, cudaStream_t s, bool prepared) {
   const int E = H * kHW;
   const Layout L = layout(B, T, E);
   int num_sms = 0;
@@ -1153,12 +1151,8 @@ cudaError_t launch_rglru_f32(const void* c, const void* pos, int pos64, const vo
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.agg_off),
                             reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + L.incl_off));
   };
-  if (n_jobs > grid && T > kUT) {
-    if (yb == nullptr) return run(rglru_f32_kernel<0, true>);
-    return y_activated ? run(rglru_f32_kernel<2, true>) : run(rglru_f32_kernel<1, true>);
-  }
-  if (yb == nullptr) return run(rglru_f32_kernel<0, false>);
-  return y_activated ? run(rglru_f32_kernel<2, false>) : run(rglru_f32_kernel<1, false>);
+  if (n_jobs > grid && T > kUT) return yb == nullptr ? run(rglru_f32_kernel<0, true>) : run(rglru_f32_kernel<1, true>);
+  return yb == nullptr ? run(rglru_f32_kernel<0, false>) : run(rglru_f32_kernel<1, false>);
 }
 
 }  // namespace rgk
