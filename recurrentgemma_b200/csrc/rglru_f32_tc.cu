@@ -454,7 +454,7 @@ __device__ __forceinline__ float look_back(const unsigned long long* agg, const 
 template <int kJoin, bool kDrawn>
 __global__ void __launch_bounds__(kThreads, 1)
 rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl,
-                 const float* __restrict__ scale, const WeightRange* ranges, const float* least,
+                 const float* w_scale, const WeightRange* ranges, const float* least,
                  const float* wx, const float* wa, float* zx_wide, float* za_wide, const float* c, const void* pos,
                  int pos64, const float* __restrict__ a_param, const float* __restrict__ bias_x,
                  const float* __restrict__ bias_a, const float* h0, const float* yb, int B, int T_, int E, int heads,
@@ -606,7 +606,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
       const int64_t at0 = ((int64_t)b * T_ + tok0) * E + e;
       // z log2(e) with the sign turned: the sigmoid is 1 / (1 + 2^that)
       const int wrow = grp * 2 * kUC + chq * 32 + lane;
-      const float kx = kNegLog2e * scale[wrow], ka = kNegLog2e * scale[wrow + kUC];
+      const float kx = kNegLog2e * w_scale[wrow], ka = kNegLog2e * w_scale[wrow + kUC];
       const float bx = kNegLog2e * bias_x[e], ba = kNegLog2e * bias_a[e];
       const float m8sp = -8.0f * softplus_(a_param[e]);
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(chq * 32) << 16) + as * 2 * kUT + th * kTokHalf;
@@ -641,7 +641,7 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
 #pragma unroll 1
           for (int q = 0; q < 2; ++q)
             place_tokens(zx_wide + at0 + (int64_t)q * 32 * E, za_wide + at0 + (int64_t)q * 32 * E, E,
-                         q == 0 ? wide.x : wide.y, st_row + q * 32, scale[wrow], scale[wrow + kUC], t_row + q * 32);
+                         q == 0 ? wide.x : wide.y, st_row + q * 32, w_scale[wrow], w_scale[wrow + kUC], t_row + q * 32);
         }
 #pragma unroll 1
         for (int k0 = 0; k0 < end; k0 += kBatch) {

@@ -35,12 +35,14 @@ def test_dependent_kernels_read_results_coherently():
         continue
       found.add(name)
       promised = set(re.findall(r"const [\w ]+\* ?__restrict__ (\w+)", params))
-      assert promised <= WEIGHTS, (name, promised - WEIGHTS)
+      # ("scale" is the weight of a norm, and of nothing else)
+      weights = WEIGHTS if "norm" in name else WEIGHTS - {"scale"}
+      assert promised <= weights, (name, promised - weights)
       cached = set(re.findall(r"__ldg\((?:reinterpret_cast<[^>]*>\()?(\w+)", body))
       assert cached <= WEIGHTS, (name, cached - WEIGHTS)
       assert ".nc." not in body, name
   assert {"attn_prefill_kernel", "gates_tf32_kernel", "rmsnorm_row_kernel", "gemm_rows_kernel",
-          "conv1d_prefill_kernel", "rglru_chan_kernel", "scan_kernel"} <= found
+          "conv1d_prefill_kernel", "rglru_chan_kernel", "rglru_f32_kernel", "scan_kernel"} <= found
   for name in ("rgk_common.cuh", "tc_common.cuh", "tma.cuh"):
     with open(os.path.join(CSRC, name)) as f:
       assert "ld.global.nc" not in re.sub(r"//[^\n]*", "", f.read()), name
