@@ -54,11 +54,14 @@ def test_rglru_layer_float32_at_config_size(rg, oracle):
   assert float(y[:, 512].abs().max()) <= float(y_r[:, 512].abs().max()) * (1 + 1e-5) + 1e-6
 
 
+@pytest.mark.parametrize("impl", ["GATES_AUTO", "GATES_TCGEN05"])
 @pytest.mark.parametrize("tokens", [1793, 2301, 2309, 4097])
-def test_rglru_layer_float32_last_wave(rg, oracle, tokens):
-  """Tiles of the float32 gate kernel that a last wave holds: 4 and 64 of 300 and 360 (launched as half
+def test_rglru_layer_float32_last_wave(rg, oracle, tokens, impl):
+  """Tiles of the float32 gate kernel (GATES_TCGEN05) that a last wave holds: 4 and 64 of 300 and 360 (launched as half
   tiles behind the others on 148 SMs), 84 of 380 (with the others), 68 of 660.  Heads at either end, the
-  last of which have their last tokens in the second launch, with an initial state."""
+  last of which have their last tokens in the second launch, with an initial state.  The same sizes in one kernel
+  (GATES_AUTO): a round and 2, 32 or 42 of 148 jobs, two rounds and 34."""
+  from recurrentgemma_b200 import _lib
   e, h = 2560, 10
   g = torch.Generator(device="cpu").manual_seed(tokens)
   p = synthetic.rglru_params(e, h, g, torch.float32)
@@ -66,7 +69,9 @@ def test_rglru_layer_float32_last_wave(rg, oracle, tokens):
   h0 = torch.randn((1, e), generator=g) * 0.5
   pos = synthetic.geometric_segment_pos(1, tokens, 300.0, 5)
   pos[:, 0] = 1
-  y, h_last = _lru(rg, p, e, h, torch.float32)(x.to(DEV), pos.to(DEV), h0.to(DEV))
+  lru = _lru(rg, p, e, h, torch.float32)
+  lru.gates_impl = getattr(_lib, impl)
+  y, h_last = lru(x.to(DEV), pos.to(DEV), h0.to(DEV))
   rg.check_status()
   for head in (0, 7, 8, 9):
     sl = slice(head * 256, (head + 1) * 256)

@@ -12,9 +12,11 @@ DEV = "cuda:0"
 @pytest.mark.parametrize("rows,heads", [(1, 1), (129, 2), (1100, 4), (1200, 4), (2300, 4), (2400, 4), (5000, 3)])
 def test_gates(rows, heads):
   import recurrentgemma_b200 as rg
+  from recurrentgemma_b200 import _lib
   torch.manual_seed(rows)
   e = heads * 256
   lru = rg.RGLRU(e, heads, device=DEV, dtype=torch.float32)
+  lru.gates_impl = _lib.GATES_TCGEN05
   for b in (lru.input_gate.b, lru.a_gate.b):
     b.data.normal_(0, 0.1)
   x = torch.randn(rows, 1, e, device=DEV)

@@ -1,6 +1,7 @@
 """The float32 RG-LRU as one kernel (tiles of 128 tokens, units of 128 channels) against float64, at the edges of
 its tiles and of its last round of work (recurrentgemma/torch/layers.py:140-191, 338-376; join of
 torch/modules.py:627-628, 646).  Needs a B200."""
+import ctypes
 import math
 
 import pytest
@@ -44,12 +45,13 @@ def _evaluate(lru, x, pos, h0, yb=None, dt=torch.float64):
   return y, h
 
 
-def _close(got, want, t):
-  # a handful of roundings of 2^-24 a token, carried along by a <= 1 and independent of one another, and a
-  # contraction good to 2^-22 of its terms
-  tol = 2.0 ** -21 * math.sqrt(t)
-  err = float((got.double() - want).norm() / want.norm())
-  assert err <= tol, (err, tol)
+def _close(got, want, plain, argument=1):
+  # No farther from float64 (2-norm) than a plain float32 evaluation of the same inputs, but for a^2, of which 1 - a^2
+  # leaves little and which carries the rounding of a twice instead of one of its own, and for 2^-21 of the contraction
+  # (48 partial sums, up to 2^-23 dropped of each, a quarter of it left by a gate, half of that by different signs) times
+  # what the gates' arguments are on the order of.
+  far = lambda v: float((v.double() - want).norm() / want.norm())
+  assert far(got) <= 2 * far(plain) + 2.0 ** -21 * argument, (far(got), far(plain))
 
 
 # one token; a tile less one, whole, and one more; whole heads and units in the last round (148 SMs: 75 jobs are dealt
@@ -66,9 +68,8 @@ def test_forward(b, t, heads, state):
   pos[:, [i for i in (63, 64, 127, 128) if i < t]] = 0
   h0 = torch.randn(b, heads * 256, device=DEV) if state else None
   y, h = lru(x, pos, h0)
-  want, want_h = _evaluate(lru, x, pos, h0)
-  _close(y, want, t)
-  _close(h, want_h, t)
+  for got, want, plain in zip((y, h), _evaluate(lru, x, pos, h0), _evaluate(lru, x, pos, h0, dt=torch.float32)):
+    _close(got, want, plain)
 
 
 @pytest.mark.parametrize("b,t,heads", [(2, 200, 3), (1, 1500, 10)])
@@ -77,14 +78,15 @@ def test_path(b, t, heads):
   x, yb = (torch.randn(b, t, heads * 256, device=DEV) for _ in range(2))
   pos = torch.arange(t, device=DEV).repeat(b, 1)
   out, cache = rg.recurrent_path(x, yb, pos, conv, lru)
-  want, want_h = _evaluate(lru, conv(x, pos)[0], pos, None, yb)
-  _close(out, want, t)
-  _close(cache.rg_lru_state, want_h, t)
+  c = conv(x, pos)[0]
+  for got, want, plain in zip((out, cache.rg_lru_state), _evaluate(lru, c, pos, None, yb),
+                              _evaluate(lru, c, pos, None, yb, torch.float32)):
+    _close(got, want, plain)
 
 
-@pytest.mark.parametrize("scale_x,scale_w", [(1e30, 1.0), (1e-30, 1.0), (1.0, 1e30), (3e4, 1e-4)])
-def test_magnitudes(scale_x, scale_w):
-  """Far outside float16: the scales of tokens and channels carry it."""
+@pytest.mark.parametrize("scale_x,scale_w,argument", [(1e30, 1.0, 1), (1e-30, 1.0, 1), (1.0, 1e30, 1), (3e4, 1e-4, 3)])
+def test_magnitudes(scale_x, scale_w, argument):
+  """Far outside float16: the scales of tokens and channels carry it.  (Gates of arguments around 1e30 are 0 or 1.)"""
   rg, lru, _ = _layer(1, 5)
   for g in (lru.input_gate, lru.a_gate):
     g.w.data.mul_(scale_w)
@@ -93,11 +95,49 @@ def test_magnitudes(scale_x, scale_w):
   x[:, ::2] *= 1e-4
   pos = torch.arange(200, device=DEV).repeat(2, 1)
   y, h = lru(x, pos)
-  want, want_h = _evaluate(lru, x, pos, None)
-  # (gates of arguments far above 1 turn a relative error of 2^-22 of an argument into as much of themselves
-  # times the argument, of which sigmoids that are not yet 0 or 1 leave some ten)
-  _close(y, want, 200 * 100)
-  _close(h, want_h, 200 * 100)
+  for got, want, plain in zip((y, h), _evaluate(lru, x, pos, None), _evaluate(lru, x, pos, None, dt=torch.float32)):
+    _close(got, want, plain, argument)
+
+
+def _rglru_forward(lru, x, pos, out, packed):
+  """The C call, with the weights packed by the call itself if `packed` is false."""
+  from recurrentgemma_b200 import _lib
+  b, t, e = x.shape
+  h_last = torch.empty(b, e, device=DEV)
+  ws = torch.zeros(_lib.workspace_bytes(b, t, e, x.dtype), dtype=torch.uint8, device=DEV)
+  p = lru._params()
+  if not packed:
+    p.gates_packed = None
+  _lib.check(_lib.load().rgk_rglru_forward(
+      x.data_ptr(), pos.data_ptr(), _lib.pos_code(pos), ctypes.byref(p), None, b, t, e, lru.num_heads, _lib.RGK_F32,
+      _lib.GATES_AUTO, out.data_ptr(), h_last.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_ptr(x.device)))
+  _lib.workspace_status(ws)
+  return h_last
+
+
+# one round of jobs, and more than one
+@pytest.mark.parametrize("b,t,heads", [(2, 300, 2), (8, 700, 5)])
+def test_weights_packed_by_the_call(b, t, heads):
+  _, lru, _ = _layer(heads, 3)
+  x, pos = torch.randn(b, t, heads * 256, device=DEV), torch.arange(t, device=DEV).repeat(b, 1)
+  y = torch.empty_like(x)
+  h = _rglru_forward(lru, x, pos, y, packed=False)
+  for got, want, plain in zip((y, h), _evaluate(lru, x, pos, None), _evaluate(lru, x, pos, None, dt=torch.float32)):
+    _close(got, want, plain)
+
+
+# the output in the input's place, and half of it in the input's second half: the two kernels, which may do that
+@pytest.mark.parametrize("shift", [0, 1])
+def test_output_over_the_input(shift):
+  from recurrentgemma_b200 import _lib
+  _, lru, _ = _layer(2, 4)
+  pos = torch.arange(300, device=DEV).repeat(2, 1)
+  buffer = torch.randn(3, 300, 512, device=DEV)
+  x, y = buffer[:2], buffer[shift:shift + 2]
+  lru.gates_impl = _lib.GATES_TCGEN05
+  want, want_h = lru(x, pos)
+  h = _rglru_forward(lru, x, pos, y, packed=True)
+  assert torch.equal(y, want) and torch.equal(h, want_h)
 
 
 def _stretch(kind, r, x, gates):
