@@ -541,7 +541,7 @@ def run_gpu(args, cfg):
               "achieved_Gops": sfu_ops * b * t * e / (kernels["rglru_fused"]["ms"] * 1e-3) / 1e9,
               "peak_Gops": 148 * 16 * 1.965, "unit": "G special-function ops/s",
               "frac": (sfu_ops * b * t * e / (kernels["rglru_fused"]["ms"] * 1e-3) / 1e9) / (148 * 16 * 1.965)},
-      "note": ("rglru_fused is bounded by instruction issue (38 warp instructions for 32 elements, 3.5 "
+      "note": ("rglru_fused is bounded by instruction issue (36 warp instructions for 32 elements, 3.5 "
                "special-function operations per element), not by HBM; frac is "
                "its algorithmic bytes over its time against the measured copy bandwidth"),
   }

@@ -57,6 +57,9 @@ enum {
   RGK_GATES_AUTO = 0,    /* the fastest kernel that covers the shape (see below; float32 with head width 256: gates,
                             gate arithmetic and scan in one kernel on three float16 products, where a token's values
                             span too wide a range for those float32 dot products, which are slow) */
+  /* (bfloat16 in one kernel, T > 128: its blocks wait for one another, all of them.  Work of streams of another priority
+     that keeps a part of them off the device until the call ends makes those waits run out, RGK_ETIMEOUT.  float32 and
+     RGK_GATES_TCGEN05 wait only for blocks that run.) */
   RGK_GATES_SIMT = 1,    /* CUDA-core gate kernel, then the scan kernel (any head width that is a
                             multiple of 16; float32 or bfloat16) */
   RGK_GATES_TCGEN05 = 2, /* tensor-core gate kernel, then the scan kernel (head width 256: bfloat16,

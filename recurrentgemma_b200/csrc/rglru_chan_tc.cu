@@ -42,11 +42,14 @@
 // for every call -> 136 without maps where chains are many -> 134 with the MMA loop on a whole warp -> 129 with
 // 112 instead of 96 registers for the epilogue warps (setmaxnreg: no spills, more pairs in flight) -> 124 with
 // table addresses in one instruction and waits that are asked once ahead of their loop -> 121 with the warp's own
-// coordinates and barriers in uniform registers (8 x 4096 tokens with a join and the conv 232 -> 226).  The path
-// 243 -> 209 us, 4 x 16384 tokens of width 4096 475 -> 395 us (one record a chain to clear instead of one a
-// tile).  Weights at rest in tensor memory instead of streamed took as long a unit: loads are not the bound.
+// coordinates and barriers in uniform registers.  With a join and the conv in front these tokens are at 232 us as the
+// workloads are timed, 200 to 224 in a loop, within which a run differs from the next.  Weights at rest in tensor
+// memory instead of streamed took as long a unit: loads are not the bound.
 // All waits (mbarriers, look-back flags) are bounded; on expiry WsHeader::status is raised, the
-// affected values are taken as zero and the kernel runs to completion.
+// affected values are taken as zero and the kernel runs to completion.  Units are dealt out to all CTAs for good, and a
+// unit waits for states that other CTAs publish: work of other streams that keeps part of the CTAs off the device until
+// this kernel ends makes those waits expire (two such calls on streams of different priority can do it to each other;
+// on streams of one priority the blocks of one are placed before those of the next).
 #include <cuda.h>
 
 #include "rgk_common.cuh"

@@ -55,10 +55,10 @@
 // 2,500 to 4,000 until the state is there, 3,500 in pass two), and there is room for two sets: 15,500 a unit.  67 warp
 // instructions for 32 elements without a join, 54 % of the issue slots.  (Cycles and instructions before the warp's
 // number was uniform, which took 5 to 7 % off the calls up to 5001 tokens.)  Width 2560, float32, us as gate and
-// scan kernels with a and the normalised input through memory / this: 2 x 1024 tokens 64 / 32, 5001 tokens 150 / 57,
-// 8 x 4096 730 / 329, 16 tokens 19 / 12; with Conv1D and join 1500 tokens 64 / 36, 4 x 4000 458 / 276.  With one
+// scan kernels with a and the normalised input through memory / this, in a loop: 2 x 1024 tokens 64 / 32, 5001 tokens
+// 150 / 60, 8 x 4096 730 / 340, 16 tokens 19 / 11; with Conv1D and join 1500 tokens 64 / 35, 4 x 4000 458 / 281.  With one
 // epilogue group of eight warps 2 x 1024 tokens took 42.  Distance of the 2-norm from a 64-bit evaluation: 9.5e-7 /
-// 5.6e-7 at 2 x 1024 tokens, and the smaller one at every size and magnitude compared.
+// 5.6e-7 at 2 x 1024 tokens, and the smaller one at every size and scale of normal data compared.
 //
 // All waits are bounded; on expiry WsHeader::status is raised, the affected values are taken as zero and the
 // kernel runs to completion.
@@ -116,7 +116,7 @@ constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kUT >> 3) << 17) | ((uint32_
 
 constexpr unsigned kLookbackSpins = 1u << 20;
 constexpr int kStartPolls = 40;          // looks at how many CTAs have started, half a microsecond apart
-constexpr int kLookback = 2;             // earlier tiles asked for per round trip (four: 8 x 4096 tokens 341 against 329 us)
+constexpr int kLookback = 2;             // earlier tiles asked for per round trip (four: 8 x 4096 tokens 4 % slower)
 constexpr unsigned long long kToken = 1ull << 32;
 
 __device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
@@ -480,8 +480,8 @@ rglru_f32_kernel(const __grid_constant__ CUtensorMap map_wh, const __grid_consta
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem + kOffAbort);
 
   // (from a lane, so that the compiler knows it to be the same in the whole warp: barriers, addresses and what the
-  // loops run over are then in uniform registers.  With the weights' loop on its whole warp, us: 2 x 1024 tokens 33.9
-  // -> 31.7, 8 x 4096 tokens 348..358 -> 332..355, 1 x 300 tokens 18.2 -> 16.8)
+  // loops run over are then in uniform registers: with the weights' loop on its whole warp 5 to 7 % off the calls of up to
+  // 5001 tokens, nothing beyond their spread off 8 x 4096)
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tiles_t = (T_ + kUT - 1) / kUT;
   const Jobs jobs(n_jobs, B * heads, heads);
